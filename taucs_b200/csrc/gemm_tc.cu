@@ -63,7 +63,15 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
-// bounded wait; false when it gave up
+// bounded wait of a whole warp; false when it gave up.  Every lane polls and
+// the loop ends by a vote, so the warp leaves it undivided: after a wait run
+// by one lane alone the warp stays split through the code that follows.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity) {
+  for (unsigned it = 0; it < TC_WAIT_LIMIT; it++)
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  return false;
+}
+// bounded wait of one thread; false when it gave up
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
   for (unsigned it = 0; it < TC_WAIT_LIMIT; it++)
     if (mbar_try(bar, parity)) return true;
@@ -229,12 +237,7 @@ k_gemm_tc(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, fl
       const int stg = kt % STAGES, use = kt / STAGES;
       if (kt + 1 < nk) load(kt + 1, an, bn);
       if (use > 0) {
-        // one lane polls the ring slot; the warp follows it
-        int got = 1;
-        if (lane == 0) got = mbar_wait(empty0 + 8 * stg, (use - 1) & 1);
-        got = __shfl_sync(0xffffffffu, got, 0);
-        __syncwarp();   // orders the lanes' stores after lane 0's acquire
-        if (!got) return false;
+        if (!mbar_wait_warp(empty0 + 8 * stg, (use - 1) & 1)) return false;
       }
       const unsigned st = sbase + stg * TC_STAGE + roff_s;
 #pragma unroll
@@ -282,10 +285,7 @@ k_gemm_tc(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, fl
       }
     };
     if (cq0 < cq1) loadC(cq0);
-    int gd = 1;
-    if (lane == 0) gd = mbar_wait(done, 0);
-    const bool got = __shfl_sync(0xffffffffu, gd, 0) != 0;
-    __syncwarp();
+    const bool got = mbar_wait_warp(done, 0);
     if (!got) record_timeout(status);
     tc_fence_after();
     // tcgen05.ld is warp-collective: the decision must be warp-uniform
@@ -478,10 +478,7 @@ k_gemm_sp(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, co
     for (int kt = 0; kt < nk; kt++) {
       const int stg = kt % STAGES, use = kt / STAGES;
       if (use > 0) {
-        int got = 1;
-        if (lane == 0) got = mbar_wait(empty0 + 8 * stg, (use - 1) & 1);
-        got = __shfl_sync(0xffffffffu, got, 0);
-        if (!got) {
+        if (!mbar_wait_warp(empty0 + 8 * stg, (use - 1) & 1)) {
           if (lane == 0) {
             record_timeout(status);
             abort_cta = 1;
@@ -497,42 +494,48 @@ k_gemm_sp(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, co
         bulk_g2s(sbase + stg * SP_STAGE + p * SP_PARTB + c * SP_CHUNK, src, SP_CHUNK, full0 + 8 * stg);
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ---- MMA issue, one thread: two MMAs of K = 2 chunks per stage
+  } else if (warp == 1) {
+    // ---- MMA issue by lane 0: two MMAs of K = 2 chunks per stage.  The
+    // warp waits together, so that it reaches its share of the epilogue
+    // undivided
     const unsigned idesc = FMT ? f16_idesc(nmma) : tc_idesc(nmma);
     bool ok = true;
     for (int kt = 0; kt < nk; kt++) {
       const int stg = kt % STAGES, use = kt / STAGES;
-      if (!mbar_wait(full0 + 8 * stg, use & 1)) {
+      if (!mbar_wait_warp(full0 + 8 * stg, use & 1)) {
         ok = false;
         break;
       }
       tc_fence_after();
-      const unsigned st = sbase + stg * SP_STAGE;
+      if (lane == 0) {
+        const unsigned st = sbase + stg * SP_STAGE;
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const unsigned o = 2 * j * SP_CHUNK;
-        const uint64_t ah = sp_desc(st + 0 * SP_PARTB + o), al = sp_desc(st + 1 * SP_PARTB + o);
-        const uint64_t bh = sp_desc(st + 2 * SP_PARTB + o), bl = sp_desc(st + 3 * SP_PARTB + o);
-        const unsigned first = (kt | j) != 0;
-        if (FMT == 0) {
-          tc_mma(tmem, al, bh, idesc, first);
-          tc_mma(tmem, ah, bl, idesc, 1u);
-          tc_mma(tmem, ah, bh, idesc, 1u);
-        } else {
-          f16_mma(tmem, ah, bh, idesc, first);
-          f16_mma(tmem + TC_TMEM_COLS, ah, bl, idesc, first);
-          f16_mma(tmem + TC_TMEM_COLS, al, bh, idesc, 1u);
+        for (int j = 0; j < 2; j++) {
+          const unsigned o = 2 * j * SP_CHUNK;
+          const uint64_t ah = sp_desc(st + 0 * SP_PARTB + o), al = sp_desc(st + 1 * SP_PARTB + o);
+          const uint64_t bh = sp_desc(st + 2 * SP_PARTB + o), bl = sp_desc(st + 3 * SP_PARTB + o);
+          const unsigned first = (kt | j) != 0;
+          if (FMT == 0) {
+            tc_mma(tmem, al, bh, idesc, first);
+            tc_mma(tmem, ah, bl, idesc, 1u);
+            tc_mma(tmem, ah, bh, idesc, 1u);
+          } else {
+            f16_mma(tmem, ah, bh, idesc, first);
+            f16_mma(tmem + TC_TMEM_COLS, ah, bl, idesc, first);
+            f16_mma(tmem + TC_TMEM_COLS, al, bh, idesc, 1u);
+          }
         }
+        tc_commit(empty0 + 8 * stg);
       }
-      tc_commit(empty0 + 8 * stg);
+      __syncwarp();
     }
-    if (!ok) {
+    if (!ok && lane == 0) {
       record_timeout(status);
       abort_cta = 1;
     }
     // done fires once every MMA issued above has completed
-    tc_commit(done);
+    if (lane == 0) tc_commit(done);
+    __syncwarp();
   }
   // ---- epilogue: warp w owns TMEM lanes (tile rows) 32 w .. 32 w + 31.
   // The first 32 columns of the old C rows are loaded before the wait for
@@ -563,10 +566,7 @@ k_gemm_sp(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, co
   };
   float oldn[32];
   load_old(0, oldn);
-  int gd = 1;
-  if (lane == 0) gd = mbar_wait(done, 0);
-  const bool got = __shfl_sync(0xffffffffu, gd, 0) != 0;
-  __syncwarp();
+  const bool got = mbar_wait_warp(done, 0);
   if (!got && lane == 0) record_timeout(status);
   tc_fence_after();
   // tcgen05.ld is warp-collective: the decision must be warp-uniform

@@ -71,13 +71,27 @@ int devplan_upload(const Plan& P, DevPlan* D, cudaStream_t st) {
       for (int b = 0; b * PANEL_NB < P.fronts[i].s; b++) dblk.push_back(int2_{i, b});
   D->n_dblk = (int) dblk.size();
   D->n_pers = (int) P.pers_fronts.size();
+  std::vector<SolveTask> stasks;
+  stasks.reserve(P.pers_fronts.size());
+  for (size_t t = 0; t < P.pers_fronts.size(); t++) {
+    const FrontDesc& F = P.fronts[P.pers_fronts[t]];
+    stasks.push_back(SolveTask{F.l_off, F.rows_off, F.s, F.f, F.child_begin, F.child_end, P.pers_parent[t]});
+  }
+  std::vector<int4> crec;
+  crec.reserve(P.children.size());
+  for (int c : P.children) {
+    const FrontDesc& C = P.fronts[c];
+    crec.push_back(make_int4(C.rows_off, C.s, C.f, C.map_off));
+  }
   bool ok = dev_upload(&D->fronts, P.fronts.data(), P.fronts.size(), st)
          && dev_upload(&D->small_num, small_num.data(), small_num.size(), st)
          && dev_upload(&D->pers_list, P.pers_fronts.data(), P.pers_fronts.size(), st)
          && dev_upload(&D->pers_parent, P.pers_parent.data(), P.pers_parent.size(), st)
          && dev_upload(&D->pers_pending0, P.pers_pending.data(), P.pers_pending.size(), st)
          && dev_upload(&D->pers_work, (const int*) nullptr, P.pers_fronts.size() + 2, st)
-         && dev_upload(&D->pers_solve, (const int*) nullptr, 2 * P.pers_fronts.size() + 2, st)
+         && dev_upload(&D->pers_solve, (const int*) nullptr, 2 * P.pers_fronts.size() + 4, st)
+         && dev_upload(&D->solve_tasks, stasks.data(), stasks.size(), st)
+         && dev_upload(&D->child_rec, crec.data(), crec.size(), st)
          && dev_upload(&D->dblk, dblk.data(), dblk.size(), st)
          && dev_upload(&D->children, P.children.data(), P.children.size(), st)
          && dev_upload(&D->rows, P.rows.data(), P.rows.size(), st)
@@ -104,7 +118,7 @@ void devplan_free(DevPlan* D) {
   tb::dfree(D->small_list); tb::dfree(D->big_list); tb::dfree(D->tiles); tb::dfree(D->tile_ch);
   tb::dfree(D->sfwd); tb::dfree(D->sbwd); tb::dfree(D->sl21); tb::dfree(D->dblk);
   tb::dfree(D->small_num); tb::dfree(D->pers_list); tb::dfree(D->pers_parent); tb::dfree(D->pers_pending0);
-  tb::dfree(D->pers_work); tb::dfree(D->pers_solve);
+  tb::dfree(D->pers_work); tb::dfree(D->pers_solve); tb::dfree(D->solve_tasks); tb::dfree(D->child_rec);
   *D = DevPlan();
 }
 

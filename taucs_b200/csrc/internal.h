@@ -65,6 +65,15 @@ struct int2_ {
   int a, b;
 };
 
+// A small front as the solve's one-warp kernels take it: one aligned 32-byte
+// record per persistent task (parent: its parent's task, -1 outside the set).
+struct alignas(16) SolveTask {
+  int64_t l_off;
+  int rows_off, s, f;             // rows_off is the work vector's offset too
+  int child_begin, child_end;
+  int parent;
+};
+
 // Dense-kernel tile for the blocked partial factorization and the update
 // of U (see numeric.cu).
 struct GemmTile {
@@ -122,15 +131,12 @@ struct LevelPlan {
   int n_fwd_diag = 0;
   std::vector<int2_> solve_bwd_blocks;   // (front, column block), last block first
   std::vector<int2_> solve_l21_tasks;    // (front, column block << 16 | row chunk)
-  // small fronts, fused kernel (sorted by order f); the first small_warp of
-  // them are small enough for the one-warp-per-front solve kernels
+  // small fronts, fused kernel (sorted by order f)
   std::vector<int> small_fronts;
   // the small fronts that the level launches of the numeric factorization
   // take (those with a big front below them); the others are factored by
   // the persistent launch (Plan::pers_fronts).  Sorted by order f.
   std::vector<int> small_numeric;
-  int small_numeric_warp = 0;      // the first ones small enough for the one-warp solve kernels
-  int small_warp = 0;
   // medium/large fronts
   std::vector<int> big_fronts;
   std::vector<Tile> build_tiles;
@@ -161,6 +167,9 @@ struct Plan {
   std::vector<int> pers_fronts, pers_parent, pers_pending;
   int pers_nwarp = 0;
   int pers_fmax = 0;               // largest order f among the second part's fronts
+  // per part, for the solve: the largest panel in shared memory (columns of
+  // f | 1 elements) and the largest order
+  int pers_slot[2] = {0, 0}, pers_wld[2] = {0, 0};
   int64_t nnz = 0;
   std::vector<FrontDesc> fronts;
   std::vector<int> children;       // device-order child indices

@@ -29,8 +29,10 @@ constexpr int GEMM_BN = 64;
 constexpr int GEMM_BK = 16;
 // right-hand sides handled per solve pass
 constexpr int SOLVE_NRHS = 8;
-// small fronts up to this order are solved by one warp each (eight per CTA)
-constexpr int SOLVE_WARP_F = 48;
+// bytes of shared memory that a warp of the solve's small-front kernels holds
+// of its front's panel at a time, at most (larger panels go through it in
+// pieces)
+constexpr int SOLVE_SLOT_BYTES = 16384;
 // rows of L21 per CTA in the backward solve's partial products
 constexpr int SOLVE_RCH = 512;
 
@@ -80,7 +82,9 @@ struct DevPlan {
   int* pers_parent = nullptr;
   int* pers_pending0 = nullptr;
   int* pers_work = nullptr;    // per factorization: pending counts (n_pers) + the two queue heads
-  int* pers_solve = nullptr;   // per solve: pending counts and done flags (n_pers each) + two queue heads
+  int* pers_solve = nullptr;   // per solve: pending counts and done flags (n_pers each) + four queue heads
+  SolveTask* solve_tasks = nullptr;   // per persistent task, in queue order
+  int4* child_rec = nullptr;   // per entry of children: work vector offset, s, f, map offset
   int n_pers = 0;
   std::vector<int> small_off, big_off, tile_off, sfwd_off, sbwd_off, sl21_off, small_num_off;  // per level (host)
   std::vector<int> lvl_max_f_small;               // per level (host)

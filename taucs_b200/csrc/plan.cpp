@@ -442,9 +442,6 @@ int build_plan(const Symbolic& S, int n, const int* colptr, const int* rowind, P
       // the fused small-front kernel is launched per size class
       std::stable_sort(LP.small_fronts.begin(), LP.small_fronts.end(),
                        [&](int a, int b) { return P.fronts[a].f < P.fronts[b].f; });
-      while (LP.small_warp < (int) LP.small_fronts.size() &&
-             P.fronts[LP.small_fronts[LP.small_warp]].f <= SOLVE_WARP_F)
-        LP.small_warp++;
     }
   }
 
@@ -465,6 +462,8 @@ int build_plan(const Symbolic& S, int n, const int* colptr, const int* rowind, P
         P.pers_fronts.push_back(i);
         P.pers_pending.push_back(F.child_end - F.child_begin);
         if (part == 1) P.pers_fmax = std::max(P.pers_fmax, F.f);
+        P.pers_slot[part] = std::max(P.pers_slot[part], (F.f | 1) * F.s);
+        P.pers_wld[part] = std::max(P.pers_wld[part], F.f);
       }
       if (part == 0) P.pers_nwarp = (int) P.pers_fronts.size();
     }
@@ -476,9 +475,6 @@ int build_plan(const Symbolic& S, int n, const int* colptr, const int* rowind, P
     for (LevelPlan& LP : P.levels) {
       for (int i : LP.small_fronts)
         if (task[i] < 0) LP.small_numeric.push_back(i);
-      while (LP.small_numeric_warp < (int) LP.small_numeric.size() &&
-             P.fronts[LP.small_numeric[LP.small_numeric_warp]].f <= SOLVE_WARP_F)
-        LP.small_numeric_warp++;
     }
   }
 

@@ -25,230 +25,332 @@ namespace tb {
 
 namespace {
 
-constexpr int SB = 32;   // substitution block (one warp)
-
-// Small fronts: G threads per front (256: one CTA; 32: one warp, eight
-// fronts per CTA for the many tiny fronts near the leaves).  The threads of
-// one front synchronise among themselves only.
-template <int G>
-__device__ __forceinline__ void group_sync() {
-  if (G == 32) __syncwarp();
-  else __syncthreads();
-}
-
-// forward step of one small front by a group of G threads; xs: the group's
-// shared staging of one substitution block
-template <typename T, int WS, int G>
-__device__ void fwd_small(const FrontDesc& F, const FrontDesc* __restrict__ fronts, const int* __restrict__ children,
-                          const int* __restrict__ maps, const int* __restrict__ rows, const T* __restrict__ L,
-                          const T* __restrict__ B, int ldb, T* __restrict__ W, int nrhs,
-                          T (&xs)[SB][SOLVE_NRHS]) {
-  const int f = F.f, s = F.s;
-  const int tid = threadIdx.x % G, nt = G, lane = tid & 31, warp = tid >> 5;
-  T* Wf = W + F.v_off * WS;
-  const int* rw = rows + F.rows_off;
-  const T* P = L + F.l_off;
-
-  for (int k = tid; k < f * nrhs; k += nt) {
-    const int r = k % f, q = k / f;
-    Wf[k] = (r < s) ? B[rw[r] + (size_t) q * ldb] : 0.0;
-  }
-  group_sync<G>();
-  for (int ci = F.child_begin; ci < F.child_end; ci++) {
-    const FrontDesc C = fronts[children[ci]];
-    const int mc = C.f - C.s;
-    const int* mp = maps + C.map_off;
-    const T* Wc = W + C.v_off * WS;
-    for (int k = tid; k < mc * nrhs; k += nt) {
-      const int i = k % mc, q = k / mc;
-      Wf[mp[i] + q * f] += Wc[C.s + i + q * C.f];
-    }
-    group_sync<G>();
-  }
-  for (int jb = 0; jb < s; jb += SB) {
-    const int bw = min(SB, s - jb);
-    if (warp == 0) {
-      // all right-hand sides advance together through one substitution chain
-      const T rd = (lane < bw) ? T(1) / P[(jb + lane) + (size_t) (jb + lane) * f] : T(0);
-      T v[SOLVE_NRHS];
-#pragma unroll
-      for (int q = 0; q < SOLVE_NRHS; q++) v[q] = (q < nrhs && lane < bw) ? Wf[jb + lane + q * f] : T(0);
-      for (int j = 0; j < bw; j++) {
-        const T rj = __shfl_sync(0xffffffffu, rd, j);
-        const T l = (lane > j && lane < bw) ? P[(jb + lane) + (size_t) (jb + j) * f] : T(0);
-#pragma unroll
-        for (int q = 0; q < SOLVE_NRHS; q++) {
-          if (q < nrhs) {
-            const T xj = __shfl_sync(0xffffffffu, v[q], j) * rj;
-            if (lane == j) v[q] = xj;
-            else v[q] -= l * xj;
-          }
-        }
-      }
-      if (lane < bw) {
-#pragma unroll
-        for (int q = 0; q < SOLVE_NRHS; q++)
-          if (q < nrhs) {
-            Wf[jb + lane + q * f] = v[q];
-            xs[lane][q] = v[q];
-          }
-      }
-    }
-    group_sync<G>();
-    for (int r = jb + bw + tid; r < f; r += nt) {
-      T acc[SOLVE_NRHS];
-#pragma unroll
-      for (int q = 0; q < SOLVE_NRHS; q++) acc[q] = 0.0;
-      for (int j = 0; j < bw; j++) {
-        const T l = P[r + (size_t) (jb + j) * f];
-#pragma unroll
-        for (int q = 0; q < SOLVE_NRHS; q++)
-          if (q < nrhs) acc[q] += l * xs[j][q];
-      }
-#pragma unroll
-      for (int q = 0; q < SOLVE_NRHS; q++)
-        if (q < nrhs) Wf[r + q * f] -= acc[q];
-    }
-    group_sync<G>();
-  }
-}
-
-template <typename T, int WS, int G>
-__global__ void __launch_bounds__(256)
-k_fwd(const int* __restrict__ list, int count, const FrontDesc* __restrict__ fronts, const int* __restrict__ children,
-      const int* __restrict__ maps, const int* __restrict__ rows, const T* __restrict__ L,
-      const T* __restrict__ B, int ldb, T* __restrict__ W, int nrhs) {
-  constexpr int GPC = 256 / G;   // fronts per CTA: one per group of G threads
-  __shared__ T xs_all[GPC][SB][SOLVE_NRHS];
-  const int grp = threadIdx.x / G, li = blockIdx.x * GPC + grp;
-  if (li >= count) return;
-  fwd_small<T, WS, G>(fronts[list[li]], fronts, children, maps, rows, L, B, ldb, W, nrhs, xs_all[grp]);
-}
-
-// backward step of one small front by a group of G threads
-template <typename T, int WS, int G>
-__device__ void bwd_small(const FrontDesc& F, const int* __restrict__ rows, const T* __restrict__ L,
-                          T* __restrict__ X, int ldx, T* __restrict__ W, int nrhs, T (&xs)[SB][SOLVE_NRHS]) {
-  const int f = F.f, s = F.s;
-  const int tid = threadIdx.x % G, nt = G, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  T* Wf = W + F.v_off * WS;
-  const int* rw = rows + F.rows_off;
-  const T* P = L + F.l_off;
-
-  // x at the update rows (final: written by ancestors)
-  for (int k = tid; k < (f - s) * nrhs; k += nt) {
-    const int i = k % (f - s), q = k / (f - s);
-    Wf[s + i + q * f] = X[rw[s + i] + (size_t) q * ldx];
-  }
-  group_sync<G>();
-  // r_j = y_j - sum_{i >= s} L[i,j] x_i
-  for (int j = warp; j < s; j += nw) {
-    T acc[SOLVE_NRHS];
-#pragma unroll
-    for (int q = 0; q < SOLVE_NRHS; q++) acc[q] = 0.0;
-    const T* pj = P + (size_t) j * f;
-    for (int i = s + lane; i < f; i += 32) {
-      const T l = pj[i];
-#pragma unroll
-      for (int q = 0; q < SOLVE_NRHS; q++)
-        if (q < nrhs) acc[q] += l * Wf[i + q * f];
-    }
-#pragma unroll
-    for (int q = 0; q < SOLVE_NRHS; q++) {
-      T v = acc[q];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      acc[q] = v;
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int q = 0; q < SOLVE_NRHS; q++)
-        if (q < nrhs) Wf[j + q * f] -= acc[q];
-    }
-  }
-  group_sync<G>();
-  // L11^T substitution, blocks from the end
-  const int nblk = (s + SB - 1) / SB;
-  for (int b = nblk - 1; b >= 0; b--) {
-    const int jb = b * SB, bw = min(SB, s - jb), je = jb + bw;
-    // contributions of the already solved x in rows [je, s)
-    if (je < s) {
-      for (int j = jb + warp; j < je; j += nw) {
-        T acc[SOLVE_NRHS];
-#pragma unroll
-        for (int q = 0; q < SOLVE_NRHS; q++) acc[q] = 0.0;
-        const T* pj = P + (size_t) j * f;
-        for (int i = je + lane; i < s; i += 32) {
-          const T l = pj[i];
-#pragma unroll
-          for (int q = 0; q < SOLVE_NRHS; q++)
-            if (q < nrhs) acc[q] += l * Wf[i + q * f];
-        }
-#pragma unroll
-        for (int q = 0; q < SOLVE_NRHS; q++) {
-          T v = acc[q];
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          acc[q] = v;
-        }
-        if (lane == 0) {
-#pragma unroll
-          for (int q = 0; q < SOLVE_NRHS; q++)
-            if (q < nrhs) Wf[j + q * f] -= acc[q];
-        }
-      }
-      group_sync<G>();
-    }
-    if (warp == 0) {
-      const T rd = (lane < bw) ? T(1) / P[(jb + lane) + (size_t) (jb + lane) * f] : T(0);
-      T v[SOLVE_NRHS];
-#pragma unroll
-      for (int q = 0; q < SOLVE_NRHS; q++) v[q] = (q < nrhs && lane < bw) ? Wf[jb + lane + q * f] : T(0);
-      for (int j = bw - 1; j >= 0; j--) {
-        const T rj = __shfl_sync(0xffffffffu, rd, j);
-        const T l = (lane < j) ? P[(jb + j) + (size_t) (jb + lane) * f] : T(0);
-#pragma unroll
-        for (int q = 0; q < SOLVE_NRHS; q++) {
-          if (q < nrhs) {
-            const T xj = __shfl_sync(0xffffffffu, v[q], j) * rj;
-            if (lane == j) v[q] = xj;
-            else v[q] -= l * xj;
-          }
-        }
-      }
-      if (lane < bw) {
-#pragma unroll
-        for (int q = 0; q < SOLVE_NRHS; q++)
-          if (q < nrhs) xs[lane][q] = v[q];
-      }
-    }
-    group_sync<G>();
-    for (int k = tid; k < bw * nrhs; k += nt) {
-      const int l = k % bw, q = k / bw;
-      Wf[jb + l + q * f] = xs[l][q];
-    }
-    group_sync<G>();
-  }
-  for (int k = tid; k < s * nrhs; k += nt) {
-    const int r = k % s, q = k / s;
-    X[rw[r] + (size_t) q * ldx] = Wf[r + q * f];
-  }
-}
-
-template <typename T, int WS, int G>
-__global__ void __launch_bounds__(256)
-k_bwd(const int* __restrict__ list, int count, const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
-      const T* __restrict__ L, T* __restrict__ X, int ldx, T* __restrict__ W,
-      int nrhs) {
-  constexpr int GPC = 256 / G;
-  __shared__ T xs_all[GPC][SB][SOLVE_NRHS];
-  const int grp = threadIdx.x / G, li = blockIdx.x * GPC + grp;
-  if (li >= count) return;
-  bwd_small<T, WS, G>(fronts[list[li]], rows, L, X, ldx, W, nrhs, xs_all[grp]);
-}
-
-__device__ __forceinline__ int ld_acquire_i(const int* p) {
+__device__ __forceinline__ int ld_acquire(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
+}
+
+constexpr int SB = 32;   // substitution block (one warp)
+
+// ------------------------------------------------------------- small fronts
+// Fronts of order f <= SMALL_F_MAX, one warp each.  What bounds them is
+// latency (a 33 x 33 grid is a chain of 8 dependent fronts each way), so a
+// front's data are on their way before its dependency is waited for: the
+// task's record (SolveTask: one 32-byte load instead of list entry, then
+// descriptor), its panel (element-wise asynchronous copies into the warp's
+// slot of shared memory, column stride f | 1 so that both the row reads of
+// the forward pass and the column reads of the backward pass are free of bank
+// conflicts), its right-hand side entries and its children's records.  After
+// the wait one round of loads fetches the neighbours' vectors, and the
+// substitution runs from shared memory and registers: lane l holds rows l,
+// l + 32, l + 64, and a step costs a shuffle and a multiply-add (the column
+// is divided by its pivot off the chain).  A panel larger than the slot goes
+// through it in column pieces.  Both persistent launches together, one
+// right-hand side: 33 x 33 grid, FP64, 140 -> 54 us forward and 72 -> 50 us
+// backward; 512 grids at once, FP32, a refined solution's three passes 12.5 ->
+// 8.7 ms.
+constexpr int SF_SLOTS = (SMALL_F_MAX + 31) / 32;   // rows per lane
+
+__device__ __forceinline__ void cp_async_elem(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned) __cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void cp_async_elem(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned) __cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void cp_async_wait_warp() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+}
+
+// the lower part of columns [ja, je) of a panel (ld f) into pan (ld f | 1)
+template <typename T>
+__device__ __forceinline__ void stage_columns(const T* P, int f, int ja, int je, T* pan) {
+  const int lane = threadIdx.x & 31, ld = f | 1;
+  for (int j = ja; j < je; j++)
+    for (int r = (j & ~31) + lane; r < f; r += 32)
+      if (r >= j) cp_async_elem(pan + (size_t) (j - ja) * ld + r, P + r + (size_t) j * f);
+}
+
+// columns a slot of `slot` elements holds of a panel of order f
+__device__ __forceinline__ int slot_columns(int slot, int f) { return slot / (f | 1); }
+
+// what a warp holds of its front before the dependency wait of the forward
+// step: the first piece of the panel on its way, b at its columns in ws (zero
+// in the other rows), and the records of the first 32 children in the lanes
+template <typename T, int NQ>
+__device__ __forceinline__ int4 fwd_front_begin(const SolveTask& K, const int4* __restrict__ child_rec,
+                                                const int* __restrict__ rows, const T* __restrict__ L,
+                                                const T* __restrict__ B, int ldb, int nrhs, T* pan, int slot, T* ws,
+                                                int wld) {
+  const int lane = threadIdx.x & 31, f = K.f, s = K.s;
+  stage_columns(L + K.l_off, f, 0, min(s, slot_columns(slot, f)), pan);
+  int g[SF_SLOTS];
+#pragma unroll
+  for (int k = 0; k < SF_SLOTS; k++) g[k] = lane + 32 * k < s ? __ldg(rows + K.rows_off + lane + 32 * k) : -1;
+  const int4 rec = lane < K.child_end - K.child_begin ? __ldg(child_rec + K.child_begin + lane) : make_int4(0, 0, 0, 0);
+#pragma unroll
+  for (int k = 0; k < SF_SLOTS; k++)
+    if (32 * k < f) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++)
+        if (lane + 32 * k < f)
+          ws[q * wld + lane + 32 * k] = (g[k] >= 0 && q < nrhs) ? B[g[k] + (size_t) q * ldb] : T(0);
+    }
+  return rec;
+}
+
+// the forward step itself, once the children are done: their update vectors
+// added in child order, then y = L11^-1 w and u = w2 - L21 y into W
+template <typename T, int NQ, int WS>
+__device__ __forceinline__ void fwd_front(const SolveTask& K, int4 rec, const int4* __restrict__ child_rec,
+                                          const int* __restrict__ maps, const T* __restrict__ L, T* __restrict__ W,
+                                          int nrhs, T* pan, int slot, T* ws, int wld) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, f = K.f, s = K.s, ld = f | 1;
+  const int nch = K.child_end - K.child_begin;
+  for (int c0 = 0; c0 < nch; c0 += 32) {
+    if (c0 > 0) rec = c0 + lane < nch ? __ldg(child_rec + K.child_begin + c0 + lane) : make_int4(0, 0, 0, 0);
+    // CB children per round: all their loads before the first add
+    constexpr int CB = NQ == 1 ? 4 : NQ <= 4 ? 2 : 1;
+    const int ce = min(32, nch - c0);
+    for (int c = 0; c < ce; c += CB) {
+      int pi[CB][SF_SLOTS];
+      T val[CB][SF_SLOTS][NQ];
+#pragma unroll
+      for (int u = 0; u < CB; u++) {
+        const int src = (c + u) & 31;
+        const int voff = __shfl_sync(FULL, rec.x, src), cs = __shfl_sync(FULL, rec.y, src),
+                  cf = __shfl_sync(FULL, rec.z, src), mo = __shfl_sync(FULL, rec.w, src);
+        const int mc = c + u < ce ? cf - cs : 0;
+        const T* Wc = W + (int64_t) voff * WS + cs;
+#pragma unroll
+        for (int k = 0; k < SF_SLOTS; k++) {
+          const int i = lane + 32 * k;
+          pi[u][k] = i < mc ? __ldg(maps + mo + i) : -1;
+#pragma unroll
+          for (int q = 0; q < NQ; q++) val[u][k][q] = (i < mc && q < nrhs) ? __ldcg(Wc + i + (size_t) q * cf) : T(0);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < CB; u++) {
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < SF_SLOTS; k++)
+          if (pi[u][k] >= 0) {
+#pragma unroll
+            for (int q = 0; q < NQ; q++) ws[q * wld + pi[u][k]] += val[u][k][q];
+          }
+      }
+    }
+  }
+  __syncwarp();
+  T v[SF_SLOTS][NQ], rd[SF_SLOTS];
+#pragma unroll
+  for (int k = 0; k < SF_SLOTS; k++)
+#pragma unroll
+    for (int q = 0; q < NQ; q++) v[k][q] = lane + 32 * k < f ? ws[q * wld + lane + 32 * k] : T(0);
+  const int cw = slot_columns(slot, f);
+#pragma unroll
+  for (int k = 0; k < SF_SLOTS; k++) rd[k] = T(0);
+  int staged = 0;   // first column of the staged piece
+  cp_async_wait_warp();
+  for (int ja = 0; ja < s;) {
+    if (ja >= staged + cw) {   // the next piece of a panel larger than the slot
+      __syncwarp();
+      stage_columns(L + K.l_off, f, ja, min(s, ja + cw), pan);
+      staged = ja;
+      cp_async_wait_warp();
+    }
+    const int je = min(min(s, staged + cw), (ja & ~31) + 32), kb = ja >> 5;
+    const T* pc = pan - (size_t) staged * ld;
+    // columns [ja, je), all in row slot kb
+#pragma unroll
+    for (int b = 0; b < SF_SLOTS; b++) {
+      if (b != kb) continue;
+      const int own = 32 * b + lane;
+      if (own >= ja && own < je) rd[b] = T(1) / pc[own + own * ld];
+      // lane l holds 1 / L_ll for the columns of this piece
+#pragma unroll 4
+      for (int j = ja; j < je; j++) {
+        const T rj = __shfl_sync(FULL, rd[b], j & 31);
+        T l[SF_SLOTS];
+#pragma unroll
+        for (int k = b; k < SF_SLOTS; k++) {
+          const int r = lane + 32 * k;
+          l[k] = (r > j && r < f) ? pc[r + j * ld] * rj : T(0);
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          const T vj = __shfl_sync(FULL, v[b][q], j & 31);
+#pragma unroll
+          for (int k = b; k < SF_SLOTS; k++) v[k][q] -= l[k] * vj;
+        }
+      }
+    }
+    ja = je;
+  }
+  T* Wf = W + (int64_t) K.rows_off * WS;
+#pragma unroll
+  for (int k = 0; k < SF_SLOTS; k++) {
+    const int r = lane + 32 * k;
+    if (r < f) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++)
+        if (q < nrhs) Wf[r + (size_t) q * f] = r < s ? v[k][q] * rd[k] : v[k][q];
+    }
+  }
+}
+
+// columns of one piece of the backward step: a block of 32, or fewer when the
+// slot does not hold the whole panel
+__device__ __forceinline__ int bwd_piece(int slot, int f, int s) {
+  const int cw = slot_columns(slot, f);
+  return cw >= s ? SB : min(SB, cw);
+}
+
+// the backward step before the wait for the parent: the last piece of the
+// panel (the whole panel when the slot holds it) on its way, y in ws, and the
+// global rows of the lane's local rows
+template <typename T, int NQ, int WS>
+__device__ __forceinline__ void bwd_front_begin(const SolveTask& K, const int* __restrict__ rows,
+                                                const T* __restrict__ L, const T* __restrict__ W, int nrhs, T* pan,
+                                                int slot, T* ws, int wld, int (&g)[SF_SLOTS]) {
+  const int lane = threadIdx.x & 31, f = K.f, s = K.s;
+  const int ja = slot_columns(slot, f) >= s ? 0 : max(0, s - bwd_piece(slot, f, s));
+  stage_columns(L + K.l_off, f, ja, s, pan);
+  const T* Wf = W + (int64_t) K.rows_off * WS;
+#pragma unroll
+  for (int k = 0; k < SF_SLOTS; k++) {
+    const int r = lane + 32 * k;
+    g[k] = r < f ? __ldg(rows + K.rows_off + r) : -1;
+    if (r < s) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++) ws[q * wld + r] = q < nrhs ? Wf[r + (size_t) q * f] : T(0);
+    }
+  }
+}
+
+// the backward step once x at the update rows is final: per piece of columns
+// from the last, r = y - L[below, piece]^T x_below (lane (column c, part p)
+// sums every 32 / columns-th row; the parts are added by shuffles), then the
+// L11^T substitution
+template <typename T, int NQ>
+__device__ __forceinline__ void bwd_front(const SolveTask& K, const T* __restrict__ L, T* __restrict__ X, int ldx,
+                                          int nrhs, T* pan, int slot, T* ws, int wld, const int (&g)[SF_SLOTS]) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, f = K.f, s = K.s, ld = f | 1;
+  {
+    T x[SF_SLOTS][NQ];
+#pragma unroll
+    for (int k = 0; k < SF_SLOTS; k++)
+#pragma unroll
+      for (int q = 0; q < NQ; q++)
+        x[k][q] = (g[k] >= 0 && lane + 32 * k >= s && q < nrhs) ? __ldcg(X + g[k] + (size_t) q * ldx) : T(0);
+#pragma unroll
+    for (int k = 0; k < SF_SLOTS; k++)
+      if (g[k] >= 0 && lane + 32 * k >= s) {
+#pragma unroll
+        for (int q = 0; q < NQ; q++) ws[q * wld + lane + 32 * k] = x[k][q];
+      }
+  }
+  const int pw = bwd_piece(slot, f, s);
+  const bool whole = slot_columns(slot, f) >= s;
+  cp_async_wait_warp();
+  for (int je = s; je > 0;) {
+    // the last piece is the ragged one when the panel goes block by block
+    const int ja = whole ? (je - 1) & ~31 : max(0, je - pw), bw = je - ja;
+    if (!whole && je < s) {
+      __syncwarp();
+      stage_columns(L + K.l_off, f, ja, je, pan);
+      cp_async_wait_warp();
+    }
+    const T* pc = whole ? pan : pan - (size_t) ja * ld;
+    int cwp = 1;
+    while (cwp < bw) cwp <<= 1;
+    const int c = lane & (cwp - 1), part = lane / cwp, np = 32 / cwp;
+    const bool own = c < bw;
+    const T* pj = pc + (ja + (own ? c : 0)) * ld;
+    T acc[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) acc[q] = T(0);
+#pragma unroll 4
+    for (int i = je + part; i < f; i += np) {
+      const T l = pj[i];
+#pragma unroll
+      for (int q = 0; q < NQ; q++) acc[q] += l * ws[q * wld + i];
+    }
+    for (int o = cwp; o < 32; o <<= 1)
+#pragma unroll
+      for (int q = 0; q < NQ; q++) acc[q] += __shfl_xor_sync(FULL, acc[q], o);
+    const T rd = own ? T(1) / pj[ja + c] : T(0);
+    T v[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) v[q] = own ? ws[q * wld + ja + c] - acc[q] : T(0);
+#pragma unroll 4
+    for (int k = bw - 1; k > 0; k--) {
+      const T rk = __shfl_sync(FULL, rd, k);
+      const T l = (own && c < k) ? pj[ja + k] * rk : T(0);
+#pragma unroll
+      for (int q = 0; q < NQ; q++) v[q] -= l * __shfl_sync(FULL, v[q], k);
+    }
+    __syncwarp();
+    if (own && part == 0) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++) ws[q * wld + ja + c] = v[q] * rd;
+    }
+    __syncwarp();
+    je = ja;
+  }
+#pragma unroll
+  for (int k = 0; k < SF_SLOTS; k++)
+    if (lane + 32 * k < s) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++)
+        if (q < nrhs) X[g[k] + (size_t) q * ldx] = ws[q * wld + lane + 32 * k];
+    }
+}
+
+// elements of a warp's slot and vectors in the dynamic shared memory of the
+// small-front kernels: wld is the largest order among the launch's fronts
+template <typename T, int NQ>
+__host__ __device__ constexpr size_t sf_warp_smem(int slot, int wld) {
+  return ((size_t) slot + (size_t) NQ * wld) * sizeof(T);
+}
+
+__device__ __forceinline__ SolveTask task_of(const FrontDesc& F) {
+  return SolveTask{F.l_off, F.rows_off, F.s, F.f, F.child_begin, F.child_end, -1};
+}
+
+// level launches: the small fronts with a big front below them (and every
+// small front of the allocation-free solve), a warp each, no waits
+template <typename T, int NQ, int WS>
+__global__ void __launch_bounds__(128)
+k_fwd(const int* __restrict__ list, int count, const FrontDesc* __restrict__ fronts, const int4* __restrict__ child_rec,
+      const int* __restrict__ maps, const int* __restrict__ rows, const T* __restrict__ L, const T* __restrict__ B,
+      int ldb, T* __restrict__ W, int nrhs, int slot, int wld) {
+  extern __shared__ __align__(16) unsigned char sfm[];
+  const int wi = threadIdx.x >> 5, li = blockIdx.x * (blockDim.x >> 5) + wi;
+  if (li >= count) return;
+  T* pan = reinterpret_cast<T*>(sfm + wi * sf_warp_smem<T, NQ>(slot, wld));
+  const SolveTask K = task_of(fronts[list[li]]);
+  const int4 rec = fwd_front_begin<T, NQ>(K, child_rec, rows, L, B, ldb, nrhs, pan, slot, pan + slot, wld);
+  fwd_front<T, NQ, WS>(K, rec, child_rec, maps, L, W, nrhs, pan, slot, pan + slot, wld);
+}
+
+template <typename T, int NQ, int WS>
+__global__ void __launch_bounds__(128)
+k_bwd(const int* __restrict__ list, int count, const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
+      const T* __restrict__ L, T* __restrict__ X, int ldx, const T* __restrict__ W, int nrhs, int slot, int wld) {
+  extern __shared__ __align__(16) unsigned char sfm[];
+  const int wi = threadIdx.x >> 5, li = blockIdx.x * (blockDim.x >> 5) + wi;
+  if (li >= count) return;
+  T* pan = reinterpret_cast<T*>(sfm + wi * sf_warp_smem<T, NQ>(slot, wld));
+  const SolveTask K = task_of(fronts[list[li]]);
+  int g[SF_SLOTS];
+  bwd_front_begin<T, NQ, WS>(K, rows, L, W, nrhs, pan, slot, pan + slot, wld, g);
+  __syncwarp();
+  bwd_front<T, NQ>(K, L, X, ldx, nrhs, pan, slot, pan + slot, wld, g);
 }
 
 // Waits (bounded) until *p holds v.  Every lane of the warp polls and the loop
@@ -258,174 +360,81 @@ __device__ __forceinline__ int ld_acquire_i(const int* p) {
 // 148 us with one lane polling, 72 us with the whole warp).
 __device__ __forceinline__ void warp_wait_value(const int* p, int v, int* status) {
   int it = 0;
-  while (!__all_sync(0xffffffffu, ld_acquire_i(p) == v)) {
+  while (!__all_sync(0xffffffffu, ld_acquire(p) == v)) {
     if (++it > (1 << 22)) {
       atomicExch(status, SOLVE_TIMEOUT);
       break;
     }
-    __nanosleep(32);
+    __nanosleep(20);
   }
 }
 
-// One-warp form of the backward small-front step for the persistent launch
-// (fronts of order f <= SMALL_F_MAX): the front's vector is kept in the
-// warp's shared rows ws[nrhs][f]; each lane holds the L entries it needs for
-// the substitution chain in registers, loaded together (in groups of eight,
-// as far as the block is wide) before the arithmetic, so that the chain
-// waits for memory once per 32-column block instead of once per column.
-// (The same form of the forward step measured slower than fwd_small.)
-constexpr int PW_SLOTS = (SMALL_F_MAX + 31) / 32;   // rows per lane
-
-// backward step of one small front by one warp: x at the update rows, then
-// per diagonal block from the last: r = y - L[below, block]^T x_below (lane
-// j takes column jb + j, the rows in batches of eight loads), and the L11^T
-// substitution chain from registers
-template <typename T, int WS>
-__device__ void bwd_warp(const FrontDesc& F, const int* __restrict__ rows, const T* __restrict__ L,
-                         T* __restrict__ X, int ldx, const T* __restrict__ W, int nrhs, T (*ws)[SMALL_F_MAX]) {
-  constexpr unsigned FULL = 0xffffffffu;
-  const int f = F.f, s = F.s, lane = threadIdx.x & 31;
-  const T* Wf = W + F.v_off * WS;
-  const int* rw = rows + F.rows_off;
-  const T* P = L + F.l_off;
-  {
-    int g[PW_SLOTS];
-#pragma unroll
-    for (int sl = 0; sl < PW_SLOTS; sl++) {
-      const int r = lane + 32 * sl;
-      g[sl] = (r >= s && r < f) ? __ldg(rw + r) : -1;
-    }
-#pragma unroll
-    for (int q = 0; q < SOLVE_NRHS; q++) {
-      if (q >= nrhs) break;
-      T v[PW_SLOTS];
-#pragma unroll
-      for (int sl = 0; sl < PW_SLOTS; sl++) {
-        const int r = lane + 32 * sl;
-        v[sl] = g[sl] >= 0 ? X[g[sl] + (size_t) q * ldx] : r < s ? Wf[r + q * f] : T(0);
-      }
-#pragma unroll
-      for (int sl = 0; sl < PW_SLOTS; sl++)
-        if (lane + 32 * sl < f) ws[q][lane + 32 * sl] = v[sl];
-    }
-  }
-  __syncwarp();
-  const int nblk = (s + SB - 1) / SB;
-  for (int b = nblk - 1; b >= 0; b--) {
-    const int jb = b * SB, bw = min(SB, s - jb), je = jb + bw;
-    const bool own = lane < bw;
-    const T* pj = P + (size_t) (jb + lane) * f;
-    // the solved rows below the block: x in rows [je, f)
-    T acc[SOLVE_NRHS];
-#pragma unroll
-    for (int q = 0; q < SOLVE_NRHS; q++) acc[q] = T(0);
-    for (int i0 = je; i0 < f; i0 += 8) {
-      T l[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++) l[u] = (own && i0 + u < f) ? pj[i0 + u] : T(0);
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        if (i0 + u >= f) break;
-#pragma unroll
-        for (int q = 0; q < SOLVE_NRHS; q++)
-          if (q < nrhs) acc[q] += l[u] * ws[q][i0 + u];
-      }
-    }
-    // lane l: column jb + l of the diagonal block
-    T lc[SB];
-#pragma unroll
-    for (int k0 = 0; k0 < SB; k0 += 8) {
-      if (k0 >= bw) break;
-#pragma unroll
-      for (int k = k0; k < k0 + 8; k++) lc[k] = (own && k > lane && k < bw) ? pj[jb + k] : T(0);
-    }
-    const T rd = own ? T(1) / pj[jb + lane] : T(0);
-    T v[SOLVE_NRHS];
-#pragma unroll
-    for (int q = 0; q < SOLVE_NRHS; q++) v[q] = (q < nrhs && own) ? ws[q][jb + lane] - acc[q] : T(0);
-#pragma unroll
-    for (int j = SB - 1; j >= 0; j--) {
-      if (j >= bw) continue;
-      const T rj = __shfl_sync(FULL, rd, j);
-#pragma unroll
-      for (int q = 0; q < SOLVE_NRHS; q++) {
-        if (q >= nrhs) break;
-        const T xj = __shfl_sync(FULL, v[q], j) * rj;
-        if (lane == j) v[q] = xj;
-        else v[q] -= lc[j] * xj;
-      }
-    }
-    if (own)
-#pragma unroll
-      for (int q = 0; q < SOLVE_NRHS; q++)
-        if (q < nrhs) ws[q][jb + lane] = v[q];
-    __syncwarp();
-  }
-#pragma unroll
-  for (int sl = 0; sl < PW_SLOTS; sl++) {
-    const int r = lane + 32 * sl;
-    if (r < s) {
-      const int g = __ldg(rw + r);
-#pragma unroll
-      for (int q = 0; q < SOLVE_NRHS; q++)
-        if (q < nrhs) X[g + (size_t) q * ldx] = ws[q][r];
-    }
-  }
-}
-
-// The small fronts with only small fronts below them (Plan::pers_fronts), in
-// one launch per direction; each warp takes the next front from a device-
-// side queue.  Forward, in level order: a front waits until its children's
-// update vectors are in place (pending count), and counts itself off at its
-// parent.  Backward, in reverse level order: a front waits until its parent
-// has written x at its update rows (done flag = epoch; parents outside the
-// set ran in the level launches before this one).  Every wait is bounded
-// (SOLVE_TIMEOUT).
-template <typename T, int WS>
-__global__ void __launch_bounds__(256)
-k_fwd_pers(const int* __restrict__ tasks, int ntask, const int* __restrict__ parent_task, int* pending, int* next,
-           const FrontDesc* __restrict__ fronts, const int* __restrict__ children, const int* __restrict__ maps,
-           const int* __restrict__ rows, const T* __restrict__ L, const T* __restrict__ B, int ldb,
-           T* __restrict__ W, int nrhs, int* status) {
-  __shared__ T xs_all[8][SB][SOLVE_NRHS];
+// The small fronts with only small fronts below them (Plan::pers_fronts),
+// tasks [t0, t1) of their queue in one launch: each warp takes the next front
+// from a device-side queue.  Forward, in level order: a front waits until its
+// children's update vectors are in place (pending count), and counts itself
+// off at its parent.  Backward, in reverse level order: a front waits until
+// its parent has written x at its update rows (done flag = epoch; parents
+// outside the set ran in the level launches before this one).  A warp claims
+// its next task before it works on the current one; the oldest unfinished
+// task is always the current one of its warp, so every wait ends.  Every wait
+// is bounded all the same (SOLVE_TIMEOUT).
+template <typename T, int NQ, int WS>
+__global__ void __launch_bounds__(256, NQ == 1 ? 4 : sizeof(T) == 4 ? 3 : 2)
+k_fwd_pers(const SolveTask* __restrict__ tasks, int t0, int t1, int* pending, int* next,
+           const int4* __restrict__ child_rec, const int* __restrict__ maps, const int* __restrict__ rows,
+           const T* __restrict__ L, const T* __restrict__ B, int ldb, T* __restrict__ W, int nrhs, int* status,
+           int slot, int wld) {
+  extern __shared__ __align__(16) unsigned char sfm[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  for (;;) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(next, 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t >= ntask) break;
-    warp_wait_value(pending + t, 0, status);
-    fwd_small<T, WS, 32>(fronts[tasks[t]], fronts, children, maps, rows, L, B, ldb, W, nrhs, xs_all[wi]);
+  T* pan = reinterpret_cast<T*>(sfm + wi * sf_warp_smem<T, NQ>(slot, wld));
+  T* ws = pan + slot;
+  int t = 0;
+  if (lane == 0) t = t0 + atomicAdd(next, 1);
+  t = __shfl_sync(0xffffffffu, t, 0);
+  while (t < t1) {
+    int tn = 0;
+    if (lane == 0) tn = t0 + atomicAdd(next, 1);
+    const SolveTask K = tasks[t];
+    const int4 rec = fwd_front_begin<T, NQ>(K, child_rec, rows, L, B, ldb, nrhs, pan, slot, ws, wld);
+    if (K.child_end > K.child_begin) warp_wait_value(pending + t, 0, status);
+    fwd_front<T, NQ, WS>(K, rec, child_rec, maps, L, W, nrhs, pan, slot, ws, wld);
     __syncwarp();
-    if (lane == 0) {
+    if (lane == 0 && K.parent >= 0) {
       __threadfence();
-      const int pt = parent_task[t];
-      if (pt >= 0) atomicSub(pending + pt, 1);
+      atomicSub(pending + K.parent, 1);
     }
+    t = __shfl_sync(0xffffffffu, tn, 0);
   }
 }
 
-template <typename T, int WS>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2)
-k_bwd_pers(const int* __restrict__ tasks, int ntask, const int* __restrict__ parent_task, int* done, int* next,
-           int epoch, const FrontDesc* __restrict__ fronts, const int* __restrict__ rows, const T* __restrict__ L,
-           T* __restrict__ X, int ldx, T* __restrict__ W, int nrhs, int* status) {
-  __shared__ T ws_all[8][SOLVE_NRHS][SMALL_F_MAX];
+template <typename T, int NQ, int WS>
+__global__ void __launch_bounds__(256, NQ == 1 ? 4 : sizeof(T) == 4 ? 3 : 2)
+k_bwd_pers(const SolveTask* __restrict__ tasks, int t0, int t1, int* done, int* next, int epoch,
+           const int* __restrict__ rows, const T* __restrict__ L, T* __restrict__ X, int ldx, const T* __restrict__ W,
+           int nrhs, int* status, int slot, int wld) {
+  extern __shared__ __align__(16) unsigned char sfm[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  for (;;) {
-    int q = 0;
-    if (lane == 0) q = atomicAdd(next, 1);
-    q = __shfl_sync(0xffffffffu, q, 0);
-    if (q >= ntask) break;
-    const int t = ntask - 1 - q;
-    const int pt = parent_task[t];
-    if (pt >= 0) warp_wait_value(done + pt, epoch, status);
-    bwd_warp<T, WS>(fronts[tasks[t]], rows, L, X, ldx, W, nrhs, ws_all[wi]);
+  T* pan = reinterpret_cast<T*>(sfm + wi * sf_warp_smem<T, NQ>(slot, wld));
+  T* ws = pan + slot;
+  int t = 0;
+  if (lane == 0) t = t1 - 1 - atomicAdd(next, 1);
+  t = __shfl_sync(0xffffffffu, t, 0);
+  while (t >= t0) {
+    int tn = 0;
+    if (lane == 0) tn = t1 - 1 - atomicAdd(next, 1);
+    const SolveTask K = tasks[t];
+    int g[SF_SLOTS];
+    bwd_front_begin<T, NQ, WS>(K, rows, L, W, nrhs, pan, slot, ws, wld, g);
+    if (K.parent >= 0) warp_wait_value(done + K.parent, epoch, status);
+    else __syncwarp();
+    bwd_front<T, NQ>(K, L, X, ldx, nrhs, pan, slot, ws, wld, g);
     __syncwarp();
-    if (lane == 0) {
+    if (lane == 0 && K.child_end > K.child_begin) {
       __threadfence();
       atomicExch(done + t, epoch);
     }
+    t = __shfl_sync(0xffffffffu, tn, 0);
   }
 }
 
@@ -443,12 +452,6 @@ constexpr int BR = PANEL_NB;   // rows per block
 // columns
 template <typename T, int NQ>
 constexpr size_t bwd_smem() { return (NQ >= 8 ? 2 : 1) * BR * (BR + 1) * sizeof(T); }
-
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 
 __device__ __forceinline__ void st_release(int* p, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
@@ -1788,8 +1791,19 @@ k_bwd_walk(const int* __restrict__ walk_fronts, int nwalk, const int2_* __restri
   }
 }
 
-// advances the walks' call counter (one thread)
-__global__ void k_walk_counter(int* counter) { *counter += 1; }
+// the start of a pass: the first nfl chain flags cleared (with them the
+// persistent set's done flags), the persistent queues' pending counts and
+// heads, and the walks' call counter advanced when there is one
+__global__ void k_solve_reset(int* flags, int nfl, const int* __restrict__ pending0, int* pers, int np, int* counter) {
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
+  for (int i = i0; i < nfl; i += n) flags[i] = 0;
+  for (int i = i0; i < np; i += n) {
+    pers[i] = pending0[i];
+    if (nfl > 0) pers[np + i] = 0;
+  }
+  if (i0 < 4) pers[2 * np + i0] = 0;
+  if (counter && i0 == 0) *counter += 1;
+}
 
 }  // namespace
 
@@ -1831,6 +1845,25 @@ static void solve_attrs() {
     cudaFuncSetAttribute(k_bwd_big<T, 8, SOLVE_NRHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 8>());
     cudaFuncSetAttribute(k_bwd_big<T, 1, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 1>());
     cudaFuncSetAttribute(k_bwd_big<T, 8, SOLVE_NRHS, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 8>());
+    auto sf = [](auto nqc) {
+      constexpr int Q = decltype(nqc)::value;
+      // the most any launch asks for: 8 warps of fronts of order <= 32, or 4
+      // warps with a full slot
+      const size_t most = std::max(8 * sf_warp_smem<T, Q>(SMALL_WARP_F * (SMALL_WARP_F + 1), SMALL_WARP_F),
+                                   4 * sf_warp_smem<T, Q>(SOLVE_SLOT_BYTES / sizeof(T), SMALL_F_MAX));
+      cudaFuncSetAttribute(k_fwd_pers<T, Q, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) most);
+      cudaFuncSetAttribute(k_bwd_pers<T, Q, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) most);
+      cudaFuncSetAttribute(k_fwd<T, Q, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) most);
+      cudaFuncSetAttribute(k_bwd<T, Q, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) most);
+    };
+    sf(std::integral_constant<int, 1>());
+    sf(std::integral_constant<int, 4>());
+    sf(std::integral_constant<int, SOLVE_NRHS>());
+    if constexpr (std::is_same<T, double>::value) {
+      const int most = (int) (4 * sf_warp_smem<T, 1>(SOLVE_SLOT_BYTES / sizeof(T), SMALL_F_MAX));
+      cudaFuncSetAttribute(k_fwd<T, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+      cudaFuncSetAttribute(k_bwd<T, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    }
     if constexpr (std::is_same<T, float>::value) {
       cudaFuncSetAttribute(k_fwd_walk<T, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int) walk_smem<T>());
@@ -1841,9 +1874,9 @@ static void solve_attrs() {
   });
 }
 
-// CTAs (eight warps each) of the persistent small-front solve launches: up
-// to four per SM, no more than the fronts need
-static int pers_solve_grid(int ntask) {
+// resident CTAs of a small-front kernel on the current device
+template <typename K>
+static int sf_resident(K kernel, int threads, size_t smem) {
   static PerDeviceOnce pd;
   static int sms[MAX_DEVICES];
   per_device_once(pd, [] {
@@ -1852,18 +1885,39 @@ static int pers_solve_grid(int ntask) {
     cudaDeviceGetAttribute(&sms[d], cudaDevAttrMultiProcessorCount, d);
     return true;
   });
-  int d = 0;
+  int d = 0, b = 0;
   cudaGetDevice(&d);
-  return std::max(1, std::min((ntask + 7) / 8, 4 * std::max(sms[d], 1)));
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, smem) != cudaSuccess) b = 1;
+  return std::max(b, 1) * std::max(sms[d], 1);
+}
+
+// slot (elements) of a small-front launch whose largest panel has `need`
+template <typename T>
+static int sf_slot(int need) {
+  return std::min((need + 3) & ~3, (int) (SOLVE_SLOT_BYTES / sizeof(T)));
+}
+
+// the queue part `part` of the persistent set: its tasks, and the warps per
+// CTA (the second part's fronts take up to 16 KB of shared memory a warp:
+// smaller CTAs fill an SM better)
+static void sf_part(const Plan& P, int np, int part, int* t0, int* t1, int* threads) {
+  *t0 = part ? P.pers_nwarp : 0;
+  *t1 = part ? np : P.pers_nwarp;
+  *threads = part ? 128 : 256;
+}
+
+// the columns of the instantiation that a pass of nq right-hand sides takes
+template <typename F>
+static void sf_dispatch(int nq, F run) {
+  if (nq <= 1) run(std::integral_constant<int, 1>());
+  else if (nq <= 4) run(std::integral_constant<int, 4>());
+  else run(std::integral_constant<int, SOLVE_NRHS>());
 }
 
 template <typename T>
 static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Dinv, int nrhs, T* X, const T* B, int ld, T* W,
                         T* part, int* flags, int* epoch, int* status, cudaStream_t st) {
   solve_attrs<T>();
-  // the handshake flags restart from zero on every call, so the epochs of a
-  // call are always 1, 2, ... and a recorded launch sequence stays valid
-  cudaMemsetAsync(flags, 0, sizeof(int) * solve_flag_words(P), st);
   // the walks: their tagged pairs, and the call counter in the word after
   // the cleared ones, advanced on the device once per call
   int* counter = flags + solve_flag_words(P);
@@ -1877,29 +1931,45 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
   };
   bool walks = false;
   for (const LevelPlan& LP : P.levels) walks = walks || walk_level(LP, true) || walk_level(LP, false);
-  if (walks) {
-    k_walk_counter<<<1, 1, 0, st>>>(counter);
-    count_launch();
-  }
   const int np = D.n_pers;
-  if (np > 0) cudaMemsetAsync(D.pers_solve, 0, sizeof(int) * (size_t) (2 * np + 2), st);
+  // the handshake flags restart from zero on every call, so the epochs of a
+  // call are always 1, 2, ... and a recorded launch sequence stays valid; one
+  // launch resets them, the persistent queues and the walks' call counter
+  auto reset = [&](bool first) {
+    const int nfl = first ? (int) solve_flag_words(P) : 0;
+    const int grid = std::max(1, std::min(148, (std::max(nfl, np) + 255) / 256));
+    k_solve_reset<<<grid, 256, 0, st>>>(flags, nfl, D.pers_pending0, D.pers_solve, np, first && walks ? counter : nullptr);
+    count_launch();
+  };
+  auto small_list = [&](int h, int nq, auto launch) {
+    const int ns = (int) P.levels[h].small_numeric.size();
+    if (ns > 0) sf_dispatch(nq, [&](auto nqc) { launch(nqc, D.small_num + D.small_num_off[h], ns); });
+  };
   int ep = 0;
   for (int q0 = 0; q0 < nrhs; q0 += SOLVE_NRHS) {
     const int nq = std::min(SOLVE_NRHS, nrhs - q0);
     const T* Bq = B + (size_t) q0 * ld;
     T* Xq = X + (size_t) q0 * ld;
     const int ef = ++ep;
-    if (np > 0) {
-      // every small front with only small fronts below it, one launch
-      cudaMemcpyAsync(D.pers_solve, D.pers_pending0, sizeof(int) * np, cudaMemcpyDeviceToDevice, st);
-      cudaMemsetAsync(D.pers_solve + 2 * np, 0, 2 * sizeof(int), st);
+    reset(q0 == 0);
+    // every small front with only small fronts below it, a launch per part
+    for (int part = 0; part < 2; part++) {
+      int t0, t1, th;
+      sf_part(P, np, part, &t0, &t1, &th);
+      if (t1 <= t0) continue;
       double by = 0.0;
       if (prof_enabled())
-        for (int i : P.pers_fronts) by += solve_pass_bytes(P.fronts[i], nq, sizeof(T));
+        for (int t = t0; t < t1; t++) by += solve_pass_bytes(P.fronts[P.pers_fronts[t]], nq, sizeof(T));
       prof_begin(KC_SOLVE_FWD, st);
-      k_fwd_pers<T, SOLVE_NRHS><<<pers_solve_grid(np), 256, 0, st>>>(
-          D.pers_list, np, D.pers_parent, D.pers_solve, D.pers_solve + 2 * np, D.fronts, D.children, D.maps, D.rows,
-          L, Bq, ld, W, nq, status);
+      sf_dispatch(nq, [&](auto nqc) {
+        constexpr int Q = decltype(nqc)::value;
+        const int slot = sf_slot<T>(P.pers_slot[part]), wld = P.pers_wld[part], nw = th / 32;
+        const size_t smem = nw * sf_warp_smem<T, Q>(slot, wld);
+        const int grid = std::min((t1 - t0 + nw - 1) / nw, sf_resident(k_fwd_pers<T, Q, SOLVE_NRHS>, th, smem));
+        k_fwd_pers<T, Q, SOLVE_NRHS><<<grid, th, smem, st>>>(D.solve_tasks, t0, t1, D.pers_solve,
+                                                             D.pers_solve + 2 * np + part, D.child_rec, D.maps, D.rows,
+                                                             L, Bq, ld, W, nq, status, slot, wld);
+      });
       prof_end(KC_SOLVE_FWD, st, 0.0, by);
       count_launch();
     }
@@ -1909,21 +1979,13 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       if (prof_enabled())
         for (int i = LP.front_begin; i < LP.front_end; i++) by += solve_pass_bytes(P.fronts[i], nq, sizeof(T));
       prof_begin(KC_SOLVE_FWD, st);
-      const int ns = (int) LP.small_numeric.size();
-      if (ns > 0) {
-        const int* sl = D.small_num + D.small_num_off[h];
-        const int nw = LP.small_numeric_warp;
-        if (nw > 0) {
-          k_fwd<T, SOLVE_NRHS, 32><<<(nw + 7) / 8, 256, 0, st>>>(sl, nw, D.fronts, D.children, D.maps, D.rows, L,
-                                                                 Bq, ld, W, nq);
-          count_launch();
-        }
-        if (ns > nw) {
-          k_fwd<T, SOLVE_NRHS, 256><<<ns - nw, 256, 0, st>>>(sl + nw, ns - nw, D.fronts, D.children, D.maps, D.rows,
-                                                             L, Bq, ld, W, nq);
-          count_launch();
-        }
-      }
+      small_list(h, nq, [&](auto nqc, const int* sl, int ns) {
+        constexpr int Q = decltype(nqc)::value;
+        const int slot = sf_slot<T>(SMALL_F_MAX * (SMALL_F_MAX + 1));
+        k_fwd<T, Q, SOLVE_NRHS><<<(ns + 3) / 4, 128, 4 * sf_warp_smem<T, Q>(slot, SMALL_F_MAX), st>>>(
+            sl, ns, D.fronts, D.child_rec, D.maps, D.rows, L, Bq, ld, W, nq, slot, SMALL_F_MAX);
+        count_launch();
+      });
       const int nb = (int) LP.solve_fwd_blocks.size();
       if (nb > 0) {
         const int2_* bl = D.sfwd + D.sfwd_off[h];
@@ -1999,29 +2061,32 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
           k_bwd_big<T, 8, SOLVE_NRHS, true><<<nb, 128, bwd_smem<T, 8>(), st>>>(bl, D.fronts, D.rows, L, Dinv, Xq, ld, W, part, nq, flags, eb, status);
         count_launch();
       }
-      const int ns = (int) LP.small_numeric.size();
-      if (ns > 0) {
-        const int* sl = D.small_num + D.small_num_off[h];
-        const int nw = LP.small_numeric_warp;
-        if (nw > 0) {
-          k_bwd<T, SOLVE_NRHS, 32><<<(nw + 7) / 8, 256, 0, st>>>(sl, nw, D.fronts, D.rows, L, Xq, ld, W, nq);
-          count_launch();
-        }
-        if (ns > nw) {
-          k_bwd<T, SOLVE_NRHS, 256><<<ns - nw, 256, 0, st>>>(sl + nw, ns - nw, D.fronts, D.rows, L, Xq, ld, W, nq);
-          count_launch();
-        }
-      }
+      small_list(h, nq, [&](auto nqc, const int* sl, int ns) {
+        constexpr int Q = decltype(nqc)::value;
+        const int slot = sf_slot<T>(SMALL_F_MAX * (SMALL_F_MAX + 1));
+        k_bwd<T, Q, SOLVE_NRHS><<<(ns + 3) / 4, 128, 4 * sf_warp_smem<T, Q>(slot, SMALL_F_MAX), st>>>(
+            sl, ns, D.fronts, D.rows, L, Xq, ld, W, nq, slot, SMALL_F_MAX);
+        count_launch();
+      });
       prof_end(KC_SOLVE_BWD, st, 0.0, by);
     }
-    if (np > 0) {
+    for (int part = 1; part >= 0; part--) {
+      int t0, t1, th;
+      sf_part(P, np, part, &t0, &t1, &th);
+      if (t1 <= t0) continue;
       double by = 0.0;
       if (prof_enabled())
-        for (int i : P.pers_fronts) by += solve_pass_bytes(P.fronts[i], nq, sizeof(T));
+        for (int t = t0; t < t1; t++) by += solve_pass_bytes(P.fronts[P.pers_fronts[t]], nq, sizeof(T));
       prof_begin(KC_SOLVE_BWD, st);
-      k_bwd_pers<T, SOLVE_NRHS><<<pers_solve_grid(np), 256, 0, st>>>(
-          D.pers_list, np, D.pers_parent, D.pers_solve + np, D.pers_solve + 2 * np + 1, eb, D.fronts, D.rows, L, Xq, ld,
-          W, nq, status);
+      sf_dispatch(nq, [&](auto nqc) {
+        constexpr int Q = decltype(nqc)::value;
+        const int slot = sf_slot<T>(P.pers_slot[part]), wld = P.pers_wld[part], nw = th / 32;
+        const size_t smem = nw * sf_warp_smem<T, Q>(slot, wld);
+        const int grid = std::min((t1 - t0 + nw - 1) / nw, sf_resident(k_bwd_pers<T, Q, SOLVE_NRHS>, th, smem));
+        k_bwd_pers<T, Q, SOLVE_NRHS><<<grid, th, smem, st>>>(D.solve_tasks, t0, t1, D.pers_solve + np,
+                                                             D.pers_solve + 2 * np + 2 + part, eb, D.rows, L, Xq, ld, W,
+                                                             nq, status, slot, wld);
+      });
       prof_end(KC_SOLVE_BWD, st, 0.0, by);
       count_launch();
     }
@@ -2100,13 +2165,14 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
                                 const double* B,
                                 int ld, double* W, int* flags, int* epoch, int* status, cudaStream_t st) {
   solve_attrs<double>();
+  const int slot = sf_slot<double>(SMALL_F_MAX * (SMALL_F_MAX + 1));
   const int ef = ++*epoch;
   for (int h = 0; h < P.n_levels; h++) {
     const LevelPlan& LP = P.levels[h];
     const int ns = (int) LP.small_fronts.size();
     if (ns > 0) {
-      k_fwd<double, 1, 256><<<ns, 256, 0, st>>>(D.small_list + D.small_off[h], ns, D.fronts, D.children, D.maps, D.rows, L, B, ld,
-                                   W, 1);
+      k_fwd<double, 1, 1><<<(ns + 3) / 4, 128, 4 * sf_warp_smem<double, 1>(slot, SMALL_F_MAX), st>>>(
+          D.small_list + D.small_off[h], ns, D.fronts, D.child_rec, D.maps, D.rows, L, B, ld, W, 1, slot, SMALL_F_MAX);
       count_launch();
     }
     const int nb = (int) LP.solve_fwd_blocks.size();
@@ -2130,7 +2196,8 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
     }
     const int ns = (int) LP.small_fronts.size();
     if (ns > 0) {
-      k_bwd<double, 1, 256><<<ns, 256, 0, st>>>(D.small_list + D.small_off[h], ns, D.fronts, D.rows, L, X, ld, W, 1);
+      k_bwd<double, 1, 1><<<(ns + 3) / 4, 128, 4 * sf_warp_smem<double, 1>(slot, SMALL_F_MAX), st>>>(
+          D.small_list + D.small_off[h], ns, D.fronts, D.rows, L, X, ld, W, 1, slot, SMALL_F_MAX);
       count_launch();
     }
   }

@@ -59,6 +59,37 @@ int devplan_upload(const Plan& P, DevPlan* D, cudaStream_t st) {
     sb.insert(sb.end(), LP.solve_bwd_blocks.begin(), LP.solve_bwd_blocks.end());
     sl.insert(sl.end(), LP.solve_l21_tasks.begin(), LP.solve_l21_tasks.end());
   }
+  // which rows of which children land in a 64-row block of a big front, per
+  // forward block in launch order and child by child (a child's map is
+  // increasing, so its rows in a block are consecutive)
+  std::vector<int2_> sfch(sf.size());
+  std::vector<int4> bch;
+  {
+    std::vector<std::vector<int4>> of;
+    std::vector<std::vector<int2_>> where(P.fronts.size());   // front -> (block, list index)
+    for (size_t k = 0; k < sf.size(); k++) where[sf[k].a].push_back(int2_{sf[k].b, (int) k});
+    for (size_t i = 0; i < P.fronts.size(); i++) {
+      if (where[i].empty()) continue;
+      const FrontDesc& F = P.fronts[i];
+      of.assign((F.f + PANEL_NB - 1) / PANEL_NB, {});
+      for (int ci = F.child_begin; ci < F.child_end; ci++) {
+        const FrontDesc& C = P.fronts[P.children[ci]];
+        const int* mp = P.maps.data() + C.map_off;
+        const int mc = C.f - C.s;
+        for (int a = 0; a < mc;) {
+          const int b = mp[a] / PANEL_NB;
+          const int e = (int) (std::lower_bound(mp + a, mp + mc, (b + 1) * PANEL_NB) - mp);
+          of[b].push_back(make_int4(C.rows_off, C.s + a, C.f << 7 | (e - a), C.map_off + a));
+          a = e;
+        }
+      }
+      for (const int2_& w : where[i]) {
+        sfch[w.b].a = (int) bch.size();
+        bch.insert(bch.end(), of[w.a].begin(), of[w.a].end());
+        sfch[w.b].b = (int) bch.size();
+      }
+    }
+  }
   // each tile's child records follow one another, one per child of its front
   int64_t nrec = 0;
   for (Tile& t : tiles) {
@@ -103,6 +134,8 @@ int devplan_upload(const Plan& P, DevPlan* D, cudaStream_t st) {
          && dev_upload(&D->big_list, big.data(), big.size(), st)
          && dev_upload(&D->tiles, tiles.data(), tiles.size(), st)
          && dev_upload(&D->sfwd, sf.data(), sf.size(), st)
+         && dev_upload(&D->sfwd_ch, sfch.data(), sfch.size(), st)
+         && dev_upload(&D->blk_child, bch.data(), bch.size(), st)
          && dev_upload(&D->sbwd, sb.data(), sb.size(), st)
          && dev_upload(&D->sl21, sl.data(), sl.size(), st)
          && dev_upload(&D->tile_ch, (const TileChild*) nullptr, (size_t) std::max<int64_t>(nrec, 1), st);
@@ -116,7 +149,7 @@ void devplan_free(DevPlan* D) {
   tb::dfree(D->fronts); tb::dfree(D->children); tb::dfree(D->rows); tb::dfree(D->maps);
   tb::dfree(D->acol_ptr); tb::dfree(D->a_rows); tb::dfree(D->a_idx);
   tb::dfree(D->small_list); tb::dfree(D->big_list); tb::dfree(D->tiles); tb::dfree(D->tile_ch);
-  tb::dfree(D->sfwd); tb::dfree(D->sbwd); tb::dfree(D->sl21); tb::dfree(D->dblk);
+  tb::dfree(D->sfwd); tb::dfree(D->sfwd_ch); tb::dfree(D->blk_child); tb::dfree(D->sbwd); tb::dfree(D->sl21); tb::dfree(D->dblk);
   tb::dfree(D->small_num); tb::dfree(D->pers_list); tb::dfree(D->pers_parent); tb::dfree(D->pers_pending0);
   tb::dfree(D->pers_work); tb::dfree(D->pers_solve); tb::dfree(D->solve_tasks); tb::dfree(D->child_rec);
   *D = DevPlan();

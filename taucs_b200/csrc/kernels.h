@@ -73,6 +73,8 @@ struct DevPlan {
   TileChild* tile_ch = nullptr;   // per build tile, one record per child of its front
   Tile* tiles = nullptr;
   int2_* sfwd = nullptr;       // solve blocks, all levels concatenated
+  int2_* sfwd_ch = nullptr;    // per forward block, the range of its child records:
+  int4* blk_child = nullptr;   // the child's work vector offset, first row there, f << 7 | rows, map offset
   int2_* sbwd = nullptr;
   int2_* sl21 = nullptr;
   int2_* dblk = nullptr;       // (front, 64-column block) of every big front's diagonal blocks

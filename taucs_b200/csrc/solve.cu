@@ -500,6 +500,55 @@ __device__ void wait_epoch(const int* flag, int epoch, int* status) {
 }
 
 
+// The children's update rows that land in a 64-row block, added into wv in
+// child order (the order of the block's records, found once per plan: the
+// kernels used to look each child's descriptor and range up, some 3 us a
+// child: forward solve at 29x24x26, FP32, three passes, 1030 -> 805 us; at
+// 64^3, FP64, 1425 -> 1285 us).  NT threads, thread t on row t % 64 of every record; the loads of
+// GC children are issued before the first add, those of the first group by
+// begin(), ahead of whatever else the block loads.
+template <typename T, int NQ, int WS, int NT>
+struct ChildGather {
+  static constexpr int GC = 4, QS = NT / BR, QN = (NQ + QS - 1) / QS;
+  int pi[GC];
+  T val[GC][QN];
+  __device__ __forceinline__ void load(const int4* __restrict__ rec, int n, const int* __restrict__ maps,
+                                       const T* __restrict__ W, int nrhs) {
+    const int i = threadIdx.x % BR, q0 = threadIdx.x / BR;
+#pragma unroll
+    for (int u = 0; u < GC; u++) {
+      const int4 R = u < n ? __ldg(rec + u) : make_int4(0, 0, 0, 0);
+      const bool in = i < (R.z & 127) && q0 < QS;   // threads past NT take no row
+      pi[u] = in ? __ldg(maps + R.w + i) : -1;
+      const T* Wc = W + (int64_t) R.x * WS + R.y + i;
+#pragma unroll
+      for (int t = 0; t < QN; t++) {
+        const int q = q0 + QS * t;
+        val[u][t] = (in && q < nrhs) ? Wc[(size_t) q * (R.z >> 7)] : T(0);
+      }
+    }
+  }
+  // adds the loaded group (already begun) and the later ones into wv rows
+  // pi - r0; every thread of the block calls it, before a barrier of its own
+  template <int LD>
+  __device__ __forceinline__ void add(const int4* __restrict__ rec, int n, const int* __restrict__ maps,
+                                      const T* __restrict__ W, int nrhs, int r0, T (*wv)[LD]) {
+    const int q0 = threadIdx.x / BR;
+    for (int c = 0; c < n; c += GC) {
+      if (c > 0) load(rec + c, n - c, maps, W, nrhs);
+#pragma unroll
+      for (int u = 0; u < GC; u++) {
+        if (c + u >= n) break;
+        if (pi[u] >= 0)
+#pragma unroll
+          for (int t = 0; t < QN; t++)
+            if (q0 + QS * t < NQ) wv[pi[u] - r0][q0 + QS * t] += val[u][t];
+        __syncthreads();
+      }
+    }
+  }
+};
+
 // Forward solve of big fronts.  Diagonal block r of L11 gives
 // y_r = L_rr^-1 (w_r - sum_{k<r} L_rk y_k), chained to block r-1 by
 // release/acquire flags; update rows i get w_i - sum_k L_ik y_k.
@@ -525,15 +574,14 @@ constexpr size_t fwd_smem() {
 
 template <typename T, int NQ, int WS, int MODE>
 __global__ void __launch_bounds__(128)
-k_fwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts,
-          const int* __restrict__ children, const int* __restrict__ maps, const int* __restrict__ rows,
+k_fwd_big(const int2_* __restrict__ blocks, const int2_* __restrict__ blk_ch, const int4* __restrict__ blk_child,
+          const FrontDesc* __restrict__ fronts, const int* __restrict__ maps, const int* __restrict__ rows,
           const T* __restrict__ L, const T* __restrict__ Dinv, const T* __restrict__ B, int ldb,
           T* __restrict__ W, int nrhs, int* __restrict__ flags, int epoch, int* status) {
   __shared__ T wv[BR][NQ];
   __shared__ T yk[BR][NQ];
   __shared__ T part[BR][NQ];
   __shared__ T ykw[4][BR / 2][NQ];   // per warp: the entries of y_k it needs
-  __shared__ int rng[2];
   // CHAIN: dg[col][row] holds L_rr^-1 in rows < bw and the front's own
   // update rows of L (last diagonal block) in rows >= bw; mx[col][row] holds
   // L_{r,r-1}, then M = L_rr^-1 L_{r,r-1} in rows < bw
@@ -553,6 +601,11 @@ k_fwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts
   constexpr bool CHAIN = MODE == FWD_CHAIN;
   const bool diag = CHAIN || (MODE == FWD_ALL && r < nbs);
   const int bw = diag ? min(BR, s - r0) : 0;
+  const int2_ cr = blk_ch[blockIdx.x];
+  const int4* rec = blk_child + cr.a;
+  const int nch = cr.b - cr.a;
+  ChildGather<T, NQ, WS, 128> cg;
+  cg.load(rec, nch, maps, W, nrhs);
 
   if (diag) {
     // staged now, off the chain's critical path
@@ -600,25 +653,7 @@ k_fwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts
     wv[i][q] = (i < nr && q < nrhs && r0 + i < s) ? B[rw[r0 + i] + (size_t) q * ldb] : 0.0;
   }
   __syncthreads();
-  for (int ci = F.child_begin; ci < F.child_end; ci++) {
-    const FrontDesc C = fronts[children[ci]];
-    const int mc = C.f - C.s;
-    const int* mp = maps + C.map_off;
-    if (warp < 2) {
-      const int x = warp_lower_bound(mp, mc, warp == 0 ? r0 : r0 + nr);
-      if (lane == 0) rng[warp] = x;
-    }
-    __syncthreads();
-    const int ia = rng[0], ib = rng[1];
-    __syncthreads();
-    if (ia >= ib) continue;
-    const T* Wc = W + C.v_off * WS;
-    for (int k = tid; k < (ib - ia) * nrhs; k += 128) {
-      const int i = ia + k % (ib - ia), q = k / (ib - ia);
-      wv[mp[i] - r0][q] += Wc[C.s + i + q * C.f];
-    }
-    __syncthreads();
-  }
+  cg.add(rec, nch, maps, W, nrhs, r0, wv);
   // contributions of the solved blocks k < kend; this thread's 32 entries of
   // L[r, k] are loaded before waiting for y_k
   T acc[NQ];
@@ -971,7 +1006,8 @@ __device__ __forceinline__ void walk_far_terms(unsigned tag, int* status, int n,
 template <typename T, int WS>
 __global__ void __maxnreg__(112)
 k_fwd_walk(const int* __restrict__ walk_fronts, int nwalk, const int2_* __restrict__ blocks,
-           const FrontDesc* __restrict__ fronts, const int* __restrict__ children, const int* __restrict__ maps,
+           const int2_* __restrict__ blk_ch, const int4* __restrict__ blk_child,
+           const FrontDesc* __restrict__ fronts, const int* __restrict__ maps,
            const int* __restrict__ rows, const T* __restrict__ L, const T* __restrict__ Dinv,
            const T* __restrict__ B, int ldb, T* __restrict__ W, unsigned long long* __restrict__ ypairs,
            unsigned long long* __restrict__ ppairs, int nrhs, int* __restrict__ flags, const int* counter, int epoch,
@@ -981,7 +1017,6 @@ k_fwd_walk(const int* __restrict__ walk_fronts, int nwalk, const int2_* __restri
   static_assert(NQ % 4 == 0, "four thread groups share the right-hand sides");
   extern __shared__ __align__(16) unsigned char wsm[];
   __shared__ T hpv[BR][NQ + 1];
-  __shared__ int rng[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int row = tid % BR, qg = tid / BR;
   const unsigned tag = walk_tag(counter, epoch);
@@ -1190,24 +1225,11 @@ k_fwd_walk(const int* __restrict__ walk_fronts, int nwalk, const int2_* __restri
     hpv[i][q] = (i < nr && q < nrhs && r0 + i < s) ? B[rw[r0 + i] + (size_t) q * ldb] : T(0);
   }
   __syncthreads();
-  for (int ci = F.child_begin; ci < F.child_end; ci++) {
-    const FrontDesc C = fronts[children[ci]];
-    const int mc = C.f - C.s;
-    const int* mp = maps + C.map_off;
-    if (warp < 2) {
-      const int x = warp_lower_bound(mp, mc, warp == 0 ? r0 : r0 + nr);
-      if (lane == 0) rng[warp] = x;
-    }
-    __syncthreads();
-    const int ia = rng[0], ib = rng[1];
-    __syncthreads();
-    if (ia >= ib) continue;
-    const T* Wc = W + C.v_off * WS;
-    for (int k = tid; k < (ib - ia) * nrhs; k += WALK_THREADS) {
-      const int i = ia + k % (ib - ia), q = k / (ib - ia);
-      hpv[mp[i] - r0][q] += Wc[C.s + i + q * C.f];
-    }
-    __syncthreads();
+  {
+    const int2_ cr = blk_ch[blockIdx.x - nwalk];
+    ChildGather<T, NQ, WS, 256> cg;
+    cg.load(blk_child + cr.a, cr.b - cr.a, maps, W, nrhs);
+    cg.add(blk_child + cr.a, cr.b - cr.a, maps, W, nrhs, r0, hpv);
   }
   // far terms k < r - WALK_D: thread (row, quarter qg) sums 16 columns of
   // each L_rk for every right-hand side
@@ -1988,7 +2010,7 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       });
       const int nb = (int) LP.solve_fwd_blocks.size();
       if (nb > 0) {
-        const int2_* bl = D.sfwd + D.sfwd_off[h];
+        const int2_ *bl = D.sfwd + D.sfwd_off[h], *bc = D.sfwd_ch + D.sfwd_off[h];
         const int nd = LP.n_fwd_diag, nu = nb - nd;
         // one right-hand side runs the two-column variant, measured faster
         // than a one-column instantiation (columns >= nrhs are skipped)
@@ -1998,22 +2020,22 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
             const int nbig = (int) LP.big_fronts.size();
             if constexpr (std::is_same<T, float>::value)
               k_fwd_walk<T, SOLVE_NRHS><<<nbig + nd, WALK_THREADS, walk_smem<T>(), st>>>(
-                  D.big_list + D.big_off[h], nbig, bl, D.fronts, D.children, D.maps, D.rows, L, Dinv, Bq, ld, W, ypairs,
+                  D.big_list + D.big_off[h], nbig, bl, bc, D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, Bq, ld, W, ypairs,
                   ppairs, nq, flags, counter, ef, status);
             if (nu)
-              k_fwd_big<T, Q, SOLVE_NRHS, FWD_UPD><<<nu, 128, 0, st>>>(bl + nd, D.fronts, D.children, D.maps, D.rows,
+              k_fwd_big<T, Q, SOLVE_NRHS, FWD_UPD><<<nu, 128, 0, st>>>(bl + nd, bc + nd, D.blk_child, D.fronts, D.maps, D.rows,
                                                                       L, Dinv, Bq, ld, W, nq, flags, ef, status);
             count_launch(nu ? 2 : 1);
           } else if (LP.max_s_big >= FWD_CHAIN_MIN_S) {
             k_fwd_big<T, Q, SOLVE_NRHS, FWD_CHAIN><<<nd, 128, fwd_smem<T, FWD_CHAIN>(), st>>>(
-                bl, D.fronts, D.children, D.maps, D.rows, L, Dinv, Bq, ld, W, nq, flags, ef, status);
+                bl, bc, D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, Bq, ld, W, nq, flags, ef, status);
             if (nu)
-              k_fwd_big<T, Q, SOLVE_NRHS, FWD_UPD><<<nu, 128, 0, st>>>(bl + nd, D.fronts, D.children, D.maps, D.rows,
+              k_fwd_big<T, Q, SOLVE_NRHS, FWD_UPD><<<nu, 128, 0, st>>>(bl + nd, bc + nd, D.blk_child, D.fronts, D.maps, D.rows,
                                                                       L, Dinv, Bq, ld, W, nq, flags, ef, status);
             count_launch(nu ? 2 : 1);
           } else {
             k_fwd_big<T, Q, SOLVE_NRHS, FWD_ALL><<<nb, 128, fwd_smem<T, FWD_ALL>(), st>>>(
-                bl, D.fronts, D.children, D.maps, D.rows, L, Dinv, Bq, ld, W, nq, flags, ef, status);
+                bl, bc, D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, Bq, ld, W, nq, flags, ef, status);
             count_launch();
           }
         };
@@ -2178,7 +2200,8 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
     const int nb = (int) LP.solve_fwd_blocks.size();
     if (nb > 0) {
       k_fwd_big<double, 1, 1, FWD_ALL><<<nb, 128, fwd_smem<double, FWD_ALL>(), st>>>(
-          D.sfwd + D.sfwd_off[h], D.fronts, D.children, D.maps, D.rows, L, Dinv, B, ld, W, 1, flags, ef, status);
+          D.sfwd + D.sfwd_off[h], D.sfwd_ch + D.sfwd_off[h], D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, B, ld, W, 1,
+          flags, ef, status);
       count_launch();
     }
   }

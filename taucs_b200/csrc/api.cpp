@@ -294,6 +294,10 @@ int ensure_device(Factor* F) {
          && cuda_ok(cudaMemsetAsync(F->dflags, 0, sizeof(int) * (solve_flag_words(P) + 1), st), "flags")
          && dev_upload(&F->dW, (const double*) nullptr, (size_t) P.v_len * SOLVE_NRHS, st)
          && dev_upload(&F->dpart, (const double*) nullptr, (size_t) P.part_len, st)
+         // the chains' published values start without a tag: the memory may
+         // hold another factor's
+         && cuda_ok(cudaMemsetAsync(F->dpart + P.fpart_off, 0, sizeof(double) * (size_t) (P.part_len - P.fpart_off), st),
+                    "published values")
          && dev_upload(&F->dX, (const double*) nullptr, (size_t) F->n * SOLVE_NRHS, st)
          && dev_upload(&F->dcolptr, F->colptr.data(), F->colptr.size(), st)
          && dev_upload(&F->drowind, F->rowind.data(), F->rowind.size(), st)

@@ -130,7 +130,8 @@ struct LevelPlan {
   std::vector<int2_> solve_fwd_blocks;   // (front, row block): the n_fwd_diag diagonal blocks first
   int n_fwd_diag = 0;
   std::vector<int2_> solve_bwd_blocks;   // (front, column block), last block first
-  std::vector<int2_> solve_l21_tasks;    // (front, column block << 16 | row chunk)
+  std::vector<int2_> solve_l21_tasks;    // (front, column block << 16 | row chunk): first those of fronts
+  int n_l21_multi = 0;                   // with more than one chunk (n_l21_multi tasks)
   // small fronts, fused kernel (sorted by order f)
   std::vector<int> small_fronts;
   // the small fronts that the level launches of the numeric factorization

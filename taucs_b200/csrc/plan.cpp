@@ -412,6 +412,7 @@ int build_plan(const Symbolic& S, int n, const int* colptr, const int* rowind, P
       while (fi < nf && P.fronts[fi].level == h) fi++;
       LP.front_end = fi;
       std::vector<int2_> fwd_upd;   // forward blocks of update rows, after the diagonal ones
+      std::vector<int2_> l21_one;   // L21 tasks of fronts with one chunk, after the others
       for (int i = LP.front_begin; i < LP.front_end; i++) {
         const FrontDesc& F = P.fronts[i];
         if (F.f <= SMALL_F_MAX) {
@@ -434,9 +435,11 @@ int build_plan(const Symbolic& S, int n, const int* colptr, const int* rowind, P
           for (int k = nbs - 1; k >= 0; k--) LP.solve_bwd_blocks.push_back(int2_{i, k});
           const int nch = (m + SOLVE_RCH - 1) / SOLVE_RCH;
           for (int k = 0; k < nbs; k++)
-            for (int c = 0; c < nch; c++) LP.solve_l21_tasks.push_back(int2_{i, (k << 16) | c});
+            for (int c = 0; c < nch; c++) (nch > 1 ? LP.solve_l21_tasks : l21_one).push_back(int2_{i, (k << 16) | c});
         }
       }
+      LP.n_l21_multi = (int) LP.solve_l21_tasks.size();
+      LP.solve_l21_tasks.insert(LP.solve_l21_tasks.end(), l21_one.begin(), l21_one.end());
       LP.n_fwd_diag = (int) LP.solve_fwd_blocks.size();
       LP.solve_fwd_blocks.insert(LP.solve_fwd_blocks.end(), fwd_upd.begin(), fwd_upd.end());
       // the fused small-front kernel is launched per size class

@@ -434,6 +434,7 @@ int numeric_fp32_device(Factor* F, const double* d_vals) {
   if (ensure_device(F) || ensure_refine(F)) return -1;
   const Plan& P = F->plan;
   cudaStream_t st = current_stream();
+  const bool fresh = !F->dpart32;
   auto al = [&](float** d, size_t n, const char* w) { return *d || cuda_ok(tb::dmalloc(d, sizeof(float) * std::max<size_t>(n, 1)), w); };
   if (!al(&F->dL32, P.l_len, "cudaMalloc(L32)") || !al(&F->dU32, P.u_len, "cudaMalloc(U32)") ||
       !al(&F->dSp32, P.sp_len, "cudaMalloc(split arena)") ||
@@ -442,6 +443,11 @@ int numeric_fp32_device(Factor* F, const double* d_vals) {
     free_numeric(F);
     return -1;
   }
+  // the chains' published values start without a tag: the memory may hold
+  // another factor's
+  if (fresh && !cuda_ok(cudaMemsetAsync(F->dpart32 + P.fpart_off, 0, sizeof(float) * (size_t) (P.part_len - P.fpart_off), st),
+                        "published values"))
+    return -1;
   F->dvals_cur = d_vals;
   k_init_status2<<<1, 1, 0, st>>>(F->dstatus);
   k_diag_scale<<<nblk(F->n, 256), 256, 0, st>>>(F->n, F->ddiagpos, d_vals, F->dscale, F->dstatus);

@@ -448,10 +448,12 @@ k_bwd_pers(const SolveTask* __restrict__ tasks, int t0, int t1, int* done, int* 
 // can hang.
 
 constexpr int BR = PANEL_NB;   // rows per block
-// dynamic shared memory: L_kk^-1, plus one staged 64x64 block of L11 for 8
-// columns
+// dynamic shared memory: L_kk^-1, then the gathered chunk of x2, or (8
+// columns) one staged 64x64 block of L11
 template <typename T, int NQ>
-constexpr size_t bwd_smem() { return (NQ >= 8 ? 2 : 1) * BR * (BR + 1) * sizeof(T); }
+constexpr size_t bwd_smem() {
+  return (BR * (BR + 1) + (NQ >= 8 ? BR * (BR + 1) : NQ * SOLVE_RCH)) * sizeof(T);
+}
 
 __device__ __forceinline__ void st_release(int* p, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
@@ -504,9 +506,9 @@ __device__ void wait_epoch(const int* flag, int epoch, int* status) {
 // child order (the order of the block's records, found once per plan: the
 // kernels used to look each child's descriptor and range up, some 3 us a
 // child: forward solve at 29x24x26, FP32, three passes, 1030 -> 805 us; at
-// 64^3, FP64, 1425 -> 1285 us).  NT threads, thread t on row t % 64 of every record; the loads of
-// GC children are issued before the first add, those of the first group by
-// begin(), ahead of whatever else the block loads.
+// 64^3, FP64, 1425 -> 1285 us).  NT threads, thread t on row t % 64 of every
+// record; the loads of GC children are issued before the first add, those of
+// the first group by load(), ahead of whatever else the block loads.
 template <typename T, int NQ, int WS, int NT>
 struct ChildGather {
   static constexpr int GC = 4, QS = NT / BR, QN = (NQ + QS - 1) / QS;
@@ -549,30 +551,16 @@ struct ChildGather {
   }
 };
 
-// Forward solve of big fronts.  Diagonal block r of L11 gives
-// y_r = L_rr^-1 (w_r - sum_{k<r} L_rk y_k), chained to block r-1 by
-// release/acquire flags; update rows i get w_i - sum_k L_ik y_k.
-//   FWD_ALL   one launch over all blocks of a level: every block waits for
-//             the blocks k it needs, one at a time (short chains);
-//   FWD_CHAIN the diagonal blocks of a level with long chains: everything
-//             but the last term is done before waiting -- M = L_rr^-1
-//             L_{r,r-1} at kernel start, the sum over k < r-1 and
-//             c = L_rr^-1 (w_r - ...) -- so after the flag of block r-1
-//             only y_r = c - M y_{r-1} remains (one 64x64 product);
-//   FWD_UPD   after FWD_CHAIN, the update-row blocks, with every y_k
-//             already published.
-// In the last diagonal block rows >= s are update rows of the same front.
-constexpr int FWD_ALL = 0, FWD_CHAIN = 1, FWD_UPD = 2;
-// levels whose largest big front has at least this many columns use
-// FWD_CHAIN + FWD_UPD (the split pays off on long chains only)
-constexpr int FWD_CHAIN_MIN_S = 2048;
+// Forward solve of big fronts, one launch over all blocks of a level (the
+// levels that do not run as chains below).  Diagonal block r of L11 gives
+// y_r = L_rr^-1 (w_r - sum_{k<r} L_rk y_k), handed on by release/acquire
+// flags; update rows i get w_i - sum_k L_ik y_k; a block waits for the blocks
+// k it needs one at a time.  In the last diagonal block rows >= s are update
+// rows of the same front.
+template <typename T>
+constexpr size_t fwd_smem() { return BR * (BR + 1) * sizeof(T); }
 
-template <typename T, int MODE>
-constexpr size_t fwd_smem() {
-  return MODE == FWD_CHAIN ? 2 * BR * (BR + 1) * sizeof(T) : MODE == FWD_ALL ? BR * (BR + 1) * sizeof(T) : 0;
-}
-
-template <typename T, int NQ, int WS, int MODE>
+template <typename T, int NQ, int WS>
 __global__ void __launch_bounds__(128)
 k_fwd_big(const int2_* __restrict__ blocks, const int2_* __restrict__ blk_ch, const int4* __restrict__ blk_child,
           const FrontDesc* __restrict__ fronts, const int* __restrict__ maps, const int* __restrict__ rows,
@@ -582,12 +570,10 @@ k_fwd_big(const int2_* __restrict__ blocks, const int2_* __restrict__ blk_ch, co
   __shared__ T yk[BR][NQ];
   __shared__ T part[BR][NQ];
   __shared__ T ykw[4][BR / 2][NQ];   // per warp: the entries of y_k it needs
-  // CHAIN: dg[col][row] holds L_rr^-1 in rows < bw and the front's own
-  // update rows of L (last diagonal block) in rows >= bw; mx[col][row] holds
-  // L_{r,r-1}, then M = L_rr^-1 L_{r,r-1} in rows < bw
+  // dg[col][row] holds L_rr^-1 in rows < bw and the front's own update rows
+  // of L (last diagonal block) in rows >= bw
   extern __shared__ __align__(16) unsigned char fsm[];
   T (*dg)[BR + 1] = reinterpret_cast<T (*)[BR + 1]>(fsm);
-  T (*mx)[BR + 1] = reinterpret_cast<T (*)[BR + 1]>(fsm) + BR;
   const int2_ bk = blocks[blockIdx.x];
   const FrontDesc F = fronts[bk.a];
   const int r = bk.b, f = F.f, s = F.s;
@@ -598,8 +584,7 @@ k_fwd_big(const int2_* __restrict__ blocks, const int2_* __restrict__ blk_ch, co
   T* Wf = W + F.v_off * WS;
   const int* rw = rows + F.rows_off;
   const T* P = L + F.l_off;
-  constexpr bool CHAIN = MODE == FWD_CHAIN;
-  const bool diag = CHAIN || (MODE == FWD_ALL && r < nbs);
+  const bool diag = r < nbs;
   const int bw = diag ? min(BR, s - r0) : 0;
   const int2_ cr = blk_ch[blockIdx.x];
   const int4* rec = blk_child + cr.a;
@@ -613,40 +598,20 @@ k_fwd_big(const int2_* __restrict__ blocks, const int2_* __restrict__ blk_ch, co
     // 16 entries of each tile per thread in flight before they are stored
 #pragma unroll 1
     for (int t0 = 0; t0 < BR * BR / 128; t0 += 16) {
-      T dv[16], mv[16];
+      T dv[16];
 #pragma unroll
       for (int t = 0; t < 16; t++) {
         const int e = tid + 128 * (t0 + t), i = e % BR, j = e / BR;
         T v = 0.0;
         if (j < bw && i < nr) v = (i < bw) ? (i >= j ? Di[i + j * BR] : T(0)) : P[(r0 + i) + (size_t) (r0 + j) * f];
         dv[t] = v;
-        mv[t] = (CHAIN && r > 0 && i < nr) ? P[(r0 + i) + (size_t) (r0 - BR + j) * f] : T(0);
       }
 #pragma unroll
       for (int t = 0; t < 16; t++) {
         const int e = tid + 128 * (t0 + t), i = e % BR, j = e / BR;
         dg[j][i] = dv[t];
-        if (CHAIN && r > 0) mx[j][i] = mv[t];
       }
     }
-  }
-  if (CHAIN && r > 0) {
-    // M = L_rr^-1 L_{r,r-1} in rows < bw (the inverse is lower triangular),
-    // at kernel start, independent of the chain
-    __syncthreads();
-    T m[BR / 2];
-#pragma unroll
-    for (int jj = 0; jj < BR / 2; jj++) m[jj] = 0.0;
-    if (row < bw)
-      for (int t = 0; t <= row; t++) {
-        const T d = dg[t][row];
-#pragma unroll
-        for (int jj = 0; jj < BR / 2; jj++) m[jj] += d * mx[half * (BR / 2) + jj][t];
-      }
-    __syncthreads();
-    if (row < bw)
-#pragma unroll
-      for (int jj = 0; jj < BR / 2; jj++) mx[half * (BR / 2) + jj][row] = m[jj];
   }
   for (int k = tid; k < BR * NQ; k += 128) {
     const int i = k % BR, q = k / BR;
@@ -659,7 +624,7 @@ k_fwd_big(const int2_* __restrict__ blocks, const int2_* __restrict__ blk_ch, co
   T acc[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; q++) acc[q] = 0.0;
-  const int kend = CHAIN ? max(r - 1, 0) : diag ? r : nbs;
+  const int kend = diag ? r : nbs;
   if constexpr (NQ >= 8) {
     // 8 columns: y_k staged once for the whole block (measured faster than
     // the warp-level loop below at 8 columns)
@@ -742,32 +707,6 @@ k_fwd_big(const int2_* __restrict__ blocks, const int2_* __restrict__ blk_ch, co
       for (int q = 0; q < NQ; q++) yk[row][q] = (row < bw) ? y[q] + part[row][q] : wv[row][q];
     __syncthreads();
   }
-  // the critical step: y_r = c - M y_{r-1} (update rows: w - L_{i,r-1} y_{r-1})
-  if (CHAIN && r > 0) {
-    wait_epoch(flags + F.blk_off + r - 1, epoch, status);
-    for (int e = tid; e < BR * NQ; e += 128) {
-      const int j = e % BR, q = e / BR;
-      wv[j][q] = (q < nrhs) ? __ldcg(Wf + (r - 1) * BR + j + (size_t) q * f) : T(0);
-    }
-    __syncthreads();
-    T u[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) u[q] = 0.0;
-#pragma unroll 8
-    for (int j = half * (BR / 2); j < half * (BR / 2) + BR / 2; j++) {
-      const T mv = mx[j][row];
-#pragma unroll
-      for (int q = 0; q < NQ; q++) u[q] += mv * wv[j][q];
-    }
-    if (half == 1)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) part[row][q] = u[q];
-    __syncthreads();
-    if (half == 0)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) yk[row][q] -= u[q] + part[row][q];
-    __syncthreads();
-  }
   if (bw < nr) {
     // update rows inside the last diagonal block: w_i -= L[i, r] y_r
     T u[NQ];
@@ -797,541 +736,623 @@ k_fwd_big(const int2_* __restrict__ blocks, const int2_* __restrict__ blk_ch, co
   if (tid == 0) st_release(flags + F.blk_off + r, epoch);
 }
 
-// Forward solve of the diagonal blocks of levels with long chains, as a
-// walk.  One walker CTA per big front runs the chain y_r = L_rr^-1 (w_r -
-// sum_{k<r} L_rk y_k) itself, block after block, keeping the last WALK_D
-// y's in shared memory: consecutive steps are linked by barriers inside one
-// CTA, not by flags between CTAs.  Helper CTAs, one per diagonal block,
-// gather w_r and subtract the far terms k < r - WALK_D as the walker
-// publishes y_k, then publish the partial p_r -- WALK_D steps ahead of the
-// walker -- and pull the walker's tiles of their block into L2; the walker
-// at step r subtracts the WALK_D near terms and applies the block's inverse.
-// Every value crossing between CTAs travels as a tagged pair (tag in the
-// high word, value in the low word, one 8-byte relaxed store): a reader
-// knows a value is current when its tag is, so neither side fences or
-// polls a flag.  The tag is (call counter << 12) | epoch, the counter being
-// advanced on the device at the start of every solve call (recorded launch
-// sequences stay valid), so a slot never holds a current-looking stale pair.
-// Inside the walker eight compute warps run the arithmetic while a ninth
-// warp loads the partials two steps ahead, handing them over through named
-// barriers (one per direction and step parity).  The tiles of step r + 1
-// (L_{r+1,k} for the near k and the next inverse) are loaded into registers
-// while step r runs.  Walkers have the lowest CTA indices and a helper waits
-// only for the walker of its front, which waits only for helpers of lower
-// index, so in-order dispatch keeps every wait finite; the waits are bounded
-// all the same.  In the last diagonal block rows >= s are update rows of the
-// same front; the walker finishes them too.  The update-row blocks follow in
-// FWD_UPD (the walker also sets the blocks' flags for it).  Right-hand sides
-// are processed eight at a time (the layout of the pairs).
-constexpr int WALK_D = 2, WALK_T = WALK_D + 1;
-constexpr int WALK_PER = WALK_T * BR * BR / 256;   // staged tile entries per compute thread
-constexpr int WALK_THREADS = 288;                   // eight compute warps and a loader warp
-constexpr int WALK_PAIRS = BR * SOLVE_NRHS;         // tagged pairs per block: [row][right-hand side]
-// levels with more big fronts keep the flag-chained kernels: every walker
-// must be resident with room to spare for helpers (two CTAs per SM)
-constexpr int WALK_MAX_FRONTS = 64;
-constexpr int BWD_WALK_MIN_S = 512;
-// named barriers of the walker (0 is __syncthreads): the compute warps
-// among themselves; partial of a step ready (+ step parity); partial buffer
-// of a step released (+ step parity)
-constexpr int WB_COMPUTE = 1, WB_READY = 2, WB_FREE = 4;
+// Forward and backward solve of a level's big fronts as chains, for levels
+// with few fronts and several 64-row blocks each.  What bounds such a level
+// is the chain of its blocks -- z_t = D_t (p_t - sum_{u<t} A_tu z_u), D_t the
+// inverse of a diagonal block (forward: blocks first to last; backward: last
+// to first, transposed) -- so the chain runs inside one cluster of CH_C CTAs:
+// CTA t mod CH_C computes block t and writes z_t into the shared memory of
+// all of them (st.async, counted by the receivers' mbarriers), one to two
+// orders faster than a hand-over through global memory.  Between its turns a
+// CTA adds the terms of the last CH_C blocks to its next one as they arrive,
+// with the tiles of L loaded into registers two terms ahead and into L2 a
+// turn ahead: per step the chain waits for one 64x64 product, one product
+// with the inverse and one hand-over.  The far terms (u < t - CH_C) and the
+// right-hand side of block t are the work of a helper CTA per block, which
+// follows the published z_u and publishes p_t about CH_C steps ahead;
+// forward, the update rows' blocks are helpers too and stream L21 while the
+// chain runs.  Values published between CTAs travel as tagged words (tag in
+// the high half, 32 bits of the value in the low half; a double takes two),
+// each one relaxed 8-byte access: a reader knows a value is current when its
+// tag is, so nothing fences or polls a flag.  The tag is (call counter <<
+// 12) | epoch, the counter being advanced on the device at the start of every
+// solve call, so recorded launch sequences stay valid.  A ring of 2 CH_C z's
+// needs no release: block t's CTA has consumed z_{t-CH_C} .. z_{t-1}, so when
+// z_{u+2 CH_C} is produced every CTA is past its last use of z_u.  Walkers have
+// the lowest CTA indices and helper t waits only for blocks whose helpers
+// come before it, so in-order dispatch keeps every wait finite; the waits are
+// bounded all the same, and no CTA of a cluster leaves before every z has
+// arrived in its shared memory.  In the last diagonal block rows >= s are
+// update rows of the same front; its CTA finishes them too (forward).
+// Measured, per 64-row step of the root level's forward chain: FP64, one right-
+// hand side (64^3) 2.3 us with flags between CTAs, 1.2 us here; FP64, eight
+// (45x47x44) 4.7 -> 1.7 us; FP32, eight (56^3) 4.2 us with one walker CTA per
+// front, 2.0 us here.
+constexpr int CH_C = 8;                       // CTAs of a cluster, and the near distance
+constexpr int CH_RING = 2 * CH_C;
+constexpr int CH_THREADS = 256;
+constexpr int CH_VALUES = BR * SOLVE_NRHS;    // values per block and array of published words
+constexpr int CH_HB = 2;                      // blocks per round of a helper's far terms
+// levels with at least CHAIN_MIN_S columns in their largest big front and at
+// most CHAIN_MAX_FRONTS big fronts run as chains
+constexpr int CHAIN_MIN_S = 256;
+template <typename T>
+constexpr int chain_max_fronts() { return sizeof(T) == 4 ? 16 : 8; }
 
-// barrier ids are immediates, so that the kernel reserves only the ids it uses
-template <int ID, int N>
-__device__ __forceinline__ void nbar_sync() {
-  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
-}
-template <int ID, int N>
-__device__ __forceinline__ void nbar_arrive() {
-  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
-}
-__device__ __forceinline__ void walk_ready_arrive(int par) {
-  if (par) nbar_arrive<WB_READY + 1, WALK_THREADS>();
-  else nbar_arrive<WB_READY, WALK_THREADS>();
-}
-__device__ __forceinline__ void walk_ready_sync(int par) {
-  if (par) nbar_sync<WB_READY + 1, WALK_THREADS>();
-  else nbar_sync<WB_READY, WALK_THREADS>();
-}
-__device__ __forceinline__ void walk_free_arrive(int par) {
-  if (par) nbar_arrive<WB_FREE + 1, WALK_THREADS>();
-  else nbar_arrive<WB_FREE, WALK_THREADS>();
-}
-__device__ __forceinline__ void walk_free_sync(int par) {
-  if (par) nbar_sync<WB_FREE + 1, WALK_THREADS>();
-  else nbar_sync<WB_FREE, WALK_THREADS>();
-}
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
+template <typename T>
+__host__ __device__ constexpr int ch_words() { return (int) sizeof(T) / 4; }   // words per published value
 
-// tagged pairs: one relaxed 8-byte access each (single-copy atomic)
-__device__ __forceinline__ void put_pair(unsigned long long* p, unsigned tag, float v) {
-  const unsigned long long x = ((unsigned long long) tag << 32) | __float_as_uint(v);
-  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
-}
-__device__ __forceinline__ unsigned long long get_pair(const unsigned long long* p) {
+// one published value
+template <typename T>
+struct Tagged;
+template <>
+struct Tagged<float> {
   unsigned long long x;
-  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(x) : "l"(p) : "memory");
-  return x;
-}
-__device__ __forceinline__ bool pair_ok(unsigned long long x, unsigned tag) { return (unsigned) (x >> 32) == tag; }
-__device__ __forceinline__ float pair_value(unsigned long long x) { return __uint_as_float((unsigned) x); }
+  __device__ __forceinline__ void load(const unsigned long long* p) {
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(x) : "l"(p) : "memory");
+  }
+  __device__ __forceinline__ bool ok(unsigned tag) const { return (unsigned) (x >> 32) == tag; }
+  __device__ __forceinline__ float value() const { return __uint_as_float((unsigned) x); }
+  __device__ __forceinline__ static void put(unsigned long long* p, unsigned tag, float v) {
+    const unsigned long long w = ((unsigned long long) tag << 32) | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+  }
+};
+template <>
+struct Tagged<double> {
+  unsigned long long x, y;   // high and low half of the value
+  __device__ __forceinline__ void load(const unsigned long long* p) {
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(p) : "memory");
+  }
+  __device__ __forceinline__ bool ok(unsigned tag) const {
+    return (unsigned) (x >> 32) == tag && (unsigned) (y >> 32) == tag;
+  }
+  __device__ __forceinline__ double value() const { return __hiloint2double((int) (unsigned) x, (int) (unsigned) y); }
+  __device__ __forceinline__ static void put(unsigned long long* p, unsigned tag, double v) {
+    const unsigned long long t = (unsigned long long) tag << 32;
+    const unsigned long long a = t | (unsigned) __double2hiint(v), b = t | (unsigned) __double2loint(v);
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+  }
+};
 
-// a row of eight FP32 values in shared memory (32-byte aligned), read as
-// two 128-bit vectors
-__device__ __forceinline__ void ld_row8(const float* p, float (&v)[8]) {
-  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-__device__ __forceinline__ void st_row8(float* p, const float (&v)[8]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
-}
-
-// the tag of a walk: the solve call's counter and the epoch
-__device__ __forceinline__ unsigned walk_tag(const int* counter, int epoch) {
-  return ((unsigned) *counter << 12) | (unsigned) epoch;
-}
-
-// waits (bounded) until pair x at p carries tag, reloading it; called by
-// whole warps, each lane with its own pair, and left together
-__device__ __forceinline__ unsigned long long wait_pair(const unsigned long long* p, unsigned long long x, unsigned tag,
-                                                        int* status) {
+// waits (bounded) until the lanes' values all carry the tag, reloading them;
+// called by whole warps and left together; lanes with need = false take part
+// without a value
+template <typename T>
+__device__ __forceinline__ void wait_tagged(const unsigned long long* p, Tagged<T>& v, bool need, unsigned tag,
+                                            int* status) {
   const int limit = g_solve_wait_limit;
   const unsigned want = tag + (unsigned) (g_solve_wait_skew << 12);
   int it = 0;
-  while (!__all_sync(0xffffffffu, pair_ok(x, want))) {
+  while (!__all_sync(0xffffffffu, !need || v.ok(want))) {
     ++it;
     if (__any_sync(0xffffffffu, it > limit || ((it & 1023) == 0 && *(volatile int*) status == SOLVE_TIMEOUT))) {
       atomicExch(status, SOLVE_TIMEOUT);
       break;
     }
-    __nanosleep(32);
-    x = get_pair(p);
+    if (it > 4) __nanosleep(20);
+    if (need) v.load(p);
   }
-  return x;
 }
 
-// dynamic shared memory of the walk: the walker's tiles of one step, its
-// ring of y's, two partial buffers, the quarters' products and the reduced
-// partial; the helpers use the first part for their partial sums and staged
-// y's
-template <typename T>
-constexpr size_t walk_smem() {
-  return (WALK_T * BR * BR + (WALK_T + 2 + 4 + 1) * BR * SOLVE_NRHS) * sizeof(T);
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned) __cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned map_rank(unsigned addr, unsigned rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
 }
-// the backward walker's tiles are [row][column], padded against bank
-// conflicts of the coalesced staging stores
-template <typename T>
-constexpr size_t bwalk_smem() {
-  return (WALK_T * BR * (BR + 1) + (WALK_T + 2 + 4 + 1) * BR * SOLVE_NRHS) * sizeof(T);
+// QL values of a lane into another CTA's shared memory, counted there
+__device__ __forceinline__ void st_async(unsigned addr, unsigned bar, const float (&v)[1]) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
+               "r"(__float_as_uint(v[0])), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async(unsigned addr, unsigned bar, const float (&v)[2]) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr),
+               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async(unsigned addr, unsigned bar, const double (&v)[1]) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+               "l"(__double_as_longlong(v[0])), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async(unsigned addr, unsigned bar, const double (&v)[2]) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(addr),
+               "l"(__double_as_longlong(v[0])), "l"(__double_as_longlong(v[1])), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// bounded wait of a whole warp for a phase of a z's barrier
+__device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, int* status) {
+  const int limit = g_solve_wait_limit;
+  int it = 0;
+  while (!__all_sync(0xffffffffu, bar_try(bar, parity))) {
+    ++it;
+    if (__any_sync(0xffffffffu, it > limit || ((it & 255) == 0 && *(volatile int*) status == SOLVE_TIMEOUT))) {
+      atomicExch(status, SOLVE_TIMEOUT);
+      break;
+    }
+  }
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// (a, b) += l (x, y): two FP32 multiply-adds in one packed instruction
+__device__ __forceinline__ void fma2(float& a, float& b, float l, float x, float y) {
+  asm("{\n\t.reg .b64 p, q, r;\n\t"
+      "mov.b64 p, {%2, %2};\n\tmov.b64 q, {%3, %4};\n\tmov.b64 r, {%0, %1};\n\t"
+      "fma.rn.f32x2 r, p, q, r;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "+f"(a), "+f"(b)
+      : "f"(l), "f"(x), "f"(y));
+}
+__device__ __forceinline__ void fma2(double& a, double& b, double l, double x, double y) {
+  a += l * x;
+  b += l * y;
 }
 
-// The far terms of a walk's helper: blocks t = 0 .. n-1 of the chain in the
-// order the walker publishes them, each adding acc[q] += sum_jj
-// load_l(t, jj) ys[qg * 16 + jj][q] with ys[i][q] the value of pair
-// [i][q] of block pairs(t).  Every round loads up to WALK_HB blocks, all
-// loads in flight at once, and uses the leading blocks whose pairs all carry
-// the tag; a round that finds none waits (bounded) for the first.  Threads
-// past the first 256 (act false) only keep the barriers.
-constexpr int WALK_HB = 4;
-template <int NQ, typename LoadL, typename Pairs>
-__device__ __forceinline__ void walk_far_terms(unsigned tag, int* status, int n, LoadL load_l, Pairs pairs,
-                                               float (*ysb)[BR][NQ], float (&acc)[NQ], int qg, bool act) {
+// A 64-row product by the CTA's eight warps, warp w the rows 8 w .. 8 w + 7.
+// Its cost is the bytes of z that the lanes take from shared memory (128 a
+// clock), so with several right-hand sides a lane covers R = 2 rows: lane
+// (i, j), j < J = 4 R, holds rows 8 w + i + (8 / R) h, h < R, and columns J t +
+// j -- a warp's loads cover whole sectors, its reads of z ([column][right-hand
+// side]) are neighbouring rows -- and the row's lanes are summed by shuffles.
+// FP64 with eight columns runs on DMMA m8n8k4 instead: its A fragment is the
+// R = 1 layout, its B fragment one value of z a lane, and its C fragment
+// leaves each lane with two columns of its row, with nothing to sum.
+// Afterwards a lane owns QL right-hand sides qb .. of row `own` (qact: of
+// several lanes with the same values only one).
+template <typename T, int NQ>
+struct ChainRow {
+  static constexpr bool DMMA = sizeof(T) == 8 && NQ == 8;
+  static constexpr int R = NQ == 1 || DMMA ? 1 : 2, J = 4 * R, NT = 16 / R;
+  static constexpr int NACC = DMMA ? 2 : R * NQ, QL = NQ >= 4 ? NQ / 4 : 1;
+  static_assert(NQ == 1 || NQ == 4 || NQ == 8, "the solve's instantiations");
+  T acc[NACC];
+  __device__ __forceinline__ static int lane() { return threadIdx.x & 31; }
+  __device__ __forceinline__ static int jq() { return lane() % J; }
+  __device__ __forceinline__ static int row(int h) { return (threadIdx.x >> 5) * 8 + lane() / J + (8 / R) * h; }
+  __device__ __forceinline__ static int own() { return row(R == 2 ? jq() >> 2 : 0); }
+  __device__ __forceinline__ static int qb() { return NQ >= 4 ? QL * (jq() & 3) : 0; }
+  __device__ __forceinline__ static bool qact() { return NQ >= 4 || jq() == 0; }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int a = 0; a < NACC; a++) acc[a] = T(0);
+  }
+  // acc += l z, l[h * NT + t] the entry of row(h), column J t + j
+  __device__ __forceinline__ void add(const T (&l)[16], const T* z) {
+    const int j = jq();
+    if constexpr (DMMA) {
+#pragma unroll
+      for (int t = 0; t < 16; t++) {
+        const double b = z[(4 * t + j) * NQ + (lane() >> 2)];
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                     : "+d"(acc[0]), "+d"(acc[1])
+                     : "d"(l[t]), "d"(b));
+      }
+    } else {
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        const T* zr = z + (J * t + j) * NQ;
+        T x[NQ];
+        if constexpr (NQ * sizeof(T) >= 16) {
+          constexpr int V = 16 / (int) sizeof(T);
+          struct alignas(16) Vec { T v[V]; };
+#pragma unroll
+          for (int q = 0; q < NQ; q += V) {
+            const Vec y = *reinterpret_cast<const Vec*>(zr + q);
+#pragma unroll
+            for (int c = 0; c < V; c++) x[q + c] = y.v[c];
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < NQ; q++) x[q] = zr[q];
+        }
+#pragma unroll
+        for (int h = 0; h < R; h++) {
+          if constexpr (sizeof(T) == 4 && NQ % 2 == 0) {
+#pragma unroll
+            for (int q = 0; q < NQ; q += 2) fma2(acc[h * NQ + q], acc[h * NQ + q + 1], l[h * NT + t], x[q], x[q + 1]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < NQ; q++) acc[h * NQ + q] += l[h * NT + t] * x[q];
+          }
+        }
+      }
+    }
+  }
+  // the sums over the row's lanes that this lane owns
+  __device__ __forceinline__ void sum(T (&out)[QL]) const {
+    constexpr unsigned FULL = 0xffffffffu;
+    if constexpr (DMMA) {
+      out[0] = acc[0];
+      out[1] = acc[1];
+    } else if constexpr (NQ == 1) {
+      T v = acc[0];
+      v += __shfl_xor_sync(FULL, v, 2);
+      out[0] = v + __shfl_xor_sync(FULL, v, 1);
+    } else {
+      // at each offset a lane keeps one half of its sums and adds its
+      // partner's copy of it: first by row (offset 4), then by column
+      T v[NACC];
+#pragma unroll
+      for (int a = 0; a < NACC; a++) v[a] = acc[a];
+#pragma unroll
+      for (int o = J / 2, h = NACC / 2; o >= 1; o >>= 1, h >>= 1) {
+        const bool up = (threadIdx.x & o) != 0;
+#pragma unroll
+        for (int a = 0; a < h; a++) v[a] = (up ? v[a + h] : v[a]) + __shfl_xor_sync(FULL, up ? v[a] : v[a + h], o);
+      }
+#pragma unroll
+      for (int q = 0; q < QL; q++) out[q] = v[q];
+    }
+  }
+};
+
+// dynamic shared memory: the ring of z's and the vector of the inverse's
+// product (walker); a round's staged z's and the block's own vector (helper)
+template <typename T, int NQ>
+constexpr size_t chain_smem() { return (size_t) (CH_RING + 1) * BR * NQ * sizeof(T); }
+
+// zp, pp: published z's and p's; forward reads B and writes W, backward reads
+// W (y) and part (L21^T x2) and writes X
+template <typename T, int NQ, int WS, bool BWD>
+__global__ void __cluster_dims__(CH_C, 1, 1) __launch_bounds__(CH_THREADS, sizeof(T) == 4 ? 2 : 1)
+k_chain(const int* __restrict__ walk_fronts, int nwalk, const int2_* __restrict__ blocks, int nblocks,
+        const int2_* __restrict__ blk_ch, const int4* __restrict__ blk_child, const FrontDesc* __restrict__ fronts,
+        const int* __restrict__ maps, const int* __restrict__ rows, const T* __restrict__ L,
+        const T* __restrict__ Dinv, const T* __restrict__ B, T* __restrict__ X, int ldx, T* __restrict__ W,
+        const T* __restrict__ part, unsigned long long* __restrict__ zp, unsigned long long* __restrict__ pp, int nrhs,
+        const int* counter, int epoch, int* status) {
+  using Row = ChainRow<T, NQ>;
+  constexpr int QL = Row::QL, WPV = ch_words<T>();
+  extern __shared__ __align__(16) unsigned char chm[];
+  __shared__ __align__(8) unsigned long long bars[CH_RING];
   __shared__ unsigned bad_s;
-  constexpr int NY = WALK_HB * BR * NQ / 256;
-  for (int t = 0; t < n;) {
-    const int nb = min(n - t, WALK_HB);
-    if (threadIdx.x == 0) bad_s = 0;
-    __syncthreads();
-    float lv[WALK_HB][BR / 4];
-    unsigned long long yv[NY];
-    if (act) {
-#pragma unroll
-      for (int b = 0; b < WALK_HB; b++)
-#pragma unroll
-        for (int jj = 0; jj < BR / 4; jj++) lv[b][jj] = (b < nb) ? load_l(t + b, jj) : 0.0f;
-#pragma unroll
-      for (int u = 0; u < NY; u++) {
-        const int e = threadIdx.x + 256 * u, b = e / (BR * NQ);
-        yv[u] = (b < nb) ? get_pair(pairs(t + b) + e % (BR * NQ)) : 0ull;
-      }
-      unsigned bad = 0;
-#pragma unroll
-      for (int u = 0; u < NY; u++) {
-        const int e = threadIdx.x + 256 * u, b = e / (BR * NQ);
-        if (b < nb && !pair_ok(yv[u], tag)) bad |= 1u << b;
-      }
-      if (bad) atomicOr(&bad_s, bad);
-    }
-    __syncthreads();
-    // the leading blocks whose pairs are all current; none: wait for the first
-    int ok = __ffs(bad_s | (1u << nb)) - 1;
-    if (ok == 0) {
-      if (act) {
-#pragma unroll
-        for (int u = 0; u < NY; u++) {
-          const int e = threadIdx.x + 256 * u, b = e / (BR * NQ);
-          if (b == 0) yv[u] = wait_pair(pairs(t) + e % (BR * NQ), yv[u], tag, status);
-        }
-      }
-      ok = 1;
-    }
-    if (act) {
-#pragma unroll
-      for (int u = 0; u < NY; u++) {
-        const int e = threadIdx.x + 256 * u, b = e / (BR * NQ), r = e % (BR * NQ);
-        ysb[b][r / NQ][r % NQ] = pair_value(yv[u]);
-      }
-    }
-    __syncthreads();
-    if (act) {
-#pragma unroll
-      for (int b = 0; b < WALK_HB; b++)
-        if (b < ok)
-#pragma unroll
-          for (int jj = 0; jj < BR / 4; jj++) {
-            float yv[NQ];
-            ld_row8(ysb[b][qg * (BR / 4) + jj], yv);
-#pragma unroll
-            for (int q = 0; q < NQ; q++) acc[q] += lv[b][jj] * yv[q];
-          }
-    }
-    __syncthreads();
-    t += ok;
+  const int tid = threadIdx.x;
+  const int rho = Row::own(), qb = Row::qb(), jq = Row::jq();
+  const bool qact = Row::qact();
+  const unsigned tag = ((unsigned) *counter << 12) | (unsigned) epoch;
+  const bool walker = blockIdx.x < (unsigned) (nwalk * CH_C);
+  int2_ bk{0, 0};
+  if (walker) {
+    bk.a = walk_fronts[blockIdx.x / CH_C];
+  } else {
+    const int h = blockIdx.x - nwalk * CH_C;
+    if (h >= nblocks) return;
+    bk = blocks[h];
   }
-}
-
-template <typename T, int WS>
-__global__ void __maxnreg__(112)
-k_fwd_walk(const int* __restrict__ walk_fronts, int nwalk, const int2_* __restrict__ blocks,
-           const int2_* __restrict__ blk_ch, const int4* __restrict__ blk_child,
-           const FrontDesc* __restrict__ fronts, const int* __restrict__ maps,
-           const int* __restrict__ rows, const T* __restrict__ L, const T* __restrict__ Dinv,
-           const T* __restrict__ B, int ldb, T* __restrict__ W, unsigned long long* __restrict__ ypairs,
-           unsigned long long* __restrict__ ppairs, int nrhs, int* __restrict__ flags, const int* counter, int epoch,
-           int* status) {
-  static_assert(sizeof(T) == 4, "the tagged pairs carry FP32 values");
-  constexpr int NQ = SOLVE_NRHS, TPT = BR * BR / 256;
-  static_assert(NQ % 4 == 0, "four thread groups share the right-hand sides");
-  extern __shared__ __align__(16) unsigned char wsm[];
-  __shared__ T hpv[BR][NQ + 1];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row = tid % BR, qg = tid / BR;
-  const unsigned tag = walk_tag(counter, epoch);
-  if (blockIdx.x < nwalk) {
-    // ---------------------------------------------------------------- walker
-    const FrontDesc F = fronts[walk_fronts[blockIdx.x]];
-    const int f = F.f, s = F.s, nbs = (s + BR - 1) / BR;
-    const T* P = L + F.l_off;
-    T* Wf = W + F.v_off * WS;
-    unsigned long long* yp = ypairs + (size_t) F.blk_off * WALK_PAIRS;
-    const unsigned long long* pp = ppairs + (size_t) F.blk_off * WALK_PAIRS;
-    // tl[j] for j < WALK_D: L_{r, r-WALK_D+j} (zero before the first block);
-    // tl[WALK_D]: the inverse of block r, and in rows >= bw of the last
-    // block the update rows' entries of L_{., r}; all column-major.  yr:
-    // the ring of the last y's; pvb: the partials of even and odd steps;
-    // red: the four j-quarters' partial products; pf: p_r after the near
-    // terms.  Rows of eight right-hand sides, 32 bytes, read as vectors.
-    T (*tl)[BR][BR] = reinterpret_cast<T (*)[BR][BR]>(wsm);
-    T (*yr)[BR][NQ] = reinterpret_cast<T (*)[BR][NQ]>(wsm + WALK_T * BR * BR * sizeof(T));
-    T (*pvb)[BR][NQ] = yr + WALK_T;   // [2]
-    T (*red)[BR][NQ] = pvb + 2;        // [4]
-    T (*pf)[NQ] = red[4];
-    if (warp == 8) {
-      // ---- loader warp: the partials two steps ahead
-      auto load_p = [&](int r, int buf) {
-        constexpr int NV = WALK_PAIRS / 32;
-        unsigned long long v[NV];
-        const unsigned long long* src = pp + (size_t) r * WALK_PAIRS;
+  const FrontDesc F = fronts[bk.a];
+  const int f = F.f, s = F.s, nbs = (s + BR - 1) / BR;
+  const T* P = L + F.l_off;
+  T* Wf = W + F.v_off * WS;
+  const int* rw = rows + F.rows_off;
+  unsigned long long* zf = zp + (size_t) F.blk_off * CH_VALUES * WPV;
+  unsigned long long* pf = pp + (size_t) F.blk_off * CH_VALUES * WPV;
+  T* zs = reinterpret_cast<T*>(chm);              // [CH_RING][BR][NQ]
+  T (*vs)[NQ] = reinterpret_cast<T (*)[NQ]>(zs + CH_RING * BR * NQ);
+  // chain position t <-> block of the front
+  auto block_of = [&](int t) { return BWD ? nbs - 1 - t : t; };
+  // this lane's 16 entries of A_tu (block row bt: rows below s may belong to
+  // the update rows of the last diagonal block, or be an update block)
+  auto tile = [&](int bt, int bu, T (&l)[16]) {
 #pragma unroll
-        for (int u = 0; u < NV; u++) v[u] = get_pair(src + lane + 32 * u);
+    for (int h = 0; h < Row::R; h++) {
+      const int r = bt * BR + Row::row(h), c = bu * BR + jq;
+      const bool rv = r < (BWD ? s : f);
+      const T* a = BWD ? P + c + (size_t) r * f : P + r + (size_t) c * f;
 #pragma unroll
-        for (int u = 0; u < NV; u++) {
-          v[u] = wait_pair(src + lane + 32 * u, v[u], tag, status);
-          const int e = lane + 32 * u;
-          pvb[buf][e / NQ][e % NQ] = pair_value(v[u]);
-        }
-        walk_ready_arrive(buf);
-      };
-      load_p(0, 0);
-      if (nbs > 1) load_p(1, 1);
-      // one wait per step of the compute warps (the last two complete the
-      // barriers of the final steps): step r - 2 released its buffer
-      for (int r = 2; r < nbs + 2; r++) {
-        walk_free_sync(r & 1);
-        if (r < nbs) load_p(r, r & 1);
-      }
-      return;
+      for (int t = 0; t < Row::NT; t++)
+        l[h * Row::NT + t] = (rv && c + Row::J * t < s) ? __ldg(a + (BWD ? Row::J * t : (size_t) (Row::J * t) * f)) : T(0);
     }
-    // ---- compute warps
-    T pre[WALK_PER];
-    auto fetch = [&](int r) {
-      const int r0 = r * BR, nr = min(BR, f - r0), bw = min(BR, s - r0);
-      const T* Di = Dinv + F.dinv_off + (size_t) r * BR * BR;
-#pragma unroll
-      for (int t = 0; t < WALK_PER; t++) {
-        const int jj = t / TPT, e = tid + 256 * (t % TPT);
-        const int i = e % BR, j = e / BR;
-        T v = 0.0;
-        if (jj < WALK_D) {
-          const int k = r - WALK_D + jj;   // a full block (k < r <= nbs - 1)
-          if (k >= 0 && i < nr) v = P[(r0 + i) + (size_t) (k * BR + j) * f];
-        } else if (j < bw && i < nr) {
-          v = (i < bw) ? (i >= j ? Di[i + j * BR] : T(0)) : P[(r0 + i) + (size_t) (r0 + j) * f];
-        }
-        pre[t] = v;
+  };
+  // the right-hand side of block t, into vs (a barrier follows inside)
+  auto own_rhs = [&](int b, const int2_ cr) {
+    const int r0 = b * BR, nr = min(BR, f - r0);
+    if (!BWD) {
+      ChildGather<T, NQ, WS, CH_THREADS> cg;
+      cg.load(blk_child + cr.a, cr.b - cr.a, maps, W, nrhs);
+      for (int e = tid; e < BR * NQ; e += CH_THREADS) {
+        const int i = e % BR, q = e / BR;
+        vs[i][q] = (i < nr && q < nrhs && r0 + i < s) ? B[rw[r0 + i] + (size_t) q * ldx] : T(0);
       }
-    };
-    auto put = [&]() {
-#pragma unroll
-      for (int t = 0; t < WALK_PER; t++) {
-        const int e = tid + 256 * (t % TPT);
-        tl[t / TPT][e / BR][e % BR] = pre[t];
-      }
-    };
-    fetch(0);
-    put();
-    // thread (row, j-quarter jq): the products of its row with 16 of the
-    // block's columns for all eight right-hand sides, reduced over the
-    // quarters in shared memory
-    const int jq = tid / BR, j0 = jq * (BR / 4);
-    for (int r = 0; r < nbs; r++) {
-      const int r0 = r * BR, nr = min(BR, f - r0), bw = min(BR, s - r0);
-      const int slot = r % WALK_T, buf = r & 1;
-      // p_r is in place (loader warp) and so are the tiles of step r (every
-      // compute thread put its share before arriving here)
-      walk_ready_sync(buf);
-      if (r + 1 < nbs) fetch(r + 1);   // in flight during the step
-      // near terms: p_r -= sum_j L_{r, r-WALK_D+j} y_{r-WALK_D+j}
-      {
-        T u[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; q++) u[q] = 0.0;
-#pragma unroll
-        for (int jj = 0; jj < WALK_D; jj++) {
-          const int k = r - WALK_D + jj;
-          if (k < 0) continue;
-          const int sl = k % WALK_T;
+      __syncthreads();
+      cg.add(blk_child + cr.a, cr.b - cr.a, maps, W, nrhs, r0, vs);
+    } else {
+      for (int e = tid; e < BR * NQ; e += CH_THREADS) {
+        const int i = e % BR, q = e / BR;
+        T v = T(0);
+        if (r0 + i < s && q < nrhs) {
+          v = Wf[r0 + i + (size_t) q * f];
+          T acc = T(0);
 #pragma unroll 4
-          for (int j = j0; j < j0 + BR / 4; j++) {
-            const T l = tl[jj][j][row];
-            T yv[NQ];
-            ld_row8(yr[sl][j], yv);
-#pragma unroll
-            for (int q = 0; q < NQ; q++) u[q] += l * yv[q];
-          }
+          for (int ch = 0; ch < F.nchunk; ch++)
+            acc += part[F.part_off + ((size_t) ch * s + r0 + i) * SOLVE_NRHS + q];
+          v -= acc;
         }
-        st_row8(red[jq][row], u);
+        vs[i][q] = v;
       }
-      nbar_sync<WB_COMPUTE, 256>();
-      // thread (row, jq) finishes right-hand sides 2 jq and 2 jq + 1
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        const int q = 2 * jq + c;
-        pf[row][q] = pvb[buf][row][q] - (red[0][row][q] + red[1][row][q] + red[2][row][q] + red[3][row][q]);
-      }
-      nbar_sync<WB_COMPUTE, 256>();
-      // the partial buffer of this step is free for the loader (step r + 2)
-      walk_free_arrive(buf);
-      // y_r = L_rr^-1 p_r in rows < bw (the inverse is lower triangular)
-      {
-        T u[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; q++) u[q] = 0.0;
-        const int je = min(j0 + BR / 4, min(row + 1, bw));
-        for (int j = j0; j < je; j++) {
-          const T d = tl[WALK_D][j][row];
-          T pv8[NQ];
-          ld_row8(pf[j], pv8);
-#pragma unroll
-          for (int q = 0; q < NQ; q++) u[q] += d * pv8[q];
-        }
-        st_row8(red[jq][row], u);
-      }
-      nbar_sync<WB_COMPUTE, 256>();
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        const int q = 2 * jq + c;
-        yr[slot][row][q] = (row < bw) ? red[0][row][q] + red[1][row][q] + red[2][row][q] + red[3][row][q] : pf[row][q];
-      }
-      nbar_sync<WB_COMPUTE, 256>();
-      if (bw < nr) {
-        // update rows inside the last diagonal block: w_i -= L[i, r] y_r
-        // (reads rows < bw of the ring slot, writes rows >= bw)
-        if (row >= bw) {
-#pragma unroll
-          for (int c = 0; c < 2; c++) {
-            const int q = 2 * jq + c;
-            T v = 0.0;
-            for (int j = 0; j < bw; j++) v += tl[WALK_D][j][row] * yr[slot][j][q];
-            yr[slot][row][q] -= v;
-          }
-        }
-        nbar_sync<WB_COMPUTE, 256>();
-      }
-      // y_r: tagged pairs for the helpers, plain values for later launches
-      {
-        unsigned long long* dst = yp + (size_t) r * WALK_PAIRS;
-#pragma unroll
-        for (int u = 0; u < WALK_PAIRS / 256; u++) {
-          const int e = tid + 256 * u;
-          put_pair(dst + e, tag, yr[slot][e / NQ][e % NQ]);
-        }
-      }
-      for (int e = tid; e < nr * nrhs; e += 256) {
-        const int i = e % nr, q = e / nr;
-        Wf[r0 + i + (size_t) q * f] = yr[slot][i][q];
-      }
-      if (tid == 0) flags[F.blk_off + r] = epoch;
-      // every read of this step's tiles is done before they are replaced
-      nbar_sync<WB_COMPUTE, 256>();
-      if (r + 1 < nbs) put();
+      __syncthreads();
     }
+  };
+
+  if (walker) {
+    // ---------------------------------------------------------------- walker
+    const unsigned rank = blockIdx.x % CH_C;
+    constexpr unsigned ZBYTES = BR * NQ * sizeof(T);
+    if (tid == 0) {
+      for (int i = 0; i < CH_RING; i++)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bars[i])) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      for (int i = 0; i < min(CH_RING, nbs); i++) bar_expect(smem_addr(&bars[i]), ZBYTES);
+    }
+    __syncthreads();
+    cluster_sync_all();
+    // z_u has arrived (each CTA waits for every u once, in order); its
+    // barrier is armed for the z that takes the slot next
+    auto wait_z = [&](int u) {
+      bar_wait(smem_addr(&bars[u % CH_RING]), (u / CH_RING) & 1, status);
+      if (tid == 0 && u + CH_RING < nbs) bar_expect(smem_addr(&bars[u % CH_RING]), ZBYTES);
+    };
+    unsigned peer[CH_C];   // offsets of the others' shared memory, the next CTA of the chain first
+#pragma unroll
+    for (int r = 0; r < CH_C; r++) peer[r] = map_rank(smem_addr(bars), (rank + 1 + r) % CH_C) - smem_addr(bars);
+    for (int t = rank; t < nbs; t += CH_C) {
+      const int b = block_of(t), r0 = b * BR, nr = min(BR, f - r0), bw = min(BR, s - r0);
+      const T* Di = Dinv + F.dinv_off + (size_t) b * BR * BR;
+      const int u0 = max(0, t - CH_C);
+      T la[16], lb[16], xd[16];
+      if (u0 < t) tile(b, block_of(u0), la);
+      if (u0 + 1 < t) tile(b, block_of(u0 + 1), lb);
+#pragma unroll
+      for (int h = 0; h < Row::R; h++)
+#pragma unroll
+        for (int i = 0; i < Row::NT; i++) {
+          const int r = Row::row(h), c = Row::J * i + jq;
+          xd[h * Row::NT + i] = BWD ? Di[c + r * BR] : Di[r + c * BR];
+        }
+      // the next turn's tiles into L2
+      if (t + CH_C < nbs) {
+        const int bn = block_of(t + CH_C);
+        constexpr int LPC = BR * (int) sizeof(T) / 128 + 1;   // lines a 64-entry column piece touches
+        for (int e = tid; e < CH_C * BR * LPC; e += CH_THREADS) {
+          const int li = e % LPC, c = e / LPC;
+          const int bu = block_of(t + c / BR);
+          const int row = (BWD ? bu : bn) * BR + min(li * (128 / (int) sizeof(T)), BR - 1);
+          const int col = (BWD ? bn : bu) * BR + c % BR;
+          if (row < f && col < s) prefetch_l2(P + row + (size_t) col * f);
+        }
+        for (int e = tid; e < BR * BR * (int) sizeof(T) / 128; e += CH_THREADS)
+          prefetch_l2(reinterpret_cast<const unsigned char*>(Dinv + F.dinv_off + (size_t) bn * BR * BR) + 128 * e);
+      }
+      T pv[QL];
+      Row acc;
+      acc.clear();
+      Tagged<T> pt[QL];
+      const unsigned long long* pq = pf + ((size_t) b * CH_VALUES + rho * NQ + qb) * WPV;
+      auto load_p = [&]() {
+#pragma unroll
+        for (int q = 0; q < QL; q++) pt[q].load(pq + q * WPV);
+      };
+      if (t == 0) load_p();
+      for (int u = u0; u < t; u += 2) {
+        if (u + 2 >= t) load_p();
+        wait_z(u);
+        acc.add(la, zs + (u % CH_RING) * BR * NQ);
+        if (u + 2 < t) tile(b, block_of(u + 2), la);
+        if (u + 1 < t) {
+          wait_z(u + 1);
+          acc.add(lb, zs + ((u + 1) % CH_RING) * BR * NQ);
+          if (u + 3 < t) tile(b, block_of(u + 3), lb);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < QL; q++) {
+        wait_tagged<T>(pq + q * WPV, pt[q], true, tag, status);
+        pv[q] = pt[q].value();
+      }
+      T z[QL];
+      acc.sum(z);
+#pragma unroll
+      for (int q = 0; q < QL; q++) {
+        pv[q] -= z[q];
+        if (qact) vs[rho][qb + q] = pv[q];
+      }
+      __syncthreads();
+      acc.clear();
+      acc.add(xd, &vs[0][0]);
+      acc.sum(z);
+      if (!BWD && bw < nr) {
+        // the last diagonal block's update rows: w_i - L[i, block] y (the
+        // inverse is zero in their rows, so y is in place first)
+        __syncthreads();
+        if (qact && rho < bw)
+#pragma unroll
+          for (int q = 0; q < QL; q++) vs[rho][qb + q] = z[q];
+        __syncthreads();
+        tile(b, b, la);
+        acc.clear();
+        acc.add(la, &vs[0][0]);
+        T uq[QL];
+        acc.sum(uq);
+        if (rho >= bw)
+#pragma unroll
+          for (int q = 0; q < QL; q++) z[q] = pv[q] - uq[q];
+      }
+      // z_t: into every CTA of the cluster, then published for the helpers,
+      // then the result
+      if (qact) {
+        const unsigned za = smem_addr(zs + ((t % CH_RING) * BR + rho) * NQ + qb), ba = smem_addr(&bars[t % CH_RING]);
+        // first to the CTA whose turn is next
+#pragma unroll
+        for (int r = 0; r < CH_C; r++) st_async(za + peer[r], ba + peer[r], z);
+        unsigned long long* dst = zf + ((size_t) b * CH_VALUES + rho * NQ + qb) * WPV;
+#pragma unroll
+        for (int q = 0; q < QL; q++) Tagged<T>::put(dst + q * WPV, tag, z[q]);
+        if (!BWD) {
+          if (rho < nr)
+#pragma unroll
+            for (int q = 0; q < QL; q++)
+              if (qb + q < nrhs) Wf[r0 + rho + (size_t) (qb + q) * f] = z[q];
+        } else if (rho < bw) {
+          const int g = __ldg(rw + r0 + rho);
+#pragma unroll
+          for (int q = 0; q < QL; q++)
+            if (qb + q < nrhs) X[g + (size_t) (qb + q) * ldx] = z[q];
+        }
+      }
+    }
+    // every z that is still on its way to this CTA's shared memory
+    const int last = (int) rank < nbs ? (int) rank + (nbs - 1 - (int) rank) / CH_C * CH_C : 0;
+    for (int u = (int) rank < nbs ? last : 0; u < nbs; u++) wait_z(u);
+    cluster_sync_all();
     return;
   }
   // ------------------------------------------------------------------ helper
-  // (the loader warp's threads only keep the barriers here)
-  const bool act = tid < 256;
-  const int2_ bk = blocks[blockIdx.x - nwalk];
-  const FrontDesc F = fronts[bk.a];
-  const int r = bk.b, f = F.f, s = F.s;
-  const int r0 = r * BR, nr = min(BR, f - r0);
-  const T* P = L + F.l_off;
-  const int* rw = rows + F.rows_off;
-  T (*red)[BR][NQ] = reinterpret_cast<T (*)[BR][NQ]>(wsm);            // [4]
-  T (*ysb)[BR][NQ] = reinterpret_cast<T (*)[BR][NQ]>(wsm) + 4;         // [WALK_HB]
-  const int kend = max(r - WALK_D, 0);
-  const unsigned long long* yp = ypairs + (size_t) F.blk_off * WALK_PAIRS;
-  // the walker's tiles of this block into L2: the near blocks' 64 columns
-  // (two 128-byte lines each, the second while it holds rows of the front)
-  // and the block's inverse
-  {
-    const int ncol = WALK_D * BR, dlines = (int) (BR * BR * sizeof(T) / 128);
-    const T* Di = Dinv + F.dinv_off + (size_t) r * BR * BR;
-    for (int e = tid; e < 2 * ncol + dlines; e += WALK_THREADS) {
-      if (e < 2 * ncol) {
-        const int c = e >> 1, half = e & 1, k = r - WALK_D + c / BR;
-        if (k >= 0 && (half == 0 || r0 + 128 / (int) sizeof(T) < f))
-          prefetch_l2(P + r0 + half * (128 / (int) sizeof(T)) + (size_t) (k * BR + c % BR) * f);
-      } else {
-        prefetch_l2(reinterpret_cast<const unsigned char*>(Di) + (size_t) (e - 2 * ncol) * 128);
-      }
+  const bool upd = !BWD && bk.b >= nbs;                  // an update-row block
+  const int t = upd ? nbs : BWD ? nbs - 1 - bk.b : bk.b;
+  const int n = upd ? nbs : max(0, t - CH_C), b = bk.b;
+  T* zst = zs;                                           // [CH_HB][BR][NQ]
+  own_rhs(b, BWD ? int2_{0, 0} : blk_ch[blockIdx.x - nwalk * CH_C]);
+  Row acc;
+  acc.clear();
+  constexpr int NV = (CH_HB * BR * NQ + CH_THREADS - 1) / CH_THREADS;
+  for (int u = 0; u < n;) {
+    // a round: up to CH_HB blocks with every load in flight; the leading
+    // blocks whose values are all current are used, or the first is waited for
+    const int nb = min(n - u, CH_HB);
+    if (tid == 0) bad_s = 0;
+    __syncthreads();
+    T l[CH_HB][16];
+#pragma unroll
+    for (int i = 0; i < CH_HB; i++)
+      if (i < nb) tile(b, block_of(u + i), l[i]);
+    Tagged<T> zv[NV];
+    auto src = [&](int e) {
+      return zf + ((size_t) block_of(u + e / (BR * NQ)) * CH_VALUES + e % (BR * NQ)) * WPV;
+    };
+    unsigned bad = 0;
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+      const int e = tid + CH_THREADS * i;
+      if (e < nb * BR * NQ) zv[i].load(src(e));
     }
-  }
-  for (int k = tid; k < BR * NQ; k += WALK_THREADS) {
-    const int i = k % BR, q = k / BR;
-    hpv[i][q] = (i < nr && q < nrhs && r0 + i < s) ? B[rw[r0 + i] + (size_t) q * ldb] : T(0);
-  }
-  __syncthreads();
-  {
-    const int2_ cr = blk_ch[blockIdx.x - nwalk];
-    ChildGather<T, NQ, WS, 256> cg;
-    cg.load(blk_child + cr.a, cr.b - cr.a, maps, W, nrhs);
-    cg.add(blk_child + cr.a, cr.b - cr.a, maps, W, nrhs, r0, hpv);
-  }
-  // far terms k < r - WALK_D: thread (row, quarter qg) sums 16 columns of
-  // each L_rk for every right-hand side
-  T acc[NQ];
 #pragma unroll
-  for (int q = 0; q < NQ; q++) acc[q] = 0.0;
-  walk_far_terms<NQ>(
-      tag, status, kend,
-      [&](int k, int jj) -> T {
-        return (row < nr) ? P[(r0 + row) + (size_t) (k * BR + qg * (BR / 4) + jj) * f] : T(0);
-      },
-      [&](int k) { return yp + (size_t) k * WALK_PAIRS; }, ysb, acc, qg, act);
-  if (act) {
+    for (int i = 0; i < NV; i++) {
+      const int e = tid + CH_THREADS * i;
+      if (e < nb * BR * NQ && !zv[i].ok(tag)) bad |= 1u << (e / (BR * NQ));
+    }
+    if (bad) atomicOr(&bad_s, bad);
+    __syncthreads();
+    int ok = __ffs(bad_s | (1u << nb)) - 1;
+    if (ok == 0) {
 #pragma unroll
-    for (int q = 0; q < NQ; q++) red[qg][row][q] = acc[q];
+      for (int i = 0; i < NV; i++) {
+        const int e = tid + CH_THREADS * i;
+        if (CH_THREADS * i < BR * NQ) wait_tagged<T>(src(e < BR * NQ ? e : 0), zv[i], e < BR * NQ, tag, status);
+      }
+      ok = 1;
+    }
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+      const int e = tid + CH_THREADS * i;
+      if (e < ok * BR * NQ) zst[e] = zv[i].value();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < CH_HB; i++)
+      if (i < ok) acc.add(l[i], zst + i * BR * NQ);
+    __syncthreads();
+    u += ok;
   }
-  __syncthreads();
-  unsigned long long* dst = ppairs + (size_t) (F.blk_off + r) * WALK_PAIRS;
-  for (int e = tid; e < WALK_PAIRS; e += WALK_THREADS) {
-    const int i = e / NQ, q = e % NQ;
-    put_pair(dst + e, tag, hpv[i][q] - (red[0][i][q] + red[1][i][q] + red[2][i][q] + red[3][i][q]));
+  T p[QL];
+  acc.sum(p);
+  if (!qact) return;
+#pragma unroll
+  for (int q = 0; q < QL; q++) p[q] = vs[rho][qb + q] - p[q];
+  if (upd) {
+    if (b * BR + rho < f)
+#pragma unroll
+      for (int q = 0; q < QL; q++)
+        if (qb + q < nrhs) Wf[b * BR + rho + (size_t) (qb + q) * f] = p[q];
+  } else {
+    unsigned long long* dst = pf + ((size_t) b * CH_VALUES + rho * NQ + qb) * WPV;
+#pragma unroll
+    for (int q = 0; q < QL; q++) Tagged<T>::put(dst + q * WPV, tag, p[q]);
   }
 }
 
-// x at the update rows of every big front of a level, gathered once into the
-// front's work vector (rows s..f-1) so the backward blocks read it coalesced
-template <typename T, int WS>
-__global__ void __launch_bounds__(128)
-k_gather_upd(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts,
-             const int* __restrict__ rows, const T* __restrict__ X, int ldx, T* __restrict__ W,
-             int nrhs) {
-  const int2_ bk = blocks[blockIdx.x];
-  const FrontDesc F = fronts[bk.a];
-  const int r0 = max(bk.b * BR, F.s), r1 = min(bk.b * BR + BR, F.f);
-  if (r0 >= r1) return;
-  T* Wf = W + F.v_off * WS;
-  const int* rw = rows + F.rows_off;
-  const int nr = r1 - r0;
-  for (int e = threadIdx.x; e < nr * nrhs; e += blockDim.x) {
-    const int i = r0 + e % nr, q = e / nr;
-    Wf[i + (size_t) q * F.f] = X[rw[i] + (size_t) q * ldx];
-  }
-}
-
-// Backward solve, L21^T x2 split over (column block, 512-row chunk) CTAs so
-// that the whole GPU streams L21; each CTA stores its partial sums, which the
-// chain kernel adds in chunk order.  The chunk of x2 is staged in shared
-// memory once ([column][row], conflict-free across lanes); each warp takes
-// its 16 columns of the block G = 32 / NQ at a time, so that the G x NQ = 32
-// sums of a pass finish with one warp reduce-scatter (31 shuffles; lane t
-// ends with sum t = column t / NQ, right-hand side t % NQ).
-template <typename T, int NQ, int WS>
-__global__ void __launch_bounds__(128)
-k_bwd_l21(const int2_* __restrict__ tasks, const FrontDesc* __restrict__ fronts, const T* __restrict__ L,
-          const T* __restrict__ W, T* __restrict__ part, int nrhs) {
-  constexpr int G = 32 / NQ;
-  static_assert(G * NQ == 32 && G <= 16, "a pass holds 32 sums of at most 16 columns");
-  __shared__ T zs[NQ][SOLVE_RCH];
-  const int2_ tk = tasks[blockIdx.x];
-  const FrontDesc F = fronts[tk.a];
-  const int k = tk.b >> 16, ch = tk.b & 0xffff;
+// Backward solve, L21^T x2 over a 64-column block and a chunk of 512 update
+// rows by a CTA of 128 threads.  The chunk of x2 is gathered into shared
+// memory once ([column][row], conflict-free across lanes); each warp takes its
+// 16 columns of the block G = 32 / NQ at a time, so that the G x NQ = 32 sums
+// of a pass finish with one warp reduce-scatter (31 shuffles; lane t ends with
+// sum t = column t / NQ, right-hand side t % NQ), which sink(column, right-hand
+// side, sum) takes.  zs may be reused after the caller's next barrier.
+template <typename T, int NQ, typename Sink>
+__device__ __forceinline__ void l21_chunk(const FrontDesc& F, const T* __restrict__ L, const int* __restrict__ rows,
+                                          const T* X, int ldx, int k, int ch, int nrhs, T (*zs)[SOLVE_RCH],
+                                          Sink sink) {
+  constexpr int G = NQ >= 2 ? 32 / NQ : 16, SUMS = G * NQ;
+  static_assert((SUMS == 32 || SUMS == 16) && G <= 16, "a pass holds 32 (one right-hand side: 16) sums");
   const int f = F.f, s = F.s, m = f - s;
   const int c0 = k * BR, bw = min(BR, s - c0);
   const int i0 = ch * SOLVE_RCH, nr = min(m - i0, SOLVE_RCH);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const T* z = W + F.v_off * WS + s + i0;
   const T* P = L + F.l_off + s + i0;
   // all of this thread's loads in flight before its first store
   {
-    constexpr int NZ = NQ * SOLVE_RCH / 128;
-    T zv[NZ];
+    constexpr int NI = SOLVE_RCH / 128;
+    const int* rw = rows + F.rows_off + s + i0;
+    int g[NI];
+    T zv[NQ][NI];
 #pragma unroll
-    for (int t = 0; t < NZ; t++) {
-      const int e = threadIdx.x + 128 * t, i = e % SOLVE_RCH, q = e / SOLVE_RCH;
-      zv[t] = (i < nr && q < nrhs) ? __ldcg(z + i + (size_t) q * f) : T(0);
-    }
+    for (int t = 0; t < NI; t++) g[t] = (int) threadIdx.x + 128 * t < nr ? __ldg(rw + threadIdx.x + 128 * t) : -1;
 #pragma unroll
-    for (int t = 0; t < NZ; t++) {
-      const int e = threadIdx.x + 128 * t;
-      zs[e / SOLVE_RCH][e % SOLVE_RCH] = zv[t];
-    }
+    for (int q = 0; q < NQ; q++)
+#pragma unroll
+      for (int t = 0; t < NI; t++) zv[q][t] = (g[t] >= 0 && q < nrhs) ? __ldcg(X + g[t] + (size_t) q * ldx) : T(0);
+#pragma unroll
+    for (int q = 0; q < NQ; q++)
+#pragma unroll
+      for (int t = 0; t < NI; t++) zs[q][threadIdx.x + 128 * t] = zv[q][t];
   }
   __syncthreads();
   for (int cg = warp * 16; cg < warp * 16 + 16; cg += G) {
-    T v[32];   // v[a * NQ + q]: column cg + a, right-hand side q
+    if (cg >= bw) break;
+    T v[SUMS];   // v[a * NQ + q]: column cg + a, right-hand side q
 #pragma unroll
-    for (int j = 0; j < 32; j++) v[j] = T(0);
+    for (int j = 0; j < SUMS; j++) v[j] = T(0);
     // RU rows per lane per round, 16 loads of the panel in flight at once
     // (one round per memory latency)
     constexpr int RU = G >= 16 ? 1 : 16 / G;
-    for (int i0 = lane; i0 < nr; i0 += 32 * RU) {
+    for (int i1 = lane; i1 < nr; i1 += 32 * RU) {
       T lv[RU][G];
 #pragma unroll
       for (int u = 0; u < RU; u++)
 #pragma unroll
         for (int a = 0; a < G; a++) {
-          const int i = i0 + 32 * u;
+          const int i = i1 + 32 * u;
           lv[u][a] = (i < nr && cg + a < bw) ? P[i + (size_t) (c0 + cg + a) * f] : T(0);
         }
 #pragma unroll
       for (int u = 0; u < RU; u++) {
-        const int i = i0 + 32 * u;
+        const int i = i1 + 32 * u;
         if (i < nr) {
           T zi[NQ];
 #pragma unroll
@@ -1346,7 +1367,11 @@ k_bwd_l21(const int2_* __restrict__ tasks, const FrontDesc* __restrict__ fronts,
     // reduce-scatter: at offset o a lane keeps the half of its remaining
     // sums that matches its bit o and adds the partner's copy of that half
 #pragma unroll
-    for (int o = 16, h = 16; o >= 1; o >>= 1, h >>= 1) {
+    for (int o = 16, h = SUMS / 2; o >= 1; o >>= 1, h >>= 1) {
+      if (h == 0) {   // 16 sums: the last pair of lanes holds the same one
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        continue;
+      }
       const bool up = (lane & o) != 0;
 #pragma unroll
       for (int j = 0; j < h; j++) {
@@ -1355,18 +1380,37 @@ k_bwd_l21(const int2_* __restrict__ tasks, const FrontDesc* __restrict__ fronts,
         v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
     }
-    const int a = lane / NQ, q = lane % NQ;
-    if (cg + a < bw && q < nrhs) part[F.part_off + ((size_t) ch * s + c0 + cg + a) * SOLVE_NRHS + q] = v[0];
+    const int t = SUMS == 32 ? lane : lane >> 1;
+    const int a = t / NQ, q = t % NQ;
+    if (cg + a < bw && q < nrhs && (SUMS == 32 || (lane & 1) == 0)) sink(cg + a, q, v[0]);
   }
 }
 
-template <typename T, int NQ, int WS, bool PARTS, bool WARPLOOP = (NQ < 8)>
+// the sums of (column block, 512-row chunk) tasks, so that the whole GPU
+// streams L21; the chain and block kernels add them in chunk order
+template <typename T, int NQ>
+__global__ void __launch_bounds__(128)
+k_bwd_l21(const int2_* __restrict__ tasks, const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
+          const T* __restrict__ L, const T* __restrict__ X, int ldx, T* __restrict__ part, int nrhs) {
+  __shared__ T zs[NQ][SOLVE_RCH];
+  const int2_ tk = tasks[blockIdx.x];
+  const FrontDesc F = fronts[tk.a];
+  const int k = tk.b >> 16, ch = tk.b & 0xffff;
+  T* out = part + F.part_off + ((size_t) ch * F.s + k * BR) * SOLVE_NRHS;
+  l21_chunk<T, NQ>(F, L, rows, X, ldx, k, ch, nrhs, zs, [&](int c, int q, T v) { out[c * SOLVE_NRHS + q] = v; });
+}
+
+// Backward solve of big fronts, one CTA per 64-column block, chained from the
+// last block by flags.  PARTS: fronts of more than one chunk of update rows
+// have their L21^T x2 from k_bwd_l21, the others (and without PARTS all) form
+// it here, before the first flag is waited for.
+template <typename T, int NQ, int WS, bool PARTS>
 __global__ void __launch_bounds__(128)
 k_bwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts,
           const int* __restrict__ rows, const T* __restrict__ L, const T* __restrict__ Dinv, T* __restrict__ X, int ldx,
           T* __restrict__ W, const T* __restrict__ part, int nrhs, int* __restrict__ flags, int epoch,
           int* status) {
-  constexpr int G = (16 / NQ) > 1 ? 16 / NQ : 1;   // columns per pass of the L21 product
+  constexpr bool WARPLOOP = NQ < 8;
   __shared__ T xv[BR][NQ];
   __shared__ T xj[BR][NQ];
   __shared__ T red[BR][NQ];
@@ -1376,7 +1420,7 @@ k_bwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts
   T (*tile)[BR + 1] = reinterpret_cast<T (*)[BR + 1]>(bsmraw) + BR;   // NQ >= 8: block of L11, [col][row]
   const int2_ bk = blocks[blockIdx.x];
   const FrontDesc F = fronts[bk.a];
-  const int k = bk.b, f = F.f, s = F.s, m = f - s;
+  const int k = bk.b, f = F.f, s = F.s;
   const int nbs = (s + BR - 1) / BR;
   const int c0 = k * BR, bw = min(BR, s - c0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1405,7 +1449,7 @@ k_bwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts
     xv[c][q] = (c < bw && q < nrhs) ? Wf[c0 + c + (size_t) q * f] : 0.0;
   }
   __syncthreads();
-  if (PARTS) {
+  if (PARTS && F.nchunk > 1) {
     // y - L21^T x2 from the per-chunk partial sums, added in chunk order
     for (int e = tid; e < bw * NQ; e += 128) {
       const int c = e % bw, q = e / bw;
@@ -1417,35 +1461,12 @@ k_bwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts
         xv[c][q] -= acc;
       }
     }
-  }
-  // y - L21^T x2: warp w owns columns 16w..16w+15, G at a time; lanes run
-  // down the update rows with one coalesced load per column per step
-  const T* z = Wf + s;
-  for (int cg = warp * 16; !PARTS && cg < warp * 16 + 16; cg += G) {
-    T acc[G][NQ];
-#pragma unroll
-    for (int a_ = 0; a_ < G; a_++)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) acc[a_][q] = 0.0;
-    for (int i = lane; i < m; i += 32) {
-      T zi[NQ];
-#pragma unroll
-      for (int q = 0; q < NQ; q++) zi[q] = (q < nrhs) ? __ldcg(z + i + (size_t) q * f) : 0.0;
-#pragma unroll
-      for (int a_ = 0; a_ < G; a_++) {
-        const T l = (cg + a_ < bw) ? P[(s + i) + (size_t) (c0 + cg + a_) * f] : 0.0;
-#pragma unroll
-        for (int q = 0; q < NQ; q++) acc[a_][q] += l * zi[q];
-      }
+  } else {
+    T (*zs)[SOLVE_RCH] = reinterpret_cast<T (*)[SOLVE_RCH]>(dgb + BR);
+    for (int ch = 0; ch < F.nchunk; ch++) {
+      l21_chunk<T, NQ>(F, L, rows, X, ldx, k, ch, nrhs, zs, [&](int c, int q, T v) { xv[c][q] -= v; });
+      __syncthreads();
     }
-#pragma unroll
-    for (int a_ = 0; a_ < G; a_++)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) {
-        T v = acc[a_][q];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0 && cg + a_ < bw) xv[cg + a_][q] -= v;
-      }
   }
   __syncthreads();
   const int col = tid % BR, half = tid / BR;
@@ -1563,256 +1584,6 @@ k_bwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts
   if (tid == 0) st_release(flags + F.blk_off + k, epoch);
 }
 
-// Backward solve of the diagonal blocks of levels with long chains, as a
-// walk: the mirror of k_fwd_walk.  The walker of a front runs
-// x_k = L_kk^-T (v_k - sum_{j>k} L_jk^T x_j) from the last block to the
-// first, subtracting the WALK_D near terms j = k+1, k+2 itself, with the
-// same split into compute warps and a loader warp; helper CTAs, one per
-// diagonal block (listed last block first), form v_k = y_k - L21^T x2 from
-// the chunk partial sums, subtract the far terms j > k + WALK_D as the
-// walker publishes x_j, publish the partial and pull the walker's tiles of
-// their block into L2.  Values cross between CTAs as tagged pairs, as in
-// the forward walk, and the same in-order dispatch argument keeps every
-// wait finite.
-template <typename T, int WS>
-__global__ void __maxnreg__(112)
-k_bwd_walk(const int* __restrict__ walk_fronts, int nwalk, const int2_* __restrict__ blocks,
-           const FrontDesc* __restrict__ fronts, const int* __restrict__ rows, const T* __restrict__ L,
-           const T* __restrict__ Dinv, T* __restrict__ X, int ldx, T* __restrict__ W,
-           const T* __restrict__ part, unsigned long long* __restrict__ ypairs,
-           unsigned long long* __restrict__ ppairs, int nrhs, int* __restrict__ flags, const int* counter, int epoch,
-           int* status) {
-  static_assert(sizeof(T) == 4, "the tagged pairs carry FP32 values");
-  constexpr int NQ = SOLVE_NRHS, TPT = BR * BR / 256;
-  extern __shared__ __align__(16) unsigned char wsm[];
-  __shared__ T hpv[BR][NQ + 1];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int col = tid % BR, qg = tid / BR;
-  const unsigned tag = walk_tag(counter, epoch);
-  if (blockIdx.x < nwalk) {
-    // ---------------------------------------------------------------- walker
-    const FrontDesc F = fronts[walk_fronts[blockIdx.x]];
-    const int f = F.f, s = F.s, nbs = (s + BR - 1) / BR;
-    const T* P = L + F.l_off;
-    T* Wf = W + F.v_off * WS;
-    const int* rw = rows + F.rows_off;
-    unsigned long long* yp = ypairs + (size_t) F.blk_off * WALK_PAIRS;
-    const unsigned long long* pp = ppairs + (size_t) F.blk_off * WALK_PAIRS;
-    // tl[j] for j < WALK_D: L_{k+1+j, k} (zero past the last block);
-    // tl[WALK_D]: the inverse of block k; all [row][column]
-    T (*tl)[BR][BR + 1] = reinterpret_cast<T (*)[BR][BR + 1]>(wsm);
-    T (*xr)[BR][NQ] = reinterpret_cast<T (*)[BR][NQ]>(wsm + WALK_T * BR * (BR + 1) * sizeof(T));
-    T (*pvb)[BR][NQ] = xr + WALK_T;   // [2]: the partials by step parity
-    T (*red)[BR][NQ] = pvb + 2;        // [4]: the i-quarters' products
-    T (*pf)[NQ] = red[4];              // p_k after the near terms
-    if (warp == 8) {
-      // ---- loader warp; step t of the walk is block nbs - 1 - t
-      auto load_p = [&](int t, int buf) {
-        constexpr int NV = WALK_PAIRS / 32;
-        unsigned long long v[NV];
-        const unsigned long long* src = pp + (size_t) (nbs - 1 - t) * WALK_PAIRS;
-#pragma unroll
-        for (int u = 0; u < NV; u++) v[u] = get_pair(src + lane + 32 * u);
-#pragma unroll
-        for (int u = 0; u < NV; u++) {
-          v[u] = wait_pair(src + lane + 32 * u, v[u], tag, status);
-          const int e = lane + 32 * u;
-          pvb[buf][e / NQ][e % NQ] = pair_value(v[u]);
-        }
-        walk_ready_arrive(buf);
-      };
-      load_p(0, 0);
-      if (nbs > 1) load_p(1, 1);
-      for (int t = 2; t < nbs + 2; t++) {
-        walk_free_sync(t & 1);
-        if (t < nbs) load_p(t, t & 1);
-      }
-      return;
-    }
-    // ---- compute warps
-    T pre[WALK_PER];
-    auto fetch = [&](int k) {
-      const int c0 = k * BR, bw = min(BR, s - c0);
-      const T* Di = Dinv + F.dinv_off + (size_t) k * BR * BR;
-#pragma unroll
-      for (int t = 0; t < WALK_PER; t++) {
-        const int jj = t / TPT, e = tid + 256 * (t % TPT);
-        const int i = e % BR, c = e / BR;
-        T v = 0.0;
-        if (jj < WALK_D) {
-          const int j = k + 1 + jj;
-          if (j < nbs && c < bw && i < min(BR, s - j * BR)) v = P[(j * BR + i) + (size_t) (c0 + c) * f];
-        } else if (c < bw && i < bw && i >= c) {
-          v = Di[i + c * BR];
-        }
-        pre[t] = v;
-      }
-    };
-    auto put = [&]() {
-#pragma unroll
-      for (int t = 0; t < WALK_PER; t++) {
-        const int e = tid + 256 * (t % TPT);
-        tl[t / TPT][e % BR][e / BR] = pre[t];
-      }
-    };
-    fetch(nbs - 1);
-    put();
-    // thread (col, i-quarter iq): the products of its column with 16 of the
-    // block's rows for all eight right-hand sides, reduced over the quarters
-    // in shared memory
-    const int iq = tid / BR, i0 = iq * (BR / 4);
-    for (int t = 0; t < nbs; t++) {
-      const int k = nbs - 1 - t;
-      const int c0 = k * BR, bw = min(BR, s - c0);
-      const int slot = k % WALK_T, buf = t & 1;
-      walk_ready_sync(buf);   // p_k and the tiles of step k are in place
-      if (k > 0) fetch(k - 1);   // in flight during the step
-      // the global row of this thread's x entry (full blocks), loaded now so
-      // that the scatter at the end of the step does not wait for it
-      const int gx = (bw == BR) ? __ldg(rw + c0 + tid % BR) : 0;
-      // near terms: p_k -= sum_j L_{k+1+j, k}^T x_{k+1+j}
-      {
-        T u[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; q++) u[q] = 0.0;
-#pragma unroll
-        for (int jj = 0; jj < WALK_D; jj++) {
-          const int j = k + 1 + jj;
-          if (j >= nbs) continue;
-          const int sl = j % WALK_T;
-#pragma unroll 4
-          for (int i = i0; i < i0 + BR / 4; i++) {
-            const T l = tl[jj][i][col];
-            T xv[NQ];
-            ld_row8(xr[sl][i], xv);
-#pragma unroll
-            for (int q = 0; q < NQ; q++) u[q] += l * xv[q];
-          }
-        }
-        st_row8(red[iq][col], u);
-      }
-      nbar_sync<WB_COMPUTE, 256>();
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        const int q = 2 * iq + c;
-        pf[col][q] = pvb[buf][col][q] - (red[0][col][q] + red[1][col][q] + red[2][col][q] + red[3][col][q]);
-      }
-      nbar_sync<WB_COMPUTE, 256>();
-      walk_free_arrive(buf);   // the partial buffer of this step is free
-      // x_k = L_kk^-T p_k (the inverse is lower triangular)
-      {
-        T u[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; q++) u[q] = 0.0;
-#pragma unroll
-        for (int ii = 0; ii < BR / 4; ii++) {
-          const int i = i0 + ii;
-          const bool ok = i >= col && i < bw;
-          const T d = tl[WALK_D][i][col];
-          T pv8[NQ];
-          ld_row8(pf[i], pv8);
-#pragma unroll
-          for (int q = 0; q < NQ; q++) u[q] += ok ? d * pv8[q] : T(0);
-        }
-        st_row8(red[iq][col], u);
-      }
-      nbar_sync<WB_COMPUTE, 256>();
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        const int q = 2 * iq + c;
-        xr[slot][col][q] = (col < bw) ? red[0][col][q] + red[1][col][q] + red[2][col][q] + red[3][col][q] : T(0);
-      }
-      nbar_sync<WB_COMPUTE, 256>();
-      {
-        unsigned long long* dst = yp + (size_t) k * WALK_PAIRS;
-#pragma unroll
-        for (int u = 0; u < WALK_PAIRS / 256; u++) {
-          const int e = tid + 256 * u;
-          put_pair(dst + e, tag, xr[slot][e / NQ][e % NQ]);
-        }
-      }
-      for (int e = tid; e < bw * nrhs; e += 256) {
-        const int c = e % bw, q = e / bw;
-        const T v = xr[slot][c][q];
-        Wf[c0 + c + (size_t) q * f] = v;
-        X[(bw == BR ? gx : rw[c0 + c]) + (size_t) q * ldx] = v;
-      }
-      if (tid == 0) flags[F.blk_off + k] = epoch;
-      // every read of this step's tiles is done before they are replaced
-      nbar_sync<WB_COMPUTE, 256>();
-      if (k > 0) put();
-    }
-    return;
-  }
-  // ------------------------------------------------------------------ helper
-  // (the loader warp's threads only keep the barriers here)
-  const bool act = tid < 256;
-  const int2_ bk = blocks[blockIdx.x - nwalk];
-  const FrontDesc F = fronts[bk.a];
-  const int k = bk.b, f = F.f, s = F.s;
-  const int nbs = (s + BR - 1) / BR;
-  const int c0 = k * BR, bw = min(BR, s - c0);
-  const T* P = L + F.l_off;
-  const T* Wf = W + F.v_off * WS;
-  T (*red)[BR][NQ] = reinterpret_cast<T (*)[BR][NQ]>(wsm);            // [4]
-  T (*ysb)[BR][NQ] = reinterpret_cast<T (*)[BR][NQ]>(wsm) + 4;         // [WALK_HB]
-  const int jlo = k + WALK_D + 1;   // far blocks j = nbs-1 .. jlo
-  const unsigned long long* yp = ypairs + (size_t) F.blk_off * WALK_PAIRS;
-  // the walker's tiles of this block into L2: the near blocks' 64-row
-  // column pieces of block column k (two 128-byte lines each, the second
-  // while it holds rows of the near block) and the block's inverse
-  {
-    const int ncol = WALK_D * BR, dlines = (int) (BR * BR * sizeof(T) / 128);
-    const T* Di = Dinv + F.dinv_off + (size_t) k * BR * BR;
-    for (int e = tid; e < 2 * ncol + dlines; e += WALK_THREADS) {
-      if (e < 2 * ncol) {
-        const int c = e >> 1, half = e & 1, j = k + 1 + c / BR;
-        const int rows_j = j < nbs ? min(BR, s - j * BR) : 0;
-        if (c % BR < bw && (half == 0 ? rows_j > 0 : rows_j > 128 / (int) sizeof(T)))
-          prefetch_l2(P + (size_t) j * BR + half * (128 / (int) sizeof(T)) + (size_t) (c0 + c % BR) * f);
-      } else {
-        prefetch_l2(reinterpret_cast<const unsigned char*>(Di) + (size_t) (e - 2 * ncol) * 128);
-      }
-    }
-  }
-  // v_k = y_k - L21^T x2, the chunk partial sums added in chunk order
-  for (int e = tid; e < BR * NQ; e += WALK_THREADS) {
-    const int c = e % BR, q = e / BR;
-    T v = 0.0;
-    if (c < bw && q < nrhs) {
-      v = Wf[c0 + c + (size_t) q * f];
-      T acc = 0.0;
-#pragma unroll 4
-      for (int ch = 0; ch < F.nchunk; ch++)
-        acc += __ldcg(part + F.part_off + ((size_t) ch * s + c0 + c) * SOLVE_NRHS + q);
-      v -= acc;
-    }
-    hpv[c][q] = v;
-  }
-  // far terms: blocks j = nbs-1 down to jlo (block t of the helper's order
-  // is j = nbs-1-t); rows past the block's last column are zero in the pairs
-  T acc[NQ];
-#pragma unroll
-  for (int q = 0; q < NQ; q++) acc[q] = 0.0;
-  walk_far_terms<NQ>(
-      tag, status, max(nbs - jlo, 0),
-      [&](int t, int tt) -> T {
-        const int j = nbs - 1 - t, i = qg * (BR / 4) + tt;
-        return (col < bw && i < min(BR, s - j * BR)) ? __ldg(P + (size_t) (c0 + col) * f + j * BR + i) : T(0);
-      },
-      [&](int t) { return yp + (size_t) (nbs - 1 - t) * WALK_PAIRS; }, ysb, acc, qg, act);
-  if (act) {
-#pragma unroll
-    for (int q = 0; q < NQ; q++) red[qg][col][q] = acc[q];
-  }
-  __syncthreads();
-  unsigned long long* dst = ppairs + (size_t) (F.blk_off + k) * WALK_PAIRS;
-  for (int e = tid; e < WALK_PAIRS; e += WALK_THREADS) {
-    const int c = e / NQ, q = e % NQ;
-    put_pair(dst + e, tag, hpv[c][q] - (red[0][c][q] + red[1][c][q] + red[2][c][q] + red[3][c][q]));
-  }
-}
-
 // the start of a pass: the first nfl chain flags cleared (with them the
 // persistent set's done flags), the persistent queues' pending counts and
 // heads, and the walks' call counter advanced when there is one
@@ -1836,16 +1607,30 @@ static double solve_pass_bytes(const FrontDesc& F, int nrhs, double esz) {
   return esz * (s * (s + 1.0) / 2.0 + m * s) + 4.0 * F.f + 2.0 * esz * nrhs * F.f;
 }
 
-// the forward and backward walks on levels with long chains of FP32
-// factors (TAUCS_B200_NO_SOLVE_WALK=1 selects the flag-chained kernels
-// instead; FP64 keeps them: the walker's staged FP64 tiles take 164
-// registers, one CTA per SM, too few resident helpers)
+// TAUCS_B200_NO_SOLVE_WALK=1 selects the flag-chained block kernels on every
+// level instead of the cluster chains
 static bool walk_enabled() {
   static const bool on = [] {
     const char* e = getenv("TAUCS_B200_NO_SOLVE_WALK");
     return !(e && *e && strcmp(e, "0") != 0);
   }();
   return on;
+}
+
+// the columns of the instantiation that a pass of nq right-hand sides takes
+template <typename F>
+static void sf_dispatch(int nq, F run) {
+  if (nq <= 1) run(std::integral_constant<int, 1>());
+  else if (nq <= 4) run(std::integral_constant<int, 4>());
+  else run(std::integral_constant<int, SOLVE_NRHS>());
+}
+
+// the same for the chains: FP64 has no four-column form (DMMA takes eight)
+template <typename T, typename F>
+static void chain_dispatch(int nq, F run) {
+  if (nq <= 1) run(std::integral_constant<int, 1>());
+  else if (nq <= 4 && sizeof(T) == 4) run(std::integral_constant<int, sizeof(T) == 4 ? 4 : SOLVE_NRHS>());
+  else run(std::integral_constant<int, SOLVE_NRHS>());
 }
 
 template <typename T>
@@ -1855,18 +1640,19 @@ static void solve_attrs() {
   per_device_once(pd, [] {
     // static + dynamic shared memory of these kernels can exceed the default
     // 48 KB (8 columns in FP64)
-    cudaFuncSetAttribute(k_fwd_big<T, 2, SOLVE_NRHS, FWD_ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T, FWD_ALL>());
-    cudaFuncSetAttribute(k_fwd_big<T, 4, SOLVE_NRHS, FWD_ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T, FWD_ALL>());
-    cudaFuncSetAttribute(k_fwd_big<T, 8, SOLVE_NRHS, FWD_ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T, FWD_ALL>());
-    cudaFuncSetAttribute(k_fwd_big<T, 1, 1, FWD_ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T, FWD_ALL>());
-    cudaFuncSetAttribute(k_fwd_big<T, 2, SOLVE_NRHS, FWD_CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T, FWD_CHAIN>());
-    cudaFuncSetAttribute(k_fwd_big<T, 4, SOLVE_NRHS, FWD_CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T, FWD_CHAIN>());
-    cudaFuncSetAttribute(k_fwd_big<T, 8, SOLVE_NRHS, FWD_CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T, FWD_CHAIN>());
-    cudaFuncSetAttribute(k_bwd_big<T, 2, SOLVE_NRHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 2>());
-    cudaFuncSetAttribute(k_bwd_big<T, 4, SOLVE_NRHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 4>());
-    cudaFuncSetAttribute(k_bwd_big<T, 8, SOLVE_NRHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 8>());
-    cudaFuncSetAttribute(k_bwd_big<T, 1, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 1>());
-    cudaFuncSetAttribute(k_bwd_big<T, 8, SOLVE_NRHS, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 8>());
+    auto big = [](auto nqc) {
+      constexpr int Q = decltype(nqc)::value;
+      cudaFuncSetAttribute(k_fwd_big<T, Q, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T>());
+      cudaFuncSetAttribute(k_bwd_big<T, Q, SOLVE_NRHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int) bwd_smem<T, Q>());
+    };
+    big(std::integral_constant<int, 2>());
+    big(std::integral_constant<int, 4>());
+    big(std::integral_constant<int, SOLVE_NRHS>());
+    if constexpr (std::is_same<T, double>::value) {
+      cudaFuncSetAttribute(k_fwd_big<T, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T>());
+      cudaFuncSetAttribute(k_bwd_big<T, 1, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 1>());
+    }
     auto sf = [](auto nqc) {
       constexpr int Q = decltype(nqc)::value;
       // the most any launch asks for: 8 warps of fronts of order <= 32, or 4
@@ -1878,6 +1664,14 @@ static void solve_attrs() {
       cudaFuncSetAttribute(k_fwd<T, Q, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) most);
       cudaFuncSetAttribute(k_bwd<T, Q, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) most);
     };
+    auto chain = [](auto nqc) {
+      constexpr int Q = decltype(nqc)::value;
+      cudaFuncSetAttribute(k_chain<T, Q, SOLVE_NRHS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int) chain_smem<T, Q>());
+      cudaFuncSetAttribute(k_chain<T, Q, SOLVE_NRHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int) chain_smem<T, Q>());
+    };
+    for (int nq : {1, 4, 8}) chain_dispatch<T>(nq, chain);
     sf(std::integral_constant<int, 1>());
     sf(std::integral_constant<int, 4>());
     sf(std::integral_constant<int, SOLVE_NRHS>());
@@ -1885,12 +1679,6 @@ static void solve_attrs() {
       const int most = (int) (4 * sf_warp_smem<T, 1>(SOLVE_SLOT_BYTES / sizeof(T), SMALL_F_MAX));
       cudaFuncSetAttribute(k_fwd<T, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
       cudaFuncSetAttribute(k_bwd<T, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    }
-    if constexpr (std::is_same<T, float>::value) {
-      cudaFuncSetAttribute(k_fwd_walk<T, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int) walk_smem<T>());
-      cudaFuncSetAttribute(k_bwd_walk<T, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int) bwalk_smem<T>());
     }
     return true;
   });
@@ -1928,31 +1716,21 @@ static void sf_part(const Plan& P, int np, int part, int* t0, int* t1, int* thre
   *threads = part ? 128 : 256;
 }
 
-// the columns of the instantiation that a pass of nq right-hand sides takes
-template <typename F>
-static void sf_dispatch(int nq, F run) {
-  if (nq <= 1) run(std::integral_constant<int, 1>());
-  else if (nq <= 4) run(std::integral_constant<int, 4>());
-  else run(std::integral_constant<int, SOLVE_NRHS>());
-}
-
 template <typename T>
 static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Dinv, int nrhs, T* X, const T* B, int ld, T* W,
                         T* part, int* flags, int* epoch, int* status, cudaStream_t st) {
   solve_attrs<T>();
-  // the walks: their tagged pairs, and the call counter in the word after
-  // the cleared ones, advanced on the device once per call
+  // the chains' published values, and their call counter in the word after the
+  // cleared flags, advanced on the device once per call
   int* counter = flags + solve_flag_words(P);
-  unsigned long long* ypairs = reinterpret_cast<unsigned long long*>(part + P.fpart_off);
-  unsigned long long* ppairs = ypairs + (size_t) P.n_blk * WALK_PAIRS;
-  // the forward walk pays off on chains of 32 blocks or more, the backward
-  // one from 8 (both measured on the 80^3 lognormal system)
-  auto walk_level = [&](const LevelPlan& LP, bool fwd) {
-    return std::is_same<T, float>::value && walk_enabled() && LP.max_s_big >= (fwd ? FWD_CHAIN_MIN_S : BWD_WALK_MIN_S) &&
-           (int) LP.big_fronts.size() <= WALK_MAX_FRONTS && LP.max_s_big < 4095 * BR;
+  unsigned long long* zpub = reinterpret_cast<unsigned long long*>(part + P.fpart_off);
+  unsigned long long* ppub = zpub + (size_t) P.n_blk * CH_VALUES * ch_words<T>();
+  auto chain_level = [&](const LevelPlan& LP) {
+    return walk_enabled() && LP.max_s_big >= CHAIN_MIN_S && (int) LP.big_fronts.size() <= chain_max_fronts<T>();
   };
+  auto chain_grid = [](int nbig, int nblocks) { return nbig * CH_C + (nblocks + CH_C - 1) / CH_C * CH_C; };
   bool walks = false;
-  for (const LevelPlan& LP : P.levels) walks = walks || walk_level(LP, true) || walk_level(LP, false);
+  for (const LevelPlan& LP : P.levels) walks = walks || chain_level(LP);
   const int np = D.n_pers;
   // the handshake flags restart from zero on every call, so the epochs of a
   // call are always 1, 2, ... and a recorded launch sequence stays valid; one
@@ -1975,9 +1753,9 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
     const int ef = ++ep;
     reset(q0 == 0);
     // every small front with only small fronts below it, a launch per part
-    for (int part = 0; part < 2; part++) {
+    for (int pt = 0; pt < 2; pt++) {
       int t0, t1, th;
-      sf_part(P, np, part, &t0, &t1, &th);
+      sf_part(P, np, pt, &t0, &t1, &th);
       if (t1 <= t0) continue;
       double by = 0.0;
       if (prof_enabled())
@@ -1985,11 +1763,11 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       prof_begin(KC_SOLVE_FWD, st);
       sf_dispatch(nq, [&](auto nqc) {
         constexpr int Q = decltype(nqc)::value;
-        const int slot = sf_slot<T>(P.pers_slot[part]), wld = P.pers_wld[part], nw = th / 32;
+        const int slot = sf_slot<T>(P.pers_slot[pt]), wld = P.pers_wld[pt], nw = th / 32;
         const size_t smem = nw * sf_warp_smem<T, Q>(slot, wld);
         const int grid = std::min((t1 - t0 + nw - 1) / nw, sf_resident(k_fwd_pers<T, Q, SOLVE_NRHS>, th, smem));
         k_fwd_pers<T, Q, SOLVE_NRHS><<<grid, th, smem, st>>>(D.solve_tasks, t0, t1, D.pers_solve,
-                                                             D.pers_solve + 2 * np + part, D.child_rec, D.maps, D.rows,
+                                                             D.pers_solve + 2 * np + pt, D.child_rec, D.maps, D.rows,
                                                              L, Bq, ld, W, nq, status, slot, wld);
       });
       prof_end(KC_SOLVE_FWD, st, 0.0, by);
@@ -2011,37 +1789,27 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       const int nb = (int) LP.solve_fwd_blocks.size();
       if (nb > 0) {
         const int2_ *bl = D.sfwd + D.sfwd_off[h], *bc = D.sfwd_ch + D.sfwd_off[h];
-        const int nd = LP.n_fwd_diag, nu = nb - nd;
-        // one right-hand side runs the two-column variant, measured faster
-        // than a one-column instantiation (columns >= nrhs are skipped)
-        auto run = [&](auto nqc) {
-          constexpr int Q = decltype(nqc)::value;
-          if (walk_level(LP, true)) {
-            const int nbig = (int) LP.big_fronts.size();
-            if constexpr (std::is_same<T, float>::value)
-              k_fwd_walk<T, SOLVE_NRHS><<<nbig + nd, WALK_THREADS, walk_smem<T>(), st>>>(
-                  D.big_list + D.big_off[h], nbig, bl, bc, D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, Bq, ld, W, ypairs,
-                  ppairs, nq, flags, counter, ef, status);
-            if (nu)
-              k_fwd_big<T, Q, SOLVE_NRHS, FWD_UPD><<<nu, 128, 0, st>>>(bl + nd, bc + nd, D.blk_child, D.fronts, D.maps, D.rows,
-                                                                      L, Dinv, Bq, ld, W, nq, flags, ef, status);
-            count_launch(nu ? 2 : 1);
-          } else if (LP.max_s_big >= FWD_CHAIN_MIN_S) {
-            k_fwd_big<T, Q, SOLVE_NRHS, FWD_CHAIN><<<nd, 128, fwd_smem<T, FWD_CHAIN>(), st>>>(
-                bl, bc, D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, Bq, ld, W, nq, flags, ef, status);
-            if (nu)
-              k_fwd_big<T, Q, SOLVE_NRHS, FWD_UPD><<<nu, 128, 0, st>>>(bl + nd, bc + nd, D.blk_child, D.fronts, D.maps, D.rows,
-                                                                      L, Dinv, Bq, ld, W, nq, flags, ef, status);
-            count_launch(nu ? 2 : 1);
-          } else {
-            k_fwd_big<T, Q, SOLVE_NRHS, FWD_ALL><<<nb, 128, fwd_smem<T, FWD_ALL>(), st>>>(
-                bl, bc, D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, Bq, ld, W, nq, flags, ef, status);
-            count_launch();
-          }
-        };
-        if (nq <= 2) run(std::integral_constant<int, 2>());
-        else if (nq <= 4) run(std::integral_constant<int, 4>());
-        else run(std::integral_constant<int, 8>());
+        if (chain_level(LP)) {
+          const int nbig = (int) LP.big_fronts.size();
+          chain_dispatch<T>(nq, [&](auto nqc) {
+            constexpr int Q = decltype(nqc)::value;
+            k_chain<T, Q, SOLVE_NRHS, false><<<chain_grid(nbig, nb), CH_THREADS, chain_smem<T, Q>(), st>>>(
+                D.big_list + D.big_off[h], nbig, bl, nb, bc, D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, Bq, Xq, ld, W,
+                part, zpub, ppub, nq, counter, ef, status);
+          });
+        } else {
+          // one right-hand side runs the two-column variant, measured faster
+          // than a one-column instantiation (columns >= nrhs are skipped)
+          auto run = [&](auto nqc) {
+            constexpr int Q = decltype(nqc)::value;
+            k_fwd_big<T, Q, SOLVE_NRHS><<<nb, 128, fwd_smem<T>(), st>>>(bl, bc, D.blk_child, D.fronts, D.maps, D.rows, L,
+                                                                        Dinv, Bq, ld, W, nq, flags, ef, status);
+          };
+          if (nq <= 2) run(std::integral_constant<int, 2>());
+          else if (nq <= 4) run(std::integral_constant<int, 4>());
+          else run(std::integral_constant<int, 8>());
+        }
+        count_launch();
       }
       prof_end(KC_SOLVE_FWD, st, 0.0, by);
     }
@@ -2054,33 +1822,39 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       prof_begin(KC_SOLVE_BWD, st);
       const int nb = (int) LP.solve_bwd_blocks.size();
       if (nb > 0) {
-        k_gather_upd<T, SOLVE_NRHS><<<(int) LP.solve_fwd_blocks.size(), 128, 0, st>>>(D.sfwd + D.sfwd_off[h], D.fronts, D.rows,
-                                                                        Xq, ld, W, nq);
-        count_launch();
-        const int nt = (int) LP.solve_l21_tasks.size();
-        const int2_* tl = D.sl21 + D.sl21_off[h];
+        // chains take all their L21^T x2 from k_bwd_l21, the block kernel
+        // that of fronts with more than one chunk of update rows
+        const bool chain = chain_level(LP);
+        const int nt = chain ? (int) LP.solve_l21_tasks.size() : LP.n_l21_multi;
+        const int2_ *tl = D.sl21 + D.sl21_off[h], *bl = D.sbwd + D.sbwd_off[h];
         if (nt > 0) {
-          if (nq <= 2) k_bwd_l21<T, 2, SOLVE_NRHS><<<nt, 128, 0, st>>>(tl, D.fronts, L, W, part, nq);
-          else if (nq <= 4) k_bwd_l21<T, 4, SOLVE_NRHS><<<nt, 128, 0, st>>>(tl, D.fronts, L, W, part, nq);
-          else k_bwd_l21<T, 8, SOLVE_NRHS><<<nt, 128, 0, st>>>(tl, D.fronts, L, W, part, nq);
+          auto run = [&](auto nqc) {
+            constexpr int Q = decltype(nqc)::value;
+            k_bwd_l21<T, Q><<<nt, 128, 0, st>>>(tl, D.fronts, D.rows, L, Xq, ld, part, nq);
+          };
+          if (nq <= 2) run(std::integral_constant<int, 2>());
+          else if (nq <= 4) run(std::integral_constant<int, 4>());
+          else run(std::integral_constant<int, 8>());
           count_launch();
         }
-        const int2_* bl = D.sbwd + D.sbwd_off[h];
-        if (walk_level(LP, false)) {
+        if (chain) {
           const int nbig = (int) LP.big_fronts.size();
-          if constexpr (std::is_same<T, float>::value)
-            k_bwd_walk<T, SOLVE_NRHS><<<nbig + nb, WALK_THREADS, bwalk_smem<T>(), st>>>(
-                D.big_list + D.big_off[h], nbig, bl, D.fronts, D.rows, L, Dinv, Xq, ld, W, part, ypairs, ppairs, nq,
-                flags, counter, eb, status);
-        } else if (nq <= 2)
-          k_bwd_big<T, 2, SOLVE_NRHS, true><<<nb, 128, bwd_smem<T, 2>(), st>>>(bl, D.fronts, D.rows, L, Dinv, Xq, ld, W, part, nq, flags, eb, status);
-        else if (nq <= 4)
-          k_bwd_big<T, 4, SOLVE_NRHS, true><<<nb, 128, bwd_smem<T, 4>(), st>>>(bl, D.fronts, D.rows, L, Dinv, Xq, ld, W, part, nq, flags, eb, status);
-        else if (LP.max_s_big >= FWD_CHAIN_MIN_S)
-          // long chains: the barrier-free warp loop (every block's iterations are on the chain)
-          k_bwd_big<T, 8, SOLVE_NRHS, true, true><<<nb, 128, bwd_smem<T, 8>(), st>>>(bl, D.fronts, D.rows, L, Dinv, Xq, ld, W, part, nq, flags, eb, status);
-        else
-          k_bwd_big<T, 8, SOLVE_NRHS, true><<<nb, 128, bwd_smem<T, 8>(), st>>>(bl, D.fronts, D.rows, L, Dinv, Xq, ld, W, part, nq, flags, eb, status);
+          chain_dispatch<T>(nq, [&](auto nqc) {
+            constexpr int Q = decltype(nqc)::value;
+            k_chain<T, Q, SOLVE_NRHS, true><<<chain_grid(nbig, nb), CH_THREADS, chain_smem<T, Q>(), st>>>(
+                D.big_list + D.big_off[h], nbig, bl, nb, nullptr, nullptr, D.fronts, D.maps, D.rows, L, Dinv, nullptr, Xq,
+                ld, W, part, zpub, ppub, nq, counter, eb, status);
+          });
+        } else {
+          auto run = [&](auto nqc) {
+            constexpr int Q = decltype(nqc)::value;
+            k_bwd_big<T, Q, SOLVE_NRHS, true><<<nb, 128, bwd_smem<T, Q>(), st>>>(bl, D.fronts, D.rows, L, Dinv, Xq, ld, W,
+                                                                                 part, nq, flags, eb, status);
+          };
+          if (nq <= 2) run(std::integral_constant<int, 2>());
+          else if (nq <= 4) run(std::integral_constant<int, 4>());
+          else run(std::integral_constant<int, 8>());
+        }
         count_launch();
       }
       small_list(h, nq, [&](auto nqc, const int* sl, int ns) {
@@ -2092,9 +1866,9 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       });
       prof_end(KC_SOLVE_BWD, st, 0.0, by);
     }
-    for (int part = 1; part >= 0; part--) {
+    for (int pt = 1; pt >= 0; pt--) {
       int t0, t1, th;
-      sf_part(P, np, part, &t0, &t1, &th);
+      sf_part(P, np, pt, &t0, &t1, &th);
       if (t1 <= t0) continue;
       double by = 0.0;
       if (prof_enabled())
@@ -2102,11 +1876,11 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       prof_begin(KC_SOLVE_BWD, st);
       sf_dispatch(nq, [&](auto nqc) {
         constexpr int Q = decltype(nqc)::value;
-        const int slot = sf_slot<T>(P.pers_slot[part]), wld = P.pers_wld[part], nw = th / 32;
+        const int slot = sf_slot<T>(P.pers_slot[pt]), wld = P.pers_wld[pt], nw = th / 32;
         const size_t smem = nw * sf_warp_smem<T, Q>(slot, wld);
         const int grid = std::min((t1 - t0 + nw - 1) / nw, sf_resident(k_bwd_pers<T, Q, SOLVE_NRHS>, th, smem));
         k_bwd_pers<T, Q, SOLVE_NRHS><<<grid, th, smem, st>>>(D.solve_tasks, t0, t1, D.pers_solve + np,
-                                                             D.pers_solve + 2 * np + 2 + part, eb, D.rows, L, Xq, ld, W,
+                                                             D.pers_solve + 2 * np + 2 + pt, eb, D.rows, L, Xq, ld, W,
                                                              nq, status, slot, wld);
       });
       prof_end(KC_SOLVE_BWD, st, 0.0, by);
@@ -2199,7 +1973,7 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
     }
     const int nb = (int) LP.solve_fwd_blocks.size();
     if (nb > 0) {
-      k_fwd_big<double, 1, 1, FWD_ALL><<<nb, 128, fwd_smem<double, FWD_ALL>(), st>>>(
+      k_fwd_big<double, 1, 1><<<nb, 128, fwd_smem<double>(), st>>>(
           D.sfwd + D.sfwd_off[h], D.sfwd_ch + D.sfwd_off[h], D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, B, ld, W, 1,
           flags, ef, status);
       count_launch();
@@ -2210,9 +1984,6 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
     const LevelPlan& LP = P.levels[h];
     const int nb = (int) LP.solve_bwd_blocks.size();
     if (nb > 0) {
-      k_gather_upd<double, 1><<<(int) LP.solve_fwd_blocks.size(), 128, 0, st>>>(D.sfwd + D.sfwd_off[h], D.fronts, D.rows,
-                                                                         X, ld, W, 1);
-      count_launch();
       k_bwd_big<double, 1, 1, false><<<nb, 128, bwd_smem<double, 1>(), st>>>(D.sbwd + D.sbwd_off[h], D.fronts, D.rows, L, Dinv, X, ld, W, nullptr, 1,
                                                  flags, eb, status);
       count_launch();

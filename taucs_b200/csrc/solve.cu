@@ -1298,18 +1298,28 @@ k_chain(const int* __restrict__ walk_fronts, int nwalk, const int2_* __restrict_
 }
 
 // Backward solve, L21^T x2 over a 64-column block and a chunk of 512 update
-// rows by a CTA of 128 threads.  The chunk of x2 is gathered into shared
-// memory once ([column][row], conflict-free across lanes); each warp takes its
-// 16 columns of the block G = 32 / NQ at a time, so that the G x NQ = 32 sums
-// of a pass finish with one warp reduce-scatter (31 shuffles; lane t ends with
-// sum t = column t / NQ, right-hand side t % NQ), which sink(column, right-hand
-// side, sum) takes.  zs may be reused after the caller's next barrier.
-template <typename T, int NQ, typename Sink>
+// rows by a CTA of NTH threads.  The chunk of x2 is gathered into shared
+// memory once ([column][row], conflict-free across lanes).  A warp takes G = 32
+// / NQ columns (16 with one right-hand side) over one of RP row parts, 16
+// loads of the panel in flight a lane, so that the G x NQ sums of a pass
+// finish with one warp reduce-scatter (31 shuffles; lane t ends with sum t =
+// column t / NQ, right-hand side t % NQ).  A round of loads is a memory
+// latency, which is what bounds a small launch: 4 warps take 16 rounds for a
+// chunk (40 us, FP64, one right-hand side, from 72 to 394 CTAs), 16 warps 4.
+// sink(column, right-hand side, row part, sum) takes the sums.
+template <int NQ, int NTH>
+struct L21Split {
+  static constexpr int G = NQ >= 2 ? 32 / NQ : 16, SUMS = G * NQ, NW = NTH / 32;
+  static constexpr int CG = BR / G;                        // column groups
+  static constexpr int RP = NW >= CG ? NW / CG : 1;        // row parts
+  static_assert((SUMS == 32 || SUMS == 16) && G <= 16, "a pass holds 32 (one right-hand side: 16) sums");
+};
+template <typename T, int NQ, int NTH, typename Sink>
 __device__ __forceinline__ void l21_chunk(const FrontDesc& F, const T* __restrict__ L, const int* __restrict__ rows,
                                           const T* X, int ldx, int k, int ch, int nrhs, T (*zs)[SOLVE_RCH],
                                           Sink sink) {
-  constexpr int G = NQ >= 2 ? 32 / NQ : 16, SUMS = G * NQ;
-  static_assert((SUMS == 32 || SUMS == 16) && G <= 16, "a pass holds 32 (one right-hand side: 16) sums");
+  using S = L21Split<NQ, NTH>;
+  constexpr int G = S::G, SUMS = S::SUMS, RP = S::RP;
   const int f = F.f, s = F.s, m = f - s;
   const int c0 = k * BR, bw = min(BR, s - c0);
   const int i0 = ch * SOLVE_RCH, nr = min(m - i0, SOLVE_RCH);
@@ -1317,12 +1327,12 @@ __device__ __forceinline__ void l21_chunk(const FrontDesc& F, const T* __restric
   const T* P = L + F.l_off + s + i0;
   // all of this thread's loads in flight before its first store
   {
-    constexpr int NI = SOLVE_RCH / 128;
+    constexpr int NI = SOLVE_RCH / NTH;
     const int* rw = rows + F.rows_off + s + i0;
     int g[NI];
     T zv[NQ][NI];
 #pragma unroll
-    for (int t = 0; t < NI; t++) g[t] = (int) threadIdx.x + 128 * t < nr ? __ldg(rw + threadIdx.x + 128 * t) : -1;
+    for (int t = 0; t < NI; t++) g[t] = (int) threadIdx.x + NTH * t < nr ? __ldg(rw + threadIdx.x + NTH * t) : -1;
 #pragma unroll
     for (int q = 0; q < NQ; q++)
 #pragma unroll
@@ -1330,18 +1340,16 @@ __device__ __forceinline__ void l21_chunk(const FrontDesc& F, const T* __restric
 #pragma unroll
     for (int q = 0; q < NQ; q++)
 #pragma unroll
-      for (int t = 0; t < NI; t++) zs[q][threadIdx.x + 128 * t] = zv[q][t];
+      for (int t = 0; t < NI; t++) zs[q][threadIdx.x + NTH * t] = zv[q][t];
   }
   __syncthreads();
-  for (int cg = warp * 16; cg < warp * 16 + 16; cg += G) {
-    if (cg >= bw) break;
+  const int part = warp / S::CG % RP;
+  for (int cg = warp % S::CG * G; cg < bw; cg += S::NW >= S::CG ? BR : S::NW * G) {
     T v[SUMS];   // v[a * NQ + q]: column cg + a, right-hand side q
 #pragma unroll
     for (int j = 0; j < SUMS; j++) v[j] = T(0);
-    // RU rows per lane per round, 16 loads of the panel in flight at once
-    // (one round per memory latency)
-    constexpr int RU = G >= 16 ? 1 : 16 / G;
-    for (int i1 = lane; i1 < nr; i1 += 32 * RU) {
+    constexpr int RU = G >= 16 ? 1 : 16 / G;   // rows per lane per round
+    for (int i1 = lane + 32 * RU * part; i1 < nr; i1 += 32 * RU * RP) {
       T lv[RU][G];
 #pragma unroll
       for (int u = 0; u < RU; u++)
@@ -1382,22 +1390,33 @@ __device__ __forceinline__ void l21_chunk(const FrontDesc& F, const T* __restric
     }
     const int t = SUMS == 32 ? lane : lane >> 1;
     const int a = t / NQ, q = t % NQ;
-    if (cg + a < bw && q < nrhs && (SUMS == 32 || (lane & 1) == 0)) sink(cg + a, q, v[0]);
+    if (cg + a < bw && q < nrhs && (SUMS == 32 || (lane & 1) == 0)) sink(cg + a, q, part, v[0]);
   }
 }
 
 // the sums of (column block, 512-row chunk) tasks, so that the whole GPU
 // streams L21; the chain and block kernels add them in chunk order
-template <typename T, int NQ>
-__global__ void __launch_bounds__(128)
+template <typename T, int NQ, int NTH>
+__global__ void __launch_bounds__(NTH)
 k_bwd_l21(const int2_* __restrict__ tasks, const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
           const T* __restrict__ L, const T* __restrict__ X, int ldx, T* __restrict__ part, int nrhs) {
+  constexpr int RP = L21Split<NQ, NTH>::RP;
   __shared__ T zs[NQ][SOLVE_RCH];
+  __shared__ T red[RP][BR][NQ];
   const int2_ tk = tasks[blockIdx.x];
   const FrontDesc F = fronts[tk.a];
   const int k = tk.b >> 16, ch = tk.b & 0xffff;
+  l21_chunk<T, NQ, NTH>(F, L, rows, X, ldx, k, ch, nrhs, zs, [&](int c, int q, int p, T v) { red[p][c][q] = v; });
+  __syncthreads();
   T* out = part + F.part_off + ((size_t) ch * F.s + k * BR) * SOLVE_NRHS;
-  l21_chunk<T, NQ>(F, L, rows, X, ldx, k, ch, nrhs, zs, [&](int c, int q, T v) { out[c * SOLVE_NRHS + q] = v; });
+  const int bw = min(BR, F.s - k * BR);
+  for (int e = threadIdx.x; e < bw * NQ; e += NTH) {
+    const int c = e / NQ, q = e % NQ;
+    T v = red[0][c][q];
+#pragma unroll
+    for (int p = 1; p < RP; p++) v += red[p][c][q];
+    if (q < nrhs) out[c * SOLVE_NRHS + q] = v;
+  }
 }
 
 // Backward solve of big fronts, one CTA per 64-column block, chained from the
@@ -1464,7 +1483,7 @@ k_bwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts
   } else {
     T (*zs)[SOLVE_RCH] = reinterpret_cast<T (*)[SOLVE_RCH]>(dgb + BR);
     for (int ch = 0; ch < F.nchunk; ch++) {
-      l21_chunk<T, NQ>(F, L, rows, X, ldx, k, ch, nrhs, zs, [&](int c, int q, T v) { xv[c][q] -= v; });
+      l21_chunk<T, NQ, 128>(F, L, rows, X, ldx, k, ch, nrhs, zs, [&](int c, int q, int, T v) { xv[c][q] -= v; });
       __syncthreads();
     }
   }
@@ -1828,13 +1847,16 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
         const int nt = chain ? (int) LP.solve_l21_tasks.size() : LP.n_l21_multi;
         const int2_ *tl = D.sl21 + D.sl21_off[h], *bl = D.sbwd + D.sbwd_off[h];
         if (nt > 0) {
-          auto run = [&](auto nqc) {
+          sf_dispatch(nq, [&](auto nqc) {
             constexpr int Q = decltype(nqc)::value;
-            k_bwd_l21<T, Q><<<nt, 128, 0, st>>>(tl, D.fronts, D.rows, L, Xq, ld, part, nq);
-          };
-          if (nq <= 2) run(std::integral_constant<int, 2>());
-          else if (nq <= 4) run(std::integral_constant<int, 4>());
-          else run(std::integral_constant<int, 8>());
+            // one CTA or less per SM: 16 warps each; the more CTAs, the
+            // fewer warps each, down to 4 (solve at 64^3, FP64, backward: 4
+            // warps always 1538 us, 16 always 1446, so 1380; mixed step at
+            // 80^3, backward: 6509, 7333, 6441)
+            if (nt <= 148) k_bwd_l21<T, Q, 512><<<nt, 512, 0, st>>>(tl, D.fronts, D.rows, L, Xq, ld, part, nq);
+            else if (nt <= 4 * 148) k_bwd_l21<T, Q, 256><<<nt, 256, 0, st>>>(tl, D.fronts, D.rows, L, Xq, ld, part, nq);
+            else k_bwd_l21<T, Q, 128><<<nt, 128, 0, st>>>(tl, D.fronts, D.rows, L, Xq, ld, part, nq);
+          });
           count_launch();
         }
         if (chain) {

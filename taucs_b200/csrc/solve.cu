@@ -15,6 +15,7 @@
 // update rows (written by ancestors in earlier launches), r = y - L21^T x2,
 // then the L11^T substitution, and scatter x at the columns.  Up to
 // SOLVE_NRHS right-hand sides share every read of L.
+#include <climits>
 #include <mutex>
 #include <type_traits>
 
@@ -440,21 +441,13 @@ k_bwd_pers(const SolveTask* __restrict__ tasks, int t0, int t1, int* done, int* 
 
 
 // ---------------------------------------------------------------- big fronts
-// One CTA per 64-row block.  Forward: block r waits for the solved blocks
-// k < r of L11 (flags, release/acquire), accumulates L[r,k] y_k, then solves
-// its own diagonal block and publishes y_r.  Backward: blocks run from the
-// last one; block k waits for x_j, j > k.  Waits are bounded: on timeout the
-// CTA records SOLVE_TIMEOUT in the status word and carries on, so no launch
-// can hang.
+// 64-row blocks.  Forward: block r needs the solved blocks k < r of L11,
+// accumulates L[r,k] y_k and applies the inverse of its diagonal block.
+// Backward: blocks run from the last one; block k needs x_j, j > k.  Waits are
+// bounded: on timeout a CTA records SOLVE_TIMEOUT in the status word and
+// carries on, so no launch can hang.
 
 constexpr int BR = PANEL_NB;   // rows per block
-// dynamic shared memory: L_kk^-1, then the gathered chunk of x2, or (8
-// columns) one staged 64x64 block of L11
-template <typename T, int NQ>
-constexpr size_t bwd_smem() {
-  return (BR * (BR + 1) + (NQ >= 8 ? BR * (BR + 1) : NQ * SOLVE_RCH)) * sizeof(T);
-}
-
 __device__ __forceinline__ void st_release(int* p, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -551,227 +544,11 @@ struct ChildGather {
   }
 };
 
-// Forward solve of big fronts, one launch over all blocks of a level (the
-// levels that do not run as chains below).  Diagonal block r of L11 gives
-// y_r = L_rr^-1 (w_r - sum_{k<r} L_rk y_k), handed on by release/acquire
-// flags; update rows i get w_i - sum_k L_ik y_k; a block waits for the blocks
-// k it needs one at a time.  In the last diagonal block rows >= s are update
-// rows of the same front.
-template <typename T>
-constexpr size_t fwd_smem() { return BR * (BR + 1) * sizeof(T); }
-
-template <typename T, int NQ, int WS>
-__global__ void __launch_bounds__(128)
-k_fwd_big(const int2_* __restrict__ blocks, const int2_* __restrict__ blk_ch, const int4* __restrict__ blk_child,
-          const FrontDesc* __restrict__ fronts, const int* __restrict__ maps, const int* __restrict__ rows,
-          const T* __restrict__ L, const T* __restrict__ Dinv, const T* __restrict__ B, int ldb,
-          T* __restrict__ W, int nrhs, int* __restrict__ flags, int epoch, int* status) {
-  __shared__ T wv[BR][NQ];
-  __shared__ T yk[BR][NQ];
-  __shared__ T part[BR][NQ];
-  __shared__ T ykw[4][BR / 2][NQ];   // per warp: the entries of y_k it needs
-  // dg[col][row] holds L_rr^-1 in rows < bw and the front's own update rows
-  // of L (last diagonal block) in rows >= bw
-  extern __shared__ __align__(16) unsigned char fsm[];
-  T (*dg)[BR + 1] = reinterpret_cast<T (*)[BR + 1]>(fsm);
-  const int2_ bk = blocks[blockIdx.x];
-  const FrontDesc F = fronts[bk.a];
-  const int r = bk.b, f = F.f, s = F.s;
-  const int nbs = (s + BR - 1) / BR;
-  const int r0 = r * BR, nr = min(BR, f - r0);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row = tid % BR, half = tid / BR;
-  T* Wf = W + F.v_off * WS;
-  const int* rw = rows + F.rows_off;
-  const T* P = L + F.l_off;
-  const bool diag = r < nbs;
-  const int bw = diag ? min(BR, s - r0) : 0;
-  const int2_ cr = blk_ch[blockIdx.x];
-  const int4* rec = blk_child + cr.a;
-  const int nch = cr.b - cr.a;
-  ChildGather<T, NQ, WS, 128> cg;
-  cg.load(rec, nch, maps, W, nrhs);
-
-  if (diag) {
-    // staged now, off the chain's critical path
-    const T* Di = Dinv + F.dinv_off + (size_t) r * BR * BR;
-    // 16 entries of each tile per thread in flight before they are stored
-#pragma unroll 1
-    for (int t0 = 0; t0 < BR * BR / 128; t0 += 16) {
-      T dv[16];
-#pragma unroll
-      for (int t = 0; t < 16; t++) {
-        const int e = tid + 128 * (t0 + t), i = e % BR, j = e / BR;
-        T v = 0.0;
-        if (j < bw && i < nr) v = (i < bw) ? (i >= j ? Di[i + j * BR] : T(0)) : P[(r0 + i) + (size_t) (r0 + j) * f];
-        dv[t] = v;
-      }
-#pragma unroll
-      for (int t = 0; t < 16; t++) {
-        const int e = tid + 128 * (t0 + t), i = e % BR, j = e / BR;
-        dg[j][i] = dv[t];
-      }
-    }
-  }
-  for (int k = tid; k < BR * NQ; k += 128) {
-    const int i = k % BR, q = k / BR;
-    wv[i][q] = (i < nr && q < nrhs && r0 + i < s) ? B[rw[r0 + i] + (size_t) q * ldb] : 0.0;
-  }
-  __syncthreads();
-  cg.add(rec, nch, maps, W, nrhs, r0, wv);
-  // contributions of the solved blocks k < kend; this thread's 32 entries of
-  // L[r, k] are loaded before waiting for y_k
-  T acc[NQ];
-#pragma unroll
-  for (int q = 0; q < NQ; q++) acc[q] = 0.0;
-  const int kend = diag ? r : nbs;
-  if constexpr (NQ >= 8) {
-    // 8 columns: y_k staged once for the whole block (measured faster than
-    // the warp-level loop below at 8 columns)
-    for (int k = 0; k < kend; k++) {
-      const int bwk = min(BR, s - k * BR);
-      T lv[BR / 2];
-      const T* pc = P + (r0 + row) + (size_t) (k * BR + half * (BR / 2)) * f;
-#pragma unroll
-      for (int j = 0; j < BR / 2; j++)
-        lv[j] = (row < nr && half * (BR / 2) + j < bwk) ? pc[(size_t) j * f] : 0.0;
-      wait_epoch(flags + F.blk_off + k, epoch, status);
-      for (int e = tid; e < BR * NQ; e += 128) {
-        const int j = e % BR, q = e / BR;
-        yk[j][q] = (j < bwk && q < nrhs) ? __ldcg(Wf + k * BR + j + (size_t) q * f) : 0.0;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int j = 0; j < BR / 2; j++)
-#pragma unroll
-        for (int q = 0; q < NQ; q++) acc[q] += lv[j] * yk[half * (BR / 2) + j][q];
-      __syncthreads();
-    }
-  } else {
-    // without block-wide barriers: each warp polls the flags itself and
-    // stages the 32 entries of y_k its rows need
-    T (*yw)[NQ] = ykw[warp];
-    for (int k = 0; k < kend; k++) {
-      const int bwk = min(BR, s - k * BR);
-      T lv[BR / 2];
-      const T* pc = P + (r0 + row) + (size_t) (k * BR + half * (BR / 2)) * f;
-  #pragma unroll
-      for (int j = 0; j < BR / 2; j++)
-        lv[j] = (row < nr && half * (BR / 2) + j < bwk) ? pc[(size_t) j * f] : 0.0;
-      poll_epoch(flags + F.blk_off + k, epoch, status);
-  #pragma unroll
-      for (int q = 0; q < NQ; q++) {
-        const int j = half * (BR / 2) + lane;
-        yw[lane][q] = (j < bwk && q < nrhs) ? __ldcg(Wf + k * BR + j + (size_t) q * f) : T(0);
-      }
-      __syncwarp();
-  #pragma unroll
-      for (int j = 0; j < BR / 2; j++)
-  #pragma unroll
-        for (int q = 0; q < NQ; q++) acc[q] += lv[j] * yw[j][q];
-      __syncwarp();
-    }
-  }
-  if (half == 1)
-#pragma unroll
-    for (int q = 0; q < NQ; q++) part[row][q] = acc[q];
-  __syncthreads();
-  if (half == 0)
-#pragma unroll
-    for (int q = 0; q < NQ; q++) wv[row][q] -= acc[q] + part[row][q];
-  __syncthreads();
-  if (!diag) {
-    for (int k = tid; k < nr * nrhs; k += 128) {
-      const int i = k % nr, q = k / nr;
-      Wf[r0 + i + (size_t) q * f] = wv[i][q];
-    }
-    return;
-  }
-  // c = L_rr^-1 w in rows < bw (into yk); update rows keep w
-  {
-    T y[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) y[q] = 0.0;
-#pragma unroll 8
-    for (int j = half * (BR / 2); j < half * (BR / 2) + BR / 2; j++) {
-      const T d = (row < bw) ? dg[j][row] : T(0);
-#pragma unroll
-      for (int q = 0; q < NQ; q++) y[q] += d * wv[j][q];
-    }
-    if (half == 1)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) part[row][q] = y[q];
-    __syncthreads();
-    if (half == 0)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) yk[row][q] = (row < bw) ? y[q] + part[row][q] : wv[row][q];
-    __syncthreads();
-  }
-  if (bw < nr) {
-    // update rows inside the last diagonal block: w_i -= L[i, r] y_r
-    T u[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) u[q] = 0.0;
-    if (row >= bw)
-      for (int j = half * (BR / 2); j < min(bw, half * (BR / 2) + BR / 2); j++) {
-        const T l = dg[j][row];
-#pragma unroll
-        for (int q = 0; q < NQ; q++) u[q] += l * yk[j][q];
-      }
-    if (half == 1)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) part[row][q] = u[q];
-    __syncthreads();
-    if (half == 0 && row >= bw)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) yk[row][q] -= u[q] + part[row][q];
-    __syncthreads();
-  }
-  for (int k = tid; k < nr * nrhs; k += 128) {
-    const int i = k % nr, q = k / nr;
-    Wf[r0 + i + (size_t) q * f] = yk[i][q];
-  }
-  __syncthreads();
-  // the barrier orders every thread's writes before thread 0's release store
-  if (tid == 0) st_release(flags + F.blk_off + r, epoch);
-}
-
-// Forward and backward solve of a level's big fronts as chains, for levels
-// with few fronts and several 64-row blocks each.  What bounds such a level
-// is the chain of its blocks -- z_t = D_t (p_t - sum_{u<t} A_tu z_u), D_t the
-// inverse of a diagonal block (forward: blocks first to last; backward: last
-// to first, transposed) -- so the chain runs inside one cluster of CH_C CTAs:
-// CTA t mod CH_C computes block t and writes z_t into the shared memory of
-// all of them (st.async, counted by the receivers' mbarriers), one to two
-// orders faster than a hand-over through global memory.  Between its turns a
-// CTA adds the terms of the last CH_C blocks to its next one as they arrive,
-// with the tiles of L loaded into registers two terms ahead and into L2 a
-// turn ahead: per step the chain waits for one 64x64 product, one product
-// with the inverse and one hand-over.  The far terms (u < t - CH_C) and the
-// right-hand side of block t are the work of a helper CTA per block, which
-// follows the published z_u and publishes p_t about CH_C steps ahead;
-// forward, the update rows' blocks are helpers too and stream L21 while the
-// chain runs.  Values published between CTAs travel as tagged words (tag in
-// the high half, 32 bits of the value in the low half; a double takes two),
-// each one relaxed 8-byte access: a reader knows a value is current when its
-// tag is, so nothing fences or polls a flag.  The tag is (call counter <<
-// 12) | epoch, the counter being advanced on the device at the start of every
-// solve call, so recorded launch sequences stay valid.  A ring of 2 CH_C z's
-// needs no release: block t's CTA has consumed z_{t-CH_C} .. z_{t-1}, so when
-// z_{u+2 CH_C} is produced every CTA is past its last use of z_u.  Walkers have
-// the lowest CTA indices and helper t waits only for blocks whose helpers
-// come before it, so in-order dispatch keeps every wait finite; the waits are
-// bounded all the same, and no CTA of a cluster leaves before every z has
-// arrived in its shared memory.  In the last diagonal block rows >= s are
-// update rows of the same front; its CTA finishes them too (forward).
-// Measured, per 64-row step of the root level's forward chain: FP64, one right-
-// hand side (64^3) 2.3 us with flags between CTAs, 1.2 us here; FP64, eight
-// (45x47x44) 4.7 -> 1.7 us; FP32, eight (56^3) 4.2 us with one walker CTA per
-// front, 2.0 us here.
 constexpr int CH_C = 8;                       // CTAs of a cluster, and the near distance
 constexpr int CH_RING = 2 * CH_C;
 constexpr int CH_THREADS = 256;
 constexpr int CH_VALUES = BR * SOLVE_NRHS;    // values per block and array of published words
+constexpr int DLD = BR + 4;                   // column stride of a staged inverse
 constexpr int CH_HB = 2;                      // blocks per round of a helper's far terms
 // levels with at least CHAIN_MIN_S columns in their largest big front and at
 // most CHAIN_MAX_FRONTS big fronts run as chains
@@ -901,11 +678,6 @@ __device__ __forceinline__ void fma2(float& a, float& b, float l, float x, float
       : "+f"(a), "+f"(b)
       : "f"(l), "f"(x), "f"(y));
 }
-__device__ __forceinline__ void fma2(double& a, double& b, double l, double x, double y) {
-  a += l * x;
-  b += l * y;
-}
-
 // A 64-row product by the CTA's eight warps, warp w the rows 8 w .. 8 w + 7.
 // Its cost is the bytes of z that the lanes take from shared memory (128 a
 // clock), so with several right-hand sides a lane covers R = 2 rows: lane
@@ -965,7 +737,7 @@ struct ChainRow {
         }
 #pragma unroll
         for (int h = 0; h < R; h++) {
-          if constexpr (sizeof(T) == 4 && NQ % 2 == 0) {
+          if constexpr (std::is_same<T, float>::value && NQ % 2 == 0) {
 #pragma unroll
             for (int q = 0; q < NQ; q += 2) fma2(acc[h * NQ + q], acc[h * NQ + q + 1], l[h * NT + t], x[q], x[q + 1]);
           } else {
@@ -1003,299 +775,6 @@ struct ChainRow {
     }
   }
 };
-
-// dynamic shared memory: the ring of z's and the vector of the inverse's
-// product (walker); a round's staged z's and the block's own vector (helper)
-template <typename T, int NQ>
-constexpr size_t chain_smem() { return (size_t) (CH_RING + 1) * BR * NQ * sizeof(T); }
-
-// zp, pp: published z's and p's; forward reads B and writes W, backward reads
-// W (y) and part (L21^T x2) and writes X
-template <typename T, int NQ, int WS, bool BWD>
-__global__ void __cluster_dims__(CH_C, 1, 1) __launch_bounds__(CH_THREADS, sizeof(T) == 4 ? 2 : 1)
-k_chain(const int* __restrict__ walk_fronts, int nwalk, const int2_* __restrict__ blocks, int nblocks,
-        const int2_* __restrict__ blk_ch, const int4* __restrict__ blk_child, const FrontDesc* __restrict__ fronts,
-        const int* __restrict__ maps, const int* __restrict__ rows, const T* __restrict__ L,
-        const T* __restrict__ Dinv, const T* __restrict__ B, T* __restrict__ X, int ldx, T* __restrict__ W,
-        const T* __restrict__ part, unsigned long long* __restrict__ zp, unsigned long long* __restrict__ pp, int nrhs,
-        const int* counter, int epoch, int* status) {
-  using Row = ChainRow<T, NQ>;
-  constexpr int QL = Row::QL, WPV = ch_words<T>();
-  extern __shared__ __align__(16) unsigned char chm[];
-  __shared__ __align__(8) unsigned long long bars[CH_RING];
-  __shared__ unsigned bad_s;
-  const int tid = threadIdx.x;
-  const int rho = Row::own(), qb = Row::qb(), jq = Row::jq();
-  const bool qact = Row::qact();
-  const unsigned tag = ((unsigned) *counter << 12) | (unsigned) epoch;
-  const bool walker = blockIdx.x < (unsigned) (nwalk * CH_C);
-  int2_ bk{0, 0};
-  if (walker) {
-    bk.a = walk_fronts[blockIdx.x / CH_C];
-  } else {
-    const int h = blockIdx.x - nwalk * CH_C;
-    if (h >= nblocks) return;
-    bk = blocks[h];
-  }
-  const FrontDesc F = fronts[bk.a];
-  const int f = F.f, s = F.s, nbs = (s + BR - 1) / BR;
-  const T* P = L + F.l_off;
-  T* Wf = W + F.v_off * WS;
-  const int* rw = rows + F.rows_off;
-  unsigned long long* zf = zp + (size_t) F.blk_off * CH_VALUES * WPV;
-  unsigned long long* pf = pp + (size_t) F.blk_off * CH_VALUES * WPV;
-  T* zs = reinterpret_cast<T*>(chm);              // [CH_RING][BR][NQ]
-  T (*vs)[NQ] = reinterpret_cast<T (*)[NQ]>(zs + CH_RING * BR * NQ);
-  // chain position t <-> block of the front
-  auto block_of = [&](int t) { return BWD ? nbs - 1 - t : t; };
-  // this lane's 16 entries of A_tu (block row bt: rows below s may belong to
-  // the update rows of the last diagonal block, or be an update block)
-  auto tile = [&](int bt, int bu, T (&l)[16]) {
-#pragma unroll
-    for (int h = 0; h < Row::R; h++) {
-      const int r = bt * BR + Row::row(h), c = bu * BR + jq;
-      const bool rv = r < (BWD ? s : f);
-      const T* a = BWD ? P + c + (size_t) r * f : P + r + (size_t) c * f;
-#pragma unroll
-      for (int t = 0; t < Row::NT; t++)
-        l[h * Row::NT + t] = (rv && c + Row::J * t < s) ? __ldg(a + (BWD ? Row::J * t : (size_t) (Row::J * t) * f)) : T(0);
-    }
-  };
-  // the right-hand side of block t, into vs (a barrier follows inside)
-  auto own_rhs = [&](int b, const int2_ cr) {
-    const int r0 = b * BR, nr = min(BR, f - r0);
-    if (!BWD) {
-      ChildGather<T, NQ, WS, CH_THREADS> cg;
-      cg.load(blk_child + cr.a, cr.b - cr.a, maps, W, nrhs);
-      for (int e = tid; e < BR * NQ; e += CH_THREADS) {
-        const int i = e % BR, q = e / BR;
-        vs[i][q] = (i < nr && q < nrhs && r0 + i < s) ? B[rw[r0 + i] + (size_t) q * ldx] : T(0);
-      }
-      __syncthreads();
-      cg.add(blk_child + cr.a, cr.b - cr.a, maps, W, nrhs, r0, vs);
-    } else {
-      for (int e = tid; e < BR * NQ; e += CH_THREADS) {
-        const int i = e % BR, q = e / BR;
-        T v = T(0);
-        if (r0 + i < s && q < nrhs) {
-          v = Wf[r0 + i + (size_t) q * f];
-          T acc = T(0);
-#pragma unroll 4
-          for (int ch = 0; ch < F.nchunk; ch++)
-            acc += part[F.part_off + ((size_t) ch * s + r0 + i) * SOLVE_NRHS + q];
-          v -= acc;
-        }
-        vs[i][q] = v;
-      }
-      __syncthreads();
-    }
-  };
-
-  if (walker) {
-    // ---------------------------------------------------------------- walker
-    const unsigned rank = blockIdx.x % CH_C;
-    constexpr unsigned ZBYTES = BR * NQ * sizeof(T);
-    if (tid == 0) {
-      for (int i = 0; i < CH_RING; i++)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bars[i])) : "memory");
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      for (int i = 0; i < min(CH_RING, nbs); i++) bar_expect(smem_addr(&bars[i]), ZBYTES);
-    }
-    __syncthreads();
-    cluster_sync_all();
-    // z_u has arrived (each CTA waits for every u once, in order); its
-    // barrier is armed for the z that takes the slot next
-    auto wait_z = [&](int u) {
-      bar_wait(smem_addr(&bars[u % CH_RING]), (u / CH_RING) & 1, status);
-      if (tid == 0 && u + CH_RING < nbs) bar_expect(smem_addr(&bars[u % CH_RING]), ZBYTES);
-    };
-    unsigned peer[CH_C];   // offsets of the others' shared memory, the next CTA of the chain first
-#pragma unroll
-    for (int r = 0; r < CH_C; r++) peer[r] = map_rank(smem_addr(bars), (rank + 1 + r) % CH_C) - smem_addr(bars);
-    for (int t = rank; t < nbs; t += CH_C) {
-      const int b = block_of(t), r0 = b * BR, nr = min(BR, f - r0), bw = min(BR, s - r0);
-      const T* Di = Dinv + F.dinv_off + (size_t) b * BR * BR;
-      const int u0 = max(0, t - CH_C);
-      T la[16], lb[16], xd[16];
-      if (u0 < t) tile(b, block_of(u0), la);
-      if (u0 + 1 < t) tile(b, block_of(u0 + 1), lb);
-#pragma unroll
-      for (int h = 0; h < Row::R; h++)
-#pragma unroll
-        for (int i = 0; i < Row::NT; i++) {
-          const int r = Row::row(h), c = Row::J * i + jq;
-          xd[h * Row::NT + i] = BWD ? Di[c + r * BR] : Di[r + c * BR];
-        }
-      // the next turn's tiles into L2
-      if (t + CH_C < nbs) {
-        const int bn = block_of(t + CH_C);
-        constexpr int LPC = BR * (int) sizeof(T) / 128 + 1;   // lines a 64-entry column piece touches
-        for (int e = tid; e < CH_C * BR * LPC; e += CH_THREADS) {
-          const int li = e % LPC, c = e / LPC;
-          const int bu = block_of(t + c / BR);
-          const int row = (BWD ? bu : bn) * BR + min(li * (128 / (int) sizeof(T)), BR - 1);
-          const int col = (BWD ? bn : bu) * BR + c % BR;
-          if (row < f && col < s) prefetch_l2(P + row + (size_t) col * f);
-        }
-        for (int e = tid; e < BR * BR * (int) sizeof(T) / 128; e += CH_THREADS)
-          prefetch_l2(reinterpret_cast<const unsigned char*>(Dinv + F.dinv_off + (size_t) bn * BR * BR) + 128 * e);
-      }
-      T pv[QL];
-      Row acc;
-      acc.clear();
-      Tagged<T> pt[QL];
-      const unsigned long long* pq = pf + ((size_t) b * CH_VALUES + rho * NQ + qb) * WPV;
-      auto load_p = [&]() {
-#pragma unroll
-        for (int q = 0; q < QL; q++) pt[q].load(pq + q * WPV);
-      };
-      if (t == 0) load_p();
-      for (int u = u0; u < t; u += 2) {
-        if (u + 2 >= t) load_p();
-        wait_z(u);
-        acc.add(la, zs + (u % CH_RING) * BR * NQ);
-        if (u + 2 < t) tile(b, block_of(u + 2), la);
-        if (u + 1 < t) {
-          wait_z(u + 1);
-          acc.add(lb, zs + ((u + 1) % CH_RING) * BR * NQ);
-          if (u + 3 < t) tile(b, block_of(u + 3), lb);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < QL; q++) {
-        wait_tagged<T>(pq + q * WPV, pt[q], true, tag, status);
-        pv[q] = pt[q].value();
-      }
-      T z[QL];
-      acc.sum(z);
-#pragma unroll
-      for (int q = 0; q < QL; q++) {
-        pv[q] -= z[q];
-        if (qact) vs[rho][qb + q] = pv[q];
-      }
-      __syncthreads();
-      acc.clear();
-      acc.add(xd, &vs[0][0]);
-      acc.sum(z);
-      if (!BWD && bw < nr) {
-        // the last diagonal block's update rows: w_i - L[i, block] y (the
-        // inverse is zero in their rows, so y is in place first)
-        __syncthreads();
-        if (qact && rho < bw)
-#pragma unroll
-          for (int q = 0; q < QL; q++) vs[rho][qb + q] = z[q];
-        __syncthreads();
-        tile(b, b, la);
-        acc.clear();
-        acc.add(la, &vs[0][0]);
-        T uq[QL];
-        acc.sum(uq);
-        if (rho >= bw)
-#pragma unroll
-          for (int q = 0; q < QL; q++) z[q] = pv[q] - uq[q];
-      }
-      // z_t: into every CTA of the cluster, then published for the helpers,
-      // then the result
-      if (qact) {
-        const unsigned za = smem_addr(zs + ((t % CH_RING) * BR + rho) * NQ + qb), ba = smem_addr(&bars[t % CH_RING]);
-        // first to the CTA whose turn is next
-#pragma unroll
-        for (int r = 0; r < CH_C; r++) st_async(za + peer[r], ba + peer[r], z);
-        unsigned long long* dst = zf + ((size_t) b * CH_VALUES + rho * NQ + qb) * WPV;
-#pragma unroll
-        for (int q = 0; q < QL; q++) Tagged<T>::put(dst + q * WPV, tag, z[q]);
-        if (!BWD) {
-          if (rho < nr)
-#pragma unroll
-            for (int q = 0; q < QL; q++)
-              if (qb + q < nrhs) Wf[r0 + rho + (size_t) (qb + q) * f] = z[q];
-        } else if (rho < bw) {
-          const int g = __ldg(rw + r0 + rho);
-#pragma unroll
-          for (int q = 0; q < QL; q++)
-            if (qb + q < nrhs) X[g + (size_t) (qb + q) * ldx] = z[q];
-        }
-      }
-    }
-    // every z that is still on its way to this CTA's shared memory
-    const int last = (int) rank < nbs ? (int) rank + (nbs - 1 - (int) rank) / CH_C * CH_C : 0;
-    for (int u = (int) rank < nbs ? last : 0; u < nbs; u++) wait_z(u);
-    cluster_sync_all();
-    return;
-  }
-  // ------------------------------------------------------------------ helper
-  const bool upd = !BWD && bk.b >= nbs;                  // an update-row block
-  const int t = upd ? nbs : BWD ? nbs - 1 - bk.b : bk.b;
-  const int n = upd ? nbs : max(0, t - CH_C), b = bk.b;
-  T* zst = zs;                                           // [CH_HB][BR][NQ]
-  own_rhs(b, BWD ? int2_{0, 0} : blk_ch[blockIdx.x - nwalk * CH_C]);
-  Row acc;
-  acc.clear();
-  constexpr int NV = (CH_HB * BR * NQ + CH_THREADS - 1) / CH_THREADS;
-  for (int u = 0; u < n;) {
-    // a round: up to CH_HB blocks with every load in flight; the leading
-    // blocks whose values are all current are used, or the first is waited for
-    const int nb = min(n - u, CH_HB);
-    if (tid == 0) bad_s = 0;
-    __syncthreads();
-    T l[CH_HB][16];
-#pragma unroll
-    for (int i = 0; i < CH_HB; i++)
-      if (i < nb) tile(b, block_of(u + i), l[i]);
-    Tagged<T> zv[NV];
-    auto src = [&](int e) {
-      return zf + ((size_t) block_of(u + e / (BR * NQ)) * CH_VALUES + e % (BR * NQ)) * WPV;
-    };
-    unsigned bad = 0;
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-      const int e = tid + CH_THREADS * i;
-      if (e < nb * BR * NQ) zv[i].load(src(e));
-    }
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-      const int e = tid + CH_THREADS * i;
-      if (e < nb * BR * NQ && !zv[i].ok(tag)) bad |= 1u << (e / (BR * NQ));
-    }
-    if (bad) atomicOr(&bad_s, bad);
-    __syncthreads();
-    int ok = __ffs(bad_s | (1u << nb)) - 1;
-    if (ok == 0) {
-#pragma unroll
-      for (int i = 0; i < NV; i++) {
-        const int e = tid + CH_THREADS * i;
-        if (CH_THREADS * i < BR * NQ) wait_tagged<T>(src(e < BR * NQ ? e : 0), zv[i], e < BR * NQ, tag, status);
-      }
-      ok = 1;
-    }
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-      const int e = tid + CH_THREADS * i;
-      if (e < ok * BR * NQ) zst[e] = zv[i].value();
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < CH_HB; i++)
-      if (i < ok) acc.add(l[i], zst + i * BR * NQ);
-    __syncthreads();
-    u += ok;
-  }
-  T p[QL];
-  acc.sum(p);
-  if (!qact) return;
-#pragma unroll
-  for (int q = 0; q < QL; q++) p[q] = vs[rho][qb + q] - p[q];
-  if (upd) {
-    if (b * BR + rho < f)
-#pragma unroll
-      for (int q = 0; q < QL; q++)
-        if (qb + q < nrhs) Wf[b * BR + rho + (size_t) (qb + q) * f] = p[q];
-  } else {
-    unsigned long long* dst = pf + ((size_t) b * CH_VALUES + rho * NQ + qb) * WPV;
-#pragma unroll
-    for (int q = 0; q < QL; q++) Tagged<T>::put(dst + q * WPV, tag, p[q]);
-  }
-}
 
 // Backward solve, L21^T x2 over a 64-column block and a chunk of 512 update
 // rows by a CTA of NTH threads.  The chunk of x2 is gathered into shared
@@ -1419,202 +898,541 @@ k_bwd_l21(const int2_* __restrict__ tasks, const FrontDesc* __restrict__ fronts,
   }
 }
 
-// Backward solve of big fronts, one CTA per 64-column block, chained from the
-// last block by flags.  PARTS: fronts of more than one chunk of update rows
-// have their L21^T x2 from k_bwd_l21, the others (and without PARTS all) form
-// it here, before the first flag is waited for.
-template <typename T, int NQ, int WS, bool PARTS>
-__global__ void __launch_bounds__(128)
-k_bwd_big(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts,
-          const int* __restrict__ rows, const T* __restrict__ L, const T* __restrict__ Dinv, T* __restrict__ X, int ldx,
-          T* __restrict__ W, const T* __restrict__ part, int nrhs, int* __restrict__ flags, int epoch,
-          int* status) {
-  constexpr bool WARPLOOP = NQ < 8;
-  __shared__ T xv[BR][NQ];
-  __shared__ T xj[BR][NQ];
-  __shared__ T red[BR][NQ];
-  __shared__ T xjw[4][BR / 2][NQ];   // per warp: the rows of x_j it needs
-  extern __shared__ __align__(16) unsigned char bsmraw[];
-  T (*dgb)[BR + 1] = reinterpret_cast<T (*)[BR + 1]>(bsmraw);                              // L_kk^-1, [row][col]
-  T (*tile)[BR + 1] = reinterpret_cast<T (*)[BR + 1]>(bsmraw) + BR;   // NQ >= 8: block of L11, [col][row]
-  const int2_ bk = blocks[blockIdx.x];
-  const FrontDesc F = fronts[bk.a];
-  const int k = bk.b, f = F.f, s = F.s;
-  const int nbs = (s + BR - 1) / BR;
-  const int c0 = k * BR, bw = min(BR, s - c0);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  T* Wf = W + F.v_off * WS;
-  const int* rw = rows + F.rows_off;
-  const T* P = L + F.l_off;
+// What the kernels of the big fronts' blocks share.  zp, pp: published z's and
+// p's; forward reads B and writes W, backward reads W (y) and, for fronts of at
+// least part_min chunks of update rows, the sums in part (L21^T x2; the other
+// fronts form it themselves), and writes X.
+template <typename T>
+struct SolveArgs {
+  const int* walk_fronts;
+  int nwalk;
+  const int2_* blocks;
+  int nblocks;
+  const int2_* blk_ch;
+  const int4* blk_child;
+  const FrontDesc* fronts;
+  const int *maps, *rows;
+  const T *L, *Dinv, *B;
+  T* X;
+  int ldx;
+  T* W;
+  const T* part;
+  int part_min;
+  unsigned long long *zp, *pp;
+  int* flags;
+  int nrhs;
+  const int* counter;
+  int epoch;
+  int* status;
+};
 
-  // stage the block's inverse now, off the chain's critical path
-  const T* Di = Dinv + F.dinv_off + (size_t) k * BR * BR;
-#pragma unroll 1
-  for (int t0 = 0; t0 < BR * BR / 128; t0 += 16) {
-    T dv[16];
-#pragma unroll
-    for (int t = 0; t < 16; t++) {
-      const int e = tid + 128 * (t0 + t), i = e % BR, c = e / BR;
-      dv[t] = (i < bw && c < bw && i >= c) ? Di[i + c * BR] : T(0);
-    }
-#pragma unroll
-    for (int t = 0; t < 16; t++) {
-      const int e = tid + 128 * (t0 + t);
-      dgb[e % BR][e / BR] = dv[t];
-    }
-  }
-  for (int e = tid; e < BR * NQ; e += 128) {
-    const int c = e % BR, q = e / BR;
-    xv[c][q] = (c < bw && q < nrhs) ? Wf[c0 + c + (size_t) q * f] : 0.0;
-  }
-  __syncthreads();
-  if (PARTS && F.nchunk > 1) {
-    // y - L21^T x2 from the per-chunk partial sums, added in chunk order
-    for (int e = tid; e < bw * NQ; e += 128) {
-      const int c = e % bw, q = e / bw;
-      if (q < nrhs) {
-        T acc = 0.0;
-#pragma unroll 4
-        for (int ch = 0; ch < F.nchunk; ch++)
-          acc += __ldcg(part + F.part_off + ((size_t) ch * s + c0 + c) * SOLVE_NRHS + q);
-        xv[c][q] -= acc;
-      }
-    }
-  } else {
-    T (*zs)[SOLVE_RCH] = reinterpret_cast<T (*)[SOLVE_RCH]>(dgb + BR);
-    for (int ch = 0; ch < F.nchunk; ch++) {
-      l21_chunk<T, NQ, 128>(F, L, rows, X, ldx, k, ch, nrhs, zs, [&](int c, int q, int, T v) { xv[c][q] -= v; });
-      __syncthreads();
-    }
-  }
-  __syncthreads();
-  const int col = tid % BR, half = tid / BR;
-  if constexpr (!WARPLOOP) {
-    // 8 columns: the block of L11 is staged in shared memory before the wait
-    // for x_j (measured faster than the warp-level loop below at 8 columns)
-    for (int j = nbs - 1; j > k; j--) {
-      const int bwj = min(BR, s - j * BR);
-#pragma unroll 1
-      for (int t0 = 0; t0 < BR * BR / 128; t0 += 16) {
-        T tv[16];
-#pragma unroll
-        for (int t = 0; t < 16; t++) {
-          const int e = tid + 128 * (t0 + t), i = e % BR, c = e / BR;
-          tv[t] = (i < bwj && c < bw) ? P[(j * BR + i) + (size_t) (c0 + c) * f] : T(0);
-        }
-#pragma unroll
-        for (int t = 0; t < 16; t++) {
-          const int e = tid + 128 * (t0 + t);
-          tile[e / BR][e % BR] = tv[t];
-        }
-      }
-      wait_epoch(flags + F.blk_off + j, epoch, status);
-      for (int e = tid; e < BR * NQ; e += 128) {
-        const int i = e % BR, q = e / BR;
-        xj[i][q] = (i < bwj && q < nrhs) ? __ldcg(Wf + j * BR + i + (size_t) q * f) : 0.0;
-      }
-      __syncthreads();
-      T acc[NQ];
-#pragma unroll
-      for (int q = 0; q < NQ; q++) acc[q] = 0.0;
-#pragma unroll 8
-      for (int i = half * (BR / 2); i < half * (BR / 2) + BR / 2; i++) {
-        const T l = tile[col][i];
-#pragma unroll
-        for (int q = 0; q < NQ; q++) acc[q] += l * xj[i][q];
-      }
-      if (half == 1)
-#pragma unroll
-        for (int q = 0; q < NQ; q++) red[col][q] = acc[q];
-      __syncthreads();
-      if (half == 0)
-#pragma unroll
-        for (int q = 0; q < NQ; q++) xv[col][q] -= acc[q] + red[col][q];
-      __syncthreads();
-    }
-  } else {
-  // solved blocks below, last first, without block-wide barriers: thread
-  // (col, half) keeps its partial sum over the rows of its half across all
-  // tiles (the 32 entries of L it needs are loaded before the wait); each
-  // warp polls the flags itself and stages the 32 rows of x_j it needs; the
-  // two halves are combined once at the end
-  {
-    T acc[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) acc[q] = 0.0;
-    const T* pcol = P + (size_t) (c0 + col) * f + half * (BR / 2);
-    T (*xw)[NQ] = xjw[warp];
-    for (int j = nbs - 1; j > k; j--) {
-      const int bwj = min(BR, s - j * BR);
-      T lv[BR / 2];
-#pragma unroll
-      for (int t = 0; t < BR / 2; t++)
-        lv[t] = (col < bw && half * (BR / 2) + t < bwj) ? __ldg(pcol + (size_t) j * BR + t) : T(0);
-      poll_epoch(flags + F.blk_off + j, epoch, status);
-#pragma unroll
-      for (int q = 0; q < NQ; q++) {
-        const int i = half * (BR / 2) + lane;
-        xw[lane][q] = (i < bwj && q < nrhs) ? __ldcg(Wf + (size_t) j * BR + i + (size_t) q * f) : T(0);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int t = 0; t < BR / 2; t++)
-#pragma unroll
-        for (int q = 0; q < NQ; q++) acc[q] += lv[t] * xw[t][q];
-      __syncwarp();
-    }
-    if (half == 1)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) red[col][q] = acc[q];
-    __syncthreads();
-    if (half == 0)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) xv[col][q] -= acc[q] + red[col][q];
-    __syncthreads();
-  }
-  }
-  // x_k = L_kk^-T v_k from the staged inverse, split over the two halves
-  {
-    T x[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) x[q] = 0.0;
-#pragma unroll 8
-    for (int i = half * (BR / 2); i < half * (BR / 2) + BR / 2; i++) {
-      const T d = dgb[i][col];
-#pragma unroll
-      for (int q = 0; q < NQ; q++) x[q] += d * xv[i][q];
-    }
-    if (half == 1)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) red[col][q] = x[q];
-    __syncthreads();
-    if (half == 0)
-#pragma unroll
-      for (int q = 0; q < NQ; q++) xj[col][q] = x[q] + red[col][q];
-    __syncthreads();
-  }
-  for (int e = tid; e < bw * nrhs; e += 128) {
-    const int c = e % bw, q = e / bw;
-    Wf[c0 + c + (size_t) q * f] = xj[c][q];
-    X[rw[c0 + c] + (size_t) q * ldx] = xj[c][q];
-  }
-  __syncthreads();
-  // the barrier orders every thread's writes before thread 0's release store
-  if (tid == 0) st_release(flags + F.blk_off + k, epoch);
+// a load of the factor that is issued where it stands (a plain read-only load
+// may be moved down to its use, past the wait that it is meant to overlap);
+// zero, and no access, without in
+__device__ __forceinline__ double load_now(const double* p, bool in) {
+  double v;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+               "@q ld.global.nc.f64 %0, [%1];\n\t}"
+               : "=d"(v)
+               : "l"(p), "r"((unsigned) in));
+  return v;
+}
+__device__ __forceinline__ float load_now(const float* p, bool in) {
+  float v;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+               "@q ld.global.nc.f32 %0, [%1];\n\t}"
+               : "=f"(v)
+               : "l"(p), "r"((unsigned) in));
+  return v;
 }
 
-// the start of a pass: the first nfl chain flags cleared (with them the
-// persistent set's done flags), the persistent queues' pending counts and
-// heads, and the walks' call counter advanced when there is one
-__global__ void k_solve_reset(int* flags, int nfl, const int* __restrict__ pending0, int* pers, int np, int* counter) {
+// One front's 64-row blocks as the kernels below work on them.  Chain
+// position t <-> block (backward: the last block first).  TAGS: the z's between
+// CTAs are published values; else (the allocation-free solve, which has no
+// room for them) they are in the work vector behind release/acquire flags.
+template <typename T, int NQ, int WS, bool BWD, bool TAGS>
+struct BigBlock {
+  using Row = ChainRow<T, NQ>;
+  static constexpr int QL = Row::QL, WPV = ch_words<T>();
+  const SolveArgs<T>& A;
+  const FrontDesc F;
+  const int f, s, nbs;
+  const T* const P;
+  T* const Wf;
+  const int* const rw;
+  unsigned long long* const zf;
+  const unsigned tag;
+  __device__ __forceinline__ BigBlock(const SolveArgs<T>& a, int front)
+      : A(a), F(a.fronts[front]), f(F.f), s(F.s), nbs((F.s + BR - 1) / BR), P(a.L + F.l_off), Wf(a.W + F.v_off * WS),
+        rw(a.rows + F.rows_off), zf(a.zp + (size_t) F.blk_off * CH_VALUES * WPV),
+        tag(TAGS ? ((unsigned) *a.counter << 12) | (unsigned) a.epoch : 0u) {}
+  __device__ __forceinline__ int block_of(int t) const { return BWD ? nbs - 1 - t : t; }
+  // this lane's 16 entries of A_tu (block row bt: rows below s may belong to
+  // the update rows of the last diagonal block, or be an update block)
+  __device__ __forceinline__ void tile(int bt, int bu, T (&l)[16]) const {
+    const int jq = Row::jq();
+#pragma unroll
+    for (int h = 0; h < Row::R; h++) {
+      const int r = bt * BR + Row::row(h), c = bu * BR + jq;
+      const bool rv = r < (BWD ? s : f);
+      const T* a = BWD ? P + c + (size_t) r * f : P + r + (size_t) c * f;
+#pragma unroll
+      for (int t = 0; t < Row::NT; t++)
+        l[h * Row::NT + t] = load_now(a + (BWD ? Row::J * t : (size_t) (Row::J * t) * f), rv && c + Row::J * t < s);
+    }
+  }
+  // the inverse of diagonal block b on its way into ds (column stride DLD:
+  // the products' reads are free of bank conflicts)
+  __device__ __forceinline__ void stage_inverse(int b, T* ds) const {
+    const T* Di = A.Dinv + F.dinv_off + (size_t) b * BR * BR;
+    constexpr int V = 16 / (int) sizeof(T), PER = BR / V;
+#pragma unroll
+    for (int e = threadIdx.x; e < BR * PER; e += CH_THREADS) {
+      const int c = e / PER, r = e % PER * V;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(ds + c * DLD + r)), "l"(Di + c * BR + r));
+    }
+  }
+  // the right-hand side of block b into vs, with a barrier after it; scr:
+  // scratch (backward: a chunk of x2 and its sums, with SUMS)
+  template <bool SUMS>
+  __device__ __forceinline__ void own_rhs(int b, const int2_ cr, T (*vs)[NQ], T* scr) const {
+    const int tid = threadIdx.x, r0 = b * BR, nr = min(BR, f - r0);
+    if constexpr (!BWD) {
+      ChildGather<T, NQ, WS, CH_THREADS> cg;
+      cg.load(A.blk_child + cr.a, cr.b - cr.a, A.maps, A.W, A.nrhs);
+      for (int e = tid; e < BR * NQ; e += CH_THREADS) {
+        const int i = e % BR, q = e / BR;
+        vs[i][q] = (i < nr && q < A.nrhs && r0 + i < s) ? A.B[rw[r0 + i] + (size_t) q * A.ldx] : T(0);
+      }
+      __syncthreads();
+      cg.add(A.blk_child + cr.a, cr.b - cr.a, A.maps, A.W, A.nrhs, r0, vs);
+    } else {
+      const bool parts = !SUMS || F.nchunk >= A.part_min;
+      for (int e = tid; e < BR * NQ; e += CH_THREADS) {
+        const int i = e % BR, q = e / BR;
+        T v = T(0);
+        if (r0 + i < s && q < A.nrhs) {
+          v = Wf[r0 + i + (size_t) q * f];
+          T acc = T(0);
+          if (parts) {
+#pragma unroll 4
+            for (int ch = 0; ch < F.nchunk; ch++)
+              acc += A.part[F.part_off + ((size_t) ch * s + r0 + i) * SOLVE_NRHS + q];
+          }
+          v -= acc;
+        }
+        vs[i][q] = v;
+      }
+      if (SUMS && !parts) {
+        constexpr int RP = L21Split<NQ, CH_THREADS>::RP;
+        T (*zs)[SOLVE_RCH] = reinterpret_cast<T (*)[SOLVE_RCH]>(scr);
+        T (*red)[BR][NQ] = reinterpret_cast<T (*)[BR][NQ]>(scr + NQ * SOLVE_RCH);
+        const int nch = (f - s + SOLVE_RCH - 1) / SOLVE_RCH, bw = min(BR, s - r0);
+        for (int ch = 0; ch < nch; ch++) {
+          l21_chunk<T, NQ, CH_THREADS>(F, A.L, A.rows, A.X, A.ldx, b, ch, A.nrhs, zs,
+                                       [&](int c, int q, int p, T v) { red[p][c][q] = v; });
+          __syncthreads();
+          for (int e = tid; e < bw * NQ; e += CH_THREADS) {
+            const int c = e / NQ, q = e % NQ;
+            T v = red[0][c][q];
+#pragma unroll
+            for (int p = 1; p < RP; p++) v += red[p][c][q];
+            if (q < A.nrhs) vs[c][q] -= v;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+  // acc += sum_{u<n} A_bu z_u as the z's appear.  A round takes up to HB blocks
+  // with every load in flight: the leading blocks whose values are all current
+  // are used, or the first is waited for.  l: the first round's tiles, already
+  // loaded.  zst: HB staged z's.
+  template <int HB>
+  __device__ __forceinline__ void terms(int b, int n, T (&l)[HB][16], Row& acc, T* zst, unsigned* bad_s) const {
+    const int tid = threadIdx.x;
+    constexpr int NV = (HB * BR * NQ + CH_THREADS - 1) / CH_THREADS;
+    for (int u = 0; u < n;) {
+      int ok = min(n - u, HB);
+      if constexpr (TAGS) {
+        const int nb = ok;
+        if (HB > 1 && tid == 0) *bad_s = 0;
+        if (HB > 1) __syncthreads();
+        Tagged<T> zv[NV];
+        auto src = [&](int e) {
+          return zf + ((size_t) block_of(u + e / (BR * NQ)) * CH_VALUES + e % (BR * NQ)) * WPV;
+        };
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+          const int e = tid + CH_THREADS * i;
+          if (e < nb * BR * NQ) zv[i].load(src(e));
+        }
+        if constexpr (HB > 1) {
+          unsigned bad = 0;
+#pragma unroll
+          for (int i = 0; i < NV; i++) {
+            const int e = tid + CH_THREADS * i;
+            if (e < nb * BR * NQ && !zv[i].ok(tag)) bad |= 1u << (e / (BR * NQ));
+          }
+          if (bad) atomicOr(bad_s, bad);
+          __syncthreads();
+          ok = __ffs(*bad_s | (1u << nb)) - 1;
+        } else {
+          ok = 0;
+        }
+        if (ok == 0) {
+#pragma unroll
+          for (int i = 0; i < NV; i++) {
+            const int e = tid + CH_THREADS * i;
+            if (CH_THREADS * i < BR * NQ) wait_tagged<T>(src(e < BR * NQ ? e : 0), zv[i], e < BR * NQ, tag, A.status);
+          }
+          ok = 1;
+        }
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+          const int e = tid + CH_THREADS * i;
+          if (e < ok * BR * NQ) zst[e] = zv[i].value();
+        }
+      } else {
+        ok = 1;
+        const int bu = block_of(u);
+        wait_epoch(A.flags + F.blk_off + bu, A.epoch, A.status);
+        for (int e = tid; e < BR * NQ; e += CH_THREADS) {
+          const int i = e / NQ, q = e % NQ;
+          zst[e] = (bu * BR + i < s && q < A.nrhs) ? __ldcg(Wf + bu * BR + i + (size_t) q * f) : T(0);
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < HB; i++)
+        if (i < ok) acc.add(l[i], zst + i * BR * NQ);
+      u += ok;
+#pragma unroll
+      for (int i = 0; i < HB; i++)
+        if (u + i < n) tile(b, block_of(u + i), l[i]);
+      __syncthreads();
+    }
+  }
+  // this lane's 16 entries of the staged inverse, once it is complete
+  __device__ __forceinline__ static void inverse(const T* ds, T (&d)[16]) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < Row::R; h++)
+#pragma unroll
+      for (int i = 0; i < Row::NT; i++) {
+        const int r = Row::row(h), c = Row::J * i + Row::jq();
+        d[h * Row::NT + i] = ds[BWD ? c + r * DLD : r + c * DLD];
+      }
+  }
+  // z = D v, v (this lane's share pv) in rows of vs; in the last diagonal block
+  // the update rows get w_i - L[i, block] y (forward)
+  __device__ __forceinline__ void diagonal(int b, const T (&d)[16], const T (&pv)[QL], T (*vs)[NQ], T (&z)[QL]) const {
+    const int rho = Row::own(), qb = Row::qb();
+    const int r0 = b * BR, nr = min(BR, f - r0), bw = min(BR, s - r0);
+    if (Row::qact())
+#pragma unroll
+      for (int q = 0; q < QL; q++) vs[rho][qb + q] = pv[q];
+    __syncthreads();
+    Row acc;
+    acc.clear();
+    acc.add(d, &vs[0][0]);
+    acc.sum(z);
+    if (!BWD && bw < nr) {
+      // the inverse is zero in the update rows: y is in place first
+      __syncthreads();
+      if (Row::qact() && rho < bw)
+#pragma unroll
+        for (int q = 0; q < QL; q++) vs[rho][qb + q] = z[q];
+      __syncthreads();
+      T l[16], uq[QL];
+      tile(b, b, l);
+      acc.clear();
+      acc.add(l, &vs[0][0]);
+      acc.sum(uq);
+      if (rho >= bw)
+#pragma unroll
+        for (int q = 0; q < QL; q++) z[q] = pv[q] - uq[q];
+    }
+  }
+  // the result of block b: forward into the work vector, backward into X
+  __device__ __forceinline__ void result(int b, const T (&z)[QL]) const {
+    const int r = b * BR + Row::own(), qb = Row::qb();
+    if (!Row::qact() || r >= (BWD ? s : f)) return;
+    if (!BWD || !TAGS) {
+#pragma unroll
+      for (int q = 0; q < QL; q++)
+        if (qb + q < A.nrhs) Wf[r + (size_t) (qb + q) * f] = z[q];
+    }
+    if (BWD) {
+      const int g = __ldg(rw + r);
+#pragma unroll
+      for (int q = 0; q < QL; q++)
+        if (qb + q < A.nrhs) A.X[g + (size_t) (qb + q) * A.ldx] = z[q];
+    }
+  }
+  // a published value array's slot of this lane in block b
+  __device__ __forceinline__ unsigned long long* slot(unsigned long long* base, int b) const {
+    return base + ((size_t) b * CH_VALUES + Row::own() * NQ + Row::qb()) * WPV;
+  }
+  __device__ __forceinline__ void publish(unsigned long long* base, int b, const T (&z)[QL]) const {
+    if (!Row::qact()) return;
+    unsigned long long* dst = slot(base, b);
+#pragma unroll
+    for (int q = 0; q < QL; q++) Tagged<T>::put(dst + q * WPV, tag, z[q]);
+  }
+};
+
+// elements of the scratch of own_rhs and terms
+template <int NQ, bool BWD, int HB>
+__host__ __device__ constexpr int block_scratch() {
+  const int rhs = BWD ? NQ * SOLVE_RCH + L21Split<NQ, CH_THREADS>::RP * BR * NQ : 0, z = HB * BR * NQ;
+  return rhs > z ? rhs : z;
+}
+
+// Forward and backward solve of a level's big fronts as chains, for levels
+// with few fronts and several 64-row blocks each.  What bounds such a level
+// is the chain of its blocks -- z_t = D_t (p_t - sum_{u<t} A_tu z_u), D_t the
+// inverse of a diagonal block (forward: blocks first to last; backward: last
+// to first, transposed) -- so the chain runs inside one cluster of CH_C CTAs:
+// CTA t mod CH_C computes block t and writes z_t into the shared memory of
+// all of them (st.async, counted by the receivers' mbarriers), one to two
+// orders faster than a hand-over through global memory.  Between its turns a
+// CTA adds the terms of the last CH_C blocks to its next one as they arrive,
+// with the tiles of L loaded into registers two terms ahead and into L2 a
+// turn ahead: per step the chain waits for one 64x64 product, one product
+// with the inverse and one hand-over.  The far terms (u < t - CH_C) and the
+// right-hand side of block t are the work of a helper CTA per block, which
+// follows the published z_u and publishes p_t about CH_C steps ahead;
+// forward, the update rows' blocks are helpers too and stream L21 while the
+// chain runs.  Values published between CTAs travel as tagged words (tag in
+// the high half, 32 bits of the value in the low half; a double takes two),
+// each one relaxed 8-byte access: a reader knows a value is current when its
+// tag is, so nothing fences or polls a flag.  The tag is (call counter <<
+// 12) | epoch, the counter being advanced on the device at the start of every
+// solve call, so recorded launch sequences stay valid.  A ring of 2 CH_C z's
+// needs no release: block t's CTA has consumed z_{t-CH_C} .. z_{t-1}, so when
+// z_{u+2 CH_C} is produced every CTA is past its last use of z_u.  Walkers have
+// the lowest CTA indices and helper t waits only for blocks whose helpers
+// come before it, so in-order dispatch keeps every wait finite; the waits are
+// bounded all the same, and no CTA of a cluster leaves before every z has
+// arrived in its shared memory.  In the last diagonal block rows >= s are
+// update rows of the same front; its CTA finishes them too (forward).
+// Measured, per 64-row step of the root level's forward chain: FP64, one right-
+// hand side (64^3) 2.3 us with flags between CTAs, 1.2 us here; FP64, eight
+// (45x47x44) 4.7 -> 1.7 us; FP32, eight (56^3) 4.2 us with one walker CTA per
+// front, 2.0 us here.
+// dynamic shared memory: the block's inverse, the ring of z's (walker) or a
+// round's staged z's and x2 (helper), and the block's vector
+template <typename T, int NQ>
+constexpr size_t chain_smem() { return (size_t) (BR * DLD + (CH_RING + 1) * BR * NQ) * sizeof(T); }
+
+template <typename T, int NQ, int WS, bool BWD>
+__global__ void __cluster_dims__(CH_C, 1, 1) __launch_bounds__(CH_THREADS, 2)
+k_chain(const __grid_constant__ SolveArgs<T> A) {
+  using BB = BigBlock<T, NQ, WS, BWD, true>;
+  using Row = ChainRow<T, NQ>;
+  constexpr int QL = Row::QL, WPV = ch_words<T>();
+  extern __shared__ __align__(16) unsigned char chm[];
+  __shared__ __align__(8) unsigned long long bars[CH_RING];
+  __shared__ unsigned bad_s;
+  const int tid = threadIdx.x;
+  const int rho = Row::own(), qb = Row::qb();
+  const bool walker = blockIdx.x < (unsigned) (A.nwalk * CH_C);
+  const int h = (int) blockIdx.x - A.nwalk * CH_C;
+  if (!walker && h >= A.nblocks) return;
+  const int2_ bk = walker ? int2_{A.walk_fronts[blockIdx.x / CH_C], 0} : A.blocks[h];
+  const BB M(A, bk.a);
+  const int f = M.f, s = M.s, nbs = M.nbs;
+  unsigned long long* pf = A.pp + (size_t) M.F.blk_off * CH_VALUES * WPV;
+  T* ds = reinterpret_cast<T*>(chm);
+  T* zs = ds + BR * DLD;                          // [CH_RING][BR][NQ]
+  T (*vs)[NQ] = reinterpret_cast<T (*)[NQ]>(zs + CH_RING * BR * NQ);
+
+  if (walker) {
+    // ---------------------------------------------------------------- walker
+    const unsigned rank = blockIdx.x % CH_C;
+    constexpr unsigned ZBYTES = BR * NQ * sizeof(T);
+    if (tid == 0) {
+      for (int i = 0; i < CH_RING; i++)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bars[i])) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      for (int i = 0; i < min(CH_RING, nbs); i++) bar_expect(smem_addr(&bars[i]), ZBYTES);
+    }
+    __syncthreads();
+    cluster_sync_all();
+    // z_u has arrived (each CTA waits for every u once, in order); its
+    // barrier is armed for the z that takes the slot next
+    auto wait_z = [&](int u) {
+      bar_wait(smem_addr(&bars[u % CH_RING]), (u / CH_RING) & 1, A.status);
+      if (tid == 0 && u + CH_RING < nbs) bar_expect(smem_addr(&bars[u % CH_RING]), ZBYTES);
+    };
+    unsigned peer[CH_C];   // offsets of the others' shared memory, the next CTA of the chain first
+#pragma unroll
+    for (int r = 0; r < CH_C; r++) peer[r] = map_rank(smem_addr(bars), (rank + 1 + r) % CH_C) - smem_addr(bars);
+    for (int t = rank; t < nbs; t += CH_C) {
+      const int b = M.block_of(t);
+      const int u0 = max(0, t - CH_C);
+      T la[16], lb[16], d[16];
+      if (u0 < t) M.tile(b, M.block_of(u0), la);
+      if (u0 + 1 < t) M.tile(b, M.block_of(u0 + 1), lb);
+      __syncthreads();   // every warp is done with the last turn's inverse
+      M.stage_inverse(b, ds);
+      // the next turn's tiles into L2
+      if (t + CH_C < nbs) {
+        const int bn = M.block_of(t + CH_C);
+        constexpr int LPC = BR * (int) sizeof(T) / 128 + 1;   // lines a 64-entry column piece touches
+        for (int e = tid; e < CH_C * BR * LPC; e += CH_THREADS) {
+          const int li = e % LPC, c = e / LPC;
+          const int bu = M.block_of(t + c / BR);
+          const int row = (BWD ? bu : bn) * BR + min(li * (128 / (int) sizeof(T)), BR - 1);
+          const int col = (BWD ? bn : bu) * BR + c % BR;
+          if (row < f && col < s) prefetch_l2(M.P + row + (size_t) col * f);
+        }
+        for (int e = tid; e < BR * BR * (int) sizeof(T) / 128; e += CH_THREADS)
+          prefetch_l2(reinterpret_cast<const unsigned char*>(A.Dinv + M.F.dinv_off + (size_t) bn * BR * BR) + 128 * e);
+      }
+      Row acc;
+      acc.clear();
+      Tagged<T> pt[QL];
+      const unsigned long long* pq = M.slot(pf, b);
+      auto load_p = [&]() {
+#pragma unroll
+        for (int q = 0; q < QL; q++) pt[q].load(pq + q * WPV);
+      };
+      if (t == 0) {
+        load_p();
+        M.inverse(ds, d);
+      }
+      for (int u = u0; u < t; u += 2) {
+        if (u + 2 >= t) {   // ahead of the waits that are on the chain
+          load_p();
+          M.inverse(ds, d);
+        }
+        wait_z(u);
+        acc.add(la, zs + (u % CH_RING) * BR * NQ);
+        if (u + 2 < t) M.tile(b, M.block_of(u + 2), la);
+        if (u + 1 < t) {
+          wait_z(u + 1);
+          acc.add(lb, zs + ((u + 1) % CH_RING) * BR * NQ);
+          if (u + 3 < t) M.tile(b, M.block_of(u + 3), lb);
+        }
+      }
+      T z[QL], pv[QL];
+      acc.sum(z);
+#pragma unroll
+      for (int q = 0; q < QL; q++) {
+        wait_tagged<T>(pq + q * WPV, pt[q], true, M.tag, A.status);
+        pv[q] = pt[q].value() - z[q];
+      }
+      M.diagonal(b, d, pv, vs, z);
+      // z_t: into every CTA of the cluster, the next of the chain first, then
+      // published for the helpers, then the result
+      if (Row::qact()) {
+        const unsigned za = smem_addr(zs + ((t % CH_RING) * BR + rho) * NQ + qb), ba = smem_addr(&bars[t % CH_RING]);
+#pragma unroll
+        for (int r = 0; r < CH_C; r++) st_async(za + peer[r], ba + peer[r], z);
+      }
+      M.publish(M.zf, b, z);
+      M.result(b, z);
+    }
+    // every z that is still on its way to this CTA's shared memory
+    for (int u = (int) rank < nbs ? (int) rank + (nbs - 1 - (int) rank) / CH_C * CH_C : 0; u < nbs; u++) wait_z(u);
+    cluster_sync_all();
+    return;
+  }
+  // ------------------------------------------------------------------ helper
+  const bool upd = !BWD && bk.b >= nbs;                  // an update-row block
+  const int b = bk.b, n = upd ? nbs : max(0, (BWD ? nbs - 1 - b : b) - CH_C);
+  T l[CH_HB][16];
+#pragma unroll
+  for (int i = 0; i < CH_HB; i++)
+    if (i < n) M.tile(b, M.block_of(i), l[i]);
+  M.template own_rhs<false>(b, BWD ? int2_{0, 0} : A.blk_ch[h], vs, zs);
+  Row acc;
+  acc.clear();
+  M.template terms<CH_HB>(b, n, l, acc, zs, &bad_s);
+  T p[QL];
+  acc.sum(p);
+#pragma unroll
+  for (int q = 0; q < QL; q++) p[q] = vs[rho][qb + q] - p[q];
+  if (upd) M.result(b, p);
+  else M.publish(pf, b, p);
+}
+
+// The big fronts of the other levels: one CTA per 64-row block, which adds the
+// terms of the blocks before it as they are published, applies its inverse and
+// publishes its own result (forward, blocks of update rows stop at the terms).
+// Blocks wait only for blocks of lower index.
+constexpr int BLK_HB = 1;
+template <typename T, int NQ, bool BWD>
+constexpr size_t block_smem() { return (size_t) (BR * DLD + block_scratch<NQ, BWD, BLK_HB>() + BR * NQ) * sizeof(T); }
+
+template <typename T, int NQ, int WS, bool BWD, bool TAGS>
+__global__ void __launch_bounds__(CH_THREADS, (sizeof(T) == 4 ? 4 : 3) - BWD)
+k_block(const __grid_constant__ SolveArgs<T> A) {
+  using BB = BigBlock<T, NQ, WS, BWD, TAGS>;
+  using Row = ChainRow<T, NQ>;
+  constexpr int QL = Row::QL;
+  extern __shared__ __align__(16) unsigned char chm[];
+  __shared__ unsigned bad_s;
+  T* ds = reinterpret_cast<T*>(chm);
+  T* scr = ds + BR * DLD;
+  T (*vs)[NQ] = reinterpret_cast<T (*)[NQ]>(scr + block_scratch<NQ, BWD, BLK_HB>());
+  const int2_ bk = A.blocks[blockIdx.x];
+  const int2_ cr = BWD ? int2_{0, 0} : A.blk_ch[blockIdx.x];
+  const BB M(A, bk.a);
+  const int b = bk.b, nbs = M.nbs;
+  const bool diag = BWD || b < nbs;
+  const int n = !diag ? nbs : BWD ? nbs - 1 - b : b;
+  T l[BLK_HB][16];
+  // forward, the first tile is on its way before the children's rows are
+  // added; backward the sums over x2 need the registers
+  auto first = [&]() {
+#pragma unroll
+    for (int i = 0; i < BLK_HB; i++)
+      if (i < n) M.tile(b, M.block_of(i), l[i]);
+  };
+  if (diag) M.stage_inverse(b, ds);
+  if (!BWD) first();
+  M.template own_rhs<true>(b, cr, vs, scr);
+  if (BWD) first();
+  Row acc;
+  acc.clear();
+  M.template terms<BLK_HB>(b, n, l, acc, scr, &bad_s);
+  T z[QL], pv[QL];
+  acc.sum(z);
+#pragma unroll
+  for (int q = 0; q < QL; q++) pv[q] = vs[Row::own()][Row::qb() + q] - z[q];
+  if (!diag) {
+    M.result(b, pv);
+    return;
+  }
+  T d[16];
+  M.inverse(ds, d);
+  M.diagonal(b, d, pv, vs, z);
+  if constexpr (TAGS) {
+    M.publish(M.zf, b, z);
+    M.result(b, z);
+  } else {
+    M.result(b, z);
+    __syncthreads();
+    // the barrier orders every thread's writes before thread 0's release store
+    if (threadIdx.x == 0) st_release(A.flags + M.F.blk_off + b, A.epoch);
+  }
+}
+
+// the start of a pass: the persistent queues' pending counts and heads; with
+// the first pass of a call also the persistent set's done flags and the call
+// counter of the published values
+__global__ void k_solve_reset(int first, const int* __restrict__ pending0, int* pers, int np, int* counter) {
   const int i0 = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
-  for (int i = i0; i < nfl; i += n) flags[i] = 0;
   for (int i = i0; i < np; i += n) {
     pers[i] = pending0[i];
-    if (nfl > 0) pers[np + i] = 0;
+    if (first) pers[np + i] = 0;
   }
   if (i0 < 4) pers[2 * np + i0] = 0;
-  if (counter && i0 == 0) *counter += 1;
+  if (first && i0 == 0) *counter += 1;
 }
 
 }  // namespace
@@ -1659,19 +1477,6 @@ static void solve_attrs() {
   per_device_once(pd, [] {
     // static + dynamic shared memory of these kernels can exceed the default
     // 48 KB (8 columns in FP64)
-    auto big = [](auto nqc) {
-      constexpr int Q = decltype(nqc)::value;
-      cudaFuncSetAttribute(k_fwd_big<T, Q, SOLVE_NRHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T>());
-      cudaFuncSetAttribute(k_bwd_big<T, Q, SOLVE_NRHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int) bwd_smem<T, Q>());
-    };
-    big(std::integral_constant<int, 2>());
-    big(std::integral_constant<int, 4>());
-    big(std::integral_constant<int, SOLVE_NRHS>());
-    if constexpr (std::is_same<T, double>::value) {
-      cudaFuncSetAttribute(k_fwd_big<T, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fwd_smem<T>());
-      cudaFuncSetAttribute(k_bwd_big<T, 1, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bwd_smem<T, 1>());
-    }
     auto sf = [](auto nqc) {
       constexpr int Q = decltype(nqc)::value;
       // the most any launch asks for: 8 warps of fronts of order <= 32, or 4
@@ -1689,6 +1494,10 @@ static void solve_attrs() {
                            (int) chain_smem<T, Q>());
       cudaFuncSetAttribute(k_chain<T, Q, SOLVE_NRHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int) chain_smem<T, Q>());
+      cudaFuncSetAttribute(k_block<T, Q, SOLVE_NRHS, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int) block_smem<T, Q, false>());
+      cudaFuncSetAttribute(k_block<T, Q, SOLVE_NRHS, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int) block_smem<T, Q, true>());
     };
     for (int nq : {1, 4, 8}) chain_dispatch<T>(nq, chain);
     sf(std::integral_constant<int, 1>());
@@ -1739,8 +1548,8 @@ template <typename T>
 static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Dinv, int nrhs, T* X, const T* B, int ld, T* W,
                         T* part, int* flags, int* epoch, int* status, cudaStream_t st) {
   solve_attrs<T>();
-  // the chains' published values, and their call counter in the word after the
-  // cleared flags, advanced on the device once per call
+  // the blocks' published values, and their call counter in the word after the
+  // flags
   int* counter = flags + solve_flag_words(P);
   unsigned long long* zpub = reinterpret_cast<unsigned long long*>(part + P.fpart_off);
   unsigned long long* ppub = zpub + (size_t) P.n_blk * CH_VALUES * ch_words<T>();
@@ -1748,16 +1557,16 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
     return walk_enabled() && LP.max_s_big >= CHAIN_MIN_S && (int) LP.big_fronts.size() <= chain_max_fronts<T>();
   };
   auto chain_grid = [](int nbig, int nblocks) { return nbig * CH_C + (nblocks + CH_C - 1) / CH_C * CH_C; };
-  bool walks = false;
-  for (const LevelPlan& LP : P.levels) walks = walks || chain_level(LP);
+  auto args = [&](int h, int nb, const int2_* bl, const int2_* bc, const T* Bq, T* Xq, int nq, int ep, int part_min) {
+    return SolveArgs<T>{D.big_list + D.big_off[h], (int) P.levels[h].big_fronts.size(), bl, nb, bc, D.blk_child, D.fronts,
+                        D.maps, D.rows, L, Dinv, Bq, Xq, ld, W, part, part_min, zpub, ppub, flags, nq, counter, ep, status};
+  };
   const int np = D.n_pers;
-  // the handshake flags restart from zero on every call, so the epochs of a
-  // call are always 1, 2, ... and a recorded launch sequence stays valid; one
-  // launch resets them, the persistent queues and the walks' call counter
+  // the epochs of a call are always 1, 2, ... and the counter advances on the
+  // device, so a recorded launch sequence stays valid
   auto reset = [&](bool first) {
-    const int nfl = first ? (int) solve_flag_words(P) : 0;
-    const int grid = std::max(1, std::min(148, (std::max(nfl, np) + 255) / 256));
-    k_solve_reset<<<grid, 256, 0, st>>>(flags, nfl, D.pers_pending0, D.pers_solve, np, first && walks ? counter : nullptr);
+    const int grid = std::max(1, std::min(148, (np + 255) / 256));
+    k_solve_reset<<<grid, 256, 0, st>>>(first, D.pers_pending0, D.pers_solve, np, counter);
     count_launch();
   };
   auto small_list = [&](int h, int nq, auto launch) {
@@ -1808,26 +1617,14 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       const int nb = (int) LP.solve_fwd_blocks.size();
       if (nb > 0) {
         const int2_ *bl = D.sfwd + D.sfwd_off[h], *bc = D.sfwd_ch + D.sfwd_off[h];
-        if (chain_level(LP)) {
-          const int nbig = (int) LP.big_fronts.size();
-          chain_dispatch<T>(nq, [&](auto nqc) {
-            constexpr int Q = decltype(nqc)::value;
-            k_chain<T, Q, SOLVE_NRHS, false><<<chain_grid(nbig, nb), CH_THREADS, chain_smem<T, Q>(), st>>>(
-                D.big_list + D.big_off[h], nbig, bl, nb, bc, D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, Bq, Xq, ld, W,
-                part, zpub, ppub, nq, counter, ef, status);
-          });
-        } else {
-          // one right-hand side runs the two-column variant, measured faster
-          // than a one-column instantiation (columns >= nrhs are skipped)
-          auto run = [&](auto nqc) {
-            constexpr int Q = decltype(nqc)::value;
-            k_fwd_big<T, Q, SOLVE_NRHS><<<nb, 128, fwd_smem<T>(), st>>>(bl, bc, D.blk_child, D.fronts, D.maps, D.rows, L,
-                                                                        Dinv, Bq, ld, W, nq, flags, ef, status);
-          };
-          if (nq <= 2) run(std::integral_constant<int, 2>());
-          else if (nq <= 4) run(std::integral_constant<int, 4>());
-          else run(std::integral_constant<int, 8>());
-        }
+        const SolveArgs<T> A = args(h, nb, bl, bc, Bq, Xq, nq, ef, 1);
+        chain_dispatch<T>(nq, [&](auto nqc) {
+          constexpr int Q = decltype(nqc)::value;
+          if (chain_level(LP))
+            k_chain<T, Q, SOLVE_NRHS, false><<<chain_grid(A.nwalk, nb), CH_THREADS, chain_smem<T, Q>(), st>>>(A);
+          else
+            k_block<T, Q, SOLVE_NRHS, false, true><<<nb, CH_THREADS, block_smem<T, Q, false>(), st>>>(A);
+        });
         count_launch();
       }
       prof_end(KC_SOLVE_FWD, st, 0.0, by);
@@ -1859,24 +1656,14 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
           });
           count_launch();
         }
-        if (chain) {
-          const int nbig = (int) LP.big_fronts.size();
-          chain_dispatch<T>(nq, [&](auto nqc) {
-            constexpr int Q = decltype(nqc)::value;
-            k_chain<T, Q, SOLVE_NRHS, true><<<chain_grid(nbig, nb), CH_THREADS, chain_smem<T, Q>(), st>>>(
-                D.big_list + D.big_off[h], nbig, bl, nb, nullptr, nullptr, D.fronts, D.maps, D.rows, L, Dinv, nullptr, Xq,
-                ld, W, part, zpub, ppub, nq, counter, eb, status);
-          });
-        } else {
-          auto run = [&](auto nqc) {
-            constexpr int Q = decltype(nqc)::value;
-            k_bwd_big<T, Q, SOLVE_NRHS, true><<<nb, 128, bwd_smem<T, Q>(), st>>>(bl, D.fronts, D.rows, L, Dinv, Xq, ld, W,
-                                                                                 part, nq, flags, eb, status);
-          };
-          if (nq <= 2) run(std::integral_constant<int, 2>());
-          else if (nq <= 4) run(std::integral_constant<int, 4>());
-          else run(std::integral_constant<int, 8>());
-        }
+        const SolveArgs<T> A = args(h, nb, bl, nullptr, nullptr, Xq, nq, eb, chain ? 1 : 2);
+        chain_dispatch<T>(nq, [&](auto nqc) {
+          constexpr int Q = decltype(nqc)::value;
+          if (chain)
+            k_chain<T, Q, SOLVE_NRHS, true><<<chain_grid(A.nwalk, nb), CH_THREADS, chain_smem<T, Q>(), st>>>(A);
+          else
+            k_block<T, Q, SOLVE_NRHS, true, true><<<nb, CH_THREADS, block_smem<T, Q, true>(), st>>>(A);
+        });
         count_launch();
       }
       small_list(h, nq, [&](auto nqc, const int* sl, int ns) {
@@ -1995,9 +1782,10 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
     }
     const int nb = (int) LP.solve_fwd_blocks.size();
     if (nb > 0) {
-      k_fwd_big<double, 1, 1><<<nb, 128, fwd_smem<double>(), st>>>(
-          D.sfwd + D.sfwd_off[h], D.sfwd_ch + D.sfwd_off[h], D.blk_child, D.fronts, D.maps, D.rows, L, Dinv, B, ld, W, 1,
-          flags, ef, status);
+      const SolveArgs<double> A{nullptr, 0, D.sfwd + D.sfwd_off[h], nb, D.sfwd_ch + D.sfwd_off[h], D.blk_child, D.fronts,
+                                D.maps, D.rows, L, Dinv, B, X, ld, W, nullptr, INT_MAX, nullptr, nullptr, flags, 1, nullptr,
+                                ef, status};
+      k_block<double, 1, 1, false, false><<<nb, CH_THREADS, block_smem<double, 1, false>(), st>>>(A);
       count_launch();
     }
   }
@@ -2006,8 +1794,9 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
     const LevelPlan& LP = P.levels[h];
     const int nb = (int) LP.solve_bwd_blocks.size();
     if (nb > 0) {
-      k_bwd_big<double, 1, 1, false><<<nb, 128, bwd_smem<double, 1>(), st>>>(D.sbwd + D.sbwd_off[h], D.fronts, D.rows, L, Dinv, X, ld, W, nullptr, 1,
-                                                 flags, eb, status);
+      const SolveArgs<double> A{nullptr, 0, D.sbwd + D.sbwd_off[h], nb, nullptr, nullptr, D.fronts, D.maps, D.rows, L, Dinv,
+                                nullptr, X, ld, W, nullptr, INT_MAX, nullptr, nullptr, flags, 1, nullptr, eb, status};
+      k_block<double, 1, 1, true, false><<<nb, CH_THREADS, block_smem<double, 1, true>(), st>>>(A);
       count_launch();
     }
     const int ns = (int) LP.small_fronts.size();

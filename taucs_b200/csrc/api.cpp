@@ -123,6 +123,8 @@ int devplan_upload(const Plan& P, DevPlan* D, cudaStream_t st) {
          && dev_upload(&D->pers_solve, (const int*) nullptr, 2 * P.pers_fronts.size() + 4, st)
          && dev_upload(&D->solve_tasks, stasks.data(), stasks.size(), st)
          && dev_upload(&D->child_rec, crec.data(), crec.size(), st)
+         && dev_upload(&D->panel_done, (const int*) nullptr, (size_t) P.n_blk, st)
+         && dev_upload(&D->panel_rdiag, (const double*) nullptr, (size_t) P.n_blk * PANEL_NB, st)
          && dev_upload(&D->dblk, dblk.data(), dblk.size(), st)
          && dev_upload(&D->children, P.children.data(), P.children.size(), st)
          && dev_upload(&D->rows, P.rows.data(), P.rows.size(), st)
@@ -152,6 +154,7 @@ void devplan_free(DevPlan* D) {
   tb::dfree(D->sfwd); tb::dfree(D->sfwd_ch); tb::dfree(D->blk_child); tb::dfree(D->sbwd); tb::dfree(D->sl21); tb::dfree(D->dblk);
   tb::dfree(D->small_num); tb::dfree(D->pers_list); tb::dfree(D->pers_parent); tb::dfree(D->pers_pending0);
   tb::dfree(D->pers_work); tb::dfree(D->pers_solve); tb::dfree(D->solve_tasks); tb::dfree(D->child_rec);
+  tb::dfree(D->panel_done); tb::dfree(D->panel_rdiag);
   *D = DevPlan();
 }
 

@@ -19,10 +19,8 @@ constexpr int SMALL_WARP_F = 32;
 // front-build tile (rows x columns of one front held in shared memory)
 constexpr int BUILD_TR = 128;
 constexpr int BUILD_TC = 32;
-// block column width of the blocked partial Cholesky of large fronts
+// block width of the solve and of the diagonal-block inverses
 constexpr int PANEL_NB = 64;
-// rows per CTA of the panel POTRF+TRSM kernel
-constexpr int TRSM_ROWS = 64;
 // GEMM tile of the trailing / update-matrix kernels
 constexpr int GEMM_BM = 64;
 constexpr int GEMM_BN = 64;
@@ -87,6 +85,8 @@ struct DevPlan {
   int* pers_solve = nullptr;   // per solve: pending counts and done flags (n_pers each) + four queue heads
   SolveTask* solve_tasks = nullptr;   // per persistent task, in queue order
   int4* child_rec = nullptr;   // per entry of children: work vector offset, s, f, map offset
+  int* panel_done = nullptr;   // per factorization: 16-column pieces finished, at FrontDesc::blk_off
+  double* panel_rdiag = nullptr;   // 1 / L_jj of the big fronts' columns, 64 per block (FP32 fronts use the first half)
   int n_pers = 0;
   std::vector<int> small_off, big_off, tile_off, sfwd_off, sbwd_off, sl21_off, small_num_off;  // per level (host)
   std::vector<int> lvl_max_f_small;               // per level (host)

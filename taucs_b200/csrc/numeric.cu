@@ -18,10 +18,10 @@
 //                   duplicate entries are summed) and the children's update
 //                   matrices in a fixed child order into shared memory and
 //                   writes the tile once;
-//   k_leaf          blocked partial Cholesky, step kb: one launch factors
-//                   the 64x64 diagonal block and applies it to every row
-//                   below it (one CTA per 64-row slab, each factoring the
-//                   diagonal block itself);
+//   k_panel         blocked partial Cholesky, step kb: one launch factors
+//                   the 128x128 diagonal block (one CTA per front) and applies
+//                   it to every row below it (a CTA per 64 or 128 rows,
+//                   following it piece by piece);
 //   k_gemm          C -= A B^T on DMMA (mma.sync m16n8k8 f64) tiles: the
 //                   panel updates of a recursive (left half, GEMM, right
 //                   half) panel factorization, and the update matrix
@@ -34,6 +34,7 @@
 // with atomicMin (the reference reports the failing column, :1139-1145).
 #include <climits>
 #include <cstdio>
+#include <type_traits>
 #include <cuda_fp16.h>
 
 #include "kernels.h"
@@ -49,7 +50,12 @@ __device__ __forceinline__ bool failed(const int* status) {
   return *(volatile const int*) status != INT_MAX;
 }
 
-__global__ void k_init_status(int* status) { *status = INT_MAX; }
+// the status word, and the panels' counters
+__global__ void k_init_status(int* status, int* done, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *status = INT_MAX;
+  if (i < n) done[i] = 0;
+}
 
 // ------------------------------------------------------------ small fronts
 
@@ -211,6 +217,19 @@ __device__ __forceinline__ void warp_wait_zero(const int* p, int* status, int ns
     }
     __nanosleep(ns);
   }
+}
+
+// the same until *p is at least v; the value seen
+__device__ __forceinline__ int warp_wait_at_least(const int* p, int v, int* status) {
+  int it = 0, x;
+  while (!__all_sync(0xffffffffu, (x = ld_acquire_gpu(p)) >= v)) {
+    if (++it > (1 << 22)) {
+      atomicMin(status, NUMERIC_TIMEOUT);
+      break;
+    }
+    __nanosleep(20);
+  }
+  return x;
 }
 
 // One front of order f <= SMALL_WARP_F by one warp: the front is assembled
@@ -524,29 +543,10 @@ k_build(const Tile* __restrict__ tiles, const TileChild* __restrict__ tile_ch, c
   }
 }
 
-// ---------------------------------------------------------- panel leaves
+// -------------------------------------------- inverses of the diagonal blocks
 
-// Panel leaf, step kb: the columns [kb, kb + w) of the level's big fronts, w =
-// min(64, s - kb), factored and applied to every row below them in ONE
-// launch (the reference's POTRF :1131 and TRSM :1150 on a 64-column piece).
-// CTA x of front y owns the 64 rows [kb + w + 64 x, ...) below the diagonal
-// block.  Every CTA of the launch reads the diagonal block as it was before
-// the step, so CTA 0 parks the factored block in the block's slot of the
-// inverse array rather than in the panel; k_dinv moves it into the panel
-// after the factorization and replaces it there by its inverse.  Every CTA
-// factors the 64x64 diagonal block itself -- a redundant Cholesky instead of
-// waiting for the CTA that owns it.  Each thread holds one row in registers
-// (threads 0-63 the slab's rows, 64-127 the diagonal block's), and the block
-// goes in four 16-column steps: the warp whose lanes hold the piece's rows
-// factors the 16x16 piece by shuffles, every row below it solves against
-// the piece by substitution, and every row updates its columns to the right
-// from the diagonal block's new rows (published row-major in shared memory).
-// The inverses of the 64x64 diagonal blocks, which the solve applies, are
-// formed afterwards for all fronts at once (k_dinv).  Nothing reads a
-// diagonal block of the panel between its leaf and k_dinv: the later
-// products read rows below it only.
 constexpr int LLD = PANEL_NB + 4;   // padded column stride of k_dinv's blocks in shared memory
-constexpr int LQ = 16;              // column step inside a leaf
+constexpr int LQ = 16;              // its pieces
 constexpr int LYD = LQ + 1;         // column stride of a 16x16 inverse
 
 template <typename T>
@@ -573,234 +573,14 @@ __device__ __forceinline__ void warp_inv16_rows(const T (&a)[LQ], T* Y) {
   }
 }
 
-// One pivot J of the 16x16 warp Cholesky of the leaf, unrolled through the
-// recursion so that every index into the row held in registers is a
-// constant: lane base + i holds row i of the piece (a[k] = L[i][k], k <= i);
-// the pivot comes by shuffle, the column is scaled by rsqrt(pivot), and the
-// columns right of J take the right-looking update.  Lanes outside the piece
-// run along on values that are never written back.
-template <typename T, int J>
-struct CholStep {
-  __device__ __forceinline__ static void run(T (&a)[LQ], int i, int base, int& bad) {
-    const T d = __shfl_sync(0xffffffffu, a[J], base + J);
-    if (!(d > T(0)) && bad < 0) bad = J;
-    const T r = rsqrt_t(d);
-    a[J] = (i == J) ? d * r : a[J] * r;
-#pragma unroll
-    for (int k = J + 1; k < LQ; k++) {
-      const T lkj = __shfl_sync(0xffffffffu, a[J], base + k);
-      if (i >= k) a[k] -= a[J] * lkj;
-    }
-    CholStep<T, J + 1>::run(a, i, base, bad);
-  }
-};
-template <typename T>
-struct CholStep<T, LQ> {
-  __device__ __forceinline__ static void run(T (&)[LQ], int, int, int&) {}
-};
-
-// The split copy of one slab row for the tensor-core products: chunks of CW
-// columns, hi and lo parts, written for chunk indices [0, nch) of the leaf
-// (columns past w are zero: the front's last leaf pads K to the products'
-// stage width).
-template <int CW>
-__device__ __forceinline__ void leaf_split_row(const float (&rw)[PANEL_NB], int w, int nch, unsigned char* base,
-                                               int64_t part, int64_t kc0, int64_t rg, int r) {
-  constexpr int CMAX = PANEL_NB / CW + 4;
-#pragma unroll
-  for (int c = 0; c < CMAX; c++) {
-    if (c >= nch) break;
-    const int64_t o = ((kc0 + c) * rg + (r >> 3)) * 128 + (r & 7) * 16;
-    if (CW == 4) {
-      unsigned h[4], l[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int k = c * 4 + q;
-        const float x = (k < PANEL_NB && k < w) ? rw[k < PANEL_NB ? k : 0] : 0.0f;
-        h[q] = __float_as_uint(x) & 0xffffe000u;
-        l[q] = __float_as_uint(x - __uint_as_float(h[q]));
-      }
-      *reinterpret_cast<uint4*>(base + o) = make_uint4(h[0], h[1], h[2], h[3]);
-      *reinterpret_cast<uint4*>(base + part + o) = make_uint4(l[0], l[1], l[2], l[3]);
-    } else {
-      unsigned short h[8], l[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const int k = c * 8 + q;
-        const float x = (k < PANEL_NB && k < w) ? rw[k < PANEL_NB ? k : 0] : 0.0f;
-        const __half hh = __float2half_rn(x);
-        h[q] = __half_as_ushort(hh);
-        l[q] = __half_as_ushort(__float2half_rn((x - __half2float(hh)) * 2048.0f));
-      }
-      uint4 vh, vl;
-      vh.x = h[0] | (unsigned) h[1] << 16; vh.y = h[2] | (unsigned) h[3] << 16;
-      vh.z = h[4] | (unsigned) h[5] << 16; vh.w = h[6] | (unsigned) h[7] << 16;
-      vl.x = l[0] | (unsigned) l[1] << 16; vl.y = l[2] | (unsigned) l[3] << 16;
-      vl.z = l[4] | (unsigned) l[5] << 16; vl.w = l[6] | (unsigned) l[7] << 16;
-      *reinterpret_cast<uint4*>(base + o) = vh;
-      *reinterpret_cast<uint4*>(base + part + o) = vl;
-    }
-  }
-}
-template <int CW>
-__device__ __forceinline__ void leaf_split_row(const double (&)[PANEL_NB], int, int, unsigned char*, int64_t, int64_t,
-                                               int64_t, int) {}
-
-template <typename T, int SPF>
-__global__ void __launch_bounds__(128)
-k_leaf(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
-       T* __restrict__ L, T* __restrict__ Dinv, float* __restrict__ sp, int kb, int* status) {
-  // SPF: the split format of the copy for the tensor-core products (one
-  // instantiation each: the fully unrolled row code is large)
-  constexpr int sp_fmt = SPF;
-  // Xt[buf][c][k]: the new L[c][c0 + k] of the diagonal block's rows c below
-  // the current piece (row-major, 16-byte aligned rows, two buffers by piece
-  // parity); Lp, rinv: the factored piece and its reciprocal diagonal
-  constexpr int XLD = sizeof(T) == 4 ? LQ + 4 : LQ + 2;
-  __shared__ __align__(16) T Xt[2][PANEL_NB][XLD];
-  __shared__ T Lp[LQ][LQ + 1];
-  __shared__ T rinv[LQ];
-  __shared__ int bad_s;
-  if (failed(status)) return;
-  const FrontDesc F = fronts[list[blockIdx.y]];
-  const int f = F.f, s = F.s;
-  if (kb >= s) return;
-  const int w = min(PANEL_NB, s - kb);
-  const int r0 = kb + w + blockIdx.x * PANEL_NB;
-  const int nr = max(0, min(PANEL_NB, f - r0));
-  if (blockIdx.x > 0 && nr == 0) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // threads 0-63: the slab's rows; threads 64-127: the diagonal block's rows
-  // (identity past w); each thread holds its row's 64 entries in registers
-  const bool is_d = tid >= PANEL_NB;
-  const int i = is_d ? tid - PANEL_NB : tid;
-  T* P = L + F.l_off;
-  T rw[PANEL_NB];
-  {
-    const size_t g = is_d ? (size_t) (kb + i) : (size_t) (r0 + i);
-    const bool rv = is_d ? (i < w) : (i < nr);
-#pragma unroll
-    for (int c = 0; c < PANEL_NB; c++) {
-      const bool in = rv && c < w && (!is_d || c <= i);
-      rw[c] = in ? P[g + (size_t) (kb + c) * f] : ((is_d && c == i) ? T(1) : T(0));
-    }
-  }
-  // the four 16-column pieces in a rolled loop over one body: the row is
-  // rotated left by 16 entries after each piece, so the current piece is
-  // always rw[0..15] and its trailing columns rw[16..63 - c0] (after the
-  // fourth rotation the row is back in column order); one copy of the row
-  // code instead of four keeps the kernel's instructions cache-resident
-#pragma unroll 1
-  for (int b = 0; b < PANEL_NB / LQ; b++) {
-    const int c0 = b * LQ;
-    // the piece's 16 rows are lanes base .. base + 15 of warp 2 + c0 / 32
-    const int base = c0 % 32;
-    if (warp == 2 + c0 / 32) {
-      const int ii = lane - base;
-      T a[LQ];
-#pragma unroll
-      for (int k = 0; k < LQ; k++) a[k] = (k <= ii) ? rw[k] : T(0);
-      int bad = -1;
-      CholStep<T, 0>::run(a, ii, base, bad);
-      if (ii >= 0 && ii < LQ) {
-        T dg = T(1);
-#pragma unroll
-        for (int k = 0; k < LQ; k++) {
-          if (k <= ii) rw[k] = a[k];
-          Lp[ii][k] = (k <= ii) ? a[k] : T(0);
-          if (k == ii) dg = a[k];
-        }
-        rinv[ii] = T(1) / dg;
-      }
-      if (lane == 0) bad_s = bad;
-    }
-    __syncthreads();
-    if (bad_s >= 0) {
-      if (tid == 0 && blockIdx.x == 0 && c0 + bad_s < w) atomicMin(status, rows[F.rows_off + kb + c0 + bad_s]);
-      return;
-    }
-    // rows below the piece: X L_p^T = M by substitution (in registers), the
-    // diagonal block's rows also published for the update below
-    const bool below = !is_d || i >= c0 + LQ;
-    T x[LQ];
-#pragma unroll
-    for (int c = 0; c < LQ; c++) x[c] = rw[c];
-    if (below) {
-#pragma unroll
-      for (int c = 0; c < LQ; c++) {
-        x[c] *= rinv[c];
-#pragma unroll
-        for (int c2 = c + 1; c2 < LQ; c2++) x[c2] -= x[c] * Lp[c2][c];
-      }
-#pragma unroll
-      for (int c = 0; c < LQ; c++) rw[c] = x[c];
-      if (is_d) {
-#pragma unroll
-        for (int c = 0; c < LQ; c++) Xt[b & 1][i][c] = x[c];
-      }
-    }
-    __syncthreads();
-    // the columns right of the piece: rw[c] -= sum_k x[k] L[c0 + c][c0 + k].
-    // A warp of the diagonal block stops at the last row it holds (the
-    // columns past it are upper-triangle entries of all its rows, never
-    // read): the warp that factors the next piece is on the chain and does
-    // the least
-    const int cmax = (is_d ? (warp - 2) * 32 + 31 : PANEL_NB - 1) - c0;
-    if (below) {
-#pragma unroll
-      for (int c = LQ; c < PANEL_NB; c++) {
-        if (c > cmax) break;
-        const T* xr = Xt[b & 1][c0 + c];
-        T acc = rw[c];
-#pragma unroll
-        for (int k = 0; k < LQ; k++) acc -= x[k] * xr[k];
-        rw[c] = acc;
-      }
-    }
-    // rotate left by one piece
-#pragma unroll
-    for (int k = 0; k < LQ; k++) x[k] = rw[k];
-#pragma unroll
-    for (int k = 0; k < PANEL_NB - LQ; k++) rw[k] = rw[k + LQ];
-#pragma unroll
-    for (int k = 0; k < LQ; k++) rw[PANEL_NB - LQ + k] = x[k];
-  }
-  if (is_d) {
-    if (blockIdx.x == 0) {
-      T* Dk = Dinv + F.dinv_off + (size_t) (kb / PANEL_NB) * PANEL_NB * PANEL_NB;
-#pragma unroll
-      for (int c = 0; c < PANEL_NB; c++) Dk[i + c * PANEL_NB] = (c <= i && i < w) ? rw[c] : T(0);
-    }
-    return;
-  }
-  if (i < nr) {
-    const size_t g = (size_t) (r0 + i);
-#pragma unroll
-    for (int c = 0; c < PANEL_NB; c++)
-      if (c < w) P[g + (size_t) (kb + c) * f] = rw[c];
-    if (sizeof(T) == 4 && sp != nullptr && F.sp_off >= 0) {
-      // the row's final values, split, into the split arena for the tensor-
-      // core products; the front's last leaf also writes the zero columns
-      // that pad K to the products' stage width
-      const int64_t rg = sp_rgroups(f), part = sp_part_bytes(F, sp_fmt);
-      unsigned char* base = reinterpret_cast<unsigned char*>(sp + F.sp_off);
-      const int cw = sp_chunk_cols(sp_fmt);
-      const int kc_end = (kb + w == s) ? (int) sp_kchunks(s, sp_fmt) : (kb + w) / cw;
-      const int nch = kc_end - kb / cw;
-      leaf_split_row<SPF ? 8 : 4>(rw, w, nch, base, part, kb / (SPF ? 8 : 4), rg, r0 + i);
-    }
-  }
-}
-
-// After the factorization, one CTA per 64x64 diagonal block of every big
-// front: the factored block L_kk that its leaf parked in the block's slot of
-// Dinv goes into the panel, and the slot receives L_kk^-1 (lower, zero
-// beyond the block's width), which the solve applies.  Warp q inverts the
-// 16x16 diagonal piece q; then warp b forms block column b below the
-// diagonal, X_cb = -X_cc sum_{b<=k<c} L_ck X_kb.
+// After the factorization, one CTA per 64x64 diagonal block L_kk of every big
+// front: its inverse (lower, zero beyond the block's width), which the solve
+// applies, into the block's slot of Dinv.  Warp q inverts the 16x16 diagonal
+// piece q; then warp b forms block column b below the diagonal, X_cb = -X_cc
+// sum_{b<=k<c} L_ck X_kb.
 template <typename T>
 __global__ void __launch_bounds__(128)
-k_dinv(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts, T* __restrict__ L,
+k_dinv(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts, const T* __restrict__ L,
        T* __restrict__ Dinv, const int* status) {
   extern __shared__ __align__(16) unsigned char smraw[];
   T* S = reinterpret_cast<T*>(smraw);   // L_kk, 64 x 64, ld LLD (identity beyond w)
@@ -811,16 +591,15 @@ k_dinv(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts, T
   const FrontDesc F = fronts[bl.a];
   const int f = F.f, kb = bl.b * PANEL_NB;
   const int w = min(PANEL_NB, F.s - kb);
-  T* P = L + F.l_off;
+  const T* P = L + F.l_off;
   T* Di = Dinv + F.dinv_off + (size_t) bl.b * PANEL_NB * PANEL_NB;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #pragma unroll 8
   for (int t = 0; t < PANEL_NB * PANEL_NB / 128; t++) {
     const int e = tid + 128 * t, i = e % PANEL_NB, j = e / PANEL_NB;
-    const T v = (i < w && j < w && i >= j) ? Di[e] : (i == j ? T(1) : T(0));
+    const T v = (i < w && j < w && i >= j) ? P[(kb + i) + (size_t) (kb + j) * f] : (i == j ? T(1) : T(0));
     S[i + j * LLD] = v;
     X[i + j * LLD] = T(0);
-    if (i < w && j < w && i >= j) P[(kb + i) + (size_t) (kb + j) * f] = v;
   }
   __syncthreads();
   {
@@ -898,6 +677,446 @@ __device__ __forceinline__ void cp_async_t(float* smem, const float* gmem, bool 
   const unsigned saddr = (unsigned) __cvta_generic_to_shared(smem);
   const int sz = pred ? 4 : 0;
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(saddr), "l"(gmem), "r"(sz));
+}
+
+// ---------------------------------------------------------------- panels
+
+// A panel step: the columns [kb, kb + w) of the level's big fronts, w = min(128,
+// s - kb), factored and applied to every row below them in ONE launch (the
+// reference's POTRF :1131 and TRSM :1150 on a 128-column piece).  What bounds
+// it is the chain of pivots, so one CTA per front (the first nb of the launch)
+// holds the w x w diagonal block in shared memory and does nothing but that
+// chain, in 16-column pieces: the first warp brings the next piece's diagonal
+// rows up to date and factors it while the others update the rest.  Each
+// finished piece goes to the panel behind a counter (release/acquire); the
+// other CTAs hold NT / 4 rows below the block each, follow the counter, solve their
+// rows against the piece and update their columns to the right.  They have
+// higher indices than every diagonal CTA and wait for nothing else, so each
+// wait ends; the waits are bounded all the same.
+//
+// The code is kept small: the kernel that this one replaced held rows in
+// registers (64 columns a launch) and ran as straight-line code, 4 warps of it
+// on an SM, which instruction fetch bounded (the 136 multiply-adds of a
+// piece's substitution took 4600 cycles, 700 when they were still in the
+// instruction cache).  Here a piece's Cholesky is a loop over pivots, products
+// are small tile loops (FP64: DMMA fragments; FP32: multiply-adds in FP32).
+// Panel steps and the products between them per factorization, before (64
+// columns a launch) and now: 64^3 FP64 10.3 + 17.2 ms -> 7.2 + 13.4, 40x41x39
+// FP64 2.96 + 2.82 -> 2.20 + 1.67, 80^3 FP32 13.3 + 11.8 -> 12.6 + 8.5,
+// 139x142 FP32 0.59 + 0.13 -> 0.43 + 0.01.
+constexpr int PW = 128;              // columns of a panel step
+constexpr int PB = 16;               // columns of a piece
+constexpr int PLDB = PW + 4;         // column stride of a piece that a row CTA reads
+// The diagonal block: piece p holds its 16 columns from row 16 p on, column
+// stride PLDD - 16 p (a multiple of four elements, and no two rows of a FP64
+// fragment in the same bank); FP32 leaves room for the rows of a 32-row unit
+// that are past the block's last
+template <typename T>
+constexpr int PLDD = PW + (sizeof(T) == 4 ? 20 : 4);
+template <typename T>
+__host__ __device__ constexpr int diag_base(int p) { return PB * (PLDD<T> * p - 8 * p * (p - 1)); }
+// rows of a row CTA of NT threads, and the column stride of their entries
+template <int NT>
+constexpr int PROWS = NT / 4;
+template <int NT>
+constexpr int PLDR = PROWS<NT> + 4;
+// shared memory of a launch whose widest step has wmax columns
+template <typename T, int NT>
+constexpr size_t panel_smem(int wmax) {
+  const int np = (wmax + PB - 1) / PB;
+  const size_t d = (size_t) diag_base<T>(np) + 2 * (PB * (PB + 1) + PB);
+  const size_t r = (size_t) np * PB * PLDR<NT> + 2 * (PB * PLDB + PB);
+  return (d > r ? d : r) * sizeof(T);
+}
+
+// Pivots J0 .. J1-1 of a piece with at most NC columns right of them.  Lane i
+// holds row i, moved one entry to the left per pivot (column J is always
+// a[0]).  The scaled column goes to the other lanes through shared memory
+// (written relative to the pivot, read back as vectors): with a shuffle per
+// column a piece took 4700 cycles in FP32 and 8000 in FP64, this way 2700 and
+// 3300.  The next pivot comes from lane J + 1's own entries by one shuffle, and
+// its reciprocal square root is on its way before the other columns are
+// updated.
+template <typename T, int NC>
+__device__ __forceinline__ void chol_pivots(T (&a)[PB], int J0, int J1, int i, T& d, T& r, T& rown, int& bad, T* buf,
+                                            T* Lp, T* col, int ldc) {
+  constexpr int V = 16 / (int) sizeof(T);
+  struct alignas(16) Vec { T v[V]; };
+#pragma unroll 1
+  for (int J = J0; J < J1; J++) {
+    if (!(d > T(0)) && bad < 0) bad = J;
+    const T l = (i == J) ? d * r : a[0] * r;
+    if (i == J) rown = r;
+    T* b = buf + (J & 1) * 32;
+    b[(i - J - 1) & 31] = l;
+    if (i >= J && i < PB) {
+      Lp[i * (PB + 1) + J] = l;
+      col[J * ldc + i] = l;
+    }
+    d = __shfl_sync(0xffffffffu, a[1] - l * l, J + 1);
+    r = rsqrt_t(d);
+    __syncwarp();
+    Vec x[(NC + 1) / V];
+#pragma unroll
+    for (int k = 0; k < (NC + 1) / V; k++) x[k] = reinterpret_cast<const Vec*>(b)[k];
+#pragma unroll
+    for (int k = 1; k <= NC; k++) a[k - 1] = a[k] - l * x[(k - 1) / V].v[(k - 1) % V];
+  }
+}
+// Cholesky factor of a 16x16 piece by one warp, lane i < 16 with row i (col:
+// its columns, stride ldc; what lies above the diagonal and in the next 16 rows
+// is read but reaches no result), into Lp
+// (row stride 17), the reciprocal diagonal into rinv and back into col; bad:
+// the first nonpositive pivot, or -1.  buf: 64 entries of the warp's own.
+template <typename T>
+__device__ __forceinline__ void chol_piece(T* col, int ldc, T* Lp, T* rinv, int* bad_out, T* buf) {
+  const int i = threadIdx.x & 31;
+  T a[PB];
+#pragma unroll
+  for (int k = 0; k < PB; k++) a[k] = col[k * ldc + i];
+  int bad = -1;
+  T d = __shfl_sync(0xffffffffu, a[0], 0), r = rsqrt_t(d), rown = T(1);
+  chol_pivots<T, PB - 1>(a, 0, PB / 2, i, d, r, rown, bad, buf, Lp, col, ldc);
+  chol_pivots<T, PB / 2 - 1>(a, PB / 2, PB, i, d, r, rown, bad, buf, Lp, col, ldc);
+  if (i < PB) rinv[i] = rown;
+  if (i == 0) *bad_out = bad;
+}
+
+// x L_p^T = m for one row of 16 entries (stride ld); Lp[i sr + k sc] the piece
+template <typename T>
+__device__ __forceinline__ void solve_row(T* m, int ld, const T* Lp, int sr, int sc, const T* rinv) {
+  T x[PB];
+#pragma unroll
+  for (int c = 0; c < PB; c++) x[c] = m[c * ld];
+#pragma unroll
+  for (int c = 0; c < PB; c++) {
+    x[c] *= rinv[c];
+#pragma unroll
+    for (int c2 = c + 1; c2 < PB; c2++) x[c2] -= x[c] * Lp[c2 * sr + c * sc];
+  }
+  // (stores between the columns would hold back the loads of the next one)
+#pragma unroll
+  for (int c = 0; c < PB; c++) m[c * ld] = x[c];
+}
+
+// C[0..RU) x [0..16) -= A B^T by one warp, K = 16: C and A column-major (row 0 of
+// the unit first), B[c + k ldb] the row c of the other operand.  run: the units
+// of the trailing updates; diag: a 16 x 16 piece.  FP64: DMMA fragments; FP32:
+// multiply-adds, four by four (a diagonal piece four by two) entries a lane.
+template <typename T>
+struct PanelUnit;
+template <>
+struct PanelUnit<double> {
+  static constexpr int RU = 16;
+  __device__ __forceinline__ static void run(double* C, int ldc, const double* A, int lda, const double* B, int ldb) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    double acc[2][4], *c0 = C + g + (2 * t) * ldc;
+#pragma unroll
+    for (int ni = 0; ni < 2; ni++) {
+      const double* c = c0 + 8 * ni * ldc;
+      acc[ni][0] = -c[0]; acc[ni][1] = -c[ldc]; acc[ni][2] = -c[8]; acc[ni][3] = -c[ldc + 8];
+    }
+#pragma unroll
+    for (int kk = 0; kk < PB; kk += 8) {
+      const double* a = A + g + (kk + t) * lda;
+      const double* b = B + g + (kk + t) * ldb;
+      const double av[4] = {a[0], a[8], a[4 * lda], a[4 * lda + 8]};
+#pragma unroll
+      for (int ni = 0; ni < 2; ni++) {
+        const double bv[2] = {b[8 * ni], b[4 * ldb + 8 * ni]};
+        dmma16888(acc[ni], av, bv);
+      }
+    }
+#pragma unroll
+    for (int ni = 0; ni < 2; ni++) {
+      double* c = c0 + 8 * ni * ldc;
+      c[0] = -acc[ni][0]; c[ldc] = -acc[ni][1]; c[8] = -acc[ni][2]; c[ldc + 8] = -acc[ni][3];
+    }
+  }
+  __device__ __forceinline__ static void diag(double* C, int ldc, const double* A, int lda) {
+    run(C, ldc, A, lda, A, lda);
+  }
+};
+template <>
+struct PanelUnit<float> {
+  static constexpr int RU = 32;
+  // R x CC entries a lane, K8 columns of both operands loaded at a time
+  template <int CC>
+  __device__ __forceinline__ static void unit(float* C, int ldc, const float* A, int lda, const float* B, int ldb, int r,
+                                              int c) {
+    float acc[CC][4] = {};
+#pragma unroll 1
+    for (int k0 = 0; k0 < PB; k0 += 8) {
+      float4 a[8];
+      float b[8][CC];
+#pragma unroll
+      for (int k = 0; k < 8; k++) a[k] = *reinterpret_cast<const float4*>(A + r + (k0 + k) * lda);
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        struct alignas(4 * CC) Vec { float v[CC]; };
+        const Vec x = *reinterpret_cast<const Vec*>(B + c + (k0 + k) * ldb);
+#pragma unroll
+        for (int j = 0; j < CC; j++) b[k][j] = x.v[j];
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+#pragma unroll
+        for (int j = 0; j < CC; j++) {
+          acc[j][0] += a[k].x * b[k][j];
+          acc[j][1] += a[k].y * b[k][j];
+          acc[j][2] += a[k].z * b[k][j];
+          acc[j][3] += a[k].w * b[k][j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < CC; j++) {
+      float4* p = reinterpret_cast<float4*>(C + r + (c + j) * ldc);
+      float4 v = *p;
+      v.x -= acc[j][0]; v.y -= acc[j][1]; v.z -= acc[j][2]; v.w -= acc[j][3];
+      *p = v;
+    }
+  }
+  __device__ __forceinline__ static void run(float* C, int ldc, const float* A, int lda, const float* B, int ldb) {
+    const int lane = threadIdx.x & 31;
+    unit<4>(C, ldc, A, lda, B, ldb, 4 * (lane & 7), 4 * (lane >> 3));
+  }
+  __device__ __forceinline__ static void diag(float* C, int ldc, const float* A, int lda) {
+    const int lane = threadIdx.x & 31;
+    unit<2>(C, ldc, A, lda, A, lda, 4 * (lane & 3), 2 * (lane >> 2));
+  }
+};
+
+// The split copy of one slab row for the tensor-core products (FP32): chunk c
+// of CW columns of row r, hi and lo parts; x: the row's entries (stride ld),
+// zero from column w on.
+template <int FMT>
+__device__ __forceinline__ void split_chunk(const float* x, int ld, int c, int w, unsigned char* dst, int64_t part) {
+  if (FMT == 0) {
+    unsigned h[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int k = c * 4 + q;
+      const float v = k < w ? x[k * ld] : 0.0f;
+      h[q] = __float_as_uint(v) & 0xffffe000u;
+      l[q] = __float_as_uint(v - __uint_as_float(h[q]));
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(dst + part) = make_uint4(l[0], l[1], l[2], l[3]);
+  } else {
+    unsigned h[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      unsigned hh = 0, ll = 0;
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int k = c * 8 + 2 * q + e;
+        const float v = k < w ? x[k * ld] : 0.0f;
+        const __half hv = __float2half_rn(v);
+        hh |= (unsigned) __half_as_ushort(hv) << (16 * e);
+        ll |= (unsigned) __half_as_ushort(__float2half_rn((v - __half2float(hv)) * 2048.0f)) << (16 * e);
+      }
+      h[q] = hh;
+      l[q] = ll;
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(dst + part) = make_uint4(l[0], l[1], l[2], l[3]);
+  }
+}
+
+template <typename T, int FMT, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT)
+k_panel(const int* __restrict__ list, int nb, int gx, const FrontDesc* __restrict__ fronts,
+        const int* __restrict__ rows, T* __restrict__ L, float* __restrict__ sp, int kb, int* __restrict__ done,
+        double* __restrict__ rdiag_all, int* status) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ __align__(16) T buf_s[64];
+  __shared__ int bad_s[2];
+  T* S = reinterpret_cast<T*>(smraw);
+  const bool is_diag = (int) blockIdx.x < nb;
+  const int y = is_diag ? (int) blockIdx.x : ((int) blockIdx.x - nb) / gx;
+  const FrontDesc F = fronts[list[y]];
+  if (__syncthreads_or(failed(status))) return;   // all threads together
+  const int f = F.f, s = F.s;
+  if (kb >= s) return;
+  const int w = min(PW, s - kb), np = (w + PB - 1) / PB;
+  T* P = L + F.l_off;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NW = NT / 32, RU = PanelUnit<T>::RU, PROWS = tb::PROWS<NT>, PLDR = tb::PLDR<NT>;
+  int* cnt = done + F.blk_off;          // pieces of the front finished so far
+  T* rdiag = reinterpret_cast<T*>(rdiag_all) + (size_t) F.blk_off * PANEL_NB;   // 1 / L_jj
+  const int first = kb / PB;            // of them before this step
+
+  if (is_diag) {
+    // -------------------------------------------------------- diagonal block
+    T* Lp0 = S + diag_base<T>(np);     // two factored pieces, by parity
+    T* rinv0 = Lp0 + 2 * PB * (PB + 1);
+    auto at = [&](int p) { return S + diag_base<T>(p); };   // row 16 p of piece p's first column
+    auto ldp = [&](int p) { return PLDD<T> - PB * p; };
+    // lower part of the block, rows and columns past w as the identity
+    const int w16 = np * PB;
+    const int crew = (warp >> 2) * 3 + (warp & 3) - 1;   // of the warps that solve and update
+    for (int j = warp; j < w16; j += NW) {
+      const int p = j / PB;
+      T* c = at(p) + (j - PB * p) * ldp(p) - PB * p;
+      for (int i = PB * p + lane; i < w16; i += 32) {
+        if (i < w && j < w) cp_async_t(c + i, P + (kb + i) + (size_t) (kb + j) * f, true);
+        else c[i] = i == j ? T(1) : T(0);
+      }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    if (warp == 0) chol_piece<T>(at(0), ldp(0), Lp0, rinv0, &bad_s[0], buf_s);
+    __syncthreads();
+    for (int p = 0; p < np; p++) {
+      const T* Lp = Lp0 + (p & 1) * PB * (PB + 1);
+      const T* rinv = rinv0 + (p & 1) * PB;
+      const int t0 = (p + 1) * PB;
+      if (bad_s[p & 1] >= 0) {
+        // the row CTAs leave on the status; the counter releases them
+        if (tid == 0) {
+          atomicMin(status, rows[F.rows_off + kb + p * PB + bad_s[p & 1]]);
+          __threadfence();
+          atomicExch(cnt, INT_MAX);
+        }
+        return;
+      }
+      T* cp = at(p) - PB * p;   // piece p by block row
+      if ((warp & 3) != 0) {
+        const int r = t0 + crew * 32 + lane;
+        if (r < w16) solve_row<T>(cp + r, ldp(p), Lp, PB + 1, 1, rinv);
+      }
+      __syncthreads();
+      // the first warp: the next piece, and nothing else.  The other warps of
+      // its scheduler do nothing (their instructions would take the chain's
+      // issue slots: with the write-out there a step was 5 % slower)
+      auto unit = [&](int r0, int q0) {   // rows r0.., the columns of the piece at q0
+        const int q = q0 / PB;
+        PanelUnit<T>::run(at(q) - q0 + r0, ldp(q), cp + r0, ldp(p), cp + q0, ldp(p));
+      };
+      if (warp == 0) {
+        if (t0 < w16) {
+          PanelUnit<T>::diag(at(p + 1), ldp(p + 1), cp + t0, ldp(p));
+          __syncwarp();
+          chol_piece<T>(at(p + 1), ldp(p + 1), Lp0 + ((p + 1) & 1) * PB * (PB + 1), rinv0 + ((p + 1) & 1) * PB,
+                        &bad_s[(p + 1) & 1], buf_s);
+        }
+      } else {
+        if ((warp & 3) != 0) {
+          // the last three of them write this piece out first
+          constexpr int PT = 96, CREW = NW / 4 * 3;
+          const int t = (crew - (CREW - 3)) * 32 + lane;
+          if (t >= 0) {
+            for (int e = t; e < PB * PW / 4; e += PT) {
+              // four rows apart: every load before the first store
+              T v[4];
+              const int j = e / (PW / 4), i = e % (PW / 4);
+#pragma unroll
+              for (int q = 0; q < 4; q++) v[q] = p * PB + j <= i + 32 * q ? cp[i + 32 * q + j * ldp(p)] : T(0);
+#pragma unroll
+              for (int q = 0; q < 4; q++) {
+                const int r = i + 32 * q, c = p * PB + j;
+                if (r >= c && r < w && c < w) P[(kb + r) + (size_t) (kb + c) * f] = v[q];
+              }
+            }
+            if (t < PB && p * PB + t < w) rdiag[(first + p) * PB + t] = rinv[t];
+            asm volatile("bar.sync 1, %0;" ::"n"(PT) : "memory");
+            if (t == 0) {
+              __threadfence();
+              asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(cnt), "r"(first + p + 1) : "memory");
+            }
+          }
+          // the other units of the trailing lower part
+          int turn = crew;
+          for (int c = t0; c < w16; c += PB)
+            for (int r0 = c == t0 ? t0 + PB : c; r0 < w16; r0 += RU) {
+              if (turn == 0) {
+                unit(r0, c);
+                turn = CREW;
+              }
+              turn--;
+            }
+        }
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  // ------------------------------------------------------------ rows below
+  const int r0 = kb + w + ((int) blockIdx.x - nb) % gx * PROWS;
+  const int nr = min(PROWS, f - r0);
+  if (nr <= 0) return;
+  for (int j = warp; j < np * PB; j += NW)
+    for (int i = lane; i < PROWS; i += 32) {
+      const bool in = i < nr && j < w;   // zero elsewhere
+      cp_async_t(S + i + j * PLDR, P + r0 + (in ? i : 0) + (size_t) (kb + (in ? j : 0)) * f, in);
+    }
+  cp_async_commit();
+  // pieces of the diagonal block, [column][row] and the reciprocal diagonal, in
+  // two buffers: the next piece's loads (from L2: the block was written during
+  // this launch) are on their way, when it is finished, during this one's work
+  constexpr int NPRE = PB * PW / NT;
+  T pre[NPRE], pri = T(0);
+  auto fetch = [&](int p) {
+    const int j0 = p * PB, i = tid % PW;
+#pragma unroll
+    for (int e = 0; e < NPRE; e++) {
+      const int j = tid / PW + e * (NT / PW);
+      pre[e] = (i < w && j0 + j < w && i >= j0 + j) ? __ldcg(P + (kb + i) + (size_t) (kb + j0 + j) * f) : T(0);
+    }
+    if (tid < PB) pri = j0 + tid < w ? __ldcg(rdiag + first * PB + j0 + tid) : T(1);
+  };
+  int have = 0;             // pieces known to be finished (the first warp's lanes)
+  bool fetched = false;     // the same on every thread: bad_s carries it
+  for (int p = 0; p < np; p++) {
+    T* Bp = S + np * PB * PLDR + (p & 1) * (PB * PLDB + PB);
+    T* rinv = Bp + PB * PLDB;
+    if (!fetched) {
+      if (warp == 0 && have <= p) have = warp_wait_at_least(cnt, first + p + 1, status) - first;
+      __syncthreads();
+      fetch(p);
+    }
+#pragma unroll
+    for (int e = 0; e < NPRE; e++) Bp[tid % PW + (tid / PW + e * (NT / PW)) * PLDB] = pre[e];
+    if (tid < PB) rinv[tid] = pri;
+    if (warp == 0 && p + 1 < np) {
+      if (have <= p + 1) have = ld_acquire_gpu(cnt) - first;
+      if (lane == 0) bad_s[p & 1] = have > p + 1;
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    fetched = p + 1 < np && bad_s[p & 1];
+    if (fetched) fetch(p + 1);
+    const int j0 = p * PB;
+    T* Sp = S + j0 * PLDR;
+    if (tid < PROWS) solve_row<T>(Sp + tid, PLDR, Bp + j0, 1, PLDB, rinv);
+    __syncthreads();
+    // one unit after the other, row groups first
+    constexpr int NR = PROWS / RU;
+    for (int u = warp; u < (np - 1 - p) * NR; u += NW) {
+      const int c = j0 + PB + u / NR * PB, r = u % NR * RU;
+      PanelUnit<T>::run(S + r + c * PLDR, PLDR, Sp + r, PLDR, Bp + c, PLDB);
+    }
+  }
+  if (__syncthreads_or(failed(status))) return;
+  for (int j = warp; j < w; j += NW)
+    for (int i = lane; i < nr; i += 32) P[r0 + i + (size_t) (kb + j) * f] = S[i + j * PLDR];
+  if constexpr (sizeof(T) == 4) {
+    if (sp != nullptr && F.sp_off >= 0) {
+      // the rows' final values, split, into the split arena for the tensor-
+      // core products; the front's last step also writes the zero columns
+      // that pad K to the products' stage width
+      const int64_t rg = sp_rgroups(f), part = sp_part_bytes(F, FMT);
+      unsigned char* base = reinterpret_cast<unsigned char*>(sp + F.sp_off);
+      constexpr int CW = FMT ? 8 : 4;
+      const int kc0 = kb / CW, kc_end = (kb + w == s) ? (int) sp_kchunks(s, FMT) : (kb + w) / CW;
+      const int i = tid % PROWS;
+      if (i < nr)
+        for (int c = tid / PROWS; c < kc_end - kc0; c += NT / PROWS)
+          split_chunk<FMT>(S + i, PLDR, c, w,
+                           base + ((int64_t) (kc0 + c) * rg + ((r0 + i) >> 3)) * 128 + ((r0 + i) & 7) * 16, part);
+    }
+  }
 }
 
 // FP64 fronts: one DMMA per fragment pair
@@ -1226,6 +1445,17 @@ static void set_smem_attrs() {
                          SMALL_F_MAX * SMALL_F_MAX * (int) sizeof(T));
     cudaFuncSetAttribute(k_small_persistent<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          SMALL_F_MAX * SMALL_F_MAX * (int) sizeof(T));
+    auto panel = [](auto fmt, auto nt) {
+      constexpr int NT = decltype(nt)::value;
+      cudaFuncSetAttribute(k_panel<T, decltype(fmt)::value, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int) panel_smem<T, NT>(PW));
+    };
+    panel(std::integral_constant<int, 0>(), std::integral_constant<int, 256>());
+    panel(std::integral_constant<int, 0>(), std::integral_constant<int, 512>());
+    if constexpr (sizeof(T) == 4) {
+      panel(std::integral_constant<int, 1>(), std::integral_constant<int, 256>());
+      panel(std::integral_constant<int, 1>(), std::integral_constant<int, 512>());
+    }
     cudaFuncSetAttribute(k_dinv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dinv_smem<T>());
     cudaFuncSetAttribute(k_gemm<T, 64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int) GemmCfg<64, 64>::smem<T>());
@@ -1239,7 +1469,7 @@ template <typename T>
 static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, T* U, T* Dinv, float* sp,
                           int sp_fmt, int* status, cudaStream_t st) {
   set_smem_attrs<T>();
-  k_init_status<<<1, 1, 0, st>>>(status);
+  k_init_status<<<(P.n_blk + 255) / 256, 256, 0, st>>>(status, D.panel_done, P.n_blk);
   count_launch();
   if (D.n_pers > 0) {
     // every small front with only small fronts below it, in two launches:
@@ -1327,19 +1557,19 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
     }
     // recursive panel factorization over aligned column intervals: factor
     // the left half, update the right half with one GEMM (K = half width),
-    // factor the right half; leaves are 64-column steps (k_leaf: POTRF of
-    // the diagonal block and TRSM of the rows below in one launch)
+    // factor the right half; the intervals of PW columns are panel steps
     const int S = LP.max_s_big;
-    int span = PANEL_NB;
+    int span = PW;
     while (span < S) span *= 2;
-    auto leaf = [&](int kb) {
-      int gx = 1;
+    auto panel = [&](int kb) {
+      int rmax = 0, wmax = 0;
       double fl = 0.0, by = 0.0;
       for (int fi : LP.big_fronts) {
         const FrontDesc& F = P.fronts[fi];
         if (kb >= F.s) continue;
-        const int w = std::min(PANEL_NB, F.s - kb);
-        gx = std::max(gx, (F.f - kb - w + PANEL_NB - 1) / PANEL_NB);
+        const int w = std::min(PW, F.s - kb);
+        wmax = std::max(wmax, w);
+        rmax = std::max(rmax, F.f - kb - w);
         if (prof_enabled()) {
           const double ww = w, below = F.f - kb - w;
           fl += ww * ww * ww / 3.0 + below * ww * ww;
@@ -1347,15 +1577,30 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
         }
       }
       prof_begin(KC_LEAF, st);
-      if (sp_fmt)
-        k_leaf<T, 1><<<dim3(gx, nb), 128, 0, st>>>(blst, D.fronts, D.rows, L, Dinv, sp, kb, status);
-      else
-        k_leaf<T, 0><<<dim3(gx, nb), 128, 0, st>>>(blst, D.fronts, D.rows, L, Dinv, sp, kb, status);
+      auto run = [&](auto fmt, auto nt) {
+        constexpr int NT = decltype(nt)::value;
+        const int gx = (rmax + PROWS<NT> - 1) / PROWS<NT>;
+        k_panel<T, decltype(fmt)::value, NT><<<nb + nb * gx, NT, panel_smem<T, NT>(wmax), st>>>(
+            blst, nb, std::max(gx, 1), D.fronts, D.rows, L, sp, kb, D.panel_done, D.panel_rdiag, status);
+      };
+      // 16 warps a CTA (128 rows) while every CTA has an SM to itself (29x24x26
+      // FP32: 0.80 ms of panels -> 0.72), 8 on fuller launches, where two CTAs
+      // share an SM and one's updates fill the other's waits
+      auto size = [&](auto fmt) {
+        if (nb + nb * ((rmax + PROWS<512> - 1) / PROWS<512>) <= 148) run(fmt, std::integral_constant<int, 512>());
+        else run(fmt, std::integral_constant<int, 256>());
+      };
+      if constexpr (sizeof(T) == 4) {
+        if (sp_fmt) size(std::integral_constant<int, 1>());
+        else size(std::integral_constant<int, 0>());
+      } else {
+        size(std::integral_constant<int, 0>());
+      }
       prof_end(KC_LEAF, st, fl, by);
       count_launch();
     };
     auto update = [&](int c_lo, int c_hi, int k_lo, int k_hi) {
-      int gx = 0, gx64 = 0, maxc = 0, maxr = 0;
+      int gx = 0, gx64 = 0;
       double fg = 0.0, bg = 0.0;
       for (int fi : LP.big_fronts) {
         const FrontDesc& F = P.fronts[fi];
@@ -1363,8 +1608,6 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
         if (c_lo >= ce) continue;
         gx = std::max(gx, trap_tiles(F.f - c_lo, ce - c_lo, 128, 128));
         gx64 = std::max(gx64, trap_tiles(F.f - c_lo, ce - c_lo, 64, 64));
-        maxc = std::max(maxc, ce - c_lo);
-        maxr = std::max(maxr, F.f - c_lo);
         if (prof_enabled()) {
           const double c = ce - c_lo, below = F.f - ce, k = k_hi - k_lo;
           const double entries = c * (c + 1.0) / 2.0 + below * c;
@@ -1374,22 +1617,21 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       }
       if (gx64 == 0) return;
       prof_begin(KC_GEMM_PANEL, st);
-      (void) maxr; (void) maxc;
       launch_gemm(gemm_alt<T>(P, h, 0), gx, gx64, nb, blst, D, L, U, c_lo, c_hi, k_lo, k_hi, 0, status, st, sp, gx, sp_fmt);
       prof_end(KC_GEMM_PANEL, st, fg, bg);
       count_launch();
     };
     struct Rec {
-      static void run(int a, int b, int S_, const decltype(leaf)& lf, const decltype(update)& up) {
+      static void run(int a, int b, int S_, const decltype(panel)& lf, const decltype(update)& up) {
         if (a >= S_) return;
-        if (b - a <= PANEL_NB) { lf(a); return; }
+        if (b - a <= PW) { lf(a); return; }
         const int mid = (a + b) / 2;
         run(a, mid, S_, lf, up);
         if (mid < S_) up(mid, b, a, mid);
         run(mid, b, S_, lf, up);
       }
     };
-    Rec::run(0, span, S, leaf, update);
+    Rec::run(0, span, S, panel, update);
     int gx_u = 0, gx_u64 = 0, gx_usp = 0, maxm = 0;
     for (int fi : LP.big_fronts) {
       const FrontDesc& F = P.fronts[fi];

@@ -103,7 +103,7 @@ size_t predict_bytes(const Plan& P) {
              + (double) sizeof(FrontDesc) * P.fronts.size() + 4.0 * (solve_flag_words(P) + 1)
              // the solve's tasks, child records and per-block child records
              + (double) sizeof(SolveTask) * P.pers_fronts.size()
-             + 16.0 * (3.0 * P.children.size() + P.maps.size() / PANEL_NB + 0.5 * P.n_blk);
+             + 16.0 * (3.0 * P.children.size() + P.maps.size() / PANEL_NB + (0.75 + 32.0) * P.n_blk);
   // the build tiles and their child records
   for (const LevelPlan& LP : P.levels)
     for (const Tile& t : LP.build_tiles)

@@ -32,6 +32,7 @@
 #include <cstdint>
 
 #include "kernels.h"
+#include "launch.h"
 
 namespace tb {
 namespace {
@@ -142,6 +143,7 @@ template <int STAGES, int MINB, int NPROD>
 __global__ void __launch_bounds__(NPROD + 32, MINB)
 k_gemm_tc(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, float* __restrict__ L,
           float* __restrict__ U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status) {
+  grid_wait();
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 1];   // full[S], empty[S], done
   __shared__ unsigned tmem_slot;
   __shared__ int abort_cta;
@@ -410,7 +412,6 @@ k_gemm_sp(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, co
   __shared__ unsigned tmem_slot;
   __shared__ int abort_cta;
   extern __shared__ __align__(16) unsigned char sp_raw[];
-  if (*(volatile const int*) status != INT_MAX) return;
   const FrontDesc F = fronts[list[blockIdx.y]];
   const int f = F.f, s = F.s, m = f - s;
   // tile grid origin (a row-group boundary), the valid rows/columns and K
@@ -450,6 +451,8 @@ k_gemm_sp(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, co
   const unsigned sbase = (smem_u32(sp_raw) + 1023u) & ~1023u;
   const unsigned full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[STAGES]),
                  done = smem_u32(&bars[2 * STAGES]);
+  grid_wait();
+  if (__syncthreads_or(*(volatile const int*) status != INT_MAX)) return;
   if (tid == 0) {
     for (int i = 0; i < STAGES; i++) {
       mbar_init(full0 + 8 * i, 1);
@@ -537,6 +540,7 @@ k_gemm_sp(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, co
     if (lane == 0) tc_commit(done);
     __syncwarp();
   }
+  grid_trigger();
   // ---- epilogue: warp w owns TMEM lanes (tile rows) 32 w .. 32 w + 31.
   // The first 32 columns of the old C rows are loaded before the wait for
   // the products (they do not depend on them), and each later group while
@@ -624,10 +628,10 @@ int gemm_sp_tiles_u(int s, int f) {
 void launch_gemm_sp(int fmt, int gx, int nb, const int* list, const FrontDesc* fronts, const float* sp, float* L,
                     float* U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st) {
   if (fmt)
-    k_gemm_sp<3, 1><<<dim3(gx, nb), 128, sp_smem<3>(), st>>>(list, fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode,
+    launch(k_gemm_sp<3, 1>, dim3(gx, nb), 128, sp_smem<3>(), st, list, fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode,
                                                              status);
   else
-    k_gemm_sp<3, 0><<<dim3(gx, nb), 128, sp_smem<3>(), st>>>(list, fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode,
+    launch(k_gemm_sp<3, 0>, dim3(gx, nb), 128, sp_smem<3>(), st, list, fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode,
                                                              status);
 }
 
@@ -654,10 +658,10 @@ int gemm_tc_tiles(int rows, int cols) {
 void launch_gemm_tc(int variant, int gx, int nb, const int* list, const FrontDesc* fronts, float* L, float* U,
                     int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st) {
   if (variant == 1)
-    k_gemm_tc<3, 2, 256><<<dim3(gx, nb), 256 + 32, tc_smem<3>(), st>>>(list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
+    launch(k_gemm_tc<3, 2, 256>, dim3(gx, nb), 256 + 32, tc_smem<3>(), st, list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
                                                                        mode, status);
   else
-    k_gemm_tc<2, 3, 128><<<dim3(gx, nb), 128 + 32, tc_smem<2>(), st>>>(list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
+    launch(k_gemm_tc<2, 3, 128>, dim3(gx, nb), 128 + 32, tc_smem<2>(), st, list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
                                                                        mode, status);
 }
 

@@ -38,6 +38,7 @@
 #include <cuda_fp16.h>
 
 #include "kernels.h"
+#include "launch.h"
 
 namespace tb {
 
@@ -50,11 +51,15 @@ __device__ __forceinline__ bool failed(const int* status) {
   return *(volatile const int*) status != INT_MAX;
 }
 
-// the status word, and the panels' counters
-__global__ void k_init_status(int* status, int* done, int n) {
+// the status word, the panels' counters and the persistent launches' pending
+// counts and queue heads
+__global__ void k_init_status(int* status, int* done, int n, const int* __restrict__ pending0, int* work, int np) {
+  grid_wait_then_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *status = INT_MAX;
   if (i < n) done[i] = 0;
+  if (i < np) work[i] = pending0[i];
+  if (np > 0 && i < 2) work[np + i] = 0;
 }
 
 // ------------------------------------------------------------ small fronts
@@ -190,6 +195,7 @@ k_small_front(const int* __restrict__ list, const FrontDesc* __restrict__ fronts
               const int* __restrict__ a_rows, const int* __restrict__ a_idx,
               const T* __restrict__ vals, T* __restrict__ L, T* __restrict__ U,
               int* status) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   if (failed(status)) return;
   small_front<T>(fronts[list[blockIdx.x]], fronts, reinterpret_cast<T*>(smraw), children, maps, rows, acol_ptr, a_rows,
@@ -339,6 +345,7 @@ k_small_warp(const int* __restrict__ tasks, int t0, int t1, const int* __restric
              const int* __restrict__ maps, const int* __restrict__ rows, const int* __restrict__ acol_ptr,
              const int* __restrict__ a_rows, const int* __restrict__ a_idx, const T* __restrict__ vals,
              T* __restrict__ L, T* __restrict__ U, int* status) {
+  grid_wait();
   __shared__ T Ws_all[4][SMALL_WARP_F][SMALL_WARP_F + 1];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   for (;;) {
@@ -375,6 +382,7 @@ k_small_persistent(const int* __restrict__ tasks, int t0, int t1, const int* __r
                    const int* __restrict__ maps, const int* __restrict__ rows, const int* __restrict__ acol_ptr,
                    const int* __restrict__ a_rows, const int* __restrict__ a_idx, const T* __restrict__ vals,
                    T* __restrict__ L, T* __restrict__ U, int* status) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int t_s, skip_s;
   T* W = reinterpret_cast<T*>(smraw);
@@ -411,6 +419,7 @@ constexpr int BUILD_THREADS = 128;
 __global__ void __launch_bounds__(128)
 k_tile_ranges(const Tile* __restrict__ tiles, const FrontDesc* __restrict__ fronts, const int* __restrict__ children,
               const int* __restrict__ maps, TileChild* __restrict__ rec) {
+  grid_wait();
   const Tile tl = tiles[blockIdx.x];
   const FrontDesc F = fronts[tl.front];
   const int f = F.f, s = F.s, m = f - s;
@@ -451,7 +460,6 @@ k_build(const Tile* __restrict__ tiles, const TileChild* __restrict__ tile_ch, c
         const int* __restrict__ a_idx, const T* __restrict__ vals,
         T* __restrict__ L, T* __restrict__ U, const int* status) {
   __shared__ T W[BUILD_TR * BUILD_TC];
-  if (failed(status)) return;
   const Tile tl = tiles[blockIdx.x];
   const FrontDesc F = fronts[tl.front];
   const int f = F.f, s = F.s, m = f - s;
@@ -486,6 +494,9 @@ k_build(const Tile* __restrict__ tiles, const TileChild* __restrict__ tile_ch, c
     }
     __syncthreads();
   }
+  // (above: nothing that a kernel of this factorization writes)
+  grid_wait();
+  if (failed(status)) return;
   // the children's shares, in child order, from the tile's records (found
   // once per plan); every load of a child's share is issued before the
   // first add (the children's update matrices were written by earlier
@@ -528,6 +539,7 @@ k_build(const Tile* __restrict__ tiles, const TileChild* __restrict__ tile_ch, c
       }
     __syncthreads();
   }
+  grid_trigger();
   if (panel) {
     T* dst = L + F.l_off;
     for (int k = tid; k < BUILD_TR * BUILD_TC; k += nt) {
@@ -582,6 +594,7 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 k_dinv(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts, const T* __restrict__ L,
        T* __restrict__ Dinv, const int* status) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   T* S = reinterpret_cast<T*>(smraw);   // L_kk, 64 x 64, ld LLD (identity beyond w)
   T* X = S + PANEL_NB * LLD;            // its inverse, ld LLD
@@ -935,9 +948,10 @@ k_panel(const int* __restrict__ list, int nb, int gx, const FrontDesc* __restric
   const bool is_diag = (int) blockIdx.x < nb;
   const int y = is_diag ? (int) blockIdx.x : ((int) blockIdx.x - nb) / gx;
   const FrontDesc F = fronts[list[y]];
-  if (__syncthreads_or(failed(status))) return;   // all threads together
   const int f = F.f, s = F.s;
   if (kb >= s) return;
+  grid_wait();
+  if (__syncthreads_or(failed(status))) return;   // all threads together
   const int w = min(PW, s - kb), np = (w + PB - 1) / PB;
   T* P = L + F.l_off;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1099,6 +1113,7 @@ k_panel(const int* __restrict__ list, int nb, int gx, const FrontDesc* __restric
     }
   }
   if (__syncthreads_or(failed(status))) return;
+  grid_trigger();
   for (int j = warp; j < w; j += NW)
     for (int i = lane; i < nr; i += 32) P[r0 + i + (size_t) (kb + j) * f] = S[i + j * PLDR];
   if constexpr (sizeof(T) == 4) {
@@ -1204,7 +1219,6 @@ k_gemm(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __
   constexpr int MI = Cfg::MI, NI = Cfg::NI, LD = Cfg::LD, NT = Cfg::THREADS;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* gsm = reinterpret_cast<T*>(smraw);   // GEMM_STAGES x {A, B} x GEMM_BK x LD
-  if (failed(status)) return;
   const FrontDesc F = fronts[list[blockIdx.y]];
   const int f = F.f, s = F.s, m = f - s;
   int rows, cols, roff, kbeg, kend, ldc;
@@ -1242,6 +1256,8 @@ k_gemm(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp % Cfg::WM, wn = warp / Cfg::WM, g = lane >> 2, t = lane & 3;
   const int wrow = wm * (BM / Cfg::WM), wcol = wn * 32;
+  grid_wait();
+  if (failed(status)) return;
   // accumulators start at -C, so acc = A B^T - C and the result is -acc
   T acc[MI][NI][4];
 #pragma unroll
@@ -1313,6 +1329,7 @@ k_gemm(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __
     }
   }
   cp_async_wait<0>();
+  grid_trigger();
 #pragma unroll
   for (int mi = 0; mi < MI; mi++)
 #pragma unroll
@@ -1373,11 +1390,11 @@ static void launch_gemm(bool big, int gx128, int gx64, int nb, const int* blst, 
                         int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st,
                         const float* = nullptr, int = 0, int = 0) {
   if (big)
-    k_gemm<T, 128, 128><<<dim3(gx128, nb), GemmCfg<128, 128>::THREADS, GemmCfg<128, 128>::smem<T>(), st>>>(
-        blst, D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status);
+    launch(k_gemm<T, 128, 128>, dim3(gx128, nb), GemmCfg<128, 128>::THREADS, GemmCfg<128, 128>::smem<T>(), st, blst,
+        D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status);
   else
-    k_gemm<T, 64, 64><<<dim3(gx64, nb), GemmCfg<64, 64>::THREADS, GemmCfg<64, 64>::smem<T>(), st>>>(
-        blst, D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status);
+    launch(k_gemm<T, 64, 64>, dim3(gx64, nb), GemmCfg<64, 64>::THREADS, GemmCfg<64, 64>::smem<T>(), st, blst,
+        D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status);
 }
 
 // FP32 fronts take the tcgen05 kernels (gemm_tc.cu): by default the one fed
@@ -1469,7 +1486,11 @@ template <typename T>
 static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, T* U, T* Dinv, float* sp,
                           int sp_fmt, int* status, cudaStream_t st) {
   set_smem_attrs<T>();
-  k_init_status<<<(P.n_blk + 255) / 256, 256, 0, st>>>(status, D.panel_done, P.n_blk);
+  {
+    const int n = std::max(std::max(P.n_blk, D.n_pers), 2);
+    launch(k_init_status, (n + 255) / 256, 256, 0, st, status, D.panel_done, P.n_blk, D.pers_pending0, D.pers_work,
+        D.n_pers);
+  }
   count_launch();
   if (D.n_pers > 0) {
     // every small front with only small fronts below it, in two launches:
@@ -1477,8 +1498,6 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
     // (tasks 0 .. nw-1), then one CTA per front for the rest (their children
     // in the first part counted themselves off in the first launch)
     const int nw = P.pers_nwarp, np = D.n_pers;
-    cudaMemcpyAsync(D.pers_work, D.pers_pending0, sizeof(int) * np, cudaMemcpyDeviceToDevice, st);
-    cudaMemsetAsync(D.pers_work + np, 0, 2 * sizeof(int), st);
     auto prof_range = [&](int t0, int t1, double& fl, double& by) {
       fl = by = 0.0;
       if (prof_enabled())
@@ -1492,7 +1511,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       const int grid = std::min((nw + 3) / 4, warp_grid<T>());
       prof_range(0, nw, fl, by);
       prof_begin(KC_SMALL, st);
-      k_small_warp<T><<<grid, 128, 0, st>>>(D.pers_list, 0, nw, D.pers_parent, D.pers_work, D.pers_work + np,
+      launch(k_small_warp<T>, grid, 128, 0, st, D.pers_list, 0, nw, D.pers_parent, D.pers_work, D.pers_work + np,
                                             D.fronts, D.children, D.maps, D.rows, D.acol_ptr, D.a_rows, D.a_idx,
                                             vals, L, U, status);
       prof_end(KC_SMALL, st, fl, by);
@@ -1503,7 +1522,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       const int grid = std::min(np - nw, pers_grid<T>(smem));
       prof_range(nw, np, fl, by);
       prof_begin(KC_SMALL, st);
-      k_small_persistent<T><<<grid, 128, smem, st>>>(D.pers_list, nw, np, D.pers_parent, D.pers_work,
+      launch(k_small_persistent<T>, grid, 128, smem, st, D.pers_list, nw, np, D.pers_parent, D.pers_work,
                                                      D.pers_work + np + 1, D.fronts, D.children, D.maps, D.rows,
                                                      D.acol_ptr, D.a_rows, D.a_idx, vals, L, U, status);
       prof_end(KC_SMALL, st, fl, by);
@@ -1533,7 +1552,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
               by += front_bytes(P, F, sizeof(T));
             }
           prof_begin(KC_SMALL, st);
-          k_small_front<T><<<e - b, 128, smem, st>>>(lst + b, D.fronts, D.children, D.maps, D.rows,
+          launch(k_small_front<T>, e - b, 128, smem, st, lst + b, D.fronts, D.children, D.maps, D.rows,
                                                    D.acol_ptr, D.a_rows, D.a_idx, vals, L, U, status);
           prof_end(KC_SMALL, st, fl, by);
           count_launch();
@@ -1550,7 +1569,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       if (prof_enabled())
         for (int fi : LP.big_fronts) by += build_bytes(P, P.fronts[fi], sizeof(T));
       prof_begin(KC_BUILD, st);
-      k_build<T><<<ntiles, BUILD_THREADS, 0, st>>>(D.tiles + D.tile_off[h], D.tile_ch, D.fronts, D.maps, D.acol_ptr,
+      launch(k_build<T>, ntiles, BUILD_THREADS, 0, st, D.tiles + D.tile_off[h], D.tile_ch, D.fronts, D.maps, D.acol_ptr,
                                       D.a_rows, D.a_idx, vals, L, U, status);
       prof_end(KC_BUILD, st, 0.0, by);
       count_launch();
@@ -1580,8 +1599,8 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       auto run = [&](auto fmt, auto nt) {
         constexpr int NT = decltype(nt)::value;
         const int gx = (rmax + PROWS<NT> - 1) / PROWS<NT>;
-        k_panel<T, decltype(fmt)::value, NT><<<nb + nb * gx, NT, panel_smem<T, NT>(wmax), st>>>(
-            blst, nb, std::max(gx, 1), D.fronts, D.rows, L, sp, kb, D.panel_done, D.panel_rdiag, status);
+        launch(k_panel<T, decltype(fmt)::value, NT>, nb + nb * gx, NT, panel_smem<T, NT>(wmax), st, blst, nb,
+            std::max(gx, 1), D.fronts, D.rows, L, sp, kb, D.panel_done, D.panel_rdiag, status);
       };
       // 16 warps a CTA (128 rows) while every CTA has an SM to itself (29x24x26
       // FP32: 0.80 ms of panels -> 0.72), 8 on fuller launches, where two CTAs
@@ -1662,7 +1681,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
   prof_tag(-1);
   if (D.n_dblk > 0) {
     prof_begin(KC_DINV, st);
-    k_dinv<T><<<D.n_dblk, 128, dinv_smem<T>(), st>>>(D.dblk, D.fronts, L, Dinv, status);
+    launch(k_dinv<T>, D.n_dblk, 128, dinv_smem<T>(), st, D.dblk, D.fronts, L, Dinv, status);
     prof_end(KC_DINV, st, (double) D.n_dblk * PANEL_NB * PANEL_NB * PANEL_NB / 3.0,
              2.0 * sizeof(T) * D.n_dblk * PANEL_NB * PANEL_NB);
     count_launch();
@@ -1671,7 +1690,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
 }
 
 int launch_tile_ranges(const DevPlan& D, int ntiles, cudaStream_t st) {
-  k_tile_ranges<<<ntiles, 128, 0, st>>>(D.tiles, D.fronts, D.children, D.maps, D.tile_ch);
+  launch(k_tile_ranges, ntiles, 128, 0, st, D.tiles, D.fronts, D.children, D.maps, D.tile_ch);
   return (int) cudaGetLastError();
 }
 

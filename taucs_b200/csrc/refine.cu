@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "factor.h"
+#include "launch.h"
 
 namespace tb {
 
@@ -27,6 +28,7 @@ namespace {
 
 __global__ void k_diag_scale(int n, const int* __restrict__ diagpos, const double* __restrict__ vals,
                              double* __restrict__ scale, int* status) {
+  grid_wait();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const double d = diagpos[j] >= 0 ? vals[diagpos[j]] : 0.0;
@@ -41,6 +43,7 @@ __global__ void k_diag_scale(int n, const int* __restrict__ diagpos, const doubl
 __global__ void k_scaled_f32(long nnz, const int* __restrict__ rowind, const int* __restrict__ colidx,
                              const double* __restrict__ vals, const double* __restrict__ scale,
                              float* __restrict__ out) {
+  grid_wait();
   const long k = (long) blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nnz) return;
   out[k] = (float) (vals[k] * scale[rowind[k]] * scale[colidx[k]]);
@@ -71,6 +74,7 @@ __global__ void k_residual(int n, const int* __restrict__ rp, const int* __restr
                            const int* __restrict__ vi, const double* __restrict__ vals,
                            const double* __restrict__ X, const double* __restrict__ B, double* __restrict__ R,
                            int ld, int ldr, int nrhs, const int* __restrict__ seg, unsigned long long* norms) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int sg = (seg && i < n) ? seg[i] : 0;
   // the row's entries eight at a time, then every column's products with
@@ -116,6 +120,7 @@ __global__ void k_residual(int n, const int* __restrict__ rp, const int* __restr
 // that the residual gathers one 64-byte row per matrix entry instead of
 // eight scattered values
 __global__ void k_interleave(int n, const double* __restrict__ X, int ld, int nrhs, double* __restrict__ Xi) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double v[SOLVE_NRHS];
@@ -134,6 +139,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_residual_i(int n, const int* __
                              const int* __restrict__ vi, const double* __restrict__ vals,
                              const double* __restrict__ Xi, const double* __restrict__ B, double* __restrict__ R,
                              int ld, int ldr, int nrhs, const int* __restrict__ seg, unsigned long long* norms) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int sg = (seg && i < n) ? seg[i] : 0;
   double acc[SOLVE_NRHS];
@@ -220,6 +226,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_residual_i(int n, const int* __
 
 __global__ void k_scale_down(int n, const double* __restrict__ R, const double* __restrict__ scale,
                              float* __restrict__ out, int ld, int nrhs) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int q = 0; q < nrhs; q++) out[i + (size_t) q * n] = (float) (R[i + (size_t) q * ld] * scale[i]);
@@ -227,6 +234,7 @@ __global__ void k_scale_down(int n, const double* __restrict__ R, const double* 
 
 __global__ void k_update32(int n, double* __restrict__ X, const float* __restrict__ D, const double* __restrict__ scale,
                            int ld, int nrhs) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int q = 0; q < nrhs; q++) X[i + (size_t) q * ld] += scale[i] * (double) D[i + (size_t) q * n];
@@ -237,6 +245,7 @@ __global__ void k_update32(int n, double* __restrict__ X, const float* __restric
 // once per pattern)
 __global__ void k_gather_values(long nnz, const int* __restrict__ vmap, const double* __restrict__ raw,
                                 double* __restrict__ out) {
+  grid_wait();
   for (long k = (long) blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (long) gridDim.x * blockDim.x)
     out[k] = raw[vmap[k]];
 }
@@ -245,6 +254,7 @@ __global__ void k_gather_values(long nnz, const int* __restrict__ vmap, const do
 // and dst[perm[i]] = src[i], nq columns, original-order vectors with ld n
 __global__ void k_perm_gather(int n, int nq, const int* __restrict__ perm, const double* __restrict__ src,
                               double* __restrict__ dst) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int pi = perm[i];
@@ -253,6 +263,7 @@ __global__ void k_perm_gather(int n, int nq, const int* __restrict__ perm, const
 
 __global__ void k_perm_scatter(int n, int nq, const int* __restrict__ perm, const double* __restrict__ src,
                                double* __restrict__ dst) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int pi = perm[i];
@@ -260,6 +271,7 @@ __global__ void k_perm_scatter(int n, int nq, const int* __restrict__ perm, cons
 }
 
 __global__ void k_update64(int n, double* __restrict__ X, const double* __restrict__ D, int ld, int ldd, int nrhs) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int q = 0; q < nrhs; q++) X[i + (size_t) q * ld] += D[i + (size_t) q * ldd];
@@ -277,6 +289,7 @@ struct Coef {
 // Y = A X for nq columns (symmetric CSR of both triangles; leading dimension n)
 __global__ void k_spmv(int n, const int* __restrict__ rp, const int* __restrict__ ci, const int* __restrict__ vi,
                        const double* __restrict__ vals, const double* __restrict__ X, double* __restrict__ Y, int nq) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int q = 0; q < nq; q++) {
@@ -289,6 +302,7 @@ __global__ void k_spmv(int n, const int* __restrict__ rp, const int* __restrict_
 // Z = D d: an FP32 correction scaled back to A's variables
 __global__ void k_scale_up(int n, const float* __restrict__ D, const double* __restrict__ scale, double* __restrict__ Z,
                            int nq) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int q = 0; q < nq; q++) Z[i + (size_t) q * n] = scale[i] * (double) D[i + (size_t) q * n];
@@ -299,6 +313,7 @@ __global__ void k_scale_up(int n, const float* __restrict__ D, const double* __r
 // adds the block sums in block order
 __global__ void __launch_bounds__(256) k_dot_part(int n, int nq, const double* __restrict__ A,
                                                   const double* __restrict__ B, double* __restrict__ part) {
+  grid_wait();
   __shared__ double sh[256];
   for (int q = 0; q < nq; q++) {
     double acc = 0.0;
@@ -316,6 +331,7 @@ __global__ void __launch_bounds__(256) k_dot_part(int n, int nq, const double* _
 }
 
 __global__ void k_dot_final(int nblocks, int nq, const double* __restrict__ part, double* __restrict__ out) {
+  grid_wait();
   const int q = threadIdx.x;
   if (q >= nq) return;
   double acc = 0.0;
@@ -325,6 +341,7 @@ __global__ void k_dot_final(int nblocks, int nq, const double* __restrict__ part
 
 // search direction: P = Z + beta P (P = Z on a (re)start)
 __global__ void k_pcg_dir(int n, int nq, const double* __restrict__ Z, double* __restrict__ Pd, Coef beta, int restart) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int q = 0; q < nq; q++) {
@@ -338,6 +355,7 @@ __global__ void k_pcg_dir(int n, int nq, const double* __restrict__ Z, double* _
 __global__ void k_pcg_step(int n, int nq, double* __restrict__ X, int ld, double* __restrict__ R,
                            const double* __restrict__ Pd, const double* __restrict__ Q, Coef alpha,
                            unsigned long long* norms) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   for (int q = 0; q < nq; q++) {
     double r = 0.0, x = 0.0;
@@ -355,12 +373,16 @@ __global__ void k_pcg_step(int n, int nq, double* __restrict__ X, int ld, double
   }
 }
 
-__global__ void k_init_status2(int* s) { *s = INT_MAX; }
+__global__ void k_init_status2(int* s) {
+  grid_wait_then_trigger();
+  *s = INT_MAX;
+}
 
 // ||A||_inf of the full symmetric matrix from the CSR of both triangles
 // ||A||_inf per segment: out[s]
 __global__ void k_anorm(int n, const int* __restrict__ rp, const int* __restrict__ vi, const double* __restrict__ vals,
                         const int* __restrict__ seg, unsigned long long* out) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int sg = (seg && i < n) ? seg[i] : 0;
   double a = 0.0;
@@ -449,9 +471,9 @@ int numeric_fp32_device(Factor* F, const double* d_vals) {
                         "published values"))
     return -1;
   F->dvals_cur = d_vals;
-  k_init_status2<<<1, 1, 0, st>>>(F->dstatus);
-  k_diag_scale<<<nblk(F->n, 256), 256, 0, st>>>(F->n, F->ddiagpos, d_vals, F->dscale, F->dstatus);
-  k_scaled_f32<<<nblk(P.nnz, 256), 256, 0, st>>>(P.nnz, F->drowind, F->dcolidx, d_vals, F->dscale, F->dA32);
+  launch(k_init_status2, 1, 1, 0, st, F->dstatus);
+  launch(k_diag_scale, nblk(F->n, 256), 256, 0, st, F->n, F->ddiagpos, d_vals, F->dscale, F->dstatus);
+  launch(k_scaled_f32, nblk(P.nnz, 256), 256, 0, st, P.nnz, F->drowind, F->dcolidx, d_vals, F->dscale, F->dA32);
   count_launch(3);
   cudaMemcpyAsync(F->hstatus, F->dstatus, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (!cuda_ok(cudaStreamSynchronize(st), "scaling")) return -1;
@@ -504,8 +526,8 @@ static int pcg_fp32(Factor* F, int nq, double* X, const double* B, int ld, doubl
   double* Z = Q + nv;
   double* R = F->dR;
   auto dots = [&](const double* a, const double* b, int slot) {
-    k_dot_part<<<DOT_BLOCKS, 256, 0, st>>>(n, nq, a, b, F->ddot_part);
-    k_dot_final<<<1, 32, 0, st>>>(DOT_BLOCKS, nq, F->ddot_part, F->ddot + slot * SOLVE_NRHS);
+    launch(k_dot_part, DOT_BLOCKS, 256, 0, st, n, nq, a, b, F->ddot_part);
+    launch(k_dot_final, 1, 32, 0, st, DOT_BLOCKS, nq, F->ddot_part, F->ddot + slot * SOLVE_NRHS);
     count_launch(2);
   };
   auto fetch = [&](void* h, const void* d, size_t bytes) {
@@ -513,7 +535,7 @@ static int pcg_fp32(Factor* F, int nq, double* X, const double* B, int ld, doubl
   };
   auto true_residual = [&]() {
     cudaMemsetAsync(F->dnorm, 0, norm_bytes(F), st);
-    k_residual<<<nblk(n, 256), 256, 0, st>>>(n, F->dcsr_ptr, F->dcsr_col, F->dcsr_val, F->dvals_cur, X, B, R, ld, n,
+    launch(k_residual, nblk(n, 256), 256, 0, st, n, F->dcsr_ptr, F->dcsr_col, F->dcsr_val, F->dvals_cur, X, B, R, ld, n,
                                              nq, nullptr, F->dnorm);
     count_launch();
     return fetch(F->hnorm, F->dnorm, norm_bytes(F)) && cuda_ok(cudaStreamSynchronize(st), "pcg residual");
@@ -538,10 +560,10 @@ static int pcg_fp32(Factor* F, int nq, double* X, const double* B, int ld, doubl
   bool restart = true;
   for (int it = 0; it < F->pcg_maxits;) {
     // z = M^-1 r and rho = r.z
-    k_scale_down<<<nblk(n, 256), 256, 0, st>>>(n, R, F->dscale, F->dV32, n, nq);
+    launch(k_scale_down, nblk(n, 256), 256, 0, st, n, R, F->dscale, F->dV32, n, nq);
     int e = launch_solve_fp32(P, F->dp, F->dL32, F->dDinv32, nq, F->dV32, F->dV32, n, F->dW32, F->dpart32, F->dflags,
                               &F->epoch, F->dstatus + 1, st);
-    k_scale_up<<<nblk(n, 256), 256, 0, st>>>(n, F->dV32, F->dscale, Z, nq);
+    launch(k_scale_up, nblk(n, 256), 256, 0, st, n, F->dV32, F->dscale, Z, nq);
     count_launch(2);
     if (e) return -2;
     dots(R, Z, 0);
@@ -552,8 +574,8 @@ static int pcg_fp32(Factor* F, int nq, double* X, const double* B, int ld, doubl
       beta.v[q] = (!restart && rho_old[q] > 0 && rho[q] > 0) ? rho[q] / rho_old[q] : 0.0;
     }
     // p = z + beta p, q = A p, alpha = rho / p.q
-    k_pcg_dir<<<nblk(n, 256), 256, 0, st>>>(n, nq, Z, Pd, beta, restart ? 1 : 0);
-    k_spmv<<<nblk(n, 256), 256, 0, st>>>(n, F->dcsr_ptr, F->dcsr_col, F->dcsr_val, F->dvals_cur, Pd, Q, nq);
+    launch(k_pcg_dir, nblk(n, 256), 256, 0, st, n, nq, Z, Pd, beta, restart ? 1 : 0);
+    launch(k_spmv, nblk(n, 256), 256, 0, st, n, F->dcsr_ptr, F->dcsr_col, F->dcsr_val, F->dvals_cur, Pd, Q, nq);
     count_launch(2);
     dots(Pd, Q, 1);
     if (!fetch(F->hdot + SOLVE_NRHS, F->ddot + SOLVE_NRHS, sizeof(double) * SOLVE_NRHS) ||
@@ -565,7 +587,7 @@ static int pcg_fp32(Factor* F, int nq, double* X, const double* B, int ld, doubl
     }
     // x += alpha p, r -= alpha q, and the norms of the updated residual
     cudaMemsetAsync(F->dnorm, 0, norm_bytes(F), st);
-    k_pcg_step<<<nblk(n, 256), 256, 0, st>>>(n, nq, X, ld, R, Pd, Q, alpha, F->dnorm);
+    launch(k_pcg_step, nblk(n, 256), 256, 0, st, n, nq, X, ld, R, Pd, Q, alpha, F->dnorm);
     count_launch();
     if (!fetch(F->hnorm, F->dnorm, norm_bytes(F)) || !cuda_ok(cudaStreamSynchronize(st), "pcg")) return -2;
     rho_old = rho;
@@ -601,9 +623,9 @@ static int refine_device(Factor* F, int nrhs, double* dX, const double* dB, int 
     // r = b - A x and the inf-norms of r and x per segment, read back
     auto residual = [&](cudaStream_t s) {
       cudaMemsetAsync(F->dnorm, 0, norm_bytes(F), s);
-      k_interleave<<<nblk(n, 256), 256, 0, s>>>(n, X, ld, nq, F->dXi);
-      k_residual_i<<<nblk(n, RES_THREADS), RES_THREADS, 0, s>>>(n, F->dcsr_ptr, F->dcsr_col, F->dcsr_val, F->dvals_cur, F->dXi, B,
-                                                F->dR, ld, n, nq, F->dseg, F->dnorm);
+      launch(k_interleave, nblk(n, 256), 256, 0, s, n, X, ld, nq, F->dXi);
+      launch(k_residual_i, nblk(n, RES_THREADS), RES_THREADS, 0, s, n, F->dcsr_ptr, F->dcsr_col, F->dcsr_val,
+          F->dvals_cur, F->dXi, B, F->dR, ld, n, nq, F->dseg, F->dnorm);
       count_launch(2);
       cudaMemcpyAsync(F->hnorm, F->dnorm, norm_bytes(F), cudaMemcpyDeviceToHost, s);
       return (int) cudaGetLastError();
@@ -614,12 +636,12 @@ static int refine_device(Factor* F, int nrhs, double* dX, const double* dB, int 
       if (u64) {
         e = launch_solve_fp64(P, F->dp, F->dL, F->dDinv, nq, F->dR, F->dR, n, F->dW, F->dpart, F->dflags, &F->epoch,
                               F->dstatus + 1, s);
-        k_update64<<<nblk(n, 256), 256, 0, s>>>(n, X, F->dR, ld, n, nq);
+        launch(k_update64, nblk(n, 256), 256, 0, s, n, X, F->dR, ld, n, nq);
       } else {
-        k_scale_down<<<nblk(n, 256), 256, 0, s>>>(n, F->dR, F->dscale, F->dV32, n, nq);
+        launch(k_scale_down, nblk(n, 256), 256, 0, s, n, F->dR, F->dscale, F->dV32, n, nq);
         e = launch_solve_fp32(P, F->dp, F->dL32, F->dDinv32, nq, F->dV32, F->dV32, n, F->dW32, F->dpart32,
                               F->dflags, &F->epoch, F->dstatus + 1, s);
-        k_update32<<<nblk(n, 256), 256, 0, s>>>(n, X, F->dV32, F->dscale, ld, nq);
+        launch(k_update32, nblk(n, 256), 256, 0, s, n, X, F->dV32, F->dscale, ld, nq);
       }
       count_launch(2);
       return e ? e : residual(s);
@@ -722,7 +744,7 @@ static int device_anorm(Factor* F, std::vector<double>* anorm) {
   cudaStream_t st = current_stream();
   const int ns = F->nseg();
   cudaMemsetAsync(F->dnorm, 0, sizeof(unsigned long long) * ns, st);
-  k_anorm<<<nblk(F->n, 256), 256, 0, st>>>(F->n, F->dcsr_ptr, F->dcsr_val, F->dvals_cur, F->dseg, F->dnorm);
+  launch(k_anorm, nblk(F->n, 256), 256, 0, st, F->n, F->dcsr_ptr, F->dcsr_val, F->dvals_cur, F->dseg, F->dnorm);
   count_launch();
   cudaMemcpyAsync(F->hnorm, F->dnorm, sizeof(unsigned long long) * ns, cudaMemcpyDeviceToHost, st);
   if (!cuda_ok(cudaStreamSynchronize(st), "norm")) return -1;
@@ -734,21 +756,21 @@ static int device_anorm(Factor* F, std::vector<double>* anorm) {
 int gather_values_device(long nnz, const int* d_vmap, const double* d_raw, double* d_out) {
   if (nnz <= 0) return 0;
   const int grid = (int) std::min<long>(nblk(nnz, 256), 148L * 16);
-  k_gather_values<<<grid, 256, 0, current_stream()>>>(nnz, d_vmap, d_raw, d_out);
+  launch(k_gather_values, grid, 256, 0, current_stream(), nnz, d_vmap, d_raw, d_out);
   count_launch();
   return cuda_ok(cudaGetLastError(), "value gather") ? 0 : -1;
 }
 
 int perm_gather_device(int n, const int* d_perm, const double* src, double* dst) {
   if (n <= 0) return 0;
-  k_perm_gather<<<nblk(n, 256), 256, 0, current_stream()>>>(n, 1, d_perm, src, dst);
+  launch(k_perm_gather, nblk(n, 256), 256, 0, current_stream(), n, 1, d_perm, src, dst);
   count_launch();
   return cuda_ok(cudaGetLastError(), "permutation") ? 0 : -1;
 }
 
 int perm_scatter_device(int n, const int* d_perm, const double* src, double* dst) {
   if (n <= 0) return 0;
-  k_perm_scatter<<<nblk(n, 256), 256, 0, current_stream()>>>(n, 1, d_perm, src, dst);
+  launch(k_perm_scatter, nblk(n, 256), 256, 0, current_stream(), n, 1, d_perm, src, dst);
   count_launch();
   return cuda_ok(cudaGetLastError(), "permutation") ? 0 : -1;
 }
@@ -765,10 +787,10 @@ int solve_refine_permuted(Factor* F, int nrhs, double* d_x, const double* d_b, c
   int worst_steps = 0;
   for (int q0 = 0; q0 < nrhs; q0 += SOLVE_NRHS) {
     const int nq = std::min(SOLVE_NRHS, nrhs - q0);
-    k_perm_gather<<<nblk(n, 256), 256, 0, st>>>(n, nq, d_perm, d_b + (size_t) q0 * n, F->dBr);
+    launch(k_perm_gather, nblk(n, 256), 256, 0, st, n, nq, d_perm, d_b + (size_t) q0 * n, F->dBr);
     count_launch();
     const int s = refine_device(F, nq, F->dXr, F->dBr, n, tol, maxits, anorm, res ? res + q0 : nullptr);
-    k_perm_scatter<<<nblk(n, 256), 256, 0, st>>>(n, nq, d_perm, F->dXr, d_x + (size_t) q0 * n);
+    launch(k_perm_scatter, nblk(n, 256), 256, 0, st, n, nq, d_perm, F->dXr, d_x + (size_t) q0 * n);
     count_launch();
     if (!cuda_ok(cudaGetLastError(), "permute")) return -1;
     if (s < 0) worst_steps = -1;

@@ -21,6 +21,7 @@
 
 #include "factor.h"
 #include "kernels.h"
+#include "launch.h"
 
 namespace tb {
 
@@ -336,6 +337,7 @@ k_fwd(const int* __restrict__ list, int count, const FrontDesc* __restrict__ fro
   T* pan = reinterpret_cast<T*>(sfm + wi * sf_warp_smem<T, NQ>(slot, wld));
   const SolveTask K = task_of(fronts[list[li]]);
   const int4 rec = fwd_front_begin<T, NQ>(K, child_rec, rows, L, B, ldb, nrhs, pan, slot, pan + slot, wld);
+  grid_wait();
   fwd_front<T, NQ, WS>(K, rec, child_rec, maps, L, W, nrhs, pan, slot, pan + slot, wld);
 }
 
@@ -343,6 +345,7 @@ template <typename T, int NQ, int WS>
 __global__ void __launch_bounds__(128)
 k_bwd(const int* __restrict__ list, int count, const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
       const T* __restrict__ L, T* __restrict__ X, int ldx, const T* __restrict__ W, int nrhs, int slot, int wld) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char sfm[];
   const int wi = threadIdx.x >> 5, li = blockIdx.x * (blockDim.x >> 5) + wi;
   if (li >= count) return;
@@ -386,6 +389,7 @@ k_fwd_pers(const SolveTask* __restrict__ tasks, int t0, int t1, int* pending, in
            const int4* __restrict__ child_rec, const int* __restrict__ maps, const int* __restrict__ rows,
            const T* __restrict__ L, const T* __restrict__ B, int ldb, T* __restrict__ W, int nrhs, int* status,
            int slot, int wld) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char sfm[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   T* pan = reinterpret_cast<T*>(sfm + wi * sf_warp_smem<T, NQ>(slot, wld));
@@ -414,6 +418,7 @@ __global__ void __launch_bounds__(256, NQ == 1 ? 4 : sizeof(T) == 4 ? 3 : 2)
 k_bwd_pers(const SolveTask* __restrict__ tasks, int t0, int t1, int* done, int* next, int epoch,
            const int* __restrict__ rows, const T* __restrict__ L, T* __restrict__ X, int ldx, const T* __restrict__ W,
            int nrhs, int* status, int slot, int wld) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char sfm[];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   T* pan = reinterpret_cast<T*>(sfm + wi * sf_warp_smem<T, NQ>(slot, wld));
@@ -885,6 +890,7 @@ k_bwd_l21(const int2_* __restrict__ tasks, const FrontDesc* __restrict__ fronts,
   const int2_ tk = tasks[blockIdx.x];
   const FrontDesc F = fronts[tk.a];
   const int k = tk.b >> 16, ch = tk.b & 0xffff;
+  grid_wait();
   l21_chunk<T, NQ, NTH>(F, L, rows, X, ldx, k, ch, nrhs, zs, [&](int c, int q, int p, T v) { red[p][c][q] = v; });
   __syncthreads();
   T* out = part + F.part_off + ((size_t) ch * F.s + k * BR) * SOLVE_NRHS;
@@ -961,11 +967,16 @@ struct BigBlock {
   T* const Wf;
   const int* const rw;
   unsigned long long* const zf;
-  const unsigned tag;
+  unsigned tag = 0;
   __device__ __forceinline__ BigBlock(const SolveArgs<T>& a, int front)
       : A(a), F(a.fronts[front]), f(F.f), s(F.s), nbs((F.s + BR - 1) / BR), P(a.L + F.l_off), Wf(a.W + F.v_off * WS),
-        rw(a.rows + F.rows_off), zf(a.zp + (size_t) F.blk_off * CH_VALUES * WPV),
-        tag(TAGS ? ((unsigned) *a.counter << 12) | (unsigned) a.epoch : 0u) {}
+        rw(a.rows + F.rows_off), zf(a.zp + (size_t) F.blk_off * CH_VALUES * WPV) {}
+  // the launches before this one have finished (a solve's first one waited for
+  // the factorization: L and the inverses may be read ahead of this)
+  __device__ __forceinline__ void begin() {
+    grid_wait();
+    if (TAGS) tag = ((unsigned) *(volatile const int*) A.counter << 12) | (unsigned) A.epoch;
+  }
   __device__ __forceinline__ int block_of(int t) const { return BWD ? nbs - 1 - t : t; }
   // this lane's 16 entries of A_tu (block row bt: rows below s may belong to
   // the update rows of the last diagonal block, or be an update block)
@@ -1242,7 +1253,7 @@ k_chain(const __grid_constant__ SolveArgs<T> A) {
   const int h = (int) blockIdx.x - A.nwalk * CH_C;
   if (!walker && h >= A.nblocks) return;
   const int2_ bk = walker ? int2_{A.walk_fronts[blockIdx.x / CH_C], 0} : A.blocks[h];
-  const BB M(A, bk.a);
+  BB M(A, bk.a);
   const int f = M.f, s = M.s, nbs = M.nbs;
   unsigned long long* pf = A.pp + (size_t) M.F.blk_off * CH_VALUES * WPV;
   T* ds = reinterpret_cast<T*>(chm);
@@ -1267,6 +1278,10 @@ k_chain(const __grid_constant__ SolveArgs<T> A) {
       bar_wait(smem_addr(&bars[u % CH_RING]), (u / CH_RING) & 1, A.status);
       if (tid == 0 && u + CH_RING < nbs) bar_expect(smem_addr(&bars[u % CH_RING]), ZBYTES);
     };
+    if ((int) rank >= nbs) {
+      M.begin();
+      grid_trigger();
+    }
     unsigned peer[CH_C];   // offsets of the others' shared memory, the next CTA of the chain first
 #pragma unroll
     for (int r = 0; r < CH_C; r++) peer[r] = map_rank(smem_addr(bars), (rank + 1 + r) % CH_C) - smem_addr(bars);
@@ -1292,6 +1307,8 @@ k_chain(const __grid_constant__ SolveArgs<T> A) {
         for (int e = tid; e < BR * BR * (int) sizeof(T) / 128; e += CH_THREADS)
           prefetch_l2(reinterpret_cast<const unsigned char*>(A.Dinv + M.F.dinv_off + (size_t) bn * BR * BR) + 128 * e);
       }
+      if (t == (int) rank) M.begin();
+      if (t + CH_C >= nbs) grid_trigger();
       Row acc;
       acc.clear();
       Tagged<T> pt[QL];
@@ -1348,10 +1365,12 @@ k_chain(const __grid_constant__ SolveArgs<T> A) {
 #pragma unroll
   for (int i = 0; i < CH_HB; i++)
     if (i < n) M.tile(b, M.block_of(i), l[i]);
+  M.begin();
   M.template own_rhs<false>(b, BWD ? int2_{0, 0} : A.blk_ch[h], vs, zs);
   Row acc;
   acc.clear();
   M.template terms<CH_HB>(b, n, l, acc, zs, &bad_s);
+  grid_trigger();
   T p[QL];
   acc.sum(p);
 #pragma unroll
@@ -1381,7 +1400,7 @@ k_block(const __grid_constant__ SolveArgs<T> A) {
   T (*vs)[NQ] = reinterpret_cast<T (*)[NQ]>(scr + block_scratch<NQ, BWD, BLK_HB>());
   const int2_ bk = A.blocks[blockIdx.x];
   const int2_ cr = BWD ? int2_{0, 0} : A.blk_ch[blockIdx.x];
-  const BB M(A, bk.a);
+  BB M(A, bk.a);
   const int b = bk.b, nbs = M.nbs;
   const bool diag = BWD || b < nbs;
   const int n = !diag ? nbs : BWD ? nbs - 1 - b : b;
@@ -1395,11 +1414,13 @@ k_block(const __grid_constant__ SolveArgs<T> A) {
   };
   if (diag) M.stage_inverse(b, ds);
   if (!BWD) first();
+  M.begin();
   M.template own_rhs<true>(b, cr, vs, scr);
   if (BWD) first();
   Row acc;
   acc.clear();
   M.template terms<BLK_HB>(b, n, l, acc, scr, &bad_s);
+  grid_trigger();
   T z[QL], pv[QL];
   acc.sum(z);
 #pragma unroll
@@ -1426,6 +1447,7 @@ k_block(const __grid_constant__ SolveArgs<T> A) {
 // the first pass of a call also the persistent set's done flags and the call
 // counter of the published values
 __global__ void k_solve_reset(int first, const int* __restrict__ pending0, int* pers, int np, int* counter) {
+  grid_wait_then_trigger();
   const int i0 = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
   for (int i = i0; i < np; i += n) {
     pers[i] = pending0[i];
@@ -1566,7 +1588,7 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
   // device, so a recorded launch sequence stays valid
   auto reset = [&](bool first) {
     const int grid = std::max(1, std::min(148, (np + 255) / 256));
-    k_solve_reset<<<grid, 256, 0, st>>>(first, D.pers_pending0, D.pers_solve, np, counter);
+    launch(k_solve_reset, grid, 256, 0, st, first, D.pers_pending0, D.pers_solve, np, counter);
     count_launch();
   };
   auto small_list = [&](int h, int nq, auto launch) {
@@ -1594,7 +1616,7 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
         const int slot = sf_slot<T>(P.pers_slot[pt]), wld = P.pers_wld[pt], nw = th / 32;
         const size_t smem = nw * sf_warp_smem<T, Q>(slot, wld);
         const int grid = std::min((t1 - t0 + nw - 1) / nw, sf_resident(k_fwd_pers<T, Q, SOLVE_NRHS>, th, smem));
-        k_fwd_pers<T, Q, SOLVE_NRHS><<<grid, th, smem, st>>>(D.solve_tasks, t0, t1, D.pers_solve,
+        launch(k_fwd_pers<T, Q, SOLVE_NRHS>, grid, th, smem, st, D.solve_tasks, t0, t1, D.pers_solve,
                                                              D.pers_solve + 2 * np + pt, D.child_rec, D.maps, D.rows,
                                                              L, Bq, ld, W, nq, status, slot, wld);
       });
@@ -1610,8 +1632,8 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       small_list(h, nq, [&](auto nqc, const int* sl, int ns) {
         constexpr int Q = decltype(nqc)::value;
         const int slot = sf_slot<T>(SMALL_F_MAX * (SMALL_F_MAX + 1));
-        k_fwd<T, Q, SOLVE_NRHS><<<(ns + 3) / 4, 128, 4 * sf_warp_smem<T, Q>(slot, SMALL_F_MAX), st>>>(
-            sl, ns, D.fronts, D.child_rec, D.maps, D.rows, L, Bq, ld, W, nq, slot, SMALL_F_MAX);
+        launch(k_fwd<T, Q, SOLVE_NRHS>, (ns + 3) / 4, 128, 4 * sf_warp_smem<T, Q>(slot, SMALL_F_MAX), st, sl, ns,
+            D.fronts, D.child_rec, D.maps, D.rows, L, Bq, ld, W, nq, slot, SMALL_F_MAX);
         count_launch();
       });
       const int nb = (int) LP.solve_fwd_blocks.size();
@@ -1621,9 +1643,9 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
         chain_dispatch<T>(nq, [&](auto nqc) {
           constexpr int Q = decltype(nqc)::value;
           if (chain_level(LP))
-            k_chain<T, Q, SOLVE_NRHS, false><<<chain_grid(A.nwalk, nb), CH_THREADS, chain_smem<T, Q>(), st>>>(A);
+            launch(k_chain<T, Q, SOLVE_NRHS, false>, chain_grid(A.nwalk, nb), CH_THREADS, chain_smem<T, Q>(), st, A);
           else
-            k_block<T, Q, SOLVE_NRHS, false, true><<<nb, CH_THREADS, block_smem<T, Q, false>(), st>>>(A);
+            launch(k_block<T, Q, SOLVE_NRHS, false, true>, nb, CH_THREADS, block_smem<T, Q, false>(), st, A);
         });
         count_launch();
       }
@@ -1650,9 +1672,10 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
             // fewer warps each, down to 4 (solve at 64^3, FP64, backward: 4
             // warps always 1538 us, 16 always 1446, so 1380; mixed step at
             // 80^3, backward: 6509, 7333, 6441)
-            if (nt <= 148) k_bwd_l21<T, Q, 512><<<nt, 512, 0, st>>>(tl, D.fronts, D.rows, L, Xq, ld, part, nq);
-            else if (nt <= 4 * 148) k_bwd_l21<T, Q, 256><<<nt, 256, 0, st>>>(tl, D.fronts, D.rows, L, Xq, ld, part, nq);
-            else k_bwd_l21<T, Q, 128><<<nt, 128, 0, st>>>(tl, D.fronts, D.rows, L, Xq, ld, part, nq);
+            if (nt <= 148) launch(k_bwd_l21<T, Q, 512>, nt, 512, 0, st, tl, D.fronts, D.rows, L, Xq, ld, part, nq);
+            else if (nt <= 4 * 148) launch(k_bwd_l21<T, Q, 256>, nt, 256, 0, st, tl, D.fronts, D.rows, L, Xq, ld,
+                                        part, nq);
+            else launch(k_bwd_l21<T, Q, 128>, nt, 128, 0, st, tl, D.fronts, D.rows, L, Xq, ld, part, nq);
           });
           count_launch();
         }
@@ -1660,17 +1683,17 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
         chain_dispatch<T>(nq, [&](auto nqc) {
           constexpr int Q = decltype(nqc)::value;
           if (chain)
-            k_chain<T, Q, SOLVE_NRHS, true><<<chain_grid(A.nwalk, nb), CH_THREADS, chain_smem<T, Q>(), st>>>(A);
+            launch(k_chain<T, Q, SOLVE_NRHS, true>, chain_grid(A.nwalk, nb), CH_THREADS, chain_smem<T, Q>(), st, A);
           else
-            k_block<T, Q, SOLVE_NRHS, true, true><<<nb, CH_THREADS, block_smem<T, Q, true>(), st>>>(A);
+            launch(k_block<T, Q, SOLVE_NRHS, true, true>, nb, CH_THREADS, block_smem<T, Q, true>(), st, A);
         });
         count_launch();
       }
       small_list(h, nq, [&](auto nqc, const int* sl, int ns) {
         constexpr int Q = decltype(nqc)::value;
         const int slot = sf_slot<T>(SMALL_F_MAX * (SMALL_F_MAX + 1));
-        k_bwd<T, Q, SOLVE_NRHS><<<(ns + 3) / 4, 128, 4 * sf_warp_smem<T, Q>(slot, SMALL_F_MAX), st>>>(
-            sl, ns, D.fronts, D.rows, L, Xq, ld, W, nq, slot, SMALL_F_MAX);
+        launch(k_bwd<T, Q, SOLVE_NRHS>, (ns + 3) / 4, 128, 4 * sf_warp_smem<T, Q>(slot, SMALL_F_MAX), st, sl, ns,
+            D.fronts, D.rows, L, Xq, ld, W, nq, slot, SMALL_F_MAX);
         count_launch();
       });
       prof_end(KC_SOLVE_BWD, st, 0.0, by);
@@ -1688,7 +1711,7 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
         const int slot = sf_slot<T>(P.pers_slot[pt]), wld = P.pers_wld[pt], nw = th / 32;
         const size_t smem = nw * sf_warp_smem<T, Q>(slot, wld);
         const int grid = std::min((t1 - t0 + nw - 1) / nw, sf_resident(k_bwd_pers<T, Q, SOLVE_NRHS>, th, smem));
-        k_bwd_pers<T, Q, SOLVE_NRHS><<<grid, th, smem, st>>>(D.solve_tasks, t0, t1, D.pers_solve + np,
+        launch(k_bwd_pers<T, Q, SOLVE_NRHS>, grid, th, smem, st, D.solve_tasks, t0, t1, D.pers_solve + np,
                                                              D.pers_solve + 2 * np + 2 + pt, eb, D.rows, L, Xq, ld, W,
                                                              nq, status, slot, wld);
       });
@@ -1776,8 +1799,9 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
     const LevelPlan& LP = P.levels[h];
     const int ns = (int) LP.small_fronts.size();
     if (ns > 0) {
-      k_fwd<double, 1, 1><<<(ns + 3) / 4, 128, 4 * sf_warp_smem<double, 1>(slot, SMALL_F_MAX), st>>>(
-          D.small_list + D.small_off[h], ns, D.fronts, D.child_rec, D.maps, D.rows, L, B, ld, W, 1, slot, SMALL_F_MAX);
+      launch(k_fwd<double, 1, 1>, (ns + 3) / 4, 128, 4 * sf_warp_smem<double, 1>(slot, SMALL_F_MAX), st,
+          D.small_list + D.small_off[h], ns, D.fronts, D.child_rec, D.maps, D.rows, L, B, ld, W, 1, slot,
+          SMALL_F_MAX);
       count_launch();
     }
     const int nb = (int) LP.solve_fwd_blocks.size();
@@ -1785,7 +1809,7 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
       const SolveArgs<double> A{nullptr, 0, D.sfwd + D.sfwd_off[h], nb, D.sfwd_ch + D.sfwd_off[h], D.blk_child, D.fronts,
                                 D.maps, D.rows, L, Dinv, B, X, ld, W, nullptr, INT_MAX, nullptr, nullptr, flags, 1, nullptr,
                                 ef, status};
-      k_block<double, 1, 1, false, false><<<nb, CH_THREADS, block_smem<double, 1, false>(), st>>>(A);
+      launch(k_block<double, 1, 1, false, false>, nb, CH_THREADS, block_smem<double, 1, false>(), st, A);
       count_launch();
     }
   }
@@ -1796,12 +1820,12 @@ static int launch_solve_noalloc(const Plan& P, const DevPlan& D, const double* L
     if (nb > 0) {
       const SolveArgs<double> A{nullptr, 0, D.sbwd + D.sbwd_off[h], nb, nullptr, nullptr, D.fronts, D.maps, D.rows, L, Dinv,
                                 nullptr, X, ld, W, nullptr, INT_MAX, nullptr, nullptr, flags, 1, nullptr, eb, status};
-      k_block<double, 1, 1, true, false><<<nb, CH_THREADS, block_smem<double, 1, true>(), st>>>(A);
+      launch(k_block<double, 1, 1, true, false>, nb, CH_THREADS, block_smem<double, 1, true>(), st, A);
       count_launch();
     }
     const int ns = (int) LP.small_fronts.size();
     if (ns > 0) {
-      k_bwd<double, 1, 1><<<(ns + 3) / 4, 128, 4 * sf_warp_smem<double, 1>(slot, SMALL_F_MAX), st>>>(
+      launch(k_bwd<double, 1, 1>, (ns + 3) / 4, 128, 4 * sf_warp_smem<double, 1>(slot, SMALL_F_MAX), st,
           D.small_list + D.small_off[h], ns, D.fronts, D.rows, L, X, ld, W, 1, slot, SMALL_F_MAX);
       count_launch();
     }

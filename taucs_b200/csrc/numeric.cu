@@ -1183,8 +1183,6 @@ __device__ __forceinline__ void mma_block(float (&acc)[MI][NI][4], const float (
     }
 }
 
-constexpr int GEMM_STAGES = 3;
-
 // number of lower-trapezoid tiles of a region with `rows` rows and `cols`
 // columns whose column tile c covers rows [c*BN, rows)
 __host__ __device__ inline int trap_tiles(int rows, int cols, int bm, int bn) {
@@ -1196,17 +1194,20 @@ __host__ __device__ inline int trap_tiles(int rows, int cols, int bm, int bn) {
 template <int BM, int BN>
 struct GemmCfg {
   static constexpr int WM = 2;                     // warps along M
-  static constexpr int WN = BN / 32;               // warps along N (32 columns each)
+  static constexpr int WN = BN > 64 ? BN / 32 : 2; // warps along N
   static constexpr int THREADS = 32 * WM * WN;
   static constexpr int MI = BM / WM / 16;          // m16 tiles per warp
-  static constexpr int NI = 4;                     // n8 tiles per warp
-  static constexpr int LD = BM + 8;                // padded k-row stride (BM >= BN)
+  static constexpr int NI = BN / WN / 8;           // n8 tiles per warp
+  static constexpr int STAGES = BM == 32 ? 5 : 3;
+  // k-row stride (BM >= BN): a FP64 fragment's 4 x 8 entries fill the banks
+  // exactly (with BM + 8 every fragment load took two passes)
+  static constexpr int LD = BM + 4;
   template <typename T>
-  static constexpr size_t smem() { return (size_t) GEMM_STAGES * 2 * GEMM_BK * LD * sizeof(T); }
+  static constexpr size_t smem() { return (size_t) STAGES * 2 * GEMM_BK * LD * sizeof(T); }
 };
 
-// C -= A B^T on DMMA m16n8k8 tiles of BM x BN (64x64: 4 warps, 128x128: 8
-// warps), GEMM_STAGES-deep cp.async pipeline, accumulators preloaded with -C.
+// C -= A B^T on DMMA m16n8k8 tiles of BM x BN (32x32 and 64x64: 4 warps, 128x128:
+// 8 warps), STAGES-deep cp.async pipeline, accumulators preloaded with -C.
 // mode 0: panel update of columns [c_lo, min(c_hi, s)) and all rows below
 //         c_lo by the panel columns [k_lo, k_hi) (one node of the recursive
 //         panel factorization);
@@ -1216,9 +1217,9 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN>::THREADS)
 k_gemm(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __restrict__ L,
        T* __restrict__ U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, const int* status) {
   using Cfg = GemmCfg<BM, BN>;
-  constexpr int MI = Cfg::MI, NI = Cfg::NI, LD = Cfg::LD, NT = Cfg::THREADS;
+  constexpr int MI = Cfg::MI, NI = Cfg::NI, LD = Cfg::LD, NT = Cfg::THREADS, STAGES = Cfg::STAGES;
   extern __shared__ __align__(16) unsigned char smraw[];
-  T* gsm = reinterpret_cast<T*>(smraw);   // GEMM_STAGES x {A, B} x GEMM_BK x LD
+  T* gsm = reinterpret_cast<T*>(smraw);   // STAGES x {A, B} x GEMM_BK x LD
   const FrontDesc F = fronts[list[blockIdx.y]];
   const int f = F.f, s = F.s, m = f - s;
   int rows, cols, roff, kbeg, kend, ldc;
@@ -1255,7 +1256,7 @@ k_gemm(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp % Cfg::WM, wn = warp / Cfg::WM, g = lane >> 2, t = lane & 3;
-  const int wrow = wm * (BM / Cfg::WM), wcol = wn * 32;
+  const int wrow = wm * (BM / Cfg::WM), wcol = wn * (BN / Cfg::WN);
   grid_wait();
   if (failed(status)) return;
   // accumulators start at -C, so acc = A B^T - C and the result is -acc
@@ -1296,17 +1297,17 @@ k_gemm(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __
 
   const int nk = (kend - kbeg + GEMM_BK - 1) / GEMM_BK;
 #pragma unroll
-  for (int st = 0; st < GEMM_STAGES - 1; st++) {
+  for (int st = 0; st < STAGES - 1; st++) {
     if (st < nk) load(st, kbeg + st * GEMM_BK);
     cp_async_commit();
   }
   for (int kt = 0; kt < nk; kt++) {
-    cp_async_wait<GEMM_STAGES - 2>();
+    cp_async_wait<STAGES - 2>();
     __syncthreads();
-    const int kn = kt + GEMM_STAGES - 1;
-    if (kn < nk) load(kn % GEMM_STAGES, kbeg + kn * GEMM_BK);
+    const int kn = kt + STAGES - 1;
+    if (kn < nk) load(kn % STAGES, kbeg + kn * GEMM_BK);
     cp_async_commit();
-    const T* As = gsm + (size_t) ((kt % GEMM_STAGES) * 2) * GEMM_BK * LD;
+    const T* As = gsm + (size_t) ((kt % STAGES) * 2) * GEMM_BK * LD;
     const T* Bs = As + GEMM_BK * LD;
 #pragma unroll
     for (int kk = 0; kk < GEMM_BK; kk += 8) {
@@ -1375,8 +1376,8 @@ static double front_bytes(const Plan& P, const FrontDesc& F, double esz) {
 
 // GEMM variant of level h for the panel updates (kind 0) or the update
 // matrix (kind 1): FP64 fronts choose between 64x64 tiles (4 warps, 3 CTAs
-// per SM; the default, 24 TF/s on the 64^3 update matrices) and 128x128
-// tiles (8 warps, one CTA per SM; 19 TF/s there), FP32 fronts between the
+// per SM; the default, 27-29 TF/s on the large 64^3 update matrices; 32x32 on
+// small launches) and 128x128 tiles (8 warps, one CTA per SM; 19 TF/s there), FP32 fronts between the
 // two tcgen05 variants.  The choice comes from the autotuner's measurements
 // (Plan::gemm_choice), the default variant otherwise.
 template <typename T>
@@ -1385,11 +1386,21 @@ static bool gemm_alt(const Plan& P, int h, int kind) {
   return (size_t) (2 * h + kind) < c.size() && c[2 * h + kind] != 0;
 }
 
+// A launch of up to this many 64x64 tiles (four waves of three CTAs an SM) takes
+// 32x32 tiles: four times the CTAs, so that every SM has several of them from the
+// first to the last wave; beyond it the larger tile's reuse is worth more.  Panel
+// products and update matrices of a 40x41x39 grid 3.44 -> 2.64 ms; of 64^3, panel
+// products 13.24 -> 11.73 (12.54 with a line at 200 tiles, 11.86 at 3200), update
+// matrices 22.96 -> 22.92 (27.3 with 32x32 tiles throughout).
+constexpr int SMALL_TILES = 4 * 3 * 148;
 template <typename T>
-static void launch_gemm(bool big, int gx128, int gx64, int nb, const int* blst, const DevPlan& D, T* L, T* U,
+static void launch_gemm(bool big, int gx128, int gx64, int gx32, int n64, int nb, const int* blst, const DevPlan& D, T* L, T* U,
                         int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st,
                         const float* = nullptr, int = 0, int = 0) {
-  if (big)
+  if (!big && n64 <= SMALL_TILES)
+    launch(k_gemm<T, 32, 32>, dim3(gx32, nb), GemmCfg<32, 32>::THREADS, GemmCfg<32, 32>::smem<T>(), st, blst, D.fronts,
+           L, U, c_lo, c_hi, k_lo, k_hi, mode, status);
+  else if (big)
     launch(k_gemm<T, 128, 128>, dim3(gx128, nb), GemmCfg<128, 128>::THREADS, GemmCfg<128, 128>::smem<T>(), st, blst,
         D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status);
   else
@@ -1400,7 +1411,7 @@ static void launch_gemm(bool big, int gx128, int gx64, int nb, const int* blst, 
 // FP32 fronts take the tcgen05 kernels (gemm_tc.cu): by default the one fed
 // from the split arena (gx_sp tiles per front), with `alt` the one whose
 // producer warps split the operands as they load them
-static void launch_gemm(bool alt, int gx128, int gx64, int nb, const int* blst, const DevPlan& D, float* L, float* U,
+static void launch_gemm(bool alt, int gx128, int gx64, int gx32, int n64, int nb, const int* blst, const DevPlan& D, float* L, float* U,
                         int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st,
                         const float* sp = nullptr, int gx_sp = 0, int sp_fmt = 0) {
   if (!alt && sp && gemm_sp_init()) {
@@ -1411,7 +1422,7 @@ static void launch_gemm(bool alt, int gx128, int gx64, int nb, const int* blst, 
     launch_gemm_tc(0, gx128, nb, blst, D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
     return;
   }
-  launch_gemm<float>(false, gx128, gx64, nb, blst, D, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
+  launch_gemm<float>(false, gx128, gx64, gx32, n64, nb, blst, D, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
 }
 
 // CTAs of the persistent small-front launch: all that fit on the device at
@@ -1474,6 +1485,8 @@ static void set_smem_attrs() {
       panel(std::integral_constant<int, 1>(), std::integral_constant<int, 512>());
     }
     cudaFuncSetAttribute(k_dinv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dinv_smem<T>());
+    cudaFuncSetAttribute(k_gemm<T, 32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int) GemmCfg<32, 32>::smem<T>());
     cudaFuncSetAttribute(k_gemm<T, 64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int) GemmCfg<64, 64>::smem<T>());
     cudaFuncSetAttribute(k_gemm<T, 128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1619,14 +1632,17 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       count_launch();
     };
     auto update = [&](int c_lo, int c_hi, int k_lo, int k_hi) {
-      int gx = 0, gx64 = 0;
+      int gx = 0, gx64 = 0, gx32 = 0, n64 = 0;
       double fg = 0.0, bg = 0.0;
       for (int fi : LP.big_fronts) {
         const FrontDesc& F = P.fronts[fi];
         const int ce = std::min(c_hi, F.s);
         if (c_lo >= ce) continue;
         gx = std::max(gx, trap_tiles(F.f - c_lo, ce - c_lo, 128, 128));
-        gx64 = std::max(gx64, trap_tiles(F.f - c_lo, ce - c_lo, 64, 64));
+        const int t64 = trap_tiles(F.f - c_lo, ce - c_lo, 64, 64);
+        n64 += t64;
+        gx64 = std::max(gx64, t64);
+        gx32 = std::max(gx32, trap_tiles(F.f - c_lo, ce - c_lo, 32, 32));
         if (prof_enabled()) {
           const double c = ce - c_lo, below = F.f - ce, k = k_hi - k_lo;
           const double entries = c * (c + 1.0) / 2.0 + below * c;
@@ -1636,7 +1652,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       }
       if (gx64 == 0) return;
       prof_begin(KC_GEMM_PANEL, st);
-      launch_gemm(gemm_alt<T>(P, h, 0), gx, gx64, nb, blst, D, L, U, c_lo, c_hi, k_lo, k_hi, 0, status, st, sp, gx, sp_fmt);
+      launch_gemm(gemm_alt<T>(P, h, 0), gx, gx64, gx32, n64, nb, blst, D, L, U, c_lo, c_hi, k_lo, k_hi, 0, status, st, sp, gx, sp_fmt);
       prof_end(KC_GEMM_PANEL, st, fg, bg);
       count_launch();
     };
@@ -1651,15 +1667,17 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       }
     };
     Rec::run(0, span, S, panel, update);
-    int gx_u = 0, gx_u64 = 0, gx_usp = 0, maxm = 0;
+    int gx_u = 0, gx_u64 = 0, gx_u32 = 0, n_u64 = 0, gx_usp = 0;
     for (int fi : LP.big_fronts) {
       const FrontDesc& F = P.fronts[fi];
       const int m = F.f - F.s;
       if (m > 0) {
         gx_u = std::max(gx_u, trap_tiles(m, m, 128, 128));
         gx_usp = std::max(gx_usp, gemm_sp_tiles_u(F.s, F.f));
-        gx_u64 = std::max(gx_u64, trap_tiles(m, m, 64, 64));
-        maxm = std::max(maxm, m);
+        const int t64 = trap_tiles(m, m, 64, 64);
+        n_u64 += t64;
+        gx_u64 = std::max(gx_u64, t64);
+        gx_u32 = std::max(gx_u32, trap_tiles(m, m, 32, 32));
       }
     }
     if (gx_u64 > 0) {
@@ -1672,8 +1690,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
           bu += 2.0 * sizeof(T) * m * (m + 1.0) / 2.0 + sizeof(T) * m * F.s;
         }
       prof_begin(KC_GEMM_U, st);
-      (void) maxm;
-      launch_gemm(gemm_alt<T>(P, h, 1), gx_u, gx_u64, nb, blst, D, L, U, 0, 0, 0, 0, 1, status, st, sp, gx_usp, sp_fmt);
+      launch_gemm(gemm_alt<T>(P, h, 1), gx_u, gx_u64, gx_u32, n_u64, nb, blst, D, L, U, 0, 0, 0, 0, 1, status, st, sp, gx_usp, sp_fmt);
       prof_end(KC_GEMM_U, st, fu, bu);
       count_launch();
     }

@@ -114,6 +114,8 @@ int devplan_upload(const Plan& P, DevPlan* D, cudaStream_t st) {
     const FrontDesc& C = P.fronts[c];
     crec.push_back(make_int4(C.rows_off, C.s, C.f, C.map_off));
   }
+  std::vector<int> step_list, work;
+  plan_launches(P, D, step_list, work);
   bool ok = dev_upload(&D->fronts, P.fronts.data(), P.fronts.size(), st)
          && dev_upload(&D->small_num, small_num.data(), small_num.size(), st)
          && dev_upload(&D->pers_list, P.pers_fronts.data(), P.pers_fronts.size(), st)
@@ -123,6 +125,8 @@ int devplan_upload(const Plan& P, DevPlan* D, cudaStream_t st) {
          && dev_upload(&D->pers_solve, (const int*) nullptr, 2 * P.pers_fronts.size() + 4, st)
          && dev_upload(&D->solve_tasks, stasks.data(), stasks.size(), st)
          && dev_upload(&D->child_rec, crec.data(), crec.size(), st)
+         && dev_upload(&D->step_list, step_list.data(), step_list.size(), st)
+         && dev_upload(&D->work, work.data(), work.size(), st)
          && dev_upload(&D->panel_done, (const int*) nullptr, (size_t) P.n_blk, st)
          && dev_upload(&D->panel_rdiag, (const double*) nullptr, (size_t) P.n_blk * PANEL_NB, st)
          && dev_upload(&D->dblk, dblk.data(), dblk.size(), st)
@@ -154,7 +158,7 @@ void devplan_free(DevPlan* D) {
   tb::dfree(D->sfwd); tb::dfree(D->sfwd_ch); tb::dfree(D->blk_child); tb::dfree(D->sbwd); tb::dfree(D->sl21); tb::dfree(D->dblk);
   tb::dfree(D->small_num); tb::dfree(D->pers_list); tb::dfree(D->pers_parent); tb::dfree(D->pers_pending0);
   tb::dfree(D->pers_work); tb::dfree(D->pers_solve); tb::dfree(D->solve_tasks); tb::dfree(D->child_rec);
-  tb::dfree(D->panel_done); tb::dfree(D->panel_rdiag);
+  tb::dfree(D->step_list); tb::dfree(D->work); tb::dfree(D->panel_done); tb::dfree(D->panel_rdiag);
   *D = DevPlan();
 }
 

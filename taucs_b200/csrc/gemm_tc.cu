@@ -141,7 +141,7 @@ __device__ __forceinline__ void record_timeout(int* status) { atomicMin(status, 
 // mode 1: U -= L21 L21^T (K = [0, s))
 template <int STAGES, int MINB, int NPROD>
 __global__ void __launch_bounds__(NPROD + 32, MINB)
-k_gemm_tc(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, float* __restrict__ L,
+k_gemm_tc(const int* __restrict__ cum, int nb, const int* __restrict__ list, const FrontDesc* __restrict__ fronts, float* __restrict__ L,
           float* __restrict__ U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status) {
   grid_wait();
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 1];   // full[S], empty[S], done
@@ -149,7 +149,8 @@ k_gemm_tc(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, fl
   __shared__ int abort_cta;
   extern __shared__ __align__(16) unsigned char tc_raw[];
   if (*(volatile const int*) status != INT_MAX) return;
-  const FrontDesc F = fronts[list[blockIdx.y]];
+  int idx;
+  const FrontDesc F = fronts[list[front_of(cum, nb, blockIdx.x, idx)]];
   const int f = F.f, s = F.s, m = f - s;
   int rows, cols, roff, kbeg, kend, ldc;
   const float* P = L + F.l_off;
@@ -169,7 +170,7 @@ k_gemm_tc(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, fl
     ldc = m;
   }
   if (kend <= kbeg) return;
-  int idx = blockIdx.x, c0 = 0;
+  int c0 = 0;
   for (;;) {
     if (c0 >= cols) return;
     const int nt_c = (rows - c0 + TC_BM - 1) / TC_BM;
@@ -405,14 +406,15 @@ __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned
 
 template <int STAGES, int FMT>
 __global__ void __launch_bounds__(128, 2)
-k_gemm_sp(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, const float* __restrict__ sp,
+k_gemm_sp(const int* __restrict__ cum, int nb, const int* __restrict__ list, const FrontDesc* __restrict__ fronts, const float* __restrict__ sp,
           float* __restrict__ L, float* __restrict__ U, int c_lo, int c_hi, int k_lo, int k_hi, int mode,
           int* status) {
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 1];   // full[S], empty[S], done
   __shared__ unsigned tmem_slot;
   __shared__ int abort_cta;
   extern __shared__ __align__(16) unsigned char sp_raw[];
-  const FrontDesc F = fronts[list[blockIdx.y]];
+  int idx;
+  const FrontDesc F = fronts[list[front_of(cum, nb, blockIdx.x, idx)]];
   const int f = F.f, s = F.s, m = f - s;
   // tile grid origin (a row-group boundary), the valid rows/columns and K
   int base, rows, cols, lo, kbeg, kend;
@@ -427,7 +429,7 @@ k_gemm_sp(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, co
     kbeg = 0; kend = s;
   }
   if (kend <= kbeg) return;
-  int idx = blockIdx.x, c0 = 0;
+  int c0 = 0;
   for (;;) {
     if (c0 >= cols) return;
     const int nt_c = (rows - c0 + TC_BM - 1) / TC_BM;
@@ -625,14 +627,14 @@ int gemm_sp_tiles_u(int s, int f) {
   return gemm_tc_tiles(n, n);
 }
 
-void launch_gemm_sp(int fmt, int gx, int nb, const int* list, const FrontDesc* fronts, const float* sp, float* L,
-                    float* U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st) {
+void launch_gemm_sp(int fmt, const LaunchWork& w, const int* work, const int* list, const FrontDesc* fronts,
+                    const float* sp, float* L, float* U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st) {
   if (fmt)
-    launch(k_gemm_sp<3, 1>, dim3(gx, nb), 128, sp_smem<3>(), st, list, fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode,
-                                                             status);
+    launch(k_gemm_sp<3, 1>, w.total, 128, sp_smem<3>(), st, work + w.off, w.nb, list, fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode,
+           status);
   else
-    launch(k_gemm_sp<3, 0>, dim3(gx, nb), 128, sp_smem<3>(), st, list, fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode,
-                                                             status);
+    launch(k_gemm_sp<3, 0>, w.total, 128, sp_smem<3>(), st, work + w.off, w.nb, list, fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode,
+           status);
 }
 
 // variant 0: two-stage ring (65 KB), 128 producers, three CTAs per SM;
@@ -655,14 +657,14 @@ int gemm_tc_tiles(int rows, int cols) {
   return t;
 }
 
-void launch_gemm_tc(int variant, int gx, int nb, const int* list, const FrontDesc* fronts, float* L, float* U,
-                    int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st) {
+void launch_gemm_tc(int variant, const LaunchWork& w, const int* work, const int* list, const FrontDesc* fronts,
+                    float* L, float* U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st) {
   if (variant == 1)
-    launch(k_gemm_tc<3, 2, 256>, dim3(gx, nb), 256 + 32, tc_smem<3>(), st, list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
-                                                                       mode, status);
+    launch(k_gemm_tc<3, 2, 256>, w.total, 256 + 32, tc_smem<3>(), st, work + w.off, w.nb, list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
+           mode, status);
   else
-    launch(k_gemm_tc<2, 3, 128>, dim3(gx, nb), 128 + 32, tc_smem<2>(), st, list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
-                                                                       mode, status);
+    launch(k_gemm_tc<2, 3, 128>, w.total, 128 + 32, tc_smem<2>(), st, work + w.off, w.nb, list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
+           mode, status);
 }
 
 }  // namespace tb

@@ -55,7 +55,36 @@ __device__ __forceinline__ int warp_lower_bound(const int* a, int n, int key) {
   const int p = lo + lane;
   return lo + __popc(__ballot_sync(0xffffffffu, p < hi && a[p] < key));
 }
+// The front that CTA b of a launch works for, and the CTA's index among that
+// front's: cum[i] = CTAs of fronts 0 .. i of the launch (see LaunchWork).  Every
+// warp finds it for itself.
+__device__ __forceinline__ int front_of(const int* __restrict__ cum, int nb, int b, int& idx) {
+  idx = b;
+  if (nb == 1) return 0;
+  const int y = warp_lower_bound(cum, nb, b + 1);
+  if (y > 0) idx -= cum[y - 1];
+  return y;
+}
 #endif
+
+// One launch over the big fronts of a level: its CTAs, front by front.  The
+// launches used to be (fronts) x (the most CTAs that one of them needs): on the
+// levels with many fronts three in four left at once, each after the status
+// word, the list and its front had come from L2 (64^3 FP64: update matrices 22.9
+// -> 22.1 ms; 80^3 FP32: 11.9 -> 11.0, panel steps 12.6 -> 12.35; the search costs
+// a launch about 0.5 us).  The fronts with the most columns come first: their
+// tiles take longest, and a panel step's fronts are the first ones of the list.
+struct LaunchWork {
+  int off = 0;     // of the cumulative counts in DevPlan::work
+  int nb = 0;      // fronts, the first ones of the level's step_list
+  int total = 0;   // CTAs
+};
+// The panel steps and products of a level; step k: columns [128 k, 128 (k + 1))
+struct LevelWork {
+  std::vector<LaunchWork> rows64, rows128;      // row CTAs of k_panel by step
+  std::vector<LaunchWork> u32, u64, u128;       // tiles of the panel product into the columns from 128 k on
+  LaunchWork m32, m64, m128, msp;               // tiles of the update matrices (msp: from the split arena)
+};
 
 // Device copies of the plan arrays.
 struct DevPlan {
@@ -87,11 +116,17 @@ struct DevPlan {
   int4* child_rec = nullptr;   // per entry of children: work vector offset, s, f, map offset
   int* panel_done = nullptr;   // per factorization: 16-column pieces finished, at FrontDesc::blk_off
   double* panel_rdiag = nullptr;   // 1 / L_jj of the big fronts' columns, 64 per block (FP32 fronts use the first half)
+  int* step_list = nullptr;    // per level (big_off) the big fronts, those with the most columns first
+  int* work = nullptr;         // cumulative CTA counts of the launches over them
+  std::vector<LevelWork> level_work;
   int n_pers = 0;
   std::vector<int> small_off, big_off, tile_off, sfwd_off, sbwd_off, sl21_off, small_num_off;  // per level (host)
   std::vector<int> lvl_max_f_small;               // per level (host)
 };
 
+// fills D->level_work (with D->big_off), and the arrays that go to D->step_list
+// and D->work
+void plan_launches(const Plan& P, DevPlan* D, std::vector<int>& step_list, std::vector<int>& work);
 int devplan_upload(const Plan& P, DevPlan* D, cudaStream_t st);
 void devplan_free(DevPlan* D);
 
@@ -125,9 +160,9 @@ int gemm_tc_tiles(int rows, int cols);
 // the tcgen05 GEMM fed from the split arena by bulk copies (same modes)
 bool gemm_sp_init();
 int gemm_sp_tiles_u(int s, int f);
-void launch_gemm_sp(int fmt, int gx, int nb, const int* list, const FrontDesc* fronts, const float* sp, float* L, float* U,
+void launch_gemm_sp(int fmt, const LaunchWork& w, const int* work, const int* list, const FrontDesc* fronts, const float* sp, float* L, float* U,
                     int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st);
-void launch_gemm_tc(int variant, int gx, int nb, const int* list, const FrontDesc* fronts, float* L, float* U,
+void launch_gemm_tc(int variant, const LaunchWork& w, const int* work, const int* list, const FrontDesc* fronts, float* L, float* U,
                     int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st);
 
 // multi-RHS solve, device vectors in permuted order: X (n x nrhs, ld) from

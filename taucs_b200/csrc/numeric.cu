@@ -32,6 +32,7 @@
 // Every kernel first reads the status word and returns when an earlier front
 // hit a nonpositive pivot; the smallest failing global column is recorded
 // with atomicMin (the reference reports the failing column, :1139-1145).
+#include <algorithm>
 #include <climits>
 #include <cstdio>
 #include <type_traits>
@@ -938,7 +939,7 @@ __device__ __forceinline__ void split_chunk(const float* x, int ld, int c, int w
 
 template <typename T, int FMT, int NT>
 __global__ void __launch_bounds__(NT, 512 / NT)
-k_panel(const int* __restrict__ list, int nb, int gx, const FrontDesc* __restrict__ fronts,
+k_panel(const int* __restrict__ cum, int nb, const int* __restrict__ list, const FrontDesc* __restrict__ fronts,
         const int* __restrict__ rows, T* __restrict__ L, float* __restrict__ sp, int kb, int* __restrict__ done,
         double* __restrict__ rdiag_all, int* status) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -946,8 +947,8 @@ k_panel(const int* __restrict__ list, int nb, int gx, const FrontDesc* __restric
   __shared__ int bad_s[2];
   T* S = reinterpret_cast<T*>(smraw);
   const bool is_diag = (int) blockIdx.x < nb;
-  const int y = is_diag ? (int) blockIdx.x : ((int) blockIdx.x - nb) / gx;
-  const FrontDesc F = fronts[list[y]];
+  int idx = 0;
+  const FrontDesc F = fronts[list[is_diag ? (int) blockIdx.x : front_of(cum, nb, (int) blockIdx.x - nb, idx)]];
   const int f = F.f, s = F.s;
   if (kb >= s) return;
   grid_wait();
@@ -1057,7 +1058,7 @@ k_panel(const int* __restrict__ list, int nb, int gx, const FrontDesc* __restric
     return;
   }
   // ------------------------------------------------------------ rows below
-  const int r0 = kb + w + ((int) blockIdx.x - nb) % gx * PROWS;
+  const int r0 = kb + w + idx * PROWS;
   const int nr = min(PROWS, f - r0);
   if (nr <= 0) return;
   for (int j = warp; j < np * PB; j += NW)
@@ -1214,13 +1215,14 @@ struct GemmCfg {
 // mode 1: U -= L21 L21^T (K = [0, s))
 template <typename T, int BM, int BN>
 __global__ void __launch_bounds__(GemmCfg<BM, BN>::THREADS)
-k_gemm(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __restrict__ L,
+k_gemm(const int* __restrict__ cum, int nb, const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __restrict__ L,
        T* __restrict__ U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, const int* status) {
   using Cfg = GemmCfg<BM, BN>;
   constexpr int MI = Cfg::MI, NI = Cfg::NI, LD = Cfg::LD, NT = Cfg::THREADS, STAGES = Cfg::STAGES;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* gsm = reinterpret_cast<T*>(smraw);   // STAGES x {A, B} x GEMM_BK x LD
-  const FrontDesc F = fronts[list[blockIdx.y]];
+  int idx;
+  const FrontDesc F = fronts[list[front_of(cum, nb, blockIdx.x, idx)]];
   const int f = F.f, s = F.s, m = f - s;
   int rows, cols, roff, kbeg, kend, ldc;
   const T* P = L + F.l_off;
@@ -1240,7 +1242,7 @@ k_gemm(const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __
     ldc = m;
   }
   // decode the lower-trapezoid tile
-  int idx = blockIdx.x, c0 = 0;
+  int c0 = 0;
   for (;;) {
     if (c0 >= cols) return;
     const int nt_c = (rows - c0 + BM - 1) / BM;
@@ -1394,35 +1396,84 @@ static bool gemm_alt(const Plan& P, int h, int kind) {
 // matrices 22.96 -> 22.92 (27.3 with 32x32 tiles throughout).
 constexpr int SMALL_TILES = 4 * 3 * 148;
 template <typename T>
-static void launch_gemm(bool big, int gx128, int gx64, int gx32, int n64, int nb, const int* blst, const DevPlan& D, T* L, T* U,
-                        int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st,
-                        const float* = nullptr, int = 0, int = 0) {
-  if (!big && n64 <= SMALL_TILES)
-    launch(k_gemm<T, 32, 32>, dim3(gx32, nb), GemmCfg<32, 32>::THREADS, GemmCfg<32, 32>::smem<T>(), st, blst, D.fronts,
-           L, U, c_lo, c_hi, k_lo, k_hi, mode, status);
-  else if (big)
-    launch(k_gemm<T, 128, 128>, dim3(gx128, nb), GemmCfg<128, 128>::THREADS, GemmCfg<128, 128>::smem<T>(), st, blst,
-        D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status);
-  else
-    launch(k_gemm<T, 64, 64>, dim3(gx64, nb), GemmCfg<64, 64>::THREADS, GemmCfg<64, 64>::smem<T>(), st, blst,
-        D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status);
+static void launch_gemm(bool big, const LaunchWork& w128, const LaunchWork& w64, const LaunchWork& w32, const int* blst,
+                        const DevPlan& D, T* L, T* U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status,
+                        cudaStream_t st) {
+  auto run = [&](auto k, const LaunchWork& w, int threads, size_t smem) {
+    launch(k, w.total, threads, smem, st, D.work + w.off, w.nb, blst, D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode,
+           status);
+  };
+  using C32 = GemmCfg<32, 32>;
+  using C64 = GemmCfg<64, 64>;
+  using C128 = GemmCfg<128, 128>;
+  if (big) run(k_gemm<T, 128, 128>, w128, C128::THREADS, C128::smem<T>());
+  else if (w64.total <= SMALL_TILES) run(k_gemm<T, 32, 32>, w32, C32::THREADS, C32::smem<T>());
+  else run(k_gemm<T, 64, 64>, w64, C64::THREADS, C64::smem<T>());
 }
 
 // FP32 fronts take the tcgen05 kernels (gemm_tc.cu): by default the one fed
-// from the split arena (gx_sp tiles per front), with `alt` the one whose
-// producer warps split the operands as they load them
-static void launch_gemm(bool alt, int gx128, int gx64, int gx32, int n64, int nb, const int* blst, const DevPlan& D, float* L, float* U,
-                        int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st,
-                        const float* sp = nullptr, int gx_sp = 0, int sp_fmt = 0) {
-  if (!alt && sp && gemm_sp_init()) {
-    launch_gemm_sp(sp_fmt, gx_sp, nb, blst, D.fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
-    return;
+// from the split arena (wsp), with `alt` the one whose producer warps split the
+// operands as they load them
+static void launch_gemm32(bool alt, const LaunchWork& wsp, const LaunchWork& w128, const LaunchWork& w64,
+                          const LaunchWork& w32, const int* blst, const DevPlan& D, float* L, float* U, int c_lo,
+                          int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st, const float* sp,
+                          int sp_fmt) {
+  if (!alt && sp && gemm_sp_init())
+    launch_gemm_sp(sp_fmt, wsp, D.work, blst, D.fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
+  else if (gemm_tc_init())
+    launch_gemm_tc(0, w128, D.work, blst, D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
+  else
+    launch_gemm<float>(false, w128, w64, w32, blst, D, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
+}
+
+void plan_launches(const Plan& P, DevPlan* D, std::vector<int>& step_list, std::vector<int>& work) {
+  D->level_work.clear();
+  step_list.clear();
+  work.clear();
+  for (const LevelPlan& LP : P.levels) {
+    LevelWork W;
+    std::vector<int> order = LP.big_fronts;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return P.fronts[a].s > P.fronts[b].s; });
+    step_list.insert(step_list.end(), order.begin(), order.end());
+    // the fronts with more than c0 columns; n(F): CTAs of front F
+    auto add = [&](int c0, auto n) {
+      LaunchWork w;
+      w.off = (int) work.size();
+      for (int fi : order) {
+        const FrontDesc& F = P.fronts[fi];
+        if (F.s <= c0) break;
+        w.total += n(F);
+        work.push_back(w.total);
+        w.nb++;
+      }
+      return w;
+    };
+    const int S = LP.max_s_big;
+    for (int c = 0; c < S; c += PW) {
+      auto below = [&](int rows) {
+        return add(c, [&](const FrontDesc& F) { return (F.f - c - std::min(PW, F.s - c) + rows - 1) / rows; });
+      };
+      W.rows64.push_back(below(PROWS<256>));
+      W.rows128.push_back(below(PROWS<512>));
+      // the product into [c, c + lowest set bit of c), of the recursion below
+      const int ce = c + (c & -c);
+      auto tiles = [&](int b) {
+        return c == 0 ? LaunchWork()
+                      : add(c, [&](const FrontDesc& F) { return trap_tiles(F.f - c, std::min(ce, F.s) - c, b, b); });
+      };
+      W.u32.push_back(tiles(32));
+      W.u64.push_back(tiles(64));
+      W.u128.push_back(tiles(128));
+    }
+    auto update = [&](int b) {
+      return add(0, [&](const FrontDesc& F) { return trap_tiles(F.f - F.s, F.f - F.s, b, b); });
+    };
+    W.m32 = update(32);
+    W.m64 = update(64);
+    W.m128 = update(128);
+    W.msp = add(0, [&](const FrontDesc& F) { return F.f > F.s ? gemm_sp_tiles_u(F.s, F.f) : 0; });
+    D->level_work.push_back(std::move(W));
   }
-  if (gemm_tc_init()) {
-    launch_gemm_tc(0, gx128, nb, blst, D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
-    return;
-  }
-  launch_gemm<float>(false, gx128, gx64, gx32, n64, nb, blst, D, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
 }
 
 // CTAs of the persistent small-front launch: all that fit on the device at
@@ -1573,9 +1624,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
         b = e;
       }
     }
-    const int nb = (int) LP.big_fronts.size();
-    if (nb == 0) continue;
-    const int* blst = D.big_list + D.big_off[h];
+    if (LP.big_fronts.empty()) continue;
     const int ntiles = (int) LP.build_tiles.size();
     {
       double by = 0.0;
@@ -1593,15 +1642,17 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
     const int S = LP.max_s_big;
     int span = PW;
     while (span < S) span *= 2;
+    const LevelWork& LW = D.level_work[h];
+    const int* slst = D.step_list + D.big_off[h];
     auto panel = [&](int kb) {
-      int rmax = 0, wmax = 0;
+      const int k = kb / PW, nsteps = LW.rows64[k].nb;
+      int wmax = 0;
       double fl = 0.0, by = 0.0;
       for (int fi : LP.big_fronts) {
         const FrontDesc& F = P.fronts[fi];
         if (kb >= F.s) continue;
         const int w = std::min(PW, F.s - kb);
         wmax = std::max(wmax, w);
-        rmax = std::max(rmax, F.f - kb - w);
         if (prof_enabled()) {
           const double ww = w, below = F.f - kb - w;
           fl += ww * ww * ww / 3.0 + below * ww * ww;
@@ -1611,15 +1662,15 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       prof_begin(KC_LEAF, st);
       auto run = [&](auto fmt, auto nt) {
         constexpr int NT = decltype(nt)::value;
-        const int gx = (rmax + PROWS<NT> - 1) / PROWS<NT>;
-        launch(k_panel<T, decltype(fmt)::value, NT>, nb + nb * gx, NT, panel_smem<T, NT>(wmax), st, blst, nb,
-            std::max(gx, 1), D.fronts, D.rows, L, sp, kb, D.panel_done, D.panel_rdiag, status);
+        const LaunchWork& w = NT == 512 ? LW.rows128[k] : LW.rows64[k];
+        launch(k_panel<T, decltype(fmt)::value, NT>, nsteps + w.total, NT, panel_smem<T, NT>(wmax), st, D.work + w.off,
+               nsteps, slst, D.fronts, D.rows, L, sp, kb, D.panel_done, D.panel_rdiag, status);
       };
       // 16 warps a CTA (128 rows) while every CTA has an SM to itself (29x24x26
       // FP32: 0.80 ms of panels -> 0.72), 8 on fuller launches, where two CTAs
       // share an SM and one's updates fill the other's waits
       auto size = [&](auto fmt) {
-        if (nb + nb * ((rmax + PROWS<512> - 1) / PROWS<512>) <= 148) run(fmt, std::integral_constant<int, 512>());
+        if (nsteps + LW.rows128[k].total <= 148) run(fmt, std::integral_constant<int, 512>());
         else run(fmt, std::integral_constant<int, 256>());
       };
       if constexpr (sizeof(T) == 4) {
@@ -1631,28 +1682,28 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       prof_end(KC_LEAF, st, fl, by);
       count_launch();
     };
+    // the product with the columns [k_lo, k_hi) into [c_lo, c_hi); c_hi - c_lo is
+    // c_lo's lowest set bit
     auto update = [&](int c_lo, int c_hi, int k_lo, int k_hi) {
-      int gx = 0, gx64 = 0, gx32 = 0, n64 = 0;
       double fg = 0.0, bg = 0.0;
-      for (int fi : LP.big_fronts) {
-        const FrontDesc& F = P.fronts[fi];
-        const int ce = std::min(c_hi, F.s);
-        if (c_lo >= ce) continue;
-        gx = std::max(gx, trap_tiles(F.f - c_lo, ce - c_lo, 128, 128));
-        const int t64 = trap_tiles(F.f - c_lo, ce - c_lo, 64, 64);
-        n64 += t64;
-        gx64 = std::max(gx64, t64);
-        gx32 = std::max(gx32, trap_tiles(F.f - c_lo, ce - c_lo, 32, 32));
-        if (prof_enabled()) {
+      if (prof_enabled())
+        for (int fi : LP.big_fronts) {
+          const FrontDesc& F = P.fronts[fi];
+          const int ce = std::min(c_hi, F.s);
+          if (c_lo >= ce) continue;
           const double c = ce - c_lo, below = F.f - ce, k = k_hi - k_lo;
           const double entries = c * (c + 1.0) / 2.0 + below * c;
           fg += 2.0 * k * entries;
           bg += 2.0 * sizeof(T) * entries + sizeof(T) * k * (F.f - c_lo);
         }
-      }
-      if (gx64 == 0) return;
+      const int k = c_lo / PW;
       prof_begin(KC_GEMM_PANEL, st);
-      launch_gemm(gemm_alt<T>(P, h, 0), gx, gx64, gx32, n64, nb, blst, D, L, U, c_lo, c_hi, k_lo, k_hi, 0, status, st, sp, gx, sp_fmt);
+      if constexpr (sizeof(T) == 4)
+        launch_gemm32(gemm_alt<T>(P, h, 0), LW.u128[k], LW.u128[k], LW.u64[k], LW.u32[k], slst, D, L, U, c_lo, c_hi,
+                      k_lo, k_hi, 0, status, st, sp, sp_fmt);
+      else
+        launch_gemm(gemm_alt<T>(P, h, 0), LW.u128[k], LW.u64[k], LW.u32[k], slst, D, L, U, c_lo, c_hi, k_lo, k_hi, 0,
+                    status, st);
       prof_end(KC_GEMM_PANEL, st, fg, bg);
       count_launch();
     };
@@ -1667,20 +1718,7 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       }
     };
     Rec::run(0, span, S, panel, update);
-    int gx_u = 0, gx_u64 = 0, gx_u32 = 0, n_u64 = 0, gx_usp = 0;
-    for (int fi : LP.big_fronts) {
-      const FrontDesc& F = P.fronts[fi];
-      const int m = F.f - F.s;
-      if (m > 0) {
-        gx_u = std::max(gx_u, trap_tiles(m, m, 128, 128));
-        gx_usp = std::max(gx_usp, gemm_sp_tiles_u(F.s, F.f));
-        const int t64 = trap_tiles(m, m, 64, 64);
-        n_u64 += t64;
-        gx_u64 = std::max(gx_u64, t64);
-        gx_u32 = std::max(gx_u32, trap_tiles(m, m, 32, 32));
-      }
-    }
-    if (gx_u64 > 0) {
+    if (LW.m64.total > 0) {
       double fu = 0.0, bu = 0.0;
       if (prof_enabled())
         for (int fi : LP.big_fronts) {
@@ -1690,7 +1728,11 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
           bu += 2.0 * sizeof(T) * m * (m + 1.0) / 2.0 + sizeof(T) * m * F.s;
         }
       prof_begin(KC_GEMM_U, st);
-      launch_gemm(gemm_alt<T>(P, h, 1), gx_u, gx_u64, gx_u32, n_u64, nb, blst, D, L, U, 0, 0, 0, 0, 1, status, st, sp, gx_usp, sp_fmt);
+      if constexpr (sizeof(T) == 4)
+        launch_gemm32(gemm_alt<T>(P, h, 1), LW.msp, LW.m128, LW.m64, LW.m32, slst, D, L, U, 0, 0, 0, 0, 1, status, st,
+                      sp, sp_fmt);
+      else
+        launch_gemm(gemm_alt<T>(P, h, 1), LW.m128, LW.m64, LW.m32, slst, D, L, U, 0, 0, 0, 0, 1, status, st);
       prof_end(KC_GEMM_U, st, fu, bu);
       count_launch();
     }

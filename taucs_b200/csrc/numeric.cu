@@ -1199,7 +1199,10 @@ struct GemmCfg {
   static constexpr int THREADS = 32 * WM * WN;
   static constexpr int MI = BM / WM / 16;          // m16 tiles per warp
   static constexpr int NI = BN / WN / 8;           // n8 tiles per warp
-  static constexpr int STAGES = BM == 32 ? 5 : 3;
+  // no more shared memory than it takes: what is left caches the operand columns
+  // that the SM's other tiles read too (64^3 update matrices with 2 / 3 / 4 stages
+  // of 64x64 tiles: 21.4 / 22.1 / 23.0 ms)
+  static constexpr int STAGES = BM == 64 ? 2 : 3;
   // k-row stride (BM >= BN): a FP64 fragment's 4 x 8 entries fill the banks
   // exactly (with BM + 8 every fragment load took two passes)
   static constexpr int LD = BM + 4;
@@ -1214,7 +1217,7 @@ struct GemmCfg {
 //         panel factorization);
 // mode 1: U -= L21 L21^T (K = [0, s))
 template <typename T, int BM, int BN>
-__global__ void __launch_bounds__(GemmCfg<BM, BN>::THREADS)
+__global__ void __launch_bounds__(GemmCfg<BM, BN>::THREADS, sizeof(T) == 4 || BM == 128 ? 1 : BM == 64 ? 4 : 6)
 k_gemm(const int* __restrict__ cum, int nb, const int* __restrict__ list, const FrontDesc* __restrict__ fronts, T* __restrict__ L,
        T* __restrict__ U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, const int* status) {
   using Cfg = GemmCfg<BM, BN>;
@@ -1377,8 +1380,8 @@ static double front_bytes(const Plan& P, const FrontDesc& F, double esz) {
 }
 
 // GEMM variant of level h for the panel updates (kind 0) or the update
-// matrix (kind 1): FP64 fronts choose between 64x64 tiles (4 warps, 3 CTAs
-// per SM; the default, 27-29 TF/s on the large 64^3 update matrices; 32x32 on
+// matrix (kind 1): FP64 fronts choose between 64x64 tiles (4 warps, 4 CTAs
+// per SM; the default, 28-30 TF/s on the large 64^3 update matrices; 32x32 on
 // small launches) and 128x128 tiles (8 warps, one CTA per SM; 19 TF/s there), FP32 fronts between the
 // two tcgen05 variants.  The choice comes from the autotuner's measurements
 // (Plan::gemm_choice), the default variant otherwise.

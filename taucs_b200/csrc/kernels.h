@@ -81,9 +81,9 @@ struct LaunchWork {
 };
 // The panel steps and products of a level; step k: columns [128 k, 128 (k + 1))
 struct LevelWork {
-  std::vector<LaunchWork> rows64, rows128;      // row CTAs of k_panel by step
-  std::vector<LaunchWork> u32, u64, u128;       // tiles of the panel product into the columns from 128 k on
-  LaunchWork m32, m64, m128, msp;               // tiles of the update matrices (msp: from the split arena)
+  std::vector<LaunchWork> rows64, rows128, rows256;   // row CTAs of k_panel by step
+  std::vector<LaunchWork> u32, u64, u128;             // tiles of the panel product into the columns from 128 k on
+  LaunchWork m32, m64, m128, msp;                     // tiles of the update matrices (msp: from the split arena)
 };
 
 // Device copies of the plan arrays.

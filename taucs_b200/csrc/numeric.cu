@@ -703,7 +703,7 @@ __device__ __forceinline__ void cp_async_t(float* smem, const float* gmem, bool 
 // chain, in 16-column pieces: the first warp brings the next piece's diagonal
 // rows up to date and factors it while the others update the rest.  Each
 // finished piece goes to the panel behind a counter (release/acquire); the
-// other CTAs hold NT / 4 rows below the block each, follow the counter, solve their
+// other CTAs hold PROWS rows below the block each, follow the counter, solve their
 // rows against the piece and update their columns to the right.  They have
 // higher indices than every diagonal CTA and wait for nothing else, so each
 // wait ends; the waits are bounded all the same.
@@ -729,17 +729,15 @@ template <typename T>
 constexpr int PLDD = PW + (sizeof(T) == 4 ? 20 : 4);
 template <typename T>
 __host__ __device__ constexpr int diag_base(int p) { return PB * (PLDD<T> * p - 8 * p * (p - 1)); }
-// rows of a row CTA of NT threads, and the column stride of their entries
-template <int NT>
-constexpr int PROWS = NT / 4;
-template <int NT>
-constexpr int PLDR = PROWS<NT> + 4;
+// column stride of the entries of a row CTA of ROWS rows
+template <int ROWS>
+constexpr int PLDR = ROWS + 4;
 // shared memory of a launch whose widest step has wmax columns
-template <typename T, int NT>
+template <typename T, int ROWS>
 constexpr size_t panel_smem(int wmax) {
   const int np = (wmax + PB - 1) / PB;
   const size_t d = (size_t) diag_base<T>(np) + 2 * (PB * (PB + 1) + PB);
-  const size_t r = (size_t) np * PB * PLDR<NT> + 2 * (PB * PLDB + PB);
+  const size_t r = (size_t) np * PB * PLDR<ROWS> + 2 * (PB * PLDB + PB);
   return (d > r ? d : r) * sizeof(T);
 }
 
@@ -937,7 +935,7 @@ __device__ __forceinline__ void split_chunk(const float* x, int ld, int c, int w
   }
 }
 
-template <typename T, int FMT, int NT>
+template <typename T, int FMT, int NT, int PROWS>
 __global__ void __launch_bounds__(NT, 512 / NT)
 k_panel(const int* __restrict__ cum, int nb, const int* __restrict__ list, const FrontDesc* __restrict__ fronts,
         const int* __restrict__ rows, T* __restrict__ L, float* __restrict__ sp, int kb, int* __restrict__ done,
@@ -956,7 +954,7 @@ k_panel(const int* __restrict__ cum, int nb, const int* __restrict__ list, const
   const int w = min(PW, s - kb), np = (w + PB - 1) / PB;
   T* P = L + F.l_off;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NW = NT / 32, RU = PanelUnit<T>::RU, PROWS = tb::PROWS<NT>, PLDR = tb::PLDR<NT>;
+  constexpr int NW = NT / 32, RU = PanelUnit<T>::RU, PLDR = tb::PLDR<PROWS>;
   int* cnt = done + F.blk_off;          // pieces of the front finished so far
   T* rdiag = reinterpret_cast<T*>(rdiag_all) + (size_t) F.blk_off * PANEL_NB;   // 1 / L_jj
   const int first = kb / PB;            // of them before this step
@@ -1456,8 +1454,9 @@ void plan_launches(const Plan& P, DevPlan* D, std::vector<int>& step_list, std::
       auto below = [&](int rows) {
         return add(c, [&](const FrontDesc& F) { return (F.f - c - std::min(PW, F.s - c) + rows - 1) / rows; });
       };
-      W.rows64.push_back(below(PROWS<256>));
-      W.rows128.push_back(below(PROWS<512>));
+      W.rows64.push_back(below(64));
+      W.rows128.push_back(below(128));
+      W.rows256.push_back(below(256));
       // the product into [c, c + lowest set bit of c), of the recursion below
       const int ce = c + (c & -c);
       auto tiles = [&](int b) {
@@ -1518,6 +1517,9 @@ static int warp_grid() {
   return grid[d];
 }
 
+template <int N>
+using Int = std::integral_constant<int, N>;
+
 template <typename T>
 static void set_smem_attrs() {
   // once per device and type (request-server workers reach this concurrently)
@@ -1527,16 +1529,18 @@ static void set_smem_attrs() {
                          SMALL_F_MAX * SMALL_F_MAX * (int) sizeof(T));
     cudaFuncSetAttribute(k_small_persistent<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          SMALL_F_MAX * SMALL_F_MAX * (int) sizeof(T));
-    auto panel = [](auto fmt, auto nt) {
-      constexpr int NT = decltype(nt)::value;
-      cudaFuncSetAttribute(k_panel<T, decltype(fmt)::value, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int) panel_smem<T, NT>(PW));
+    auto panel = [](auto fmt, auto nt, auto rows) {
+      constexpr int NT = decltype(nt)::value, ROWS = decltype(rows)::value;
+      cudaFuncSetAttribute(k_panel<T, decltype(fmt)::value, NT, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int) panel_smem<T, ROWS>(PW));
     };
-    panel(std::integral_constant<int, 0>(), std::integral_constant<int, 256>());
-    panel(std::integral_constant<int, 0>(), std::integral_constant<int, 512>());
+    panel(Int<0>(), Int<256>(), Int<64>());
+    panel(Int<0>(), Int<512>(), Int<128>());
     if constexpr (sizeof(T) == 4) {
-      panel(std::integral_constant<int, 1>(), std::integral_constant<int, 256>());
-      panel(std::integral_constant<int, 1>(), std::integral_constant<int, 512>());
+      panel(Int<0>(), Int<512>(), Int<256>());
+      panel(Int<1>(), Int<256>(), Int<64>());
+      panel(Int<1>(), Int<512>(), Int<128>());
+      panel(Int<1>(), Int<512>(), Int<256>());
     }
     cudaFuncSetAttribute(k_dinv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dinv_smem<T>());
     cudaFuncSetAttribute(k_gemm<T, 32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1663,24 +1667,30 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
         }
       }
       prof_begin(KC_LEAF, st);
-      auto run = [&](auto fmt, auto nt) {
-        constexpr int NT = decltype(nt)::value;
-        const LaunchWork& w = NT == 512 ? LW.rows128[k] : LW.rows64[k];
-        launch(k_panel<T, decltype(fmt)::value, NT>, nsteps + w.total, NT, panel_smem<T, NT>(wmax), st, D.work + w.off,
-               nsteps, slst, D.fronts, D.rows, L, sp, kb, D.panel_done, D.panel_rdiag, status);
+      auto run = [&](auto fmt, auto nt, auto rows) {
+        constexpr int NT = decltype(nt)::value, ROWS = decltype(rows)::value;
+        const LaunchWork& w = ROWS == 64 ? LW.rows64[k] : ROWS == 128 ? LW.rows128[k] : LW.rows256[k];
+        launch(k_panel<T, decltype(fmt)::value, NT, ROWS>, nsteps + w.total, NT, panel_smem<T, ROWS>(wmax), st,
+               D.work + w.off, nsteps, slst, D.fronts, D.rows, L, sp, kb, D.panel_done, D.panel_rdiag, status);
       };
-      // 16 warps a CTA (128 rows) while every CTA has an SM to itself (29x24x26
-      // FP32: 0.80 ms of panels -> 0.72), 8 on fuller launches, where two CTAs
-      // share an SM and one's updates fill the other's waits
+      // 16 warps a CTA and 128 rows while every CTA has an SM to itself (29x24x26
+      // FP32: 0.80 ms of panels -> 0.72); on fuller launches 8 warps and 64 rows,
+      // where two CTAs share an SM and one's updates fill the other's waits, or
+      // (FP32: they fit) 16 warps and 256 rows.  64 rows take 35 us for the first
+      // wave, which ends with the chain of pivots, and 28 for each further one; 256
+      // rows 43 a wave.  80^3 FP32: panel steps 12.3 -> 10.9 ms
       auto size = [&](auto fmt) {
-        if (nsteps + LW.rows128[k].total <= 148) run(fmt, std::integral_constant<int, 512>());
-        else run(fmt, std::integral_constant<int, 256>());
+        if (nsteps + LW.rows128[k].total <= 148) return run(fmt, Int<512>(), Int<128>());
+        if constexpr (sizeof(T) == 4)
+          if (43 * ((nsteps + LW.rows256[k].total + 147) / 148) < 7 + 28 * ((nsteps + LW.rows64[k].total + 295) / 296))
+            return run(fmt, Int<512>(), Int<256>());
+        run(fmt, Int<256>(), Int<64>());
       };
       if constexpr (sizeof(T) == 4) {
-        if (sp_fmt) size(std::integral_constant<int, 1>());
-        else size(std::integral_constant<int, 0>());
+        if (sp_fmt) size(Int<1>());
+        else size(Int<0>());
       } else {
-        size(std::integral_constant<int, 0>());
+        size(Int<0>());
       }
       prof_end(KC_LEAF, st, fl, by);
       count_launch();

@@ -106,7 +106,7 @@ size_t predict_bytes(const Plan& P) {
              + 16.0 * (3.0 * P.children.size() + P.maps.size() / PANEL_NB + (0.75 + 32.0) * P.n_blk);
   // the build tiles and their child records; the panel steps' fronts and CTA counts
   for (const LevelPlan& LP : P.levels) {
-    for (int fi : LP.big_fronts) b += 4.0 * (5.0 + 5.0 * ((P.fronts[fi].s + 127) / 128));
+    for (int fi : LP.big_fronts) b += 4.0 * (5.0 + 6.0 * ((P.fronts[fi].s + 127) / 128));
     for (const Tile& t : LP.build_tiles)
       b += sizeof(Tile) + sizeof(TileChild) * (double) (P.fronts[t.front].child_end - P.fronts[t.front].child_begin);
   }

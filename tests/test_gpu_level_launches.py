@@ -1,7 +1,9 @@
 """Panel steps and products over a level of many fronts of different sizes (each
 launch's CTAs are counted front by front): 33, 40 and 70 dense blocks of 97 to
 300 columns, coupled to one dense root block of 40 rows, so that the number of
-fronts falls from step to step and is on both sides of one search round (32).
+fronts falls from step to step and is on both sides of one search round (32);
+30 blocks with a root block of 577 and 640 rows, for which FP32 steps take row
+CTAs of 256 rows (two waves of 64 rows, one of 256), the last one not full.
 FP64 against NumPy's Cholesky, FP32 fronts against FP64's factor of the scaled
 matrix; bars as in test_gpu_panel (100 n 2^-53 and 100 n 2^-24, relative
 Frobenius, diagonally dominant matrices).
@@ -39,9 +41,9 @@ def blocks(tb, count, r, seed):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("count", [33, 40, 70])
-def test_levels_of_many_fronts(tb, count):
-    A = blocks(tb, count, 40, seed=count)
+@pytest.mark.parametrize("count, root", [(33, 40), (40, 40), (70, 40), (30, 577), (30, 640)])
+def test_levels_of_many_fronts(tb, count, root):
+    A = blocks(tb, count, root, seed=count)
     n, cp, ri, _ = A.arrays()
     F = tb.factor_symbolic(A)
     assert F.numeric(A) == 0, tb.last_error()

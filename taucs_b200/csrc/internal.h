@@ -154,8 +154,8 @@ struct Plan {
   int64_t v_len = 0;               // doubles of per-front work vectors (1 rhs)
   int64_t dinv_len = 0;            // doubles of diagonal-block inverses
   int n_blk = 0;                   // solve flags
-  int64_t part_len = 0;            // doubles of partial sums: the backward ones, then the forward walk's
-  int64_t fpart_off = 0;           // start of the walks' tagged pairs (2 x n_blk x 64 x SOLVE_NRHS, 8 bytes each)
+  int64_t part_len = 0;            // doubles of partial sums: the backward ones, then the published values
+  int64_t fpart_off = 0;           // start of the published values, tagged pairs (2 x n_blk x 64 x SOLVE_NRHS, 8 bytes each)
   int64_t sp_len = 0;              // floats of the split arena (the largest level's split copies)
   // small fronts whose whole subtree is small: first those whose subtree
   // has only fronts of order <= SMALL_WARP_F (pers_nwarp of them, factored
@@ -190,9 +190,9 @@ struct Plan {
   std::vector<uint8_t> gemm_choice[2];
 };
 
-// words of the solve's handshake array cleared by every solve call: a chain
-// flag per 64-row block; one more word follows, the walks' call counter
-// (never cleared)
+// words of the solve's handshake array ahead of its call counter: a chain flag
+// per 64-row block, which the allocation-free solve's kernels use; the word that
+// follows them counts the solve calls (the published values' tags; never cleared)
 inline size_t solve_flag_words(const Plan& P) { return (size_t) P.n_blk; }
 
 int build_plan(const Symbolic& S, int n, const int* colptr, const int* rowind, Plan* P);

@@ -88,6 +88,7 @@ struct LevelWork {
 
 // Device copies of the plan arrays.
 struct DevPlan {
+  void* arena = nullptr;       // the allocation that holds all of them
   FrontDesc* fronts = nullptr;
   int* children = nullptr;
   int* rows = nullptr;
@@ -168,9 +169,9 @@ void launch_gemm_tc(int variant, const LaunchWork& w, const int* work, const int
 // multi-RHS solve, device vectors in permuted order: X (n x nrhs, ld) from
 // B (n x nrhs, ld); W scratch of P.v_len * SOLVE_NRHS doubles, Y n *
 // SOLVE_NRHS doubles
-// flags (P.n_blk ints) carry release/acquire handshakes between the CTAs of
-// a big front; epoch must differ from every value they hold; status gets
-// SOLVE_TIMEOUT if a bounded wait gave up
+// the word after flags' P.n_blk ints counts the solve calls (the tag of the
+// values that a big front's CTAs publish for one another, with the call's
+// epochs); status gets SOLVE_TIMEOUT if a bounded wait gave up
 constexpr int SOLVE_TIMEOUT = -2;
 // Dinv: the factor's 64x64 diagonal-block inverses (FrontDesc::dinv_off)
 int launch_solve_fp64(const Plan& P, const DevPlan& D, const double* L, const double* Dinv, int nrhs, double* X,

@@ -1389,7 +1389,7 @@ static bool gemm_alt(const Plan& P, int h, int kind) {
   return (size_t) (2 * h + kind) < c.size() && c[2 * h + kind] != 0;
 }
 
-// A launch of up to this many 64x64 tiles (four waves of three CTAs an SM) takes
+// A launch of up to this many 64x64 tiles (three waves of four CTAs an SM) takes
 // 32x32 tiles: four times the CTAs, so that every SM has several of them from the
 // first to the last wave; beyond it the larger tile's reuse is worth more.  Panel
 // products and update matrices of a 40x41x39 grid 3.44 -> 2.64 ms; of 64^3, panel

@@ -376,8 +376,8 @@ int build_plan(const Symbolic& S, int n, const int* colptr, const int* rowind, P
         F.part_off = -1;
       }
     }
-    // the walks' tagged values follow, 8-byte aligned: per 64-row block
-    // the chain's 64 x 8 results, then the helpers' 64 x 8 partial sums, as
+    // the published values of the solve's blocks follow, 8-byte aligned: per
+    // 64-row block its 64 x 8 results, then the chains' 64 x 8 partial sums, as
     // (tag, value) pairs of 8 bytes (two FP32 elements each)
     poff = (poff + 1) & ~int64_t(1);
     P.fpart_off = poff;

@@ -12,8 +12,8 @@ a capture command needs to know.
                                                        one's largest update-matrix product (for
                                                        ncu -k/-s)
     python -m taucs_b200.profile_case leaf G            the same two factorizations; prints the
-                                                       index, among the panel-leaf launches of the
-                                                       process, of the second one's first leaf of
+                                                       index, among the panel-step launches of the
+                                                       process, of the second one's first step of
                                                        the root front's level (the root front's
                                                        supernode is the largest)
     python -m taucs_b200.profile_case batch K           one FP32-front factorization and refinement
@@ -114,11 +114,11 @@ def main(argv):
     elif case == "leaf":
         F, _, (kc, ms) = _factor(tb, torch, P, True)
         leaves = [float(t) for k, t in zip(kc, ms) if k == 2]
-        # the root's level runs last: its first leaf (the largest grid) is
-        # the first of the final run of leaf launches of the root's width
+        # the root's level runs last: its first step (the largest grid) is the
+        # first of the root's ceil(s / 128) panel steps
         s_root = int(F.info().max_sn_size)
-        first = max(0, len(leaves) - (s_root + 63) // 64)
-        print("leaf launches", len(leaves), "first leaf of the root level: index", len(leaves) + first,
+        first = max(0, len(leaves) - (s_root + 127) // 128)
+        print("panel step launches", len(leaves), "first step of the root level: index", len(leaves) + first,
               "ms", leaves[first] if leaves else 0.0)
     else:
         raise SystemExit(__doc__)

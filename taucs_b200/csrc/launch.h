@@ -18,8 +18,8 @@
 //   and stay there.  With triggers at the start a factorization of a 40x41x39 grid
 //   went from 6.56 to 7.00 ms and a solve with 64^3's factor from 2.07 to 2.41.
 // CTAs that leave count as triggered.
-// Whole steps, before and now: 139x142 mixed 1.78 -> 1.67 ms, 29x24x26 mixed 2.14
-// -> 2.04, 80^3 mixed 50.8 -> 49.8, 100x100 FP64 1.17 -> 1.15.
+// Whole steps without and with it: 139x142 mixed 1.75 and 1.65 ms, 29x24x26 mixed
+// 2.22 and 2.13, 100x100 FP64 1.15 and 1.11; solves with 64^3's factor the same.
 #pragma once
 
 #include <cuda_runtime.h>

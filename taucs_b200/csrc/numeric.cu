@@ -20,7 +20,7 @@
 //                   writes the tile once;
 //   k_panel         blocked partial Cholesky, step kb: one launch factors
 //                   the 128x128 diagonal block (one CTA per front) and applies
-//                   it to every row below it (a CTA per 64 or 128 rows,
+//                   it to every row below it (a CTA per 64 to 256 rows,
 //                   following it piece by piece);
 //   k_gemm          C -= A B^T on DMMA (mma.sync m16n8k8 f64) tiles: the
 //                   panel updates of a recursive (left half, GEMM, right
@@ -715,9 +715,10 @@ __device__ __forceinline__ void cp_async_t(float* smem, const float* gmem, bool 
 // instruction cache).  Here a piece's Cholesky is a loop over pivots, products
 // are small tile loops (FP64: DMMA fragments; FP32: multiply-adds in FP32).
 // Panel steps and the products between them per factorization, before (64
-// columns a launch) and now: 64^3 FP64 10.3 + 17.2 ms -> 7.2 + 13.4, 40x41x39
-// FP64 2.96 + 2.82 -> 2.20 + 1.67, 80^3 FP32 13.3 + 11.8 -> 12.6 + 8.5,
-// 139x142 FP32 0.59 + 0.13 -> 0.43 + 0.01.
+// columns a launch) and now: 64^3 FP64 10.3 + 17.2 ms -> 7.1 + 10.8, 40x41x39
+// FP64 2.96 + 2.82 -> 2.20 + 0.93, 80^3 FP32 13.3 + 11.8 -> 10.9 + 8.3,
+// 139x142 FP32 0.59 + 0.13 -> 0.44 + 0.01.  A step takes 35 us while its CTAs
+// have an SM each, of which the eight pieces' own pivots are about 16.
 constexpr int PW = 128;              // columns of a panel step
 constexpr int PB = 16;               // columns of a piece
 constexpr int PLDB = PW + 4;         // column stride of a piece that a row CTA reads
@@ -1392,9 +1393,10 @@ static bool gemm_alt(const Plan& P, int h, int kind) {
 // A launch of up to this many 64x64 tiles (three waves of four CTAs an SM) takes
 // 32x32 tiles: four times the CTAs, so that every SM has several of them from the
 // first to the last wave; beyond it the larger tile's reuse is worth more.  Panel
-// products and update matrices of a 40x41x39 grid 3.44 -> 2.64 ms; of 64^3, panel
-// products 13.24 -> 11.73 (12.54 with a line at 200 tiles, 11.86 at 3200), update
-// matrices 22.96 -> 22.92 (27.3 with 32x32 tiles throughout).
+// products and update matrices of a 40x41x39 grid without and with them 3.44 and
+// 2.64 ms; of 64^3, panel products 13.2 and 11.7, update matrices 27.3 instead of
+// 22.9 if all took them.  Factor and solve with the line at 1184, 1776, 2368 and 3552
+// tiles: 40x41x39 5.35, 5.32, 5.33, 5.33 ms; 64^3 42.8, 42.8, 42.8, 43.0.
 constexpr int SMALL_TILES = 4 * 3 * 148;
 template <typename T>
 static void launch_gemm(bool big, const LaunchWork& w128, const LaunchWork& w64, const LaunchWork& w32, const int* blst,

@@ -21,9 +21,7 @@ constexpr int BUILD_TR = 128;
 constexpr int BUILD_TC = 32;
 // block width of the solve and of the diagonal-block inverses
 constexpr int PANEL_NB = 64;
-// GEMM tile of the trailing / update-matrix kernels
-constexpr int GEMM_BM = 64;
-constexpr int GEMM_BN = 64;
+// columns of a pipeline stage of the FP64 products
 constexpr int GEMM_BK = 16;
 // right-hand sides handled per solve pass
 constexpr int SOLVE_NRHS = 8;
@@ -122,7 +120,6 @@ struct DevPlan {
   std::vector<LevelWork> level_work;
   int n_pers = 0;
   std::vector<int> small_off, big_off, tile_off, sfwd_off, sbwd_off, sl21_off, small_num_off;  // per level (host)
-  std::vector<int> lvl_max_f_small;               // per level (host)
 };
 
 // fills D->level_work (with D->big_off), and the arrays that go to D->step_list

@@ -226,7 +226,8 @@ __device__ __forceinline__ void warp_wait_zero(const int* p, int* status, int ns
   }
 }
 
-// the same until *p is at least v; the value seen
+// the same until *p is at least v; the value that lane 0 saw, on every lane (the
+// lanes' loads may see different ones, and callers branch on it around votes)
 __device__ __forceinline__ int warp_wait_at_least(const int* p, int v, int* status) {
   int it = 0, x;
   while (!__all_sync(0xffffffffu, (x = ld_acquire_gpu(p)) >= v)) {
@@ -236,7 +237,7 @@ __device__ __forceinline__ int warp_wait_at_least(const int* p, int v, int* stat
     }
     __nanosleep(20);
   }
-  return x;
+  return __shfl_sync(0xffffffffu, x, 0);
 }
 
 // One front of order f <= SMALL_WARP_F by one warp: the front is assembled
@@ -1080,7 +1081,8 @@ k_panel(const int* __restrict__ cum, int nb, const int* __restrict__ list, const
     }
     if (tid < PB) pri = j0 + tid < w ? __ldcg(rdiag + first * PB + j0 + tid) : T(1);
   };
-  int have = 0;             // pieces known to be finished (the first warp's lanes)
+  int have = 0;             // pieces known to be finished (the first warp: lane 0's load on every
+                            // lane, since the waits that it guards vote over the whole warp)
   bool fetched = false;     // the same on every thread: bad_s carries it
   for (int p = 0; p < np; p++) {
     T* Bp = S + np * PB * PLDR + (p & 1) * (PB * PLDB + PB);
@@ -1094,7 +1096,7 @@ k_panel(const int* __restrict__ cum, int nb, const int* __restrict__ list, const
     for (int e = 0; e < NPRE; e++) Bp[tid % PW + (tid / PW + e * (NT / PW)) * PLDB] = pre[e];
     if (tid < PB) rinv[tid] = pri;
     if (warp == 0 && p + 1 < np) {
-      if (have <= p + 1) have = ld_acquire_gpu(cnt) - first;
+      if (have <= p + 1) have = __shfl_sync(0xffffffffu, ld_acquire_gpu(cnt), 0) - first;
       if (lane == 0) bad_s[p & 1] = have > p + 1;
     }
     cp_async_wait<0>();

@@ -226,12 +226,16 @@ __device__ __forceinline__ void warp_wait_zero(const int* p, int* status, int ns
   }
 }
 
-// the same until *p is at least v; the value that lane 0 saw, on every lane (the
-// lanes' loads may see different ones, and callers branch on it around votes)
+// The same until *p is at least v, or the factorization has failed (then without
+// a timeout of its own: the failing column stays in the status word).  Returns
+// the value that lane 0 saw, on every lane (the lanes' loads may see different
+// ones, and callers branch on it around votes).
 __device__ __forceinline__ int warp_wait_at_least(const int* p, int v, int* status) {
   int it = 0, x;
   while (!__all_sync(0xffffffffu, (x = ld_acquire_gpu(p)) >= v)) {
-    if (++it > (1 << 22)) {
+    ++it;
+    if ((it & 63) == 0 && __any_sync(0xffffffffu, failed(status))) break;
+    if (it > (1 << 22)) {
       atomicMin(status, NUMERIC_TIMEOUT);
       break;
     }
@@ -952,12 +956,24 @@ k_panel(const int* __restrict__ cum, int nb, const int* __restrict__ list, const
   const int f = F.f, s = F.s;
   if (kb >= s) return;
   grid_wait();
-  if (__syncthreads_or(failed(status))) return;   // all threads together
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int* cnt = done + F.blk_off;          // pieces of the front finished so far
+  // the row CTAs leave on the status; a diagonal CTA that does not come to its
+  // pieces releases those of them that are past this check (another front of the
+  // launch may fail between their look at the status and its own)
+  auto release = [&]() {
+    if (tid == 0) {
+      __threadfence();
+      atomicExch(cnt, INT_MAX);
+    }
+  };
+  if (__syncthreads_or(failed(status))) {   // all threads together
+    if (is_diag) release();
+    return;
+  }
   const int w = min(PW, s - kb), np = (w + PB - 1) / PB;
   T* P = L + F.l_off;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NW = NT / 32, RU = PanelUnit<T>::RU, PLDR = tb::PLDR<PROWS>;
-  int* cnt = done + F.blk_off;          // pieces of the front finished so far
   T* rdiag = reinterpret_cast<T*>(rdiag_all) + (size_t) F.blk_off * PANEL_NB;   // 1 / L_jj
   const int first = kb / PB;            // of them before this step
 
@@ -988,12 +1004,8 @@ k_panel(const int* __restrict__ cum, int nb, const int* __restrict__ list, const
       const T* rinv = rinv0 + (p & 1) * PB;
       const int t0 = (p + 1) * PB;
       if (bad_s[p & 1] >= 0) {
-        // the row CTAs leave on the status; the counter releases them
-        if (tid == 0) {
-          atomicMin(status, rows[F.rows_off + kb + p * PB + bad_s[p & 1]]);
-          __threadfence();
-          atomicExch(cnt, INT_MAX);
-        }
+        if (tid == 0) atomicMin(status, rows[F.rows_off + kb + p * PB + bad_s[p & 1]]);
+        release();
         return;
       }
       T* cp = at(p) - PB * p;   // piece p by block row

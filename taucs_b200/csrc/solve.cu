@@ -459,10 +459,10 @@ __device__ __forceinline__ void st_release(int* p, int v) {
 
 }  // namespace
 
-// Controls of the handshake waits on this device: the polling limit, and an
-// offset added to the flag value waited for (0; any other value makes every
-// wait run out -- a testing aid for the timeout reporting, set through
-// taucs_b200_debug_waits).
+// Controls of the handshake waits through global memory on this device: the
+// polling limit, and an offset added to the flag value waited for (0; any other
+// value makes every wait run out -- a testing aid for the timeout reporting, set
+// through taucs_b200_debug_waits).
 __device__ int g_solve_wait_limit = 1 << 22;
 __device__ int g_solve_wait_skew = 0;
 
@@ -658,17 +658,29 @@ __device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
-// bounded wait of a whole warp for a phase of a z's barrier
-__device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, int* status) {
-  const int limit = g_solve_wait_limit;
-  int it = 0;
-  while (!__all_sync(0xffffffffu, bar_try(bar, parity))) {
-    ++it;
-    if (__any_sync(0xffffffffu, it > limit || ((it & 255) == 0 && *(volatile int*) status == SOLVE_TIMEOUT))) {
+// Bounded wait of a whole warp for a phase of a z's barrier; false when it gave
+// up.  Neither the polling limit above nor the status word ends it: every z is
+// sent, also after other waits ran out (their values are then wrong, and the
+// status says so), and a CTA that did not wait for one would leave with stores
+// to its shared memory still on their way.  Its own limit, some 30 seconds, is
+// far above what the waits of the CTAs that it depends on can add up to.
+constexpr int BAR_SPIN = 4096;          // before the warp sleeps between its tries
+constexpr int BAR_LIMIT = 1 << 25;
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, int* status) {
+  for (int it = 0; !__all_sync(0xffffffffu, bar_try(bar, parity)); it++) {
+    if (it < BAR_SPIN) continue;
+    if (it > BAR_LIMIT) {
       atomicExch(status, SOLVE_TIMEOUT);
-      break;
+      return false;
     }
+    __nanosleep(1000);
   }
+  return true;
+}
+// about a millisecond, for stores from other CTAs that nothing counts any more
+__device__ __forceinline__ void settle() {
+  const long long t0 = clock64();
+  for (int it = 0; it < (1 << 16) && clock64() - t0 < (1 << 21); it++) __nanosleep(1000);
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -1226,9 +1238,11 @@ __host__ __device__ constexpr int block_scratch() {
 // z_{u+2 CH_C} is produced every CTA is past its last use of z_u.  Walkers have
 // the lowest CTA indices and helper t waits only for blocks whose helpers
 // come before it, so in-order dispatch keeps every wait finite; the waits are
-// bounded all the same, and no CTA of a cluster leaves before every z has
-// arrived in its shared memory.  In the last diagonal block rows >= s are
-// update rows of the same front; its CTA finishes them too (forward).
+// bounded all the same.  No CTA of a cluster leaves before every z has arrived
+// in its shared memory, also when the waits for published values give up: the
+// walkers carry on with what they have and send every z.  In the last diagonal
+// block rows >= s are update rows of the same front; its CTA finishes them too
+// (forward).
 // Measured, per 64-row step of the root level's forward chain: FP64, one right-
 // hand side (64^3) 2.3 us with flags between CTAs, 1.2 us here; FP64, eight
 // (45x47x44) 4.7 -> 1.7 us; FP32, eight (56^3) 4.2 us with one walker CTA per
@@ -1273,10 +1287,13 @@ k_chain(const __grid_constant__ SolveArgs<T> A) {
     __syncthreads();
     cluster_sync_all();
     // z_u has arrived (each CTA waits for every u once, in order); its
-    // barrier is armed for the z that takes the slot next
+    // barrier is armed for the z that takes the slot next.  A warp whose wait
+    // gave up waits, arms and sends no more: its z's stay incomplete, so that
+    // no slot is written, and no barrier armed, a second time within a phase
+    bool alive = true;
     auto wait_z = [&](int u) {
-      bar_wait(smem_addr(&bars[u % CH_RING]), (u / CH_RING) & 1, A.status);
-      if (tid == 0 && u + CH_RING < nbs) bar_expect(smem_addr(&bars[u % CH_RING]), ZBYTES);
+      if (alive) alive = bar_wait(smem_addr(&bars[u % CH_RING]), (u / CH_RING) & 1, A.status);
+      if (tid == 0 && alive && u + CH_RING < nbs) bar_expect(smem_addr(&bars[u % CH_RING]), ZBYTES);
     };
     if ((int) rank >= nbs) {
       M.begin();
@@ -1345,7 +1362,7 @@ k_chain(const __grid_constant__ SolveArgs<T> A) {
       M.diagonal(b, d, pv, vs, z);
       // z_t: into every CTA of the cluster, the next of the chain first, then
       // published for the helpers, then the result
-      if (Row::qact()) {
+      if (alive && Row::qact()) {
         const unsigned za = smem_addr(zs + ((t % CH_RING) * BR + rho) * NQ + qb), ba = smem_addr(&bars[t % CH_RING]);
 #pragma unroll
         for (int r = 0; r < CH_C; r++) st_async(za + peer[r], ba + peer[r], z);
@@ -1356,6 +1373,8 @@ k_chain(const __grid_constant__ SolveArgs<T> A) {
     // every z that is still on its way to this CTA's shared memory
     for (int u = (int) rank < nbs ? (int) rank + (nbs - 1 - (int) rank) / CH_C * CH_C : 0; u < nbs; u++) wait_z(u);
     cluster_sync_all();
+    // (a z that was cut short completes no phase: what was sent of it)
+    if (!alive) settle();
     return;
   }
   // ------------------------------------------------------------------ helper

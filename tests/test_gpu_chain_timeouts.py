@@ -8,6 +8,7 @@ before.
 import numpy as np
 import pytest
 
+from tests.helpers import scaled_residual
 from tests.test_gpu_front_shapes import blocks_and_separator
 from tests.test_gpu_small_solve import star
 from tests.test_gpu_timeouts import DEFAULT_LIMIT
@@ -54,8 +55,11 @@ def test_chains_that_give_up_fp32(tb, nrhs):
     assert 0 <= its <= 4 and res.max() <= 1e-12
     assert tb.lib().taucs_b200_debug_waits(2000, 1) == 0
     try:
-        # wrong corrections: neither factor's refinement can reach the tolerance
-        assert G.solve_refine(A, B, tol=1e-12, maxits=3)[1] == -1
+        # corrections from values that no tag vouches for (right or wrong): the
+        # residual decides, never a wrong answer with success
+        Y, its2, res = G.solve_refine(A, B, tol=1e-12, maxits=3)
+        assert its2 == -1 or res.max() <= 1e-12
+        assert its2 == -1 or max(scaled_residual(A, Y[:, q], B[:, q]) for q in range(nrhs)) <= 1e-12
     finally:
         assert tb.lib().taucs_b200_debug_waits(DEFAULT_LIMIT, 0) == 0
     assert G.numeric(A) == 0, tb.last_error()

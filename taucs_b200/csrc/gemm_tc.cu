@@ -406,7 +406,7 @@ __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned
 
 template <int STAGES, int FMT>
 __global__ void __launch_bounds__(128, 2)
-k_gemm_sp(const int* __restrict__ cum, int nb, const int* __restrict__ list, const FrontDesc* __restrict__ fronts, const float* __restrict__ sp,
+k_gemm_sp(const int* __restrict__ cum, int nb, const int* __restrict__ list, const FrontDesc* __restrict__ fronts, const float* sp,
           float* __restrict__ L, float* __restrict__ U, int c_lo, int c_hi, int k_lo, int k_hi, int mode,
           int* status) {
   __shared__ __align__(8) unsigned long long bars[2 * STAGES + 1];   // full[S], empty[S], done

@@ -13,10 +13,16 @@
 // * grid_trigger(), which lets the next kernel's CTAs start, only after its own
 //   grid_wait(): so whatever the kernel before the previous one wrote may be read
 //   ahead of the wait (A's values, the plan, in a solve L and the inverses);
-// * and late, when its CTAs are about to write their results: CTAs that arrive
-//   while the grid still works are stacked on the SMs that happen to have room,
-//   and stay there.  With triggers at the start a factorization of a 40x41x39 grid
-//   went from 6.56 to 7.00 ms and a solve with 64^3's factor from 2.07 to 2.41.
+// * what the kernel before may still be writing when this one starts (update
+//   matrices and panels, work vectors, iterates, residuals) is read by plain or
+//   L2 loads (__ldcg) only: not by __ldg, and not through a const __restrict__
+//   pointer, which the compiler turns into the same read-only loads.  Those are
+//   for data that nobody writes while the kernel lives, and may be moved;
+// * the trigger late, when its CTAs are about to write their results: CTAs that
+//   arrive while the grid still works are stacked on the SMs that happen to have
+//   room, and stay there.  With triggers at the start a factorization of a
+//   40x41x39 grid went from 6.56 to 7.00 ms and a solve with 64^3's factor from
+//   2.07 to 2.41.
 // CTAs that leave count as triggered.
 // Whole steps without and with it: 139x142 mixed 1.75 and 1.65 ms, 29x24x26 mixed
 // 2.22 and 2.13, 100x100 FP64 1.15 and 1.11; solves with 64^3's factor the same.

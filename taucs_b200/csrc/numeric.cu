@@ -122,7 +122,7 @@ __device__ void small_front(const FrontDesc& F, const FrontDesc* __restrict__ fr
 #pragma unroll
         for (int v = 0; v < SV; v++) {
           const int i = lane + 32 * v;
-          val[u][v] = (j < mc && i >= j && i < mc) ? __ldg(Uc + i + (size_t) j * mc) : T(0);
+          val[u][v] = (j < mc && i >= j && i < mc) ? __ldcg(Uc + i + (size_t) j * mc) : T(0);
         }
       }
 #pragma unroll
@@ -289,7 +289,7 @@ __device__ void warp_front(const FrontDesc& F, const FrontDesc* __restrict__ fro
     const int pi = lane < mc ? __ldg(maps + C.map_off + lane) : 0;
     T v[WF];
 #pragma unroll
-    for (int j = 0; j < WF; j++) v[j] = (j <= lane && lane < mc) ? __ldg(Uc + lane + (size_t) j * mc) : T(0);
+    for (int j = 0; j < WF; j++) v[j] = (j <= lane && lane < mc) ? __ldcg(Uc + lane + (size_t) j * mc) : T(0);
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < WF; j++) {
@@ -533,7 +533,7 @@ k_build(const Tile* __restrict__ tiles, const TileChild* __restrict__ tile_ch, c
 #pragma unroll
       for (int v = 0; v < IU; v++) {
         const int i = ia + lane + 32 * v;
-        val[u][v] = (jv && i < ib && i >= j) ? __ldg(Uc + (size_t) j * mc + i) : T(0);
+        val[u][v] = (jv && i < ib && i >= j) ? __ldcg(Uc + (size_t) j * mc + i) : T(0);
       }
     }
 #pragma unroll
@@ -598,7 +598,7 @@ __device__ __forceinline__ void warp_inv16_rows(const T (&a)[LQ], T* Y) {
 // sum_{b<=k<c} L_ck X_kb.
 template <typename T>
 __global__ void __launch_bounds__(128)
-k_dinv(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts, const T* __restrict__ L,
+k_dinv(const int2_* __restrict__ blocks, const FrontDesc* __restrict__ fronts, const T* L,
        T* __restrict__ Dinv, const int* status) {
   grid_wait();
   extern __shared__ __align__(16) unsigned char smraw[];

@@ -41,7 +41,7 @@ __global__ void k_diag_scale(int n, const int* __restrict__ diagpos, const doubl
 }
 
 __global__ void k_scaled_f32(long nnz, const int* __restrict__ rowind, const int* __restrict__ colidx,
-                             const double* __restrict__ vals, const double* __restrict__ scale,
+                             const double* __restrict__ vals, const double* scale,
                              float* __restrict__ out) {
   grid_wait();
   const long k = (long) blockIdx.x * blockDim.x + threadIdx.x;
@@ -72,7 +72,7 @@ __device__ __forceinline__ void seg_max(unsigned long long* slots, int sg, int s
 // (r) and [.. + 1] (x); seg == NULL: one segment
 __global__ void k_residual(int n, const int* __restrict__ rp, const int* __restrict__ ci,
                            const int* __restrict__ vi, const double* __restrict__ vals,
-                           const double* __restrict__ X, const double* __restrict__ B, double* __restrict__ R,
+                           const double* X, const double* B, double* __restrict__ R,
                            int ld, int ldr, int nrhs, const int* __restrict__ seg, unsigned long long* norms) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -119,7 +119,7 @@ __global__ void k_residual(int n, const int* __restrict__ rp, const int* __restr
 // the iterate's rows interleaved: Xi[i][q] = X[i + q ld] (zero past nrhs), so
 // that the residual gathers one 64-byte row per matrix entry instead of
 // eight scattered values
-__global__ void k_interleave(int n, const double* __restrict__ X, int ld, int nrhs, double* __restrict__ Xi) {
+__global__ void k_interleave(int n, const double* X, int ld, int nrhs, double* __restrict__ Xi) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -137,7 +137,7 @@ constexpr int RES_THREADS = 256;   // the block size k_residual_i is launched wi
 
 __global__ void __launch_bounds__(RES_THREADS) k_residual_i(int n, const int* __restrict__ rp, const int* __restrict__ ci,
                              const int* __restrict__ vi, const double* __restrict__ vals,
-                             const double* __restrict__ Xi, const double* __restrict__ B, double* __restrict__ R,
+                             const double* Xi, const double* B, double* __restrict__ R,
                              int ld, int ldr, int nrhs, const int* __restrict__ seg, unsigned long long* norms) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(RES_THREADS) k_residual_i(int n, const int* __
   }
 }
 
-__global__ void k_scale_down(int n, const double* __restrict__ R, const double* __restrict__ scale,
+__global__ void k_scale_down(int n, const double* R, const double* scale,
                              float* __restrict__ out, int ld, int nrhs) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -232,7 +232,7 @@ __global__ void k_scale_down(int n, const double* __restrict__ R, const double* 
   for (int q = 0; q < nrhs; q++) out[i + (size_t) q * n] = (float) (R[i + (size_t) q * ld] * scale[i]);
 }
 
-__global__ void k_update32(int n, double* __restrict__ X, const float* __restrict__ D, const double* __restrict__ scale,
+__global__ void k_update32(int n, double* __restrict__ X, const float* D, const double* scale,
                            int ld, int nrhs) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -243,7 +243,7 @@ __global__ void k_update32(int n, double* __restrict__ X, const float* __restric
 // value k of P A P^T is value vmap[k] of A as given (the value map of
 // taucs_ccs_permute_symmetrically, src/taucs_ccs_ops.c:174-257, precomputed
 // once per pattern)
-__global__ void k_gather_values(long nnz, const int* __restrict__ vmap, const double* __restrict__ raw,
+__global__ void k_gather_values(long nnz, const int* __restrict__ vmap, const double* raw,
                                 double* __restrict__ out) {
   grid_wait();
   for (long k = (long) blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (long) gridDim.x * blockDim.x)
@@ -252,7 +252,7 @@ __global__ void k_gather_values(long nnz, const int* __restrict__ vmap, const do
 
 // P b and its inverse (src/taucs_vec_base.c:194-206): dst[i] = src[perm[i]]
 // and dst[perm[i]] = src[i], nq columns, original-order vectors with ld n
-__global__ void k_perm_gather(int n, int nq, const int* __restrict__ perm, const double* __restrict__ src,
+__global__ void k_perm_gather(int n, int nq, const int* __restrict__ perm, const double* src,
                               double* __restrict__ dst) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -261,7 +261,7 @@ __global__ void k_perm_gather(int n, int nq, const int* __restrict__ perm, const
   for (int q = 0; q < nq; q++) dst[i + (size_t) q * n] = src[pi + (size_t) q * n];
 }
 
-__global__ void k_perm_scatter(int n, int nq, const int* __restrict__ perm, const double* __restrict__ src,
+__global__ void k_perm_scatter(int n, int nq, const int* __restrict__ perm, const double* src,
                                double* __restrict__ dst) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -270,7 +270,7 @@ __global__ void k_perm_scatter(int n, int nq, const int* __restrict__ perm, cons
   for (int q = 0; q < nq; q++) dst[pi + (size_t) q * n] = src[i + (size_t) q * n];
 }
 
-__global__ void k_update64(int n, double* __restrict__ X, const double* __restrict__ D, int ld, int ldd, int nrhs) {
+__global__ void k_update64(int n, double* __restrict__ X, const double* D, int ld, int ldd, int nrhs) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -288,7 +288,7 @@ struct Coef {
 
 // Y = A X for nq columns (symmetric CSR of both triangles; leading dimension n)
 __global__ void k_spmv(int n, const int* __restrict__ rp, const int* __restrict__ ci, const int* __restrict__ vi,
-                       const double* __restrict__ vals, const double* __restrict__ X, double* __restrict__ Y, int nq) {
+                       const double* __restrict__ vals, const double* X, double* __restrict__ Y, int nq) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -300,7 +300,7 @@ __global__ void k_spmv(int n, const int* __restrict__ rp, const int* __restrict_
 }
 
 // Z = D d: an FP32 correction scaled back to A's variables
-__global__ void k_scale_up(int n, const float* __restrict__ D, const double* __restrict__ scale, double* __restrict__ Z,
+__global__ void k_scale_up(int n, const float* D, const double* scale, double* __restrict__ Z,
                            int nq) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -311,8 +311,8 @@ __global__ void k_scale_up(int n, const float* __restrict__ D, const double* __r
 // a_q . b_q for nq columns in two fixed-order stages: every block sums a
 // fixed set of rows with a shared-memory tree, then one thread per column
 // adds the block sums in block order
-__global__ void __launch_bounds__(256) k_dot_part(int n, int nq, const double* __restrict__ A,
-                                                  const double* __restrict__ B, double* __restrict__ part) {
+__global__ void __launch_bounds__(256) k_dot_part(int n, int nq, const double* A,
+                                                  const double* B, double* __restrict__ part) {
   grid_wait();
   __shared__ double sh[256];
   for (int q = 0; q < nq; q++) {
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256) k_dot_part(int n, int nq, const double* _
   }
 }
 
-__global__ void k_dot_final(int nblocks, int nq, const double* __restrict__ part, double* __restrict__ out) {
+__global__ void k_dot_final(int nblocks, int nq, const double* part, double* __restrict__ out) {
   grid_wait();
   const int q = threadIdx.x;
   if (q >= nq) return;
@@ -340,7 +340,7 @@ __global__ void k_dot_final(int nblocks, int nq, const double* __restrict__ part
 }
 
 // search direction: P = Z + beta P (P = Z on a (re)start)
-__global__ void k_pcg_dir(int n, int nq, const double* __restrict__ Z, double* __restrict__ Pd, Coef beta, int restart) {
+__global__ void k_pcg_dir(int n, int nq, const double* Z, double* __restrict__ Pd, Coef beta, int restart) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -353,7 +353,7 @@ __global__ void k_pcg_dir(int n, int nq, const double* __restrict__ Z, double* _
 // X += alpha P, R -= alpha Q, and the inf-norms of R and X per column (the
 // one-segment layout of k_residual's norms)
 __global__ void k_pcg_step(int n, int nq, double* __restrict__ X, int ld, double* __restrict__ R,
-                           const double* __restrict__ Pd, const double* __restrict__ Q, Coef alpha,
+                           const double* Pd, const double* Q, Coef alpha,
                            unsigned long long* norms) {
   grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

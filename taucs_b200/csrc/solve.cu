@@ -216,7 +216,7 @@ __device__ __forceinline__ int bwd_piece(int slot, int f, int s) {
 // global rows of the lane's local rows
 template <typename T, int NQ, int WS>
 __device__ __forceinline__ void bwd_front_begin(const SolveTask& K, const int* __restrict__ rows,
-                                                const T* __restrict__ L, const T* __restrict__ W, int nrhs, T* pan,
+                                                const T* __restrict__ L, const T* W, int nrhs, T* pan,
                                                 int slot, T* ws, int wld, int (&g)[SF_SLOTS]) {
   const int lane = threadIdx.x & 31, f = K.f, s = K.s;
   const int ja = slot_columns(slot, f) >= s ? 0 : max(0, s - bwd_piece(slot, f, s));
@@ -344,7 +344,7 @@ k_fwd(const int* __restrict__ list, int count, const FrontDesc* __restrict__ fro
 template <typename T, int NQ, int WS>
 __global__ void __launch_bounds__(128)
 k_bwd(const int* __restrict__ list, int count, const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
-      const T* __restrict__ L, T* __restrict__ X, int ldx, const T* __restrict__ W, int nrhs, int slot, int wld) {
+      const T* __restrict__ L, T* __restrict__ X, int ldx, const T* W, int nrhs, int slot, int wld) {
   grid_wait();
   extern __shared__ __align__(16) unsigned char sfm[];
   const int wi = threadIdx.x >> 5, li = blockIdx.x * (blockDim.x >> 5) + wi;
@@ -416,7 +416,7 @@ k_fwd_pers(const SolveTask* __restrict__ tasks, int t0, int t1, int* pending, in
 template <typename T, int NQ, int WS>
 __global__ void __launch_bounds__(256, NQ == 1 ? 4 : sizeof(T) == 4 ? 3 : 2)
 k_bwd_pers(const SolveTask* __restrict__ tasks, int t0, int t1, int* done, int* next, int epoch,
-           const int* __restrict__ rows, const T* __restrict__ L, T* __restrict__ X, int ldx, const T* __restrict__ W,
+           const int* __restrict__ rows, const T* __restrict__ L, T* __restrict__ X, int ldx, const T* W,
            int nrhs, int* status, int slot, int wld) {
   grid_wait();
   extern __shared__ __align__(16) unsigned char sfm[];
@@ -513,7 +513,7 @@ struct ChildGather {
   int pi[GC];
   T val[GC][QN];
   __device__ __forceinline__ void load(const int4* __restrict__ rec, int n, const int* __restrict__ maps,
-                                       const T* __restrict__ W, int nrhs) {
+                                       const T* W, int nrhs) {
     const int i = threadIdx.x % BR, q0 = threadIdx.x / BR;
 #pragma unroll
     for (int u = 0; u < GC; u++) {
@@ -532,7 +532,7 @@ struct ChildGather {
   // pi - r0; every thread of the block calls it, before a barrier of its own
   template <int LD>
   __device__ __forceinline__ void add(const int4* __restrict__ rec, int n, const int* __restrict__ maps,
-                                      const T* __restrict__ W, int nrhs, int r0, T (*wv)[LD]) {
+                                      const T* W, int nrhs, int r0, T (*wv)[LD]) {
     const int q0 = threadIdx.x / BR;
     for (int c = 0; c < n; c += GC) {
       if (c > 0) load(rec + c, n - c, maps, W, nrhs);
@@ -895,7 +895,7 @@ __device__ __forceinline__ void l21_chunk(const FrontDesc& F, const T* __restric
 template <typename T, int NQ, int NTH>
 __global__ void __launch_bounds__(NTH)
 k_bwd_l21(const int2_* __restrict__ tasks, const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
-          const T* __restrict__ L, const T* __restrict__ X, int ldx, T* __restrict__ part, int nrhs) {
+          const T* __restrict__ L, const T* X, int ldx, T* __restrict__ part, int nrhs) {
   constexpr int RP = L21Split<NQ, NTH>::RP;
   __shared__ T zs[NQ][SOLVE_RCH];
   __shared__ T red[RP][BR][NQ];

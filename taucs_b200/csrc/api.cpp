@@ -463,16 +463,25 @@ int numeric_host(Factor* F, taucs_ccs_matrix* A) {
   return rc;
 }
 
-int solve_device(Factor* F, int nrhs, double* dX, const double* dB, int ld) {
-  if (!F->has_numeric) { set_error("solve: the factor has no numeric part"); return -1; }
-  cudaStream_t st = current_stream();
-  if (!cuda_ok(cudaMemsetAsync(F->dstatus + 1, 0, sizeof(int), st), "solve status")) return -1;
+// the status word of the solves, at the start of a call: the blocks of a call
+// share it, and one that timed out must not be forgotten by the next
+static bool clear_solve_status(Factor* F, cudaStream_t st) {
+  return cuda_ok(cudaMemsetAsync(F->dstatus + 1, 0, sizeof(int), st), "solve status");
+}
+
+static int enqueue_solve(Factor* F, int nrhs, double* dX, const double* dB, int ld, cudaStream_t st) {
   int e = run_graphed(F, GraphKey{3, (uint64_t) nrhs, (uint64_t) dX, (uint64_t) dB, (uint64_t) ld, 0}, st,
                       [&](cudaStream_t s) {
                         return launch_solve_fp64(F->plan, F->dp, F->dL, F->dDinv, nrhs, dX, dB, ld, F->dW, F->dpart,
                                                  F->dflags, &F->epoch, F->dstatus + 1, s);
                       });
   return cuda_ok((cudaError_t) e, "solve launch") ? 0 : -1;
+}
+
+int solve_device(Factor* F, int nrhs, double* dX, const double* dB, int ld) {
+  if (!F->has_numeric) { set_error("solve: the factor has no numeric part"); return -1; }
+  cudaStream_t st = current_stream();
+  return clear_solve_status(F, st) ? enqueue_solve(F, nrhs, dX, dB, ld, st) : -1;
 }
 
 // reads the solve status word after the stream has drained
@@ -496,11 +505,12 @@ int solve_host(Factor* F, int nrhs, double* X, const double* B) {
   if (!F || !F->has_numeric) { set_error("solve: the factor has no numeric part"); return -1; }
   cudaStream_t st = current_stream();
   const int n = F->n;
+  if (!clear_solve_status(F, st)) return -1;
   for (int q0 = 0; q0 < nrhs; q0 += SOLVE_NRHS) {
     const int nq = std::min(SOLVE_NRHS, nrhs - q0);
     if (!cuda_ok(cudaMemcpyAsync(F->dX, B + (size_t) q0 * n, sizeof(double) * (size_t) n * nq,
                                  cudaMemcpyHostToDevice, st), "rhs upload")) return -1;
-    if (solve_device(F, nq, F->dX, F->dX, n)) return -1;
+    if (enqueue_solve(F, nq, F->dX, F->dX, n, st)) return -1;
     if (!cuda_ok(cudaMemcpyAsync(X + (size_t) q0 * n, F->dX, sizeof(double) * (size_t) n * nq,
                                  cudaMemcpyDeviceToHost, st), "solution download")) return -1;
   }

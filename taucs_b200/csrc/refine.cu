@@ -615,6 +615,8 @@ static int refine_device(Factor* F, int nrhs, double* dX, const double* dB, int 
   int total = 0;
   F->last_fallback = 0;
   F->last_pcg_its = 0;
+  // a timeout that an earlier call left would cut this one's waits short
+  if (!cuda_ok(cudaMemsetAsync(F->dstatus + 1, 0, sizeof(int), st), "solve status")) return -1;
   for (int q0 = 0; q0 < nrhs; q0 += SOLVE_NRHS) {
     const int nq = std::min(SOLVE_NRHS, nrhs - q0);
     double* X = dX + (size_t) q0 * ld;

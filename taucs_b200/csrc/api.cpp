@@ -312,7 +312,7 @@ static void free_device(Factor* F) {
   if (F->hdot) tb::hfree(F->hdot);
   F->hdot = nullptr;
   F->refine_ready = false;
-  tb::dfree(F->dflags); F->dflags = nullptr;
+  tb::dfree(F->dcalls); F->dcalls = nullptr;
   if (F->hstatus) tb::hfree(F->hstatus);
   F->hstatus = nullptr;
   F->dev_ready = false;
@@ -336,8 +336,8 @@ int ensure_device(Factor* F) {
   const Plan& P = F->plan;
   bool ok = dev_upload(&F->dA, (const double*) nullptr, (size_t) P.nnz, st)
          && dev_upload(&F->dstatus, (const int*) nullptr, 2, st)
-         && dev_upload(&F->dflags, (const int*) nullptr, solve_flag_words(P) + 1, st)
-         && cuda_ok(cudaMemsetAsync(F->dflags, 0, sizeof(int) * (solve_flag_words(P) + 1), st), "flags")
+         && dev_upload(&F->dcalls, (const int*) nullptr, 1, st)
+         && cuda_ok(cudaMemsetAsync(F->dcalls, 0, sizeof(int), st), "call counter")
          && dev_upload(&F->dW, (const double*) nullptr, (size_t) P.v_len * SOLVE_NRHS, st)
          && dev_upload(&F->dpart, (const double*) nullptr, (size_t) P.part_len, st)
          // the chains' published values start without a tag: the memory may
@@ -473,7 +473,7 @@ static int enqueue_solve(Factor* F, int nrhs, double* dX, const double* dB, int 
   int e = run_graphed(F, GraphKey{3, (uint64_t) nrhs, (uint64_t) dX, (uint64_t) dB, (uint64_t) ld, 0}, st,
                       [&](cudaStream_t s) {
                         return launch_solve_fp64(F->plan, F->dp, F->dL, F->dDinv, nrhs, dX, dB, ld, F->dW, F->dpart,
-                                                 F->dflags, &F->epoch, F->dstatus + 1, s);
+                                                 F->dcalls, F->dstatus + 1, s);
                       });
   return cuda_ok((cudaError_t) e, "solve launch") ? 0 : -1;
 }

@@ -32,8 +32,7 @@ struct Factor {
   double* dX = nullptr;        // solve staging (n * SOLVE_NRHS)
   int* hstatus = nullptr;      // pinned status readback (2 ints: factor, solve)
   double* dDinv = nullptr;     // inverses of the big fronts' 64x64 diagonal blocks
-  int* dflags = nullptr;       // solve handshake flags (plan.n_blk)
-  int epoch = 0;               // last epoch written into dflags
+  int* dcalls = nullptr;       // the solves' call counter (the published values' tags)
   bool has_numeric = false;
   int precision = 0;           // 0 FP64, 1 FP32 fronts
 

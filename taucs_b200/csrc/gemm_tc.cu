@@ -637,17 +637,13 @@ void launch_gemm_sp(int fmt, const LaunchWork& w, const int* work, const int* li
            status);
 }
 
-// variant 0: two-stage ring (65 KB), 128 producers, three CTAs per SM;
-// variant 1: three-stage ring (97 KB), 256 producers, two CTAs per SM
+// two-stage ring (65 KB), 128 producers, three CTAs per SM
 bool gemm_tc_init() {
   // once per device (request-server workers reach this concurrently)
   static PerDeviceOnce pd;
   return per_device_once(pd, [] {
-    const cudaError_t e0 = cudaFuncSetAttribute(k_gemm_tc<2, 3, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int) tc_smem<2>());
-    const cudaError_t e1 = cudaFuncSetAttribute(k_gemm_tc<3, 2, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int) tc_smem<3>());
-    return e0 == cudaSuccess && e1 == cudaSuccess;
+    return cudaFuncSetAttribute(k_gemm_tc<2, 3, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int) tc_smem<2>()) == cudaSuccess;
   });
 }
 
@@ -657,14 +653,10 @@ int gemm_tc_tiles(int rows, int cols) {
   return t;
 }
 
-void launch_gemm_tc(int variant, const LaunchWork& w, const int* work, const int* list, const FrontDesc* fronts,
-                    float* L, float* U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st) {
-  if (variant == 1)
-    launch(k_gemm_tc<3, 2, 256>, w.total, 256 + 32, tc_smem<3>(), st, work + w.off, w.nb, list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
-           mode, status);
-  else
-    launch(k_gemm_tc<2, 3, 128>, w.total, 128 + 32, tc_smem<2>(), st, work + w.off, w.nb, list, fronts, L, U, c_lo, c_hi, k_lo, k_hi,
-           mode, status);
+void launch_gemm_tc(const LaunchWork& w, const int* work, const int* list, const FrontDesc* fronts, float* L, float* U,
+                    int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st) {
+  launch(k_gemm_tc<2, 3, 128>, w.total, 128 + 32, tc_smem<2>(), st, work + w.off, w.nb, list, fronts, L, U, c_lo, c_hi,
+         k_lo, k_hi, mode, status);
 }
 
 }  // namespace tb

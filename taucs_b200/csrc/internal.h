@@ -74,20 +74,13 @@ struct alignas(16) SolveTask {
   int parent;
 };
 
-// Dense-kernel tile for the blocked partial factorization and the update
-// of U (see numeric.cu).
-struct GemmTile {
-  int front;
-  int i0, j0;
-};
-
 // One supernode in device order.
 struct FrontDesc {
   int64_t l_off;      // panel offset (doubles) in the L arena; panel f x s, ld f
   int64_t u_off;      // update matrix offset in the U arena; m x m, ld m (-1 if m == 0)
   int64_t v_off;      // solve work-vector offset (f entries per right-hand side)
   int64_t dinv_off;   // inverses of the 64x64 diagonal blocks (big fronts), -1 otherwise
-  int blk_off;        // solve flags: first of ceil(s/64) per big front, -1 otherwise
+  int blk_off;        // first of the front's ceil(s/64) blocks of 64 columns (big fronts; -1 otherwise)
   int nchunk;         // solve: row chunks of L21 for the backward partial products
   int64_t part_off;   // solve: partial sums (nchunk x s x SOLVE_NRHS doubles), -1 if none
   int s, f;           // columns, front order (m = f - s)
@@ -153,7 +146,7 @@ struct Plan {
   int64_t u_len = 0;               // doubles in U arena (peak of planned lifetimes)
   int64_t v_len = 0;               // doubles of per-front work vectors (1 rhs)
   int64_t dinv_len = 0;            // doubles of diagonal-block inverses
-  int n_blk = 0;                   // solve flags
+  int n_blk = 0;                   // blocks of 64 columns of the big fronts
   int64_t part_len = 0;            // doubles of partial sums: the backward ones, then the published values
   int64_t fpart_off = 0;           // start of the published values, tagged pairs (2 x n_blk x 64 x SOLVE_NRHS, 8 bytes each)
   int64_t sp_len = 0;              // floats of the split arena (the largest level's split copies)
@@ -189,11 +182,6 @@ struct Plan {
   // the default variant; set by the autotuner from measured times.
   std::vector<uint8_t> gemm_choice[2];
 };
-
-// words of the solve's handshake array ahead of its call counter: a chain flag
-// per 64-row block, which the allocation-free solve's kernels use; the word that
-// follows them counts the solve calls (the published values' tags; never cleared)
-inline size_t solve_flag_words(const Plan& P) { return (size_t) P.n_blk; }
 
 int build_plan(const Symbolic& S, int n, const int* colptr, const int* rowind, Plan* P);
 

@@ -150,9 +150,6 @@ constexpr int NUMERIC_TIMEOUT = -4;
 // accumulator); same modes and arguments as the mma.sync GEMM.
 // gemm_tc_init() sets the kernel's shared-memory limit once and reports
 // whether the kernel is usable; gemm_tc_tiles() = CTAs per front.
-// variant 0: 2-stage ring, 128 producer threads, 3 CTAs per SM; variant 1:
-// 3-stage ring, 256 producer threads, 2 CTAs per SM (chosen per level and
-// product by the autotuner)
 bool gemm_tc_init();
 int gemm_tc_tiles(int rows, int cols);
 // the tcgen05 GEMM fed from the split arena by bulk copies (same modes)
@@ -160,23 +157,22 @@ bool gemm_sp_init();
 int gemm_sp_tiles_u(int s, int f);
 void launch_gemm_sp(int fmt, const LaunchWork& w, const int* work, const int* list, const FrontDesc* fronts, const float* sp, float* L, float* U,
                     int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st);
-void launch_gemm_tc(int variant, const LaunchWork& w, const int* work, const int* list, const FrontDesc* fronts, float* L, float* U,
+void launch_gemm_tc(const LaunchWork& w, const int* work, const int* list, const FrontDesc* fronts, float* L, float* U,
                     int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status, cudaStream_t st);
 
 // multi-RHS solve, device vectors in permuted order: X (n x nrhs, ld) from
 // B (n x nrhs, ld); W scratch of P.v_len * SOLVE_NRHS doubles, Y n *
 // SOLVE_NRHS doubles
-// the word after flags' P.n_blk ints counts the solve calls (the tag of the
-// values that a big front's CTAs publish for one another, with the call's
-// epochs); status gets SOLVE_TIMEOUT if a bounded wait gave up
+// calls counts the solve calls (the tag of the values that a big front's CTAs
+// publish for one another, with the call's epochs; never cleared); status gets SOLVE_TIMEOUT if a bounded wait gave up
 constexpr int SOLVE_TIMEOUT = -2;
 // Dinv: the factor's 64x64 diagonal-block inverses (FrontDesc::dinv_off)
 int launch_solve_fp64(const Plan& P, const DevPlan& D, const double* L, const double* Dinv, int nrhs, double* X,
-                      const double* B, int ld, double* W, double* part, int* flags, int* epoch, int* status,
+                      const double* B, int ld, double* W, double* part, int* calls, int* status,
                       cudaStream_t st);
 // the same solve on an FP32 factor with FP32 vectors
 int launch_solve_fp32(const Plan& P, const DevPlan& D, const float* L, const float* Dinv, int nrhs, float* X,
-                      const float* B, int ld, float* W, float* part, int* flags, int* epoch, int* status,
+                      const float* B, int ld, float* W, float* part, int* calls, int* status,
                       cudaStream_t st);
 
 // sets the polling limit and the test offset of the solve's handshake waits

@@ -1438,7 +1438,7 @@ static void launch_gemm32(bool alt, const LaunchWork& wsp, const LaunchWork& w12
   if (!alt && sp && gemm_sp_init())
     launch_gemm_sp(sp_fmt, wsp, D.work, blst, D.fronts, sp, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
   else if (gemm_tc_init())
-    launch_gemm_tc(0, w128, D.work, blst, D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
+    launch_gemm_tc(w128, D.work, blst, D.fronts, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
   else
     launch_gemm<float>(false, w128, w64, w32, blst, D, L, U, c_lo, c_hi, k_lo, k_hi, mode, status, st);
 }

@@ -561,8 +561,8 @@ static int pcg_fp32(Factor* F, int nq, double* X, const double* B, int ld, doubl
   for (int it = 0; it < F->pcg_maxits;) {
     // z = M^-1 r and rho = r.z
     launch(k_scale_down, nblk(n, 256), 256, 0, st, n, R, F->dscale, F->dV32, n, nq);
-    int e = launch_solve_fp32(P, F->dp, F->dL32, F->dDinv32, nq, F->dV32, F->dV32, n, F->dW32, F->dpart32, F->dflags,
-                              &F->epoch, F->dstatus + 1, st);
+    int e = launch_solve_fp32(P, F->dp, F->dL32, F->dDinv32, nq, F->dV32, F->dV32, n, F->dW32, F->dpart32, F->dcalls,
+                              F->dstatus + 1, st);
     launch(k_scale_up, nblk(n, 256), 256, 0, st, n, F->dV32, F->dscale, Z, nq);
     count_launch(2);
     if (e) return -2;
@@ -636,13 +636,13 @@ static int refine_device(Factor* F, int nrhs, double* dX, const double* dB, int 
     auto correction = [&](cudaStream_t s, bool u64) {
       int e;
       if (u64) {
-        e = launch_solve_fp64(P, F->dp, F->dL, F->dDinv, nq, F->dR, F->dR, n, F->dW, F->dpart, F->dflags, &F->epoch,
+        e = launch_solve_fp64(P, F->dp, F->dL, F->dDinv, nq, F->dR, F->dR, n, F->dW, F->dpart, F->dcalls,
                               F->dstatus + 1, s);
         launch(k_update64, nblk(n, 256), 256, 0, s, n, X, F->dR, ld, n, nq);
       } else {
         launch(k_scale_down, nblk(n, 256), 256, 0, s, n, F->dR, F->dscale, F->dV32, n, nq);
         e = launch_solve_fp32(P, F->dp, F->dL32, F->dDinv32, nq, F->dV32, F->dV32, n, F->dW32, F->dpart32,
-                              F->dflags, &F->epoch, F->dstatus + 1, s);
+                              F->dcalls, F->dstatus + 1, s);
         launch(k_update32, nblk(n, 256), 256, 0, s, n, X, F->dV32, F->dscale, ld, nq);
       }
       count_launch(2);

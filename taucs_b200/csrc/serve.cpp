@@ -100,7 +100,7 @@ size_t predict_bytes(const Plan& P) {
              + 8.0 * nnz * 2 + 4.0 * nnz * 6                            // A (FP64, FP32), pattern, CSR
              + 8.0 * n * SOLVE_NRHS * 4 + 4.0 * n * SOLVE_NRHS + 16.0 * n  // R, Xr, Br, X, V32, scale
              + 4.0 * ((double) P.rows.size() + P.maps.size() + P.acol_ptr.size() + 2.0 * P.a_rows.size())
-             + (double) sizeof(FrontDesc) * P.fronts.size() + 4.0 * (solve_flag_words(P) + 1)
+             + (double) sizeof(FrontDesc) * P.fronts.size() + 4.0
              // the solve's tasks, child records and per-block child records
              + (double) sizeof(SolveTask) * P.pers_fronts.size()
              + 16.0 * (3.0 * P.children.size() + P.maps.size() / PANEL_NB + (0.75 + 32.0) * P.n_blk);

@@ -1587,11 +1587,9 @@ static void sf_part(const Plan& P, int np, int part, int* t0, int* t1, int* thre
 
 template <typename T>
 static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Dinv, int nrhs, T* X, const T* B, int ld, T* W,
-                        T* part, int* flags, int* epoch, int* status, cudaStream_t st) {
+                        T* part, int* counter, int* status, cudaStream_t st) {
   solve_attrs<T>();
-  // the blocks' published values, and their call counter in the word after the
-  // flags
-  int* counter = flags + solve_flag_words(P);
+  // the blocks' published values
   unsigned long long* zpub = reinterpret_cast<unsigned long long*>(part + P.fpart_off);
   unsigned long long* ppub = zpub + (size_t) P.n_blk * CH_VALUES * ch_words<T>();
   auto chain_level = [&](const LevelPlan& LP) {
@@ -1600,7 +1598,7 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
   auto chain_grid = [](int nbig, int nblocks) { return nbig * CH_C + (nblocks + CH_C - 1) / CH_C * CH_C; };
   auto args = [&](int h, int nb, const int2_* bl, const int2_* bc, const T* Bq, T* Xq, int nq, int ep, int part_min) {
     return SolveArgs<T>{D.big_list + D.big_off[h], (int) P.levels[h].big_fronts.size(), bl, nb, bc, D.blk_child, D.fronts,
-                        D.maps, D.rows, L, Dinv, Bq, Xq, ld, W, part, part_min, zpub, ppub, flags, nq, counter, ep, status};
+                        D.maps, D.rows, L, Dinv, Bq, Xq, ld, W, part, part_min, zpub, ppub, nullptr, nq, counter, ep, status};
   };
   const int np = D.n_pers;
   // the epochs of a call are always 1, 2, ... and the counter advances on the
@@ -1738,20 +1736,19 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
       count_launch();
     }
   }
-  (void) epoch;
   return (int) cudaGetLastError();
 }
 
 int launch_solve_fp64(const Plan& P, const DevPlan& D, const double* L, const double* Dinv, int nrhs, double* X,
-                      const double* B, int ld, double* W, double* part, int* flags, int* epoch, int* status,
+                      const double* B, int ld, double* W, double* part, int* calls, int* status,
                       cudaStream_t st) {
-  return launch_solve<double>(P, D, L, Dinv, nrhs, X, B, ld, W, part, flags, epoch, status, st);
+  return launch_solve<double>(P, D, L, Dinv, nrhs, X, B, ld, W, part, calls, status, st);
 }
 
 int launch_solve_fp32(const Plan& P, const DevPlan& D, const float* L, const float* Dinv, int nrhs, float* X,
-                      const float* B, int ld, float* W, float* part, int* flags, int* epoch, int* status,
+                      const float* B, int ld, float* W, float* part, int* calls, int* status,
                       cudaStream_t st) {
-  return launch_solve<float>(P, D, L, Dinv, nrhs, X, B, ld, W, part, flags, epoch, status, st);
+  return launch_solve<float>(P, D, L, Dinv, nrhs, X, B, ld, W, part, calls, status, st);
 }
 
 }  // namespace tb

@@ -98,7 +98,7 @@ def main(argv):
         return
     P = _system(tb, g)
     if case == "factor-refine":
-        F, _, _ = _factor(tb, torch, P, False)
+        F, dv, _ = _factor(tb, torch, P, False)   # (the residual reads A's values)
         n, nrhs = P.n, 8
         db = torch.from_numpy(np.random.default_rng(0).uniform(-1, 1, n * nrhs)).cuda()
         dx = torch.zeros_like(db)

@@ -37,9 +37,11 @@ static bool dev_upload(T** dst, const T* src, size_t n, cudaStream_t st) {
   return true;
 }
 
-// The plan's arrays in one allocation, the small ones in one copy: 29 allocations
-// took 2.5 ms of a small system's first factorization (a 20^3 grid's linsolve 18.9
-// -> 16.4 ms).
+// The plan's arrays in one allocation, the small ones in one copy.  With the 29
+// allocations instead, a 20^3 grid's first factorization takes 8.8 ms instead of
+// 5.6, its linsolve 19.5 to 20.7 instead of 16.9 to 17.8 (medians of 60 calls, three
+// times in turn on one machine, quartiles within 2 ms; single calls on a busy host
+// take ten times as long, and there the difference does not show).
 class PlanArena {
  public:
   template <class T>

@@ -25,6 +25,9 @@ constexpr int PANEL_NB = 64;
 constexpr int GEMM_BK = 16;
 // right-hand sides handled per solve pass
 constexpr int SOLVE_NRHS = 8;
+// SMs of a whole B200, on which the launch rules' lines were measured (a
+// partition of one gets the same results by the same rules)
+constexpr int GPU_SMS = 148;
 // bytes of shared memory that a warp of the solve's small-front kernels holds
 // of its front's panel at a time, at most (larger panels go through it in
 // pieces)

@@ -1411,7 +1411,7 @@ static bool gemm_alt(const Plan& P, int h, int kind) {
 // 2.64 ms; of 64^3, panel products 13.2 and 11.7, update matrices 27.3 instead of
 // 22.9 if all took them.  Factor and solve with the line at 1184, 1776, 2368 and 3552
 // tiles: 40x41x39 5.35, 5.32, 5.33, 5.33 ms; 64^3 42.8, 42.8, 42.8, 43.0.
-constexpr int SMALL_TILES = 4 * 3 * 148;
+constexpr int SMALL_TILES = 4 * 3 * GPU_SMS;
 template <typename T>
 static void launch_gemm(bool big, const LaunchWork& w128, const LaunchWork& w64, const LaunchWork& w32, const int* blst,
                         const DevPlan& D, T* L, T* U, int c_lo, int c_hi, int k_lo, int k_hi, int mode, int* status,
@@ -1696,10 +1696,13 @@ static int launch_numeric(const Plan& P, const DevPlan& D, const T* vals, T* L, 
       // wave, which ends with the chain of pivots, and 28 for each further one; 256
       // rows 43 a wave.  80^3 FP32: panel steps 12.3 -> 10.9 ms
       auto size = [&](auto fmt) {
-        if (nsteps + LW.rows128[k].total <= 148) return run(fmt, Int<512>(), Int<128>());
+        if (nsteps + LW.rows128[k].total <= GPU_SMS) return run(fmt, Int<512>(), Int<128>());
         if constexpr (sizeof(T) == 4)
-          if (43 * ((nsteps + LW.rows256[k].total + 147) / 148) < 7 + 28 * ((nsteps + LW.rows64[k].total + 295) / 296))
+        {
+          auto waves = [&](const LaunchWork& w, int at_once) { return (nsteps + w.total + at_once - 1) / at_once; };
+          if (43 * waves(LW.rows256[k], GPU_SMS) < 7 + 28 * waves(LW.rows64[k], 2 * GPU_SMS))
             return run(fmt, Int<512>(), Int<256>());
+        }
         run(fmt, Int<256>(), Int<64>());
       };
       if constexpr (sizeof(T) == 4) {

@@ -279,7 +279,7 @@ __global__ void k_update64(int n, double* __restrict__ X, const double* D, int l
 
 // ---- preconditioned conjugate gradients (fallback of the refinement)
 
-constexpr int DOT_BLOCKS = 296;   // fixed grid, so the summation order never changes
+constexpr int DOT_BLOCKS = 2 * GPU_SMS;   // fixed grid, so the summation order never changes
 constexpr int PCG_STALL = 10;     // iterations over which PCG must at least halve its residual
 
 struct Coef {
@@ -757,7 +757,7 @@ static int device_anorm(Factor* F, std::vector<double>* anorm) {
 
 int gather_values_device(long nnz, const int* d_vmap, const double* d_raw, double* d_out) {
   if (nnz <= 0) return 0;
-  const int grid = (int) std::min<long>(nblk(nnz, 256), 148L * 16);
+  const int grid = (int) std::min<long>(nblk(nnz, 256), GPU_SMS * 16L);
   launch(k_gather_values, grid, 256, 0, current_stream(), nnz, d_vmap, d_raw, d_out);
   count_launch();
   return cuda_ok(cudaGetLastError(), "value gather") ? 0 : -1;

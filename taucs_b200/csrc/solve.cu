@@ -555,8 +555,16 @@ constexpr int CH_THREADS = 256;
 constexpr int CH_VALUES = BR * SOLVE_NRHS;    // values per block and array of published words
 constexpr int DLD = BR + 4;                   // column stride of a staged inverse
 constexpr int CH_HB = 2;                      // blocks per round of a helper's far terms
-// levels with at least CHAIN_MIN_S columns in their largest big front and at
-// most CHAIN_MAX_FRONTS big fronts run as chains
+// Levels with at least CHAIN_MIN_S columns in their largest big front and at
+// most chain_max_fronts() big fronts run as chains.  The number of fronts is
+// bounded by residency: walkers wait for helpers of the same launch, and 16
+// clusters of 8 are 128 of the 296 CTAs that the GPU holds at two an SM.  Within
+// that the lines lie on flat ground.  ms with chains from 128, 256 and 512
+// columns on, on no level, and with half the fronts: solve with 64^3's factor 2.00,
+// 2.00, 2.00, 2.15, 2.02; 32 columns at 45x47x44 4.50, 4.50, 4.48, 4.56, 4.44; refined
+// solution at 56^3 5.27, 5.27, 5.22, 5.56, 5.22; mixed step at 80^3 46.0, 46.0, 46.0,
+// 46.5, 46.0, at 29x24x26 2.14, 2.16, 2.16, 2.16, 2.16.  FP64 with 16 fronts: 45x47x44
+// 4.55.
 constexpr int CHAIN_MIN_S = 256;
 template <typename T>
 constexpr int chain_max_fronts() { return sizeof(T) == 4 ? 16 : 8; }
@@ -1233,16 +1241,20 @@ __host__ __device__ constexpr int block_scratch() {
 // each one relaxed 8-byte access: a reader knows a value is current when its
 // tag is, so nothing fences or polls a flag.  The tag is (call counter <<
 // 12) | epoch, the counter being advanced on the device at the start of every
-// solve call, so recorded launch sequences stay valid.  A ring of 2 CH_C z's
-// needs no release: block t's CTA has consumed z_{t-CH_C} .. z_{t-1}, so when
-// z_{u+2 CH_C} is produced every CTA is past its last use of z_u.  Walkers have
-// the lowest CTA indices and helper t waits only for blocks whose helpers
-// come before it, so in-order dispatch keeps every wait finite; the waits are
-// bounded all the same.  No CTA of a cluster leaves before every z has arrived
-// in its shared memory, also when the waits for published values give up: the
-// walkers carry on with what they have and send every z.  In the last diagonal
-// block rows >= s are update rows of the same front; its CTA finishes them too
-// (forward).
+// solve call, so recorded launch sequences stay valid.  No stale word can carry
+// a pass's tag: forward epochs are odd and backward ones even, in bit 0 also
+// when an epoch outgrows its 12 bits or the counter wraps; a pass writes every
+// word that it reads, in both directions; so its forward step finds even tags
+// everywhere, and its backward step nothing but its own forward tags.  A ring
+// of 2 CH_C z's needs no release: block t's CTA has consumed z_{t-CH_C} ..
+// z_{t-1}, so when z_{u+2 CH_C} is produced every CTA is past its last use of
+// z_u.  Walkers have the lowest CTA indices and helper t waits only for blocks
+// whose helpers come before it, so in-order dispatch keeps every wait finite;
+// the waits are bounded all the same.  No CTA of a cluster leaves before every
+// z has arrived in its shared memory, also when the waits for published values
+// give up: the walkers carry on with what they have and send every z.  In the
+// last diagonal block rows >= s are update rows of the same front; its CTA
+// finishes them too (forward).
 // Measured, per 64-row step of the root level's forward chain: FP64, one right-
 // hand side (64^3) 2.3 us with flags between CTAs, 1.2 us here; FP64, eight
 // (45x47x44) 4.7 -> 1.7 us; FP32, eight (56^3) 4.2 us with one walker CTA per
@@ -1485,8 +1497,8 @@ static double solve_pass_bytes(const FrontDesc& F, int nrhs, double esz) {
   return esz * (s * (s + 1.0) / 2.0 + m * s) + 4.0 * F.f + 2.0 * esz * nrhs * F.f;
 }
 
-// TAUCS_B200_NO_SOLVE_WALK=1 selects the flag-chained block kernels on every
-// level instead of the cluster chains
+// TAUCS_B200_NO_SOLVE_WALK=1 selects the block kernels (k_block) on every level
+// instead of the cluster chains
 static bool walk_enabled() {
   static const bool on = [] {
     const char* e = getenv("TAUCS_B200_NO_SOLVE_WALK");
@@ -1604,7 +1616,7 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
   // the epochs of a call are always 1, 2, ... and the counter advances on the
   // device, so a recorded launch sequence stays valid
   auto reset = [&](bool first) {
-    const int grid = std::max(1, std::min(148, (np + 255) / 256));
+    const int grid = std::max(1, std::min(GPU_SMS, (np + 255) / 256));
     launch(k_solve_reset, grid, 256, 0, st, first, D.pers_pending0, D.pers_solve, np, counter);
     count_launch();
   };
@@ -1689,8 +1701,8 @@ static int launch_solve(const Plan& P, const DevPlan& D, const T* L, const T* Di
             // fewer warps each, down to 4 (solve at 64^3, FP64, backward: 4
             // warps always 1538 us, 16 always 1446, so 1380; mixed step at
             // 80^3, backward: 6509, 7333, 6441)
-            if (nt <= 148) launch(k_bwd_l21<T, Q, 512>, nt, 512, 0, st, tl, D.fronts, D.rows, L, Xq, ld, part, nq);
-            else if (nt <= 4 * 148) launch(k_bwd_l21<T, Q, 256>, nt, 256, 0, st, tl, D.fronts, D.rows, L, Xq, ld,
+            if (nt <= GPU_SMS) launch(k_bwd_l21<T, Q, 512>, nt, 512, 0, st, tl, D.fronts, D.rows, L, Xq, ld, part, nq);
+            else if (nt <= 4 * GPU_SMS) launch(k_bwd_l21<T, Q, 256>, nt, 256, 0, st, tl, D.fronts, D.rows, L, Xq, ld,
                                         part, nq);
             else launch(k_bwd_l21<T, Q, 128>, nt, 128, 0, st, tl, D.fronts, D.rows, L, Xq, ld, part, nq);
           });

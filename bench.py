@@ -56,9 +56,9 @@ TENSOR_KC = {"gemm_panel", "gemm_u"}
 # DRAM traffic per algorithmic byte of a kernel class, from one ncu capture
 # of a 56^3 update-matrix launch (FP32 fronts, FP16x3 products, the largest
 # update product of the 56^3 factorization: one front, 630 tiles): dram read
-# + write 101.1 + 11.0 MB against 129.9 MB of L21 read once and U read and
+# + write 100.3 + 11.1 MB against 129.9 MB of L21 read once and U read and
 # written once; the bench scales it to its own per-launch algorithmic bytes
-TRAFFIC_PER_ALG_BYTE = {"gemm_u": (112.1 / 129.9, "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 56^3 "
+TRAFFIC_PER_ALG_BYTE = {"gemm_u": (111.3 / 129.9, "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 56^3 "
                                                   "update-matrix launch (python -m taucs_b200.profile_case "
                                                   "update-gemm 56), scaled by algorithmic bytes (L21 read once, "
                                                   "U read and written once) to this launch size")}
